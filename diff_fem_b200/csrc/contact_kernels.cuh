@@ -1470,9 +1470,10 @@ __global__ void __launch_bounds__(128, DFEM_ADJ_MIN_BLOCKS) k_cadj_local(SceneDe
                                                     const double* __restrict__ xt, const double* __restrict__ act_all,
                                                     const int* step, double* __restrict__ slot, double* gE,
                                                     double* gnu, double* mg, Gate gate) {
+  __shared__ double tape[kVolTape * 128];
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (gate.skip(cons_part(d, t))) return;
-  adj_local_item(d, t, ori, a.yb, act_all + (size_t)(*step) * d.nseg, slot, gE, gnu, mg, nullptr, xt);
+  adj_local_item(d, t, ori, a.yb, act_all + (size_t)(*step) * d.nseg, slot, gE, gnu, mg, nullptr, xt, tape);
 }
 
 // orib = (sum of the slots) - C^T yb; x_t bar += (M/h^2 - Hs_ii) yb_i; the
@@ -1864,6 +1865,7 @@ __global__ void __launch_bounds__(128) k_cadj_fused(SceneDev d, ContactDev c, Co
                                                     const double* act_all, const int* step, double* slot, double* gE,
                                                     double* gnu, double* mg, double* gact, int base, int top, double cv,
                                                     double* io_a, double* io_b) {
+  __shared__ double tape[kVolTape * 128];
   namespace cg = cooperative_groups;
   cg::grid_group grid = cg::this_grid();
   const int tid = blockIdx.x * blockDim.x + threadIdx.x, nthr = gridDim.x * blockDim.x;
@@ -1891,7 +1893,7 @@ __global__ void __launch_bounds__(128) k_cadj_fused(SceneDev d, ContactDev c, Co
     grid.sync();
     for (int i = tid; i < d.N; i += nthr) cadj_rhs_item(d, c, a, i, slot, xt, ori, prev, first, rcnt, rn);
     grid.sync();
-    for (int t = tid; t < ncons; t += nthr) adj_local_item(d, t, ori, a.yb, act_row, slot, gE, gnu, mg, nullptr, xt);
+    for (int t = tid; t < ncons; t += nthr) adj_local_item(d, t, ori, a.yb, act_row, slot, gE, gnu, mg, nullptr, xt, tape);
     grid.sync();
     for (int i = tid; i < d.N; i += nthr) {  // k_adj_gather_seq, then k_cadj_hs on the same vertex
       Vec3<double> acc = mk3(0.0, 0.0, 0.0);
@@ -1923,6 +1925,7 @@ __global__ void __launch_bounds__(128) k_cadj_fused_parts(SceneDev d, ContactDev
                                                           const double* act_all, const int* step, double* slot,
                                                           double* gE, double* gnu, double* mg, double* gact, int base,
                                                           const int* top, double cv, double* io_a, double* io_b) {
+  __shared__ double tape[kVolTape * 128];
   namespace cg = cooperative_groups;
   cg::grid_group grid = cg::this_grid();
   const int tid = blockIdx.x * blockDim.x + threadIdx.x, nthr = gridDim.x * blockDim.x;
@@ -1956,7 +1959,7 @@ __global__ void __launch_bounds__(128) k_cadj_fused_parts(SceneDev d, ContactDev
     }
     grid.sync();
     for (int t = tid; t < ncons; t += nthr)
-      if (j <= top[cons_part(d, t)]) adj_local_item(d, t, ori, a.yb, act_row, slot, gE, gnu, mg, nullptr, xt);
+      if (j <= top[cons_part(d, t)]) adj_local_item(d, t, ori, a.yb, act_row, slot, gE, gnu, mg, nullptr, xt, tape);
     grid.sync();
     for (int i = tid; i < d.N; i += nthr) {  // k_adj_gather_seq, then k_cadj_hs on the same vertex
       if (j > top[vpart_of(d, i)]) continue;

@@ -76,11 +76,11 @@ __global__ void k_noalloc_tets(int N, int T, const double* __restrict__ x, const
   Mat3<double> F, md, mdv;
 #pragma unroll
   for (int j = 0; j < 3; ++j) F.c[j] = G[0][j] * xv[0] + G[1][j] * xv[1] + G[2][j] * xv[2] + G[3][j] * xv[3];
-  corot_project(F, md, mdv);
+  corot_project_polar(F, md, mdv);
   double wr = w_rot[t], wv = w_vol[t];
   Vec3<double> P[3];
 #pragma unroll
-  for (int j = 0; j < 3; ++j) P[j] = wr * md.c[j] + wv * mdv.c[j];
+  for (int j = 0; j < 3; ++j) P[j] = rn_axpy(wr, md.c[j], rn_scale(wv, mdv.c[j]));
 #pragma unroll
   for (int a = 0; a < 4; ++a) {
     Vec3<double> f = G[a][0] * P[0] + G[a][1] * P[1] + G[a][2] * P[2];

@@ -82,20 +82,19 @@ __device__ __forceinline__ Mat3<double> deformation(const double G[4][3], const 
 
 // Minimum resident CTAs per SM asked of the register allocator for the
 // heaviest per-constraint kernels (128 threads each): more resident warps hide
-// the FP64 latency chains better than the registers they give up (the
-// adjoint local step of the 256-scene batch: 1.12 ms at 174 registers, 0.85 ms
-// at 128 with spills to L1; the mixed force step, then with an FP32 tail after
-// its SVD, 0.315 -> 0.282 ms, the FP64 local step 0.411 -> 0.383 ms; the
-// mixed force step with its FP64 tail takes 0.311 ms at 96 registers).  With
-// the adjoint's projection and VJP sharing one SVD, three CTAs (168 registers,
-// 40 bytes of spills) beat four (128, 360 bytes of spills) and two (255):
-// 32-scene batch 104.6 / 107.1 / 135.3 us, inverse-stiffness beam 13.6 /
-// 14.5 / 13.6 us per launch.
+// the FP64 latency chains better than the registers they give up (the mixed
+// force step takes 0.311 ms on the 256-scene batch at 96 registers, 0.34 ms at
+// more).  The projection by polar and matrix iterations (pd_math.cuh) needs
+// fewer live values than the SVD it replaced: the adjoint local step runs two
+// CTAs at 222 registers without spills (three CTAs, 168 registers, 128 bytes
+// of spills: the same times); inverse-stiffness beam 14.4 -> 12.3 us per
+// launch, local step 10.3 -> 8.2 us, 24-scene batch 45.6 -> 48.1 and 19.3 ->
+// 19.5 us, where the FP64 pipe bounds both.
 #ifndef DFEM_FORCE_MIN_BLOCKS
 #define DFEM_FORCE_MIN_BLOCKS 5
 #endif
 #ifndef DFEM_ADJ_MIN_BLOCKS
-#define DFEM_ADJ_MIN_BLOCKS 3
+#define DFEM_ADJ_MIN_BLOCKS 2
 #endif
 #ifndef DFEM_LOCAL_MIN_BLOCKS
 #define DFEM_LOCAL_MIN_BLOCKS 5
@@ -192,11 +191,11 @@ __device__ __forceinline__ void local_item(const SceneDev& d, int t, const doubl
     double G[4][3];
     load_g(d.tinv, d.T, t, G);
     Mat3<double> F = deformation(G, xv), md, mdv;
-    corot_project(F, md, mdv);
+    corot_project_polar(F, md, mdv);
     double wr = d.twr[t], wv = d.twv[t];
     Vec3<double> P[3];
 #pragma unroll
-    for (int j = 0; j < 3; ++j) P[j] = wr * md.c[j] + wv * mdv.c[j];
+    for (int j = 0; j < 3; ++j) P[j] = rn_axpy(wr, md.c[j], rn_scale(wv, mdv.c[j]));
     int4 sl = d.tslot[t];
     const int sv[4] = {sl.x, sl.y, sl.z, sl.w};
 #pragma unroll
@@ -1237,11 +1236,12 @@ __device__ __noinline__ void muscle_vjp(const SceneDev& d, int t, const double* 
   for (int a = 0; a < 4; ++a) st3(slot, sv[a], ((1.0 - a_act) * c[a]) * db);
 }
 
+// tape_sh: kVolTape doubles of shared memory per thread of the CTA.
 // (Plain pointers: k_cadj_fused writes yb earlier in the same launch; the
 // kernels that call it keep their parameters restrict-qualified.)
 __device__ __forceinline__ void adj_local_item(const SceneDev& d, int t, const double* x, const double* yb,
                                                const double* act_row, double* slot, double* gE, double* gnu,
-                                               double* mg, const double* x1, const double* xt) {
+                                               double* mg, const double* x1, const double* xt, double* tape_sh) {
   if (t < d.T) {
     int4 v = d.tv[t];
     const int vi[4] = {v.x, v.y, v.z, v.w};
@@ -1250,13 +1250,11 @@ __device__ __forceinline__ void adj_local_item(const SceneDev& d, int t, const d
     for (int a = 0; a < 4; ++a) { xv[a] = ld3(x, vi[a]); yv[a] = ld3(yb, vi[a]); }
     double G[4][3];
     load_g(d.tinv, d.T, t, G);
-    Mat3<double> F = deformation(G, xv), Y = deformation(G, yv), md, mdv;
+    const Mat3<double> F = deformation(G, xv), Y = deformation(G, yv);
     double E = d.tE[t], nu = d.tnu[t], vol = d.tvol[t];
-    const Svd3<double> fsv = svd3(F);  // one SVD for the projection and its VJP
-    corot_project_sv(fsv, F, md, mdv);
-    double yr = 0, yvv = 0, yh = 0;
-#pragma unroll
-    for (int j = 0; j < 3; ++j) { yr += dot3(Y.c[j], md.c[j]); yvv += dot3(Y.c[j], mdv.c[j]); }
+    double yr, yvv, yh = 0;
+    Mat3<double> gF;
+    corot_adjoint_polar(F, Y, d.twr[t], d.twv[t], yr, yvv, gF, tape_sh + threadIdx.x, blockDim.x);
     if (x1) {
       Vec3<double> x1v[4] = {ld3(x1, vi[0]), ld3(x1, vi[1]), ld3(x1, vi[2]), ld3(x1, vi[3])};
       Mat3<double> F1 = deformation(G, x1v);
@@ -1274,11 +1272,6 @@ __device__ __forceinline__ void adj_local_item(const SceneDev& d, int t, const d
     double opn = 1.0 + nu;
     if (gE) gE[t] += vol / opn * (yr + nu * yvv) - vol * yh;
     if (gnu) gnu[t] += E * vol / (opn * opn) * (yvv - yr);
-    double wr = d.twr[t], wv = d.twv[t];
-    Mat3<double> gmd, gmdv;
-#pragma unroll
-    for (int j = 0; j < 3; ++j) { gmd.c[j] = wr * Y.c[j]; gmdv.c[j] = wv * Y.c[j]; }
-    Mat3<double> gF = corot_vjp_sv(fsv, F, gmd, gmdv);
     int4 sl = d.tslot[t];
     const int sv[4] = {sl.x, sl.y, sl.z, sl.w};
 #pragma unroll
@@ -1332,6 +1325,7 @@ __global__ void __launch_bounds__(128, DFEM_ADJ_MIN_BLOCKS) k_adj_local(SceneDev
                                                    const double* __restrict__ yb,
                                                    double* bb, const double* __restrict__ act_all,
                                                    double* __restrict__ slot, double* gE, double* gnu, double* mg) {
+  __shared__ double tape[kVolTape * 128];
   const int k = *kptr;
   hist += (size_t)(*step) * hist_step;
   const double* x = hist + (size_t)k * 3 * d.N;
@@ -1339,7 +1333,7 @@ __global__ void __launch_bounds__(128, DFEM_ADJ_MIN_BLOCKS) k_adj_local(SceneDev
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t < d.N && !gate.skip(vpart_of(d, t))) st3(bb, t, ld3(bb, t) + ld3(yb, t));
   if (gate.skip(cons_part(d, t))) return;
-  adj_local_item(d, t, x, yb, act_all + (size_t)(*step) * d.nseg, slot, gE, gnu, mg, x1, nullptr);
+  adj_local_item(d, t, x, yb, act_all + (size_t)(*step) * d.nseg, slot, gE, gnu, mg, x1, nullptr, tape);
 }
 
 // xbar^k = sum of the slots (constraints without x dependence contribute nothing)

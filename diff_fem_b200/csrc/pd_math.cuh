@@ -191,6 +191,165 @@ __device__ __forceinline__ void corot_project(const Mat3<T>& F, Mat3<T>& md, Mat
   corot_project_sv(sv, F, md, mdv, s_ratio);
 }
 
+// ------------------------------------ corotated projection without an SVD ---
+//
+// The FP64 projection and its VJP need only the polar factor Q = U V^T and
+// md_volume = U diag(S + D) V^T, and both have iterations on the 3x3 matrix
+// itself (no singular vectors):
+//   Q: Newton's iteration X <- (zeta X + X^-T / zeta) / 2 (Higham), X^-T =
+//      cof(X) / det(X), from X = F; the scaling zeta = (|X^-T| / |X|)^(1/2)
+//      (an FP32 estimate: any positive value keeps U and V) runs while it is
+//      far from 1, then the plain iteration converges quadratically.
+//   md_volume: with P = F + D = U diag(s + D) V^T the reference's step
+//      D_i <- c g_i, g_i = prod_{j != i} (s_j + D_j), is D <- c C with
+//      C = sigma cof(P), sigma = sign(det F) (U, V orthogonal with
+//      det(U) det(V) = sigma), c = (C : D - (sigma det(P) - 1)) / (C : C): the
+//      same five iterates, written in matrix form.
+// One division per iteration and short FMA chains: the one-sided Jacobi SVD
+// takes two square roots, two divisions and a reciprocal square root per
+// rotation, three rotations per sweep, about five sweeps for an element at
+// ordinary strain, all dependent.  Elements near a lower rank (|det F| <
+// 0.01 (|F|^2/3)^(3/2): X^-T loses digits there) and non-finite ones keep the
+// SVD.  Products and sums that feed both the step and its VJP are written
+// with explicitly rounded operations, so every kernel that inlines them
+// computes the same bits.
+__device__ __forceinline__ Vec3<double> rn_cross(Vec3<double> a, Vec3<double> b) {
+  return {__fma_rn(a.y, b.z, -__dmul_rn(a.z, b.y)), __fma_rn(a.z, b.x, -__dmul_rn(a.x, b.z)),
+          __fma_rn(a.x, b.y, -__dmul_rn(a.y, b.x))};
+}
+__device__ __forceinline__ double rn_dot(Vec3<double> a, Vec3<double> b) {
+  return __fma_rn(a.x, b.x, __fma_rn(a.y, b.y, __dmul_rn(a.z, b.z)));
+}
+__device__ __forceinline__ double rn_dot(const Mat3<double>& a, const Mat3<double>& b) {
+  return __dadd_rn(rn_dot(a.c[0], b.c[0]), __dadd_rn(rn_dot(a.c[1], b.c[1]), rn_dot(a.c[2], b.c[2])));
+}
+__device__ __forceinline__ Vec3<double> rn_scale(double s, Vec3<double> a) {
+  return {__dmul_rn(s, a.x), __dmul_rn(s, a.y), __dmul_rn(s, a.z)};
+}
+__device__ __forceinline__ Vec3<double> rn_axpy(double s, Vec3<double> a, Vec3<double> b) {  // s a + b
+  return {__fma_rn(s, a.x, b.x), __fma_rn(s, a.y, b.y), __fma_rn(s, a.z, b.z)};
+}
+__device__ __forceinline__ Vec3<double> rn_add(Vec3<double> a, Vec3<double> b) {
+  return {__dadd_rn(a.x, b.x), __dadd_rn(a.y, b.y), __dadd_rn(a.z, b.z)};
+}
+__device__ __forceinline__ void rn_cof(const Mat3<double>& a, Mat3<double>& c) {  // a^-T det(a)
+  c.c[0] = rn_cross(a.c[1], a.c[2]);
+  c.c[1] = rn_cross(a.c[2], a.c[0]);
+  c.c[2] = rn_cross(a.c[0], a.c[1]);
+}
+
+// Polar factor of F (C = cof(F) and det = det(F) given); false when the
+// element is near a lower rank (or not finite).
+constexpr int kPolarIterations = 16;
+__device__ __forceinline__ bool polar_newton(const Mat3<double>& F, Mat3<double> C, double det, Mat3<double>& Q) {
+  const double q = __dmul_rn(rn_dot(F, F), 1.0 / 3.0);
+  if (!(__dmul_rn(det, det) > __dmul_rn(1e-4, __dmul_rn(q, __dmul_rn(q, q)))) || !isfinite(det)) return false;
+  Q = F;
+  double d2 = 1.0;
+#pragma unroll 1
+  for (int it = 0; it < kPolarIterations; ++it) {
+    if (it > 0) {
+      rn_cof(Q, C);
+      det = rn_dot(Q.c[0], C.c[0]);
+    }
+    const double inv = 1.0 / det;
+    double a = 0.5, b = __dmul_rn(0.5, inv);
+    bool scaled = false;
+    if (d2 > 0.1) {  // the first iteration, and the next ones of a strongly deformed element
+      const float fi = (float)inv, r = (float)rn_dot(C, C) * fi * fi / (float)rn_dot(Q, Q);  // (|X^-T| / |X|)^2
+      scaled = !(r > 0.8f && r < 1.25f);
+      if (scaled) {
+        const float z = sqrtf(sqrtf(r));
+        a = __dmul_rn(a, (double)z);
+        b = __dmul_rn(b, (double)(1.0f / z));
+      }
+    }
+    d2 = 0.0;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      const Vec3<double> x = rn_axpy(a, Q.c[j], rn_scale(b, C.c[j]));
+      const Vec3<double> d = rn_axpy(-1.0, Q.c[j], x);
+      d2 = __dadd_rn(d2, rn_dot(d, d));
+      Q.c[j] = x;
+    }
+    if (!scaled && d2 < 1e-17) return true;  // quadratic: the error left is about d2 / 2
+  }
+  return false;
+}
+
+// The five steps of the volume projection.  Its VJP's tape: D before steps
+// 1 .. 4 (it is 0 before step 0), c and 1 / (C : C) of every step, in kVolTape
+// doubles of shared memory per thread (value q at sh[q * stride]; in registers
+// they would spill).
+constexpr int kVolTape = 46;
+struct VolTape {
+  double* sh;
+  int stride;
+};
+__device__ __forceinline__ void tape_store(const VolTape& t, int k, const Mat3<double>& D) {
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    double* o = t.sh + (9 * k + 3 * j) * t.stride;
+    o[0] = D.c[j].x; o[t.stride] = D.c[j].y; o[2 * t.stride] = D.c[j].z;
+  }
+}
+__device__ __forceinline__ void tape_load(const VolTape& t, int k, Mat3<double>& D) {
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    const double* o = t.sh + (9 * k + 3 * j) * t.stride;
+    D.c[j] = mk3(o[0], o[t.stride], o[2 * t.stride]);
+  }
+}
+template <bool TAPE>
+__device__ __forceinline__ void volume_newton(const Mat3<double>& F, Mat3<double> C, double det, Mat3<double>& D,
+                                              VolTape* tape) {
+  const double sg = det < 0.0 ? -1.0 : 1.0;
+#pragma unroll
+  for (int j = 0; j < 3; ++j) D.c[j] = mk3(0.0, 0.0, 0.0);
+#pragma unroll 1
+  for (int it = 0; it < 5; ++it) {
+    double num = __fma_rn(-sg, det, 1.0);
+    if (it > 0) {
+      Mat3<double> P;
+#pragma unroll
+      for (int j = 0; j < 3; ++j) P.c[j] = rn_add(F.c[j], D.c[j]);
+      rn_cof(P, C);
+      num = __dadd_rn(__fma_rn(-sg, rn_dot(P.c[0], C.c[0]), 1.0), __dmul_rn(sg, rn_dot(C, D)));
+    }
+    const double iden = 1.0 / rn_dot(C, C), c = __dmul_rn(num, iden), cs = __dmul_rn(sg, c);
+    if (TAPE) {
+      if (it > 0) tape_store(*tape, it - 1, D);
+      tape->sh[(36 + it) * tape->stride] = c;
+      tape->sh[(41 + it) * tape->stride] = iden;
+    }
+#pragma unroll
+    for (int j = 0; j < 3; ++j) D.c[j] = rn_scale(cs, C.c[j]);
+  }
+}
+
+static __device__ __noinline__ void corot_project_svd(const Mat3<double>& F, Mat3<double>& md, Mat3<double>& mdv) {
+  corot_project(F, md, mdv);
+}
+
+// md (reflected rotation) and md_volume of an element.
+__device__ __forceinline__ void corot_project_polar(const Mat3<double>& F, Mat3<double>& md, Mat3<double>& mdv) {
+  Mat3<double> C;
+  rn_cof(F, C);
+  const double det = rn_dot(F.c[0], C.c[0]);
+  if (!polar_newton(F, C, det, md)) {
+    Mat3<double> f = F, a, b;  // the call takes addresses: keep the common path's values in registers
+    corot_project_svd(f, a, b);
+    md = a;
+    mdv = b;
+    return;
+  }
+  if (det < 0.0) md.c[2] = rn_scale(-1.0, md.c[2]);
+  Mat3<double> D;
+  volume_newton<false>(F, C, det, D, nullptr);
+#pragma unroll
+  for (int j = 0; j < 3; ++j) mdv.c[j] = rn_add(F.c[j], D.c[j]);
+}
+
 // Near-degenerate test for the mixed form: an element whose smallest singular
 // value is below kDegenerateRatio of its largest (nearly flat or inverted)
 // has a badly conditioned U/V in FP32 and is recomputed in FP64.
@@ -387,6 +546,116 @@ template <typename T>
 __device__ __forceinline__ Mat3<T> corot_vjp(const Mat3<T>& F, Mat3<T> gmd, const Mat3<T>& gmdv) {
   const Svd3<T> sv = svd3(F);
   return corot_vjp_sv(sv, F, gmd, gmdv);
+}
+
+static __device__ __noinline__ void corot_adjoint_svd(const Mat3<double>& F, const Mat3<double>& Y, double wr, double wv,
+                                               double& yr, double& yv, Mat3<double>& gF) {
+  Mat3<double> md, mdv, gmd, gmdv;
+  const Svd3<double> sv = svd3(F);  // one SVD for the projection and its VJP
+  corot_project_sv(sv, F, md, mdv);
+  yr = yv = 0.0;
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    yr += dot3(Y.c[j], md.c[j]);
+    yv += dot3(Y.c[j], mdv.c[j]);
+    gmd.c[j] = wr * Y.c[j];
+    gmdv.c[j] = wv * Y.c[j];
+  }
+  gF = corot_vjp_sv(sv, F, gmd, gmdv);
+}
+
+// Adjoint of an element: yr = Y : md, yv = Y : md_volume and the VJP
+// gF = (d md / dF)^T (wr Y) + (d md_volume / dF)^T (wv Y).
+//   polar factor F = Q S: dQ = Q [w]x, (tr(S) I - S) w = ax(Q^T dF), so with
+//   b = ax(Q^T gQ) and z = (tr(S) I - S)^-1 b its VJP is Q [z]x;
+//   volume steps in reverse, D' = c C, c = num / (C : C):
+//     gc = gD' : C,  gC = c gD' + gc / (C : C) (D - 2 c C),
+//     gP = sigma cofT(P, gC) - gc / (C : C) C,  gD = gc / (C : C) C + gP, gF += gP.
+__device__ __forceinline__ void corot_adjoint_polar(const Mat3<double>& F, const Mat3<double>& Y, double wr, double wv,
+                                                    double& yr, double& yv, Mat3<double>& gF, double* tape_sh,
+                                                    int stride) {
+  Mat3<double> C, Q;
+  rn_cof(F, C);
+  const double det = rn_dot(F.c[0], C.c[0]);
+  if (!polar_newton(F, C, det, Q)) {
+    Mat3<double> f = F, y = Y, g;
+    double a, b;
+    corot_adjoint_svd(f, y, wr, wv, a, b, g);
+    yr = a;
+    yv = b;
+    gF = g;
+    return;
+  }
+  const double sg = det < 0.0 ? -1.0 : 1.0;
+  {  // rotation
+    const Vec3<double> g2 = rn_scale(sg, Y.c[2]);  // md's column 2 is sigma times Q's
+    yr = __dadd_rn(rn_dot(Y.c[0], Q.c[0]), __dadd_rn(rn_dot(Y.c[1], Q.c[1]), rn_dot(g2, Q.c[2])));
+    const double b0 = __dadd_rn(rn_dot(Q.c[2], Y.c[1]), -rn_dot(Q.c[1], g2));
+    const double b1 = __dadd_rn(rn_dot(Q.c[0], g2), -rn_dot(Q.c[2], Y.c[0]));
+    const double b2 = __dadd_rn(rn_dot(Q.c[1], Y.c[0]), -rn_dot(Q.c[0], Y.c[1]));
+    const double s00 = rn_dot(Q.c[0], F.c[0]), s11 = rn_dot(Q.c[1], F.c[1]), s22 = rn_dot(Q.c[2], F.c[2]);
+    const double k01 = __dmul_rn(-0.5, __dadd_rn(rn_dot(Q.c[0], F.c[1]), rn_dot(Q.c[1], F.c[0])));
+    const double k02 = __dmul_rn(-0.5, __dadd_rn(rn_dot(Q.c[0], F.c[2]), rn_dot(Q.c[2], F.c[0])));
+    const double k12 = __dmul_rn(-0.5, __dadd_rn(rn_dot(Q.c[1], F.c[2]), rn_dot(Q.c[2], F.c[1])));
+    const double k00 = __dadd_rn(s11, s22), k11 = __dadd_rn(s00, s22), k22 = __dadd_rn(s00, s11);
+    // the symmetric 3x3 system by its cofactors
+    const double a00 = __fma_rn(k11, k22, -__dmul_rn(k12, k12)), a01 = __fma_rn(k02, k12, -__dmul_rn(k01, k22));
+    const double a02 = __fma_rn(k01, k12, -__dmul_rn(k02, k11)), a11 = __fma_rn(k00, k22, -__dmul_rn(k02, k02));
+    const double a12 = __fma_rn(k01, k02, -__dmul_rn(k00, k12)), a22 = __fma_rn(k00, k11, -__dmul_rn(k01, k01));
+    const double w = wr / rn_dot(mk3(k00, k01, k02), mk3(a00, a01, a02));
+    const Vec3<double> b = mk3(b0, b1, b2);
+    const double z0 = __dmul_rn(w, rn_dot(mk3(a00, a01, a02), b)), z1 = __dmul_rn(w, rn_dot(mk3(a01, a11, a12), b)),
+                 z2 = __dmul_rn(w, rn_dot(mk3(a02, a12, a22), b));
+    gF.c[0] = rn_axpy(z2, Q.c[1], rn_scale(-z1, Q.c[2]));
+    gF.c[1] = rn_axpy(z0, Q.c[2], rn_scale(-z2, Q.c[0]));
+    gF.c[2] = rn_axpy(z1, Q.c[0], rn_scale(-z0, Q.c[1]));
+  }
+  VolTape tape;
+  tape.sh = tape_sh;
+  tape.stride = stride;
+  Mat3<double> gD;
+  {
+    Mat3<double> D;
+    volume_newton<true>(F, C, det, D, &tape);
+    yv = 0.0;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      yv = __dadd_rn(yv, rn_dot(Y.c[j], rn_add(F.c[j], D.c[j])));
+      gD.c[j] = rn_scale(wv, Y.c[j]);
+      gF.c[j] = rn_add(gF.c[j], gD.c[j]);
+    }
+  }
+#pragma unroll 1
+  for (int it = 4; it >= 0; --it) {
+    Mat3<double> P, D, gC;
+    if (it > 0) {
+      tape_load(tape, it - 1, D);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 3; ++j) D.c[j] = mk3(0.0, 0.0, 0.0);
+    }
+#pragma unroll
+    for (int j = 0; j < 3; ++j) P.c[j] = rn_add(F.c[j], D.c[j]);
+    rn_cof(P, C);  // sigma times the step's C
+    const double c = tape.sh[(36 + it) * stride], gn = __dmul_rn(__dmul_rn(sg, rn_dot(gD, C)), tape.sh[(41 + it) * stride]);
+    const double sn = __dmul_rn(sg, gn);
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      gC.c[j] = rn_axpy(c, gD.c[j], rn_scale(__dmul_rn(-2.0, __dmul_rn(sn, c)), C.c[j]));
+      gC.c[j] = rn_scale(sg, rn_axpy(gn, D.c[j], gC.c[j]));
+    }
+    Mat3<double> gP;
+    gP.c[0] = rn_add(rn_cross(P.c[1], gC.c[2]), rn_cross(gC.c[1], P.c[2]));
+    gP.c[1] = rn_add(rn_cross(P.c[2], gC.c[0]), rn_cross(gC.c[2], P.c[0]));
+    gP.c[2] = rn_add(rn_cross(P.c[0], gC.c[1]), rn_cross(gC.c[0], P.c[1]));
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      const Vec3<double> nc = rn_scale(sn, C.c[j]);  // gc / (C : C) times the step's C
+      const Vec3<double> g = rn_axpy(-1.0, nc, gP.c[j]);
+      gF.c[j] = rn_add(gF.c[j], g);
+      gD.c[j] = rn_add(nc, g);
+    }
+  }
 }
 
 }  // namespace dfem
