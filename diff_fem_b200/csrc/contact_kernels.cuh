@@ -595,6 +595,7 @@ __global__ void __launch_bounds__(128) k_contact_fused(SceneDev d, ContactDev c,
   __shared__ double s_m;
   const int tid = blockIdx.x * blockDim.x + threadIdx.x, nthr = gridDim.x * blockDim.x;
   const bool lead = tid == 0;
+  const double* act_row = act_all + (size_t)(*step) * d.nseg;
   const int ncons = d.T + d.M + d.S + d.B, nv = max(d.N, c.nc);
   for (int i = tid; i < nv; i += nthr) contact_begin_item(d, c, i, xt, xk);
   if (lead)
@@ -643,7 +644,7 @@ __global__ void __launch_bounds__(128) k_contact_fused(SceneDev d, ContactDev c,
     if (conv) {
       mode = 0;  // back to detection
     } else {
-      for (int t = tid; t < ncons; t += nthr) local_item(d, t, xk, act_all, step, slot);
+      for (int t = tid; t < ncons; t += nthr) local_item(d, t, xk, act_row, slot);
       grid.sync();
       for (int i = tid; i < d.N; i += nthr) contact_rhs_item(d, c, i, slot, xt, xk, it == 0, rk);
       grid.sync();
@@ -699,6 +700,7 @@ __global__ void __launch_bounds__(128) k_contact_fused_parts(SceneDev d, Contact
   int* s_run = sp + PS_RUN * np;
   const int tid = blockIdx.x * blockDim.x + threadIdx.x, nthr = gridDim.x * blockDim.x;
   const bool lead = tid == 0;
+  const double* act_row = act_all + (size_t)(*step) * d.nseg;
   const int ncons = d.T + d.M + d.S + d.B, nv = max(d.N, c.nc);
   for (int i = tid; i < nv; i += nthr) contact_begin_item(d, c, i, xt, xk);
   for (int q = tid; q < 2 * np; q += nthr) { c.pany[q] = 0; c.pe[q] = 0ull; }
@@ -778,7 +780,7 @@ __global__ void __launch_bounds__(128) k_contact_fused_parts(SceneDev d, Contact
       for (int p = 0; p < np; ++p) c.pe[((rounds + 1) & 1) * np + p] = 0ull;
     __syncthreads();
     for (int t = tid; t < ncons; t += nthr)
-      if (s_run[cons_part(d, t)]) local_item(d, t, xk, act_all, step, slot);
+      if (s_run[cons_part(d, t)]) local_item(d, t, xk, act_row, slot);
     grid.sync();
     for (int i = tid; i < d.N; i += nthr) {
       const int p = vpart_of(d, i);
@@ -1473,7 +1475,7 @@ __global__ void __launch_bounds__(128, DFEM_ADJ_MIN_BLOCKS) k_cadj_local(SceneDe
   __shared__ double tape[kVolTape * 128];
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (gate.skip(cons_part(d, t))) return;
-  adj_local_item(d, t, ori, a.yb, act_all + (size_t)(*step) * d.nseg, slot, gE, gnu, mg, nullptr, xt, tape);
+  adj_local_item(d, t, ori, a.yb, act_all + (size_t)(*step) * d.nseg, slot, gE, gnu, mg, nullptr, xt, tape + threadIdx.x, 128);
 }
 
 // orib = (sum of the slots) - C^T yb; x_t bar += (M/h^2 - Hs_ii) yb_i; the
@@ -1889,11 +1891,11 @@ __global__ void __launch_bounds__(128) k_cadj_fused(SceneDev d, ContactDev c, Co
     const int* rcnt = c.rec_cnt + r * c.nc;
     const double* rn = c.rec_n + r * c.nc * kMaxImpactsPerVertex * 3;
     const int first = c.rec_first[r];
-    for (int t = tid; t < ncons; t += nthr) local_item(d, t, ori, act_all, step, slot);
+    for (int t = tid; t < ncons; t += nthr) local_item(d, t, ori, act_row, slot);
     grid.sync();
     for (int i = tid; i < d.N; i += nthr) cadj_rhs_item(d, c, a, i, slot, xt, ori, prev, first, rcnt, rn);
     grid.sync();
-    for (int t = tid; t < ncons; t += nthr) adj_local_item(d, t, ori, a.yb, act_row, slot, gE, gnu, mg, nullptr, xt, tape);
+    for (int t = tid; t < ncons; t += nthr) adj_local_item(d, t, ori, a.yb, act_row, slot, gE, gnu, mg, nullptr, xt, tape + threadIdx.x, 128);
     grid.sync();
     for (int i = tid; i < d.N; i += nthr) {  // k_adj_gather_seq, then k_cadj_hs on the same vertex
       Vec3<double> acc = mk3(0.0, 0.0, 0.0);
@@ -1951,7 +1953,7 @@ __global__ void __launch_bounds__(128) k_cadj_fused_parts(SceneDev d, ContactDev
     const int* rcnt = c.rec_cnt + r * c.nc;
     const double* rn = c.rec_n + r * c.nc * kMaxImpactsPerVertex * 3;
     for (int t = tid; t < ncons; t += nthr)
-      if (j <= top[cons_part(d, t)]) local_item(d, t, ori, act_all, step, slot);
+      if (j <= top[cons_part(d, t)]) local_item(d, t, ori, act_row, slot);
     grid.sync();
     for (int i = tid; i < d.N; i += nthr) {
       const int p = vpart_of(d, i);
@@ -1959,7 +1961,7 @@ __global__ void __launch_bounds__(128) k_cadj_fused_parts(SceneDev d, ContactDev
     }
     grid.sync();
     for (int t = tid; t < ncons; t += nthr)
-      if (j <= top[cons_part(d, t)]) adj_local_item(d, t, ori, a.yb, act_row, slot, gE, gnu, mg, nullptr, xt, tape);
+      if (j <= top[cons_part(d, t)]) adj_local_item(d, t, ori, a.yb, act_row, slot, gE, gnu, mg, nullptr, xt, tape + threadIdx.x, 128);
     grid.sync();
     for (int i = tid; i < d.N; i += nthr) {  // k_adj_gather_seq, then k_cadj_hs on the same vertex
       if (j > top[vpart_of(d, i)]) continue;

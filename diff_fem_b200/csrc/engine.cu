@@ -26,6 +26,8 @@
 #include "skeleton_kernels.cuh"
 #include "skeleton_adjoint.cuh"
 #include "dense_solve.cuh"
+#include "block_inverse.cuh"
+#include "step_kernels.cuh"
 #include "resident_plan.h"
 #include "scene.h"
 
@@ -157,13 +159,31 @@ struct dfem_scene {
   int split_cut = 0;                     // the autotune's best split (0: none)
   double solve_ms[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};  // autotune timings (ms per solve): levels, persistent,
                                                           // best split, cluster, resident, dense
-  // dense-inverse form (solve_cut = -3): X = Hs^-1 rebuilt after every refactorisation
-  bool dense_ok = false;                 // the scene qualifies (single part, N <= kDenseMaxN)
-  bool dense_built = false;
+  // block-inverse ("dense") form (solve_cut = -3), built by every refactorisation while it is in use
+  bool dense_ok = false;                 // the scene qualifies (single part, the plan fits)
+  bool dense_built = false;              // the products belong to the current moduli
+  bool tri_built = false;                // the supernodal factor does (built on demand while the dense form is in use)
   double dense_build_ms = 0.0;
+  // mixed scenes: X = Hs^-1 from the supernodal factor (dense_solve.cuh); FP64 scenes: blocks (block_inverse.cuh)
   DBuf<double> dn_A, dn_W, dn_T, dn_Linv;
   DenseDev dd{};
   int dense_grid = 1;                    // CTAs of the dense solve (one per SM at most)
+  BlockPlan bplan;
+  DBuf<BlockInfo> bl_blk;
+  DBuf<BlockTile> bl_tiles;
+  DBuf<BlockKid> bl_kids;
+  DBuf<BlockChunk> bl_chunks;
+  DBuf<int> bl_tier_tile, bl_hs_idx, bl_hs_loc, bl_cols, bl_rows, bl_rmap, bl_cslot, bl_vptr, bl_share;
+  DBuf<double> bl_front, bl_panel, bl_sol, bl_piv, bl_contrib;
+  DBuf<unsigned> bl_bar;
+  BlockDev bd{};
+  bool bl_cluster = false;               // the solve runs in one cluster (small scenes), else on the whole grid
+  // steps in one launch (step_kernels.cuh)
+  bool ps_ok = false;
+  int ps_tab = 0, ps_res_f = 0, ps_res_a = 0, ps_tape_warps = 1;
+  size_t ps_smem_f = 0, ps_smem_a = 0;
+  DBuf<double> xk2, ps_partial;
+  int bf_grid = 1;                       // CTAs of the build
   DBuf<int> lvl_ptr_d, lvl_warp_d;       // cluster form: level starts, end of each level's warp-sized supernodes
   size_t shm_cluster = 0;
   int shm_cluster_warp = 0;              // doubles of shared memory per warp item
@@ -709,27 +729,77 @@ static int upload_refactor_plan(dfem_scene* sc) {
   return DFEM_OK;
 }
 
-// Largest single scene (vertices) served by the dense-inverse form: X and its
-// workspace take 2 N_p^2 doubles (268 MB at 4,096 vertices).
-constexpr int kDenseMaxN = 4096;
 // The dense form is kept when its saving per solve, over this many solves,
-// exceeds the time to rebuild X after a refactorisation.
+// exceeds the time to rebuild it after a refactorisation.
 constexpr double kDenseAmortSolves = 100.0;
+// Largest mixed scene (vertices) served by X = Hs^-1: X and its workspace take
+// 2 N_p^2 doubles (268 MB at 4,096 vertices).
+constexpr int kDenseMaxN = 4096;
+// The dense form of mixed scenes is one product with X, of FP64 scenes the
+// block-inverse form.  The mixed form rounds its forces to FP32, so a solve
+// that differs in its last bits changes which way forces round, and the
+// trajectory at the size of that rounding (1e-8 after tens of steps): its
+// scenes keep the arithmetic of X and their results bit for bit.
+static bool dense_is_x(const dfem_scene* sc) { return sc->hs.precision == DFEM_PREC_MIXED; }
+constexpr int kBlockClusterCtas = 16;
 
 static void dense_release(dfem_scene* sc) {
   sc->dn_A.alloc(0);
   sc->dn_W.alloc(0);
   sc->dn_T.alloc(0);
   sc->dn_Linv.alloc(0);
-  sc->dense_built = false;
   sc->dd = DenseDev{};
+  sc->bl_front.alloc(0);
+  sc->bl_panel.alloc(0);
+  sc->bl_sol.alloc(0);
+  sc->bl_piv.alloc(0);
+  sc->bl_contrib.alloc(0);
+  sc->dense_built = false;
+  sc->bd = BlockDev{};
 }
 
-// X = Hs^-1 from the current GPU factor (dense_solve.cuh), on the scene's stream.
-static int dense_build(dfem_scene* sc) {
+template <class... Args>
+static cudaError_t launch_coop(cudaStream_t st, void (*fn)(Args...), int grid, int block, size_t smem, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, fn, args...);
+}
+
+template <class... Args>
+static cudaError_t launch_cluster(cudaStream_t st, void (*fn)(Args...), int ctas, int block, size_t smem, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = ctas;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, fn, args...);
+}
+
+// Buffers of X = Hs^-1 (single mixed scenes of at most kDenseMaxN vertices
+// whose arrays take at most an eighth of the free memory).
+static int dense_x_prepare(dfem_scene* sc, bool* ok) {
   const int N = sc->hs.N, nb = (N + kDenseTile - 1) / kDenseTile, Np = nb * kDenseTile;
   const size_t nn = (size_t)Np * Np;
+  if (N > kDenseMaxN) return DFEM_OK;
   if (!sc->dn_A.p || !sc->dn_W.p || !sc->dn_T.p || !sc->dn_Linv.p || sc->dn_A.n != nn) {
+    size_t free_b = 0, total_b = 0;
+    CK(cudaMemGetInfo(&free_b, &total_b));
+    if (2 * nn * sizeof(double) > free_b / 8) return DFEM_OK;
     CK(raise_smem_limit((const void*)k_dense_tile_inv, kDenseSmem));
     CK(raise_smem_limit((const void*)k_dense_trtri_t, kDenseSmem));
     CK(raise_smem_limit((const void*)k_dense_trtri_w, kDenseSmem));
@@ -750,7 +820,14 @@ static int dense_build(dfem_scene* sc) {
     }
   }
   sc->dd = DenseDev{N, Np, nb, sc->dn_A.p, sc->dn_W.p, sc->dn_T.p, sc->dn_Linv.p};
-  CK(cudaMemsetAsync(sc->dn_A.p, 0, nn * sizeof(double), sc->stream));
+  *ok = true;
+  return DFEM_OK;
+}
+
+// X = Hs^-1 from the current supernodal factor, on the scene's stream.
+static int dense_x_build(dfem_scene* sc) {
+  const int nb = sc->dd.nb;
+  CK(cudaMemsetAsync(sc->dn_A.p, 0, sc->dn_A.n * sizeof(double), sc->stream));
   k_dense_scatter<<<sc->hs.F.nsuper, 256, 0, sc->stream>>>(sc->dd, sc->fd, sc->Ldw.p, sc->sn_dofs.p);
   k_dense_tile_inv<<<nb, kDenseThreads, kDenseSmem, sc->stream>>>(sc->dd);
   int levels = 0;
@@ -762,48 +839,188 @@ static int dense_build(dfem_scene* sc) {
   k_dense_lauum<<<nb * (nb + 1) / 2, kDenseThreads, kDenseSmem, sc->stream>>>(sc->dd);
   sc->launches += 3 + 2 * levels;
   CK(cudaGetLastError());
-  sc->dense_built = true;
   return DFEM_OK;
 }
 
-// Materials from E_in / nu_in (device), Hs values, and the factor on the GPU.
-// A part whose factorisation meets a non-positive pivot is retried with the
-// reference's regularisation sequence (0, 1e-5, x10 ..., 25 attempts); the
-// other parts keep their regularisation, so their factors are unchanged.
-static int gpu_refactor(dfem_scene* sc) {
+static size_t block_solve_smem(const dfem_scene* sc) { return sizeof(double) * block_solve_doubles(sc->bd.vec); }
+
+// Shared memory of the step kernels: the index tables and rows of a CTA's
+// shares (as many rows as fit), and the adjoint's tape.
+static int plan_steps(dfem_scene* sc, int vec, int G, const std::vector<BlockChunk>& chunks,
+                      const std::vector<int>& share) {
   const HostScene& s = sc->hs;
-  const int np = s.nparts;
-  CK(cudaMemsetAsync(sc->part_fail.p, 0, sizeof(int) * (np + 1), sc->stream));
-  if (s.T > 0) k_materials<<<(s.T + 127) / 128, 128, 0, sc->stream>>>(sc->rd, sc->E_in.p, sc->nu_in.p, np);
-  k_hs_values<<<(sc->rd.nnz + 255) / 256, 256, 0, sc->stream>>>(sc->rd);
-  sc->launches += (s.T > 0 ? 1 : 0) + 1;
-  std::vector<int> failh(np + 1);
-  CK(cudaMemcpyAsync(failh.data(), sc->part_fail.p, sizeof(int) * (np + 1), cudaMemcpyDeviceToHost, sc->stream));
-  CK(cudaStreamSynchronize(sc->stream));
-  if (failh[np]) return fail(DFEM_ERR_INVALID, "invalid material (non-finite E or nu, or nu <= -1)");
-  std::fill(sc->part_reg_h.begin(), sc->part_reg_h.end(), 0.0);
+  const BlockPlan& P = sc->bplan;
+  const int phases = 2 * P.tiers - 1;
+  constexpr size_t kMaxSmem = 224 * 1024 / sizeof(double);  // doubles
+  constexpr int kMaxTab = 8192;
+  sc->ps_ok = false;
+  int tab = 0;
+  size_t rows = 0;
+  for (int c = 0; c < G; ++c) {
+    int nch = 0, ti = 0;
+    size_t rd = 0;
+    for (int p = 0; p < phases; ++p)
+      for (int k = share[(size_t)p * (G + 1) + c]; k < share[(size_t)p * (G + 1) + c + 1]; ++k) {
+        const BlockInfo& B = P.blk[chunks[k].blk];
+        const bool fwd = p < P.tiers;
+        ++nch;
+        ti += ((fwd && B.tier > 0) ? 3 : 1) * (fwd ? B.n : B.r);
+        rd += (size_t)chunks[k].rows * (fwd ? B.ldx : B.ldr);
+      }
+    if (nch > kPsChunks) return DFEM_OK;
+    tab = std::max(tab, ti);
+    rows = std::max(rows, rd);
+  }
+  if (phases > 31) return DFEM_OK;
+  sc->ps_tab = std::min((tab + 3) & ~3, kMaxTab);
+  const int ncons = s.T + s.M + s.S + s.B;
+  sc->ps_tape_warps = std::max(1, std::min(8, (ncons + 32 * G - 1) / (32 * G)));
+  const size_t fixed = ps_fixed_doubles(vec) + sc->ps_tab / 2, tape = (size_t)kVolTape * 32 * sc->ps_tape_warps;
+  if (fixed + tape > kMaxSmem) return DFEM_OK;
+  rows = (rows + 1) & ~size_t(1);
+  sc->ps_res_f = (int)std::min(rows, kMaxSmem - fixed);
+  sc->ps_res_a = (int)std::min(rows, kMaxSmem - fixed - tape);
+  sc->ps_smem_f = (fixed + sc->ps_res_f) * sizeof(double);
+  sc->ps_smem_a = (fixed + tape + sc->ps_res_a) * sizeof(double);
+  for (auto fn : {(const void*)k_pd_forward<GridBarrier, false>, (const void*)k_pd_forward<GridBarrier, true>,
+                  (const void*)k_pd_forward<ClusterBarrier, false>, (const void*)k_pd_forward<ClusterBarrier, true>})
+    CK(raise_smem_limit(fn, sc->ps_smem_f));
+  for (auto fn : {(const void*)k_pd_adjoint<GridBarrier>, (const void*)k_pd_adjoint<ClusterBarrier>})
+    CK(raise_smem_limit(fn, sc->ps_smem_a));
+  for (auto fn : {(const void*)k_pd_forward<ClusterBarrier, false>, (const void*)k_pd_forward<ClusterBarrier, true>,
+                  (const void*)k_pd_adjoint<ClusterBarrier>})
+    CK(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  CK(sc->xk2.alloc(3 * (size_t)s.N));
+  CK(sc->ps_partial.alloc(2 * (size_t)G));
+  sc->ps_ok = true;
+  return DFEM_OK;
+}
+
+// Buffers, tables and launch shapes of the dense form (block-inverse: single
+// scenes whose plan fits an eighth of the free memory); false: not a candidate.
+static int dense_prepare(dfem_scene* sc, bool* ok) {
+  *ok = false;
+  if (sc->hs.nparts != 1 || sc->hs.F.nsuper == 0) return DFEM_OK;
+  if (dense_is_x(sc)) return dense_x_prepare(sc, ok);
+  BlockPlan& P = sc->bplan;
+  if (sc->bd.blk == nullptr) {
+    size_t free_b = 0, total_b = 0;
+    CK(cudaMemGetInfo(&free_b, &total_b));
+    if (!plan_blocks(sc->hs.F, sc->hs.Hs, (int64_t)(free_b / 8 / sizeof(double)), P)) return DFEM_OK;
+    int vec = 2, coop = 0, nsm = 1, occ = 0;
+    for (const BlockInfo& B : P.blk) vec = std::max({vec, B.ldx, B.ldr});
+    CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, sc->device));
+    CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, sc->device));
+    const size_t smem = sizeof(double) * block_solve_doubles(vec);
+    if (!coop || smem > 220 * 1024) return DFEM_OK;
+    CK(raise_smem_limit((const void*)k_block_factor, kBfSmem));
+    CK(raise_smem_limit((const void*)k_block_solve<GridBarrier>, smem));
+    CK(raise_smem_limit((const void*)k_block_solve<ClusterBarrier>, smem));
+    CK(cudaFuncSetAttribute((const void*)k_block_solve<ClusterBarrier>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_block_factor, kBfThreads, kBfSmem));
+    if (occ < 1) return DFEM_OK;
+    int most = 1;
+    for (int t = 0; t < P.tiers; ++t) most = std::max(most, P.tier_tile[t + 1] - P.tier_tile[t]);
+    sc->bf_grid = std::min(nsm * occ, most);
+    sc->bl_cluster = getenv("DFEM_CL") && sc->hs.N <= atoi(getenv("DFEM_CL"));
+    const int G = sc->bl_cluster ? kBlockClusterCtas : nsm;
+    std::vector<BlockChunk> chunks;
+    std::vector<int> share;
+    block_shares(P, G, chunks, share);
+    if (chunks.empty()) return DFEM_OK;
+    auto some = [](std::vector<int> v) { if (v.empty()) v.push_back(0); return v; };
+    if (P.kids.empty()) P.kids.push_back(BlockKid{0, 0, 0, 0, 0});
+    CK(sc->bl_blk.upload(P.blk));
+    CK(sc->bl_tiles.upload(P.tiles));
+    CK(sc->bl_kids.upload(P.kids));
+    CK(sc->bl_chunks.upload(chunks));
+    CK(sc->bl_share.upload(share));
+    CK(sc->bl_tier_tile.upload(P.tier_tile));
+    CK(sc->bl_hs_idx.upload(some(P.hs_idx)));
+    CK(sc->bl_hs_loc.upload(some(P.hs_loc)));
+    CK(sc->bl_cols.upload(P.cols));
+    CK(sc->bl_rows.upload(some(P.rows)));
+    CK(sc->bl_rmap.upload(some(P.rmap)));
+    CK(sc->bl_cslot.upload(some(P.cslot)));
+    CK(sc->bl_vptr.upload(P.vptr));
+    // all buffers or none: a failed allocation leaves none behind
+    cudaError_t e = sc->bl_front.alloc(P.front_doubles);
+    if (e == cudaSuccess) e = sc->bl_panel.alloc(P.panel_doubles);
+    if (e == cudaSuccess) e = sc->bl_sol.alloc(P.solve_doubles);
+    if (e == cudaSuccess) e = sc->bl_piv.alloc(2 * P.blk.size() * kBlkPivot * kBlkPivot);
+    if (e == cudaSuccess) e = sc->bl_contrib.alloc(3 * std::max<size_t>(1, P.rows.size()));
+    if (e == cudaSuccess) e = sc->bl_bar.alloc(2);
+    if (e == cudaSuccess) e = cudaMemset(sc->bl_bar.p, 0, 2 * sizeof(unsigned));
+    if (e == cudaSuccess) e = cudaMemset(sc->bl_sol.p, 0, P.solve_doubles * sizeof(double));  // the rows' padding stays 0
+    if (e != cudaSuccess) {
+      dense_release(sc);
+      CK(e);
+    }
+    RC(plan_steps(sc, vec, G, chunks, share));
+    BlockDev d{};
+    d.N = sc->hs.N; d.tiers = P.tiers; d.nblk = (int)P.blk.size(); d.G = G;
+    d.blk = sc->bl_blk.p; d.tiles = sc->bl_tiles.p; d.tier_tile = sc->bl_tier_tile.p; d.kids = sc->bl_kids.p;
+    d.hs_idx = sc->bl_hs_idx.p; d.hs_loc = sc->bl_hs_loc.p; d.cols = sc->bl_cols.p; d.rows = sc->bl_rows.p;
+    d.rmap = sc->bl_rmap.p; d.cslot = sc->bl_cslot.p; d.vptr = sc->bl_vptr.p; d.chunks = sc->bl_chunks.p;
+    d.share = sc->bl_share.p; d.front = sc->bl_front.p; d.panel = sc->bl_panel.p; d.sol = sc->bl_sol.p;
+    d.piv = sc->bl_piv.p; d.contrib = sc->bl_contrib.p; d.bar = sc->bl_bar.p; d.status = sc->status.p; d.vec = vec;
+    sc->bd = d;
+  }
+  *ok = true;
+  return DFEM_OK;
+}
+
+// X_B and P_B of every block from the current Hs values (block_inverse.cuh),
+// on the scene's stream; a pivot that is not positive raises part_fail[0].
+static int dense_build(dfem_scene* sc) {
+  CK(launch_coop(sc->stream, k_block_factor, sc->bf_grid, kBfThreads, kBfSmem, sc->bd, (const double*)sc->hs_val.p,
+                 (const double*)sc->part_reg.p, sc->part_fail.p));
+  sc->launches += 1;
+  return DFEM_OK;
+}
+
+// Levels of the supernodal factor from the current Hs values.
+static int enqueue_triangular_factor(dfem_scene* sc) {
   const int L = (int)sc->lvl_ptr.size() - 1;
+  for (int l = 0; l < L; ++l) {
+    const int cnt = sc->lvl_ptr[l + 1] - sc->lvl_ptr[l], p0 = sc->lvl_ptr[l];
+    const int sh = sc->split_factor ? sc->fact_shares[l] : 0;
+    if (sh == 0) {
+      k_factor_level<<<cnt, 256, sc->shm_fact_lvl[l], sc->stream>>>(sc->rd, p0);
+      sc->launches += 1;
+      continue;
+    }
+    const size_t w = (size_t)sc->fact_w[l];
+    k_factor_scatter<<<cnt, 256, 0, sc->stream>>>(sc->rd, p0);
+    k_factor_update<<<dim3(cnt, sh), 256, 0, sc->stream>>>(sc->rd, p0);
+    k_factor_diag<<<cnt, 256, 2 * w * w * sizeof(double), sc->stream>>>(sc->rd, p0);
+    k_factor_trsm<<<dim3(cnt, sh), 256, (w * w + kTrsmRows * w) * sizeof(double), sc->stream>>>(sc->rd, p0);
+    sc->launches += 4;
+  }
+  CK(cudaGetLastError());
+  return DFEM_OK;
+}
+
+// Factors the current Hs for the triangular forms or (dense) the block-inverse
+// form.  A part whose factorisation meets a non-positive pivot is retried with
+// the reference's regularisation sequence (0, 1e-5, x10 ..., 25 attempts); the
+// other parts keep their regularisation, so their factors are unchanged.
+static int factor_values(dfem_scene* sc, bool dense) {
+  const int np = sc->hs.nparts;
+  if (dense && dense_is_x(sc)) {  // from the supernodal factor
+    if (!sc->tri_built) RC(factor_values(sc, false));
+    RC(dense_x_build(sc));
+    sc->dense_built = true;
+    return DFEM_OK;
+  }
+  std::vector<int> failh(np + 1);
   for (int attempt = 0; attempt < 25; ++attempt) {
     CK(cudaMemcpyAsync(sc->part_reg.p, sc->part_reg_h.data(), sizeof(double) * np, cudaMemcpyHostToDevice, sc->stream));
-    CK(cudaMemsetAsync(sc->part_fail.p, 0, sizeof(int) * np, sc->stream));
-    for (int l = 0; l < L; ++l) {
-      const int cnt = sc->lvl_ptr[l + 1] - sc->lvl_ptr[l], p0 = sc->lvl_ptr[l];
-      const int sh = sc->split_factor ? sc->fact_shares[l] : 0;
-      if (sh == 0) {
-        k_factor_level<<<cnt, 256, sc->shm_fact_lvl[l], sc->stream>>>(sc->rd, p0);
-        sc->launches += 1;
-        continue;
-      }
-      const size_t w = (size_t)sc->fact_w[l];
-      k_factor_scatter<<<cnt, 256, 0, sc->stream>>>(sc->rd, p0);
-      k_factor_update<<<dim3(cnt, sh), 256, 0, sc->stream>>>(sc->rd, p0);
-      k_factor_diag<<<cnt, 256, 2 * w * w * sizeof(double), sc->stream>>>(sc->rd, p0);
-      k_factor_trsm<<<dim3(cnt, sh), 256, (w * w + kTrsmRows * w) * sizeof(double), sc->stream>>>(sc->rd, p0);
-      sc->launches += 4;
-    }
-    CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(failh.data(), sc->part_fail.p, sizeof(int) * np, cudaMemcpyDeviceToHost, sc->stream));
+    if (attempt > 0) CK(cudaMemsetAsync(sc->part_fail.p, 0, sizeof(int) * np, sc->stream));
+    RC(dense ? dense_build(sc) : enqueue_triangular_factor(sc));
+    CK(cudaMemcpyAsync(failh.data(), sc->part_fail.p, sizeof(int) * (np + 1), cudaMemcpyDeviceToHost, sc->stream));
     CK(cudaStreamSynchronize(sc->stream));
+    if (failh[np]) return fail(DFEM_ERR_INVALID, "invalid material (non-finite E or nu, or nu <= -1)");
     bool any = false;
     for (int p = 0; p < np; ++p)
       if (failh[p]) {
@@ -811,13 +1028,40 @@ static int gpu_refactor(dfem_scene* sc) {
         sc->part_reg_h[p] = sc->part_reg_h[p] == 0.0 ? 1e-5 : sc->part_reg_h[p] * 10.0;
       }
     if (!any) {
-      pack_resident(sc);
-      sc->dense_built = false;  // X follows the factor (only while the dense form is in use)
-      if (sc->solve_cut == -3) RC(dense_build(sc));
+      (dense ? sc->dense_built : sc->tri_built) = true;
+      if (!dense) pack_resident(sc);
       return DFEM_OK;
     }
+    (dense ? sc->tri_built : sc->dense_built) = false;  // the other form's factor has another regularisation
   }
   return fail(DFEM_ERR_FACTOR, "Cholesky factorisation failed after 25 regularisation retries");
+}
+
+// The factor of the solve form in use (solve_cut), for the current moduli.
+static int ensure_factor(dfem_scene* sc) {
+  const bool dense = sc->solve_cut == -3;
+  if (dense ? sc->dense_built : sc->tri_built) return DFEM_OK;
+  CK(cudaMemsetAsync(sc->part_fail.p, 0, sizeof(int) * (sc->hs.nparts + 1), sc->stream));
+  return factor_values(sc, dense);
+}
+
+static int ensure_triangular(dfem_scene* sc) {
+  if (sc->tri_built) return DFEM_OK;
+  CK(cudaMemsetAsync(sc->part_fail.p, 0, sizeof(int) * (sc->hs.nparts + 1), sc->stream));
+  return factor_values(sc, false);
+}
+
+// Materials from E_in / nu_in (device), Hs values, and the factor on the GPU.
+static int gpu_refactor(dfem_scene* sc) {
+  const HostScene& s = sc->hs;
+  const int np = s.nparts;
+  CK(cudaMemsetAsync(sc->part_fail.p, 0, sizeof(int) * (np + 1), sc->stream));
+  if (s.T > 0) k_materials<<<(s.T + 127) / 128, 128, 0, sc->stream>>>(sc->rd, sc->E_in.p, sc->nu_in.p, np);
+  k_hs_values<<<(sc->rd.nnz + 255) / 256, 256, 0, sc->stream>>>(sc->rd);
+  sc->launches += (s.T > 0 ? 1 : 0) + 1;
+  std::fill(sc->part_reg_h.begin(), sc->part_reg_h.end(), 0.0);
+  sc->dense_built = sc->tri_built = false;
+  return factor_values(sc, sc->solve_cut == -3);
 }
 
 // Uniform grid over the static obstacle faces for the detection's broad phase
@@ -1003,7 +1247,7 @@ static int upload_scene(dfem_scene* sc) {
   CK(sc->xk.alloc(n3)); CK(sc->rhs.alloc(n3)); CK(sc->y.alloc(n3)); CK(sc->io_a.alloc(n3)); CK(sc->io_b.alloc(n3));
   CK(sc->slot.alloc(3 * (size_t)std::max(1, s.nslots)));
   CK(sc->xkb.alloc(n3)); CK(sc->xtb.alloc(n3)); CK(sc->bb.alloc(n3));
-  CK(sc->gE.alloc(std::max(1, s.T))); CK(sc->gnu.alloc(std::max(1, s.T))); CK(sc->mg.alloc(std::max(1, s.M + (s.sch.empty() ? 0 : s.S))));
+  CK(sc->gE.alloc(std::max(1, s.T))); CK(sc->gnu.alloc(std::max(1, s.T))); CK(sc->mg.alloc(std::max(1, 2 * (s.M + (s.sch.empty() ? 0 : s.S)))));
   sc->nblk_v = (s.N + 127) / 128;
   // part tables: part-aligned blocks of the reducing vertex kernels
   const int np = s.nparts;
@@ -1358,9 +1602,15 @@ static cudaError_t launch_resident_solve(dfem_scene* sc, cudaStream_t st, Gate g
 // the cluster launch's return value is also kept for the autotune, which drops
 // the cluster form when the device refuses its launch.
 static void enqueue_solve_cut(dfem_scene* sc, cudaStream_t st, Gate gate, const double* rhs, double* y, int c) {
-  if (c == -3) {  // the dense-inverse form
-    k_dense_solve<<<sc->dense_grid, kDenseSolveThreads, 3 * (size_t)sc->dd.Np * sizeof(double), st>>>(
-        sc->dd, gate, rhs, y);
+  if (c == -3 && dense_is_x(sc)) {  // X = Hs^-1
+    k_dense_solve<<<sc->dense_grid, kDenseSolveThreads, 3 * (size_t)sc->dd.Np * sizeof(double), st>>>(sc->dd, gate, rhs, y);
+    return;
+  }
+  if (c == -3) {  // the block-inverse form
+    const cudaError_t e =
+        sc->bl_cluster ? launch_cluster(st, k_block_solve<ClusterBarrier>, sc->bd.G, kBsThreads, block_solve_smem(sc), sc->bd, gate, rhs, y)
+                       : launch_coop(st, k_block_solve<GridBarrier>, sc->bd.G, kBsThreads, block_solve_smem(sc), sc->bd, gate, rhs, y);
+    if (e != cudaSuccess) sc->cluster_launch_err = e;
     return;
   }
   if (c < 0) {  // -1: cluster form, -2: resident form
@@ -1522,6 +1772,49 @@ static void launch_adj_gather(dfem_scene* sc, cudaStream_t st, Gate g) {
     k_adj_gather_t<<<sc->nblk_v, 128, 0, st>>>(sc->hs.N, g, sc->vpart.p, sc->vslot_ptr.p, sc->slot.p, sc->xkb.p);
   else
     k_adj_gather<<<(sc->hs.N + 3) / 4, 128, 0, st>>>(sc->hs.N, g, sc->vpart.p, sc->vslot_ptr.p, sc->slot.p, sc->xkb.p);
+}
+
+// Scenes whose steps run in one launch: the block-inverse solve, no links, drag
+// or soft contact.
+static bool one_launch(const dfem_scene* sc) {
+  return sc->solve_cut == -3 && sc->ps_ok && sc->bd.blk && sc->hs.nparts == 1 && !sc->skel_on && sc->nF == 0 && !sc->self_contact;
+}
+
+static PdSteps steps_args(dfem_scene* sc, int n, int s0) {
+  PdSteps a{};
+  a.n = n; a.s0 = s0; a.K = sc->hs.K; a.end = 1;
+  a.ckpt_every = std::max(1, sc->hs.checkpoint_every);
+  a.xt = sc->xt.p; a.vt = sc->vt.p; a.qn = sc->qn.p; a.c0 = sc->c0.p; a.xk = sc->xk.p; a.xk2 = sc->xk2.p;
+  a.rhs = sc->rhs.p; a.y = sc->y.p; a.slot = sc->slot.p; a.hist = sc->hist.p; a.hist_step = sc->hist_step;
+  a.ckpt_x = sc->ckpt_x.p; a.ckpt_v = sc->ckpt_v.p; a.act_all = sc->act_all.p; a.partial = sc->ps_partial.p;
+  a.iters = sc->iters.p; a.status = sc->status.p; a.vwc = sc->has_contact ? sc->vwc.p : nullptr;
+  a.to_user = sc->to_user.p; a.tab_ints = sc->ps_tab;
+  a.xkb = sc->xkb.p; a.xtb = sc->xtb.p; a.bb = sc->bb.p; a.gE = sc->gE.p; a.gnu = sc->gnu.p; a.mg = sc->mg.p;
+  a.gact = sc->gact.p; a.io_a = sc->io_a.p; a.io_b = sc->io_b.p; a.tape_warps = sc->ps_tape_warps;
+  return a;
+}
+
+static cudaError_t launch_steps(dfem_scene* sc, cudaStream_t st, PdSteps a, bool adjoint) {
+  a.res_doubles = adjoint ? sc->ps_res_a : sc->ps_res_f;
+  const size_t smem = adjoint ? sc->ps_smem_a : sc->ps_smem_f;
+  const int G = sc->bd.G;
+  const bool mx = sc->hs.precision == DFEM_PREC_MIXED;
+  sc->launches += 1;
+  if (sc->bl_cluster) {
+    auto fn = adjoint ? k_pd_adjoint<ClusterBarrier> : mx ? k_pd_forward<ClusterBarrier, true> : k_pd_forward<ClusterBarrier, false>;
+    return launch_cluster(st, fn, G, kPsThreads, smem, sc->sd, sc->bd, a);
+  }
+  auto fn = adjoint ? k_pd_adjoint<GridBarrier> : mx ? k_pd_forward<GridBarrier, true> : k_pd_forward<GridBarrier, false>;
+  return launch_coop(st, fn, G, kPsThreads, smem, sc->sd, sc->bd, a);
+}
+
+// the local-global iterations of a step with contact (the graph's first part)
+static void step_loop(dfem_scene* sc, cudaStream_t st, cudaGraphConditionalHandle) {
+  PdSteps a = steps_args(sc, 1, 0);
+  a.step = sc->step.p;
+  a.end = 0;
+  const cudaError_t e = launch_steps(sc, st, a, false);
+  if (e != cudaSuccess) sc->cur_capture_err = e;
 }
 
 static void step_pre(dfem_scene* sc, cudaStream_t st, cudaGraphConditionalHandle h) {
@@ -1692,7 +1985,8 @@ struct LoopStage {
 };
 
 // Graph = for each stage: pre kernels, then a conditional WHILE node with the
-// stage's body; then the post kernels.  Each stage has its own condition handle.
+// stage's body; then the post kernels.  Each stage has its own condition handle; a stage
+// without a body is its pre kernels alone.
 static int build_loop_graph(dfem_scene* sc, const std::vector<LoopStage>& stages, PostFn post, LoopGraph* out) {
   cudaGraph_t g = nullptr;
   CK(cudaGraphCreate(&g, 0));
@@ -1709,6 +2003,12 @@ static int build_loop_graph(dfem_scene* sc, const std::vector<LoopStage>& stages
       cudaGraph_t cg = nullptr;
       e = cudaStreamGetCaptureInfo(sc->stream, &st, nullptr, &cg, &deps, &nd);
       cudaGraphConditionalHandle h{};
+      if (!stage.body) {  // no loop
+        sc->cur_capture_err = cudaSuccess;
+        stage.pre(sc, sc->stream, h);
+        if (e == cudaSuccess) e = sc->cur_capture_err;
+        continue;
+      }
       if (e == cudaSuccess) e = cudaGraphConditionalHandleCreate(&h, cg, 1, cudaGraphCondAssignDefault);
       if (e != cudaSuccess) { where = "conditional handle"; break; }
       stage.pre(sc, sc->stream, h);
@@ -1754,9 +2054,10 @@ static int build_loop_graph(dfem_scene* sc, const std::vector<LoopStage>& stages
     out->outside = top - bodies.size();  // conditional nodes launch nothing themselves
     for (size_t k = 0; k < 2; ++k) {
       size_t inner = 0;
-      if (k < bodies.size()) cudaGraphGetNodes(bodies[k], nullptr, &inner);
+      const size_t j = stages[0].body ? k : k - 1;  // bodies skip a first stage without a loop
+      if (j < bodies.size()) cudaGraphGetNodes(bodies[j], nullptr, &inner);
       // an IF node of the solve form: its tuned branch's kernels instead of the node
-      if (k < alt_less.size() && alt_less[k] > 0)
+      if (j < alt_less.size() && alt_less[j] > 0)
         inner += (size_t)solve_launches(sc) - 1;
       (k == 0 ? out->body : out->body2) = inner;
     }
@@ -1770,12 +2071,35 @@ static int build_loop_graph(dfem_scene* sc, const std::vector<LoopStage>& stages
 }
 
 static int ensure_graphs(dfem_scene* sc) {
+  if (one_launch(sc) && !sc->has_contact) return DFEM_OK;  // no graphs: k_pd_forward / k_pd_adjoint
   if (!sc->g_step.exec) {
-    std::vector<LoopStage> st{{step_pre, step_body}};
+    std::vector<LoopStage> st;
+    if (one_launch(sc)) st.push_back({step_loop, nullptr});
+    else st.push_back({step_pre, step_body});
     if (sc->has_contact && !fused_contact(sc)) st.push_back({contact_pre, contact_body});
     RC(build_loop_graph(sc, st, step_post, &sc->g_step));
   }
-  if (!sc->g_adj.exec) RC(build_loop_graph(sc, {{adj_pre, adj_body}}, adj_post, &sc->g_adj));
+  if (!sc->g_adj.exec && !one_launch(sc)) RC(build_loop_graph(sc, {{adj_pre, adj_body}}, adj_post, &sc->g_adj));
+  return DFEM_OK;
+}
+
+// One time step from xt / vt (the step index: sc->step, set by the caller).
+static int run_step(dfem_scene* sc, int st) {
+  if (one_launch(sc) && !sc->has_contact) {
+    CK(launch_steps(sc, sc->stream, steps_args(sc, 1, st), false));
+    return DFEM_OK;
+  }
+  CK(cudaGraphLaunch(sc->g_step.exec, sc->stream));
+  return DFEM_OK;
+}
+
+// The reverse of step st's iterations, in place on io_a / io_b.
+static int run_adjoint(dfem_scene* sc, int st) {
+  if (one_launch(sc)) {
+    CK(launch_steps(sc, sc->stream, steps_args(sc, 1, st), true));
+    return DFEM_OK;
+  }
+  CK(cudaGraphLaunch(sc->g_adj.exec, sc->stream));
   return DFEM_OK;
 }
 
@@ -2071,6 +2395,8 @@ static int status_error(const int st4[4]) {
   if (st4[0] == DFEM_ERR_CAP && st4[2] > 0 && st4[2] <= 9)
     return fail(DFEM_ERR_CAP, std::string(what[st4[2]]) + " gave up (supernode " + std::to_string(st4[1]) + ", " +
                                   std::to_string(st4[3]) + " blocks)");
+  if (st4[0] == DFEM_ERR_CAP && st4[2] == kWaitGrid)
+    return fail(DFEM_ERR_CAP, "a grid-wide barrier gave up (" + std::to_string(st4[3]) + " blocks)");
   if (st4[0] == DFEM_ERR_CAP && st4[2] == kCapContactPasses)
     return fail(DFEM_ERR_CAP, "the contact phase still found new impacts after its last detection pass (pass cap)");
   if (st4[0] == DFEM_ERR_CAP && st4[2] == kCapImpacts)
@@ -2082,6 +2408,16 @@ static int status_error(const int st4[4]) {
   if (st4[0] == DFEM_ERR_CAP) return fail(DFEM_ERR_CAP, "a bounded loop gave up (contact impacts per vertex)");
   if (st4[0]) return fail(DFEM_ERR_NONFINITE, "non-finite value in the PD iteration");
   return DFEM_OK;
+}
+
+// status_error for a call's status; a barrier that gave up leaves its counters
+// behind, so they are cleared for the next launch.
+static int check_status(dfem_scene* sc, const int st4[4]) {
+  if (st4[0] == DFEM_ERR_CAP && st4[2] == kWaitGrid && sc->bl_bar.p) {
+    CK(cudaStreamSynchronize(sc->stream));
+    CK(cudaMemset(sc->bl_bar.p, 0, 2 * sizeof(unsigned)));
+  }
+  return status_error(st4);
 }
 
 // Batches: while the parts still iterating hold much of the work, the tuned
@@ -2159,6 +2495,7 @@ constexpr int kClusterMaxSupernodes = 4096;
 // fastest, then tune the per-iteration selection of batches.
 static int autotune_solve(dfem_scene* sc) {
   const size_t n3 = 3 * (size_t)sc->hs.N;
+  RC(ensure_triangular(sc));
   CK(cudaMemsetAsync(sc->rhs.p, 0, n3 * sizeof(double), sc->stream));
   reset_solve_state(sc);
   cudaEvent_t e0, e1;
@@ -2246,31 +2583,35 @@ static int autotune_solve(dfem_scene* sc) {
       rc = DFEM_OK;
     }
   }
-  // the dense-inverse form: single scenes up to kDenseMaxN vertices whose X
-  // and workspace take at most an eighth of the free memory
+  // the block-inverse form
   sc->solve_ms[5] = 0.0;
   sc->dense_build_ms = 0.0;
-  {
-    const size_t np = (size_t)((sc->hs.N + kDenseTile - 1) / kDenseTile) * kDenseTile;
-    size_t free_b = 0, total_b = 0;
-    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) free_b = 0;
-    sc->dense_ok = sc->hs.nparts == 1 && sc->hs.N <= kDenseMaxN && 2 * np * np * sizeof(double) <= free_b / 8;
-  }
-  if (rc == DFEM_OK && sc->dense_ok) {
-    int rb = dense_build(sc);  // allocates X and its workspace; the rebuild after a refactorisation is timed
-    cudaEventRecord(e0, sc->stream);
-    if (rb == DFEM_OK) rb = dense_build(sc);
-    cudaEventRecord(e1, sc->stream);
-    float tb = 0.0f;
-    if (rb == DFEM_OK && (cudaEventSynchronize(e1) != cudaSuccess || cudaEventElapsedTime(&tb, e0, e1) != cudaSuccess))
-      rb = DFEM_ERR_CUDA;
-    sc->dense_build_ms = tb;
-    if (rb == DFEM_OK) rb = time_cut(-3, &sc->solve_ms[5]);
+  if (rc == DFEM_OK) {
+    bool ok = false;
+    int rb = dense_prepare(sc, &ok);
+    sc->dense_ok = rb == DFEM_OK && ok;
+    if (sc->dense_ok) {
+      sc->solve_cut = -3;
+      sc->dense_built = false;
+      sc->cluster_launch_err = cudaSuccess;
+      rb = ensure_factor(sc);  // then the rebuild after a refactorisation, timed
+      cudaEventRecord(e0, sc->stream);
+      if (rb == DFEM_OK) rb = dense_is_x(sc) ? dense_x_build(sc) : dense_build(sc);
+      cudaEventRecord(e1, sc->stream);
+      float tb = 0.0f;
+      if (rb == DFEM_OK && (cudaEventSynchronize(e1) != cudaSuccess || cudaEventElapsedTime(&tb, e0, e1) != cudaSuccess))
+        rb = DFEM_ERR_CUDA;
+      sc->dense_build_ms = tb;
+      if (rb == DFEM_OK) rb = time_cut(-3, &sc->solve_ms[5]);
+      if (rb == DFEM_OK && sc->cluster_launch_err != cudaSuccess) rb = DFEM_ERR_CUDA;
+    }
     if (rb != DFEM_OK) {  // no room or a refused launch: not a candidate
       cudaGetLastError();
       g_last_error.clear();
+      sc->cluster_launch_err = cudaSuccess;
       dense_release(sc);
       sc->solve_ms[5] = 0.0;
+      sc->dense_ok = false;
     }
   }
   cudaEventDestroy(e0);
@@ -2287,7 +2628,7 @@ static int autotune_solve(dfem_scene* sc) {
     if (sc->solve_ms[4] > 0.0 && sc->solve_ms[4] < best) { sc->solve_cut = -2; best = sc->solve_ms[4]; }
     if (sc->solve_ms[5] > 0.0 && (best - sc->solve_ms[5]) * kDenseAmortSolves > sc->dense_build_ms) sc->solve_cut = -3;
   }
-  if (sc->solve_cut != -3 && sc->dn_A.p) dense_release(sc);
+  if (sc->solve_cut != -3 && (sc->bl_sol.p || sc->dn_A.p)) dense_release(sc);
   RC(tune_solve_select(sc));
   invalidate_graphs(sc);
   return DFEM_OK;
@@ -2509,6 +2850,32 @@ int dfem_step_forward(dfem_scene* sc, const double* x, const double* v, const do
                            sc->stream));
     }
   }
+  if (one_launch(sc) && !sc->has_contact) {
+    PdSteps a = steps_args(sc, n_steps, 0);
+    a.zero = 1;
+    a.x_in = x; a.v_in = v; a.x_out = x_out; a.v_out = v_out;
+    if (mem != DFEM_MEM_DEVICE) {
+      RC(copy_in(sc, x, n3, sc->io_a.p, mem));
+      RC(copy_in(sc, v, n3, sc->io_b.p, mem));
+      a.x_in = a.x_out = sc->io_a.p;
+      a.v_in = a.v_out = sc->io_b.p;
+    }
+    a.traj = traj_x ? (mem == DFEM_MEM_DEVICE ? traj_x : sc->traj.p) : nullptr;
+    CK(launch_steps(sc, sc->stream, a, false));
+    if (mem != DFEM_MEM_DEVICE) {
+      RC(copy_out(sc, sc->io_a.p, n3, x_out, mem));
+      RC(copy_out(sc, sc->io_b.p, n3, v_out, mem));
+      if (traj_x) RC(copy_out(sc, sc->traj.p, n3 * n_steps, traj_x, mem));
+    }
+    int st4[4] = {0, 0, 0, 0};
+    CK(cudaMemcpyAsync(st4, sc->status.p, sizeof(st4), cudaMemcpyDeviceToHost, sc->stream));
+    sc->rec_iters.assign(n_steps, 0);
+    CK(cudaMemcpyAsync(sc->rec_iters.data(), sc->iters.p, n_steps * sizeof(int), cudaMemcpyDeviceToHost, sc->stream));
+    CK(cudaStreamSynchronize(sc->stream));
+    sc->rec_passes.assign(2 * (size_t)n_steps, 0);
+    sc->rec_steps = n_steps;
+    return check_status(sc, st4);
+  }
   RC(copy_in(sc, x, n3, sc->io_a.p, mem));
   RC(copy_in(sc, v, n3, sc->io_b.p, mem));
   const int nb = sc->nblk_v;
@@ -2606,7 +2973,7 @@ int dfem_step_forward(dfem_scene* sc, const double* x, const double* v, const do
     sc->launches += (int64_t)(sc->g_step.outside + (size_t)sc->rec_iters[st] * sc->g_step.body +
                               (size_t)sc->rec_passes[2 * st + 1] * sc->g_step.body2);
   sc->rec_steps = n_steps;
-  RC(status_error(st4));
+  RC(check_status(sc, st4));
   return DFEM_OK;
 }
 
@@ -2670,6 +3037,31 @@ int dfem_step_backward(dfem_scene* sc, const double* gx_out, const double* gv_ou
   const HostScene& s = sc->hs;
   const size_t n3 = 3 * (size_t)s.N;
   const int nb = sc->nblk_v;
+  if (one_launch(sc) && !sc->has_contact && sc->hist_step != 0) {  // every step's iterates are stored: one launch
+    PdSteps a = steps_args(sc, sc->rec_steps, 0);
+    a.zero = 1;
+    a.x_in = gx_out; a.v_in = gv_out; a.x_out = gx; a.v_out = gv;
+    if (mem == DFEM_MEM_DEVICE) {
+      a.gE_out = g_youngs; a.gnu_out = g_poisson; a.gact_out = s.nseg > 0 ? g_act : nullptr;
+    } else {
+      RC(copy_in(sc, gx_out, n3, sc->io_a.p, mem));
+      RC(copy_in(sc, gv_out, n3, sc->io_b.p, mem));
+      a.x_in = a.x_out = sc->io_a.p;
+      a.v_in = a.v_out = sc->io_b.p;
+    }
+    CK(launch_steps(sc, sc->stream, a, true));
+    if (mem != DFEM_MEM_DEVICE) {
+      RC(copy_out(sc, sc->io_a.p, n3, gx, mem));
+      RC(copy_out(sc, sc->io_b.p, n3, gv, mem));
+      if (g_youngs) RC(copy_out(sc, sc->gE.p, s.T, g_youngs, mem));
+      if (g_poisson) RC(copy_out(sc, sc->gnu.p, s.T, g_poisson, mem));
+      if (g_act && s.nseg > 0) RC(copy_out(sc, sc->gact.p, (size_t)sc->rec_steps * s.nseg, g_act, mem));
+    }
+    int st4[4] = {0, 0, 0, 0};
+    CK(cudaMemcpyAsync(st4, sc->status.p, sizeof(st4), cudaMemcpyDeviceToHost, sc->stream));
+    CK(cudaStreamSynchronize(sc->stream));
+    return check_status(sc, st4);
+  }
   // incoming cotangents -> internal order (staged through rhs / c0)
   RC(copy_in(sc, gx_out, n3, sc->rhs.p, mem));
   RC(copy_in(sc, gv_out, n3, sc->c0.p, mem));
@@ -2714,7 +3106,7 @@ int dfem_step_backward(dfem_scene* sc, const double* gx_out, const double* gv_ou
                            cudaMemcpyDeviceToDevice, sc->stream));
         if (q + 1 < seg_end) {
           k_set_int<<<1, 1, 0, sc->stream>>>(sc->step.p, q);
-          CK(cudaGraphLaunch(sc->g_step.exec, sc->stream));
+          RC(run_step(sc, q));
           rerun[q] += 1;
           ++recomputed;
         }
@@ -2730,7 +3122,7 @@ int dfem_step_backward(dfem_scene* sc, const double* gx_out, const double* gv_ou
         CK(cudaMemcpyAsync(sc->vt.p, sv(st), n3 * sizeof(double), cudaMemcpyDeviceToDevice, sc->stream));
         if (sc->skel_on) RC(joint_state_at(st));
         k_set_int<<<1, 1, 0, sc->stream>>>(sc->step.p, st);
-        CK(cudaGraphLaunch(sc->g_step.exec, sc->stream));
+        RC(run_step(sc, st));
         rerun[st] += 1;
         ++recomputed;
       }
@@ -2742,7 +3134,7 @@ int dfem_step_backward(dfem_scene* sc, const double* gx_out, const double* gv_ou
         sc->launches += 1 + (sc->nF > 0 ? 1 : 0);
       }
       if (contact_step) RC(contact_adjoint_step(sc, st, recorded[st] != 0, rbase, sx(st)));
-      CK(cudaGraphLaunch(sc->g_adj.exec, sc->stream));
+      RC(run_adjoint(sc, st));
       if (contact_step) {
         const ContactAdj a = make_cadj(sc);
         k_cadj_finish<<<nb, 128, 0, sc->stream>>>(s.N, a, sc->io_a.p, sc->io_b.p);
@@ -2788,7 +3180,7 @@ int dfem_step_backward(dfem_scene* sc, const double* gx_out, const double* gv_ou
     sc->sel_seen[0] = sel[0];
     sc->sel_seen[1] = sel[1];
   }
-  return status_error(st4);
+  return check_status(sc, st4);
 }
 
 int dfem_eval_local(dfem_scene* sc, const double* x, double* jd_out, int mem) {
@@ -2855,6 +3247,7 @@ int dfem_profile_levels(dfem_scene* sc, int32_t reps, int32_t cap, int32_t* n_se
   const int G = (int)sc->segs.size();
   *n_segments = G;
   if (!ms_fwd || !ms_bwd || cap < G) return DFEM_OK;
+  RC(ensure_triangular(sc));
   cudaEvent_t e0, e1;
   CK(cudaEventCreate(&e0));
   CK(cudaEventCreate(&e1));
@@ -2906,10 +3299,9 @@ int dfem_solve_mode(dfem_scene* sc, int32_t request, int32_t* chosen, double* ms
     if (request == 5 && !sc->res_ok) return fail(DFEM_ERR_INVALID, "no resident form for this scene");
     if (request == 6) {
       if (!sc->dense_ok) return fail(DFEM_ERR_INVALID, "no dense form for this scene (a batch, or too many vertices)");
-      if (!sc->dense_built) {
-        CK(cudaStreamSynchronize(sc->stream));
-        RC(dense_build(sc));
-      }
+      bool ok = false;
+      RC(dense_prepare(sc, &ok));
+      if (!ok) return fail(DFEM_ERR_NOMEM, "no room for the dense form");
     }
     const int c = request == 1 ? n_levels(sc) : request == 2 ? 0 : request == 3 ? sc->split_cut : request == 4 ? -1
                 : request == 5 ? -2 : -3;
@@ -2918,6 +3310,7 @@ int dfem_solve_mode(dfem_scene* sc, int32_t request, int32_t* chosen, double* ms
       sc->solve_select = false;
       invalidate_graphs(sc);
     }
+    RC(ensure_factor(sc));  // the forms' factors are built on demand
   }
   if (chosen) *chosen = solve_form(sc);
   if (ms) { ms[0] = sc->solve_ms[0]; ms[1] = sc->solve_ms[1]; }

@@ -182,8 +182,8 @@ __device__ __forceinline__ double spring_length(const SceneDev& d, int t, const 
 // pointers are not restrict-qualified: a kernel that writes x in an earlier
 // phase of the same launch (k_contact_fused) must not read it through the
 // read-only data path.
-__device__ __forceinline__ void local_item(const SceneDev& d, int t, const double* x, const double* act_all,
-                                           const int* step, double* slot) {
+__device__ __forceinline__ void local_item(const SceneDev& d, int t, const double* x, const double* act_row,
+                                           double* slot) {
   if (t < d.T) {
     // corotated FEM (CorotateFEMConstraint::EvaluateDVector + EvaluateJMatrix)
     int4 v = d.tv[t];
@@ -217,7 +217,7 @@ __device__ __forceinline__ void local_item(const SceneDev& d, int t, const doubl
       c[a] = G[a][0] * f.x + G[a][1] * f.y + G[a][2] * f.z;
       Ff = Ff + c[a] * xv[a];
     }
-    double a_act = act_all[(size_t)(*step) * d.nseg + d.mseg[t]];
+    double a_act = act_row[d.mseg[t]];
     Vec3<double> p0 = (1.0 - a_act) * Ff;
     double w = d.mw[t];
     int4 sl = d.mslot[t];
@@ -232,7 +232,7 @@ __device__ __forceinline__ void local_item(const SceneDev& d, int t, const doubl
     // pneumatic spring (PneumaticConstraint::EvaluateDVector): rest * activation
     int2 v = d.sv[t];
     Vec3<double> e = ld3(x, v.x) - ld3(x, v.y);
-    Vec3<double> dd = (spring_length(d, t, act_all + (size_t)(*step) * d.nseg) * rsqrt(dot3(e, e))) * e;
+    Vec3<double> dd = (spring_length(d, t, act_row) * rsqrt(dot3(e, e))) * e;
     double w = d.ssw[t];
     int2 sl = d.sslot[t];
     st3(slot, sl.x, w * dd);
@@ -260,7 +260,7 @@ __global__ void __launch_bounds__(128, DFEM_LOCAL_MIN_BLOCKS) k_local(SceneDev d
                                                double* __restrict__ slot) {
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (gate.skip(cons_part(d, t))) return;
-  local_item(d, t, x, act_all, step, slot);
+  local_item(d, t, x, act_all + (size_t)(*step) * d.nseg, slot);
 }
 
 // ---- mixed form: FP32 projections, FP32 slots and accumulation ----------------
@@ -286,11 +286,8 @@ __device__ __forceinline__ Vec3<float> ld3f(const float* p, int i) { return mk3(
 // in FP64 first; each slot is rounded to FP32 once, from an FP64 value, and a
 // vertex's slots are summed in FP64.
 
-__global__ void __launch_bounds__(128, DFEM_FORCE_MIN_BLOCKS) k_force_f32(SceneDev d, Gate gate, const double* __restrict__ x,
-                                                   const double* __restrict__ act_all, const int* step,
-                                                   float* __restrict__ slot) {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (gate.skip(cons_part(d, t))) return;
+// Force slots of constraint t (plain pointers: see local_item).
+__device__ __forceinline__ void force_item(const SceneDev& d, int t, const double* x, const double* act_row, float* slot) {
   if (t < d.T) {
     int4 v = d.tv[t];
     Vec3<double> xv[4] = {ld3(x, v.x), ld3(x, v.y), ld3(x, v.z), ld3(x, v.w)};
@@ -328,7 +325,7 @@ __global__ void __launch_bounds__(128, DFEM_FORCE_MIN_BLOCKS) k_force_f32(SceneD
       c[0] -= ck;
       Ff = Ff + ck * ds[k];
     }
-    const double a_act = act_all[(size_t)(*step) * d.nseg + d.mseg[t]];
+    const double a_act = act_row[d.mseg[t]];
     const Vec3<double> p = (-a_act * d.mw[t]) * Ff;
     int4 sl = d.mslot[t];
     const int sv[4] = {sl.x, sl.y, sl.z, sl.w};
@@ -342,7 +339,7 @@ __global__ void __launch_bounds__(128, DFEM_FORCE_MIN_BLOCKS) k_force_f32(SceneD
     const Vec3<double> e = ld3(x, v.x) - ld3(x, v.y);
     const double len = sqrt(dot3(e, e));
     const Vec3<float> fs =
-        to_f((d.ssw[t] * (spring_length(d, t, act_all + (size_t)(*step) * d.nseg) / len - 1.0)) * e);
+        to_f((d.ssw[t] * (spring_length(d, t, act_row) / len - 1.0)) * e);
     int2 sl = d.sslot[t];
     st3f(slot, sl.x, fs);
     st3f(slot, sl.y, (-1.0f) * fs);
@@ -359,6 +356,14 @@ __global__ void __launch_bounds__(128, DFEM_FORCE_MIN_BLOCKS) k_force_f32(SceneD
     const Vec3<double> fl = sc * lap;
     for (int k = o0; k < o1; ++k) st3f(slot, d.bslot[k], to_f(d.bbeta[k] * fl));
   }
+}
+
+__global__ void __launch_bounds__(128, DFEM_FORCE_MIN_BLOCKS) k_force_f32(SceneDev d, Gate gate, const double* __restrict__ x,
+                                                   const double* __restrict__ act_all, const int* step,
+                                                   float* __restrict__ slot) {
+  int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (gate.skip(cons_part(d, t))) return;
+  force_item(d, t, x, act_all + (size_t)(*step) * d.nseg, slot);
 }
 
 // r_i = m_i/h^2 (q_i - x_i) + attach_jd_i - attach_k_i x_i + the sum of vertex i's FP32 force
@@ -1236,12 +1241,13 @@ __device__ __noinline__ void muscle_vjp(const SceneDev& d, int t, const double* 
   for (int a = 0; a < 4; ++a) st3(slot, sv[a], ((1.0 - a_act) * c[a]) * db);
 }
 
-// tape_sh: kVolTape doubles of shared memory per thread of the CTA.
+// tape: this thread's first value of the VJP's tape (kVolTape values, stride apart, in shared memory).
 // (Plain pointers: k_cadj_fused writes yb earlier in the same launch; the
 // kernels that call it keep their parameters restrict-qualified.)
 __device__ __forceinline__ void adj_local_item(const SceneDev& d, int t, const double* x, const double* yb,
                                                const double* act_row, double* slot, double* gE, double* gnu,
-                                               double* mg, const double* x1, const double* xt, double* tape_sh) {
+                                               double* mg, const double* x1, const double* xt, double* tape,
+                                               int stride) {
   if (t < d.T) {
     int4 v = d.tv[t];
     const int vi[4] = {v.x, v.y, v.z, v.w};
@@ -1254,7 +1260,7 @@ __device__ __forceinline__ void adj_local_item(const SceneDev& d, int t, const d
     double E = d.tE[t], nu = d.tnu[t], vol = d.tvol[t];
     double yr, yvv, yh = 0;
     Mat3<double> gF;
-    corot_adjoint_polar(F, Y, d.twr[t], d.twv[t], yr, yvv, gF, tape_sh + threadIdx.x, blockDim.x);
+    corot_adjoint_polar(F, Y, d.twr[t], d.twv[t], yr, yvv, gF, tape, stride);
     if (x1) {
       Vec3<double> x1v[4] = {ld3(x1, vi[0]), ld3(x1, vi[1]), ld3(x1, vi[2]), ld3(x1, vi[3])};
       Mat3<double> F1 = deformation(G, x1v);
@@ -1333,7 +1339,7 @@ __global__ void __launch_bounds__(128, DFEM_ADJ_MIN_BLOCKS) k_adj_local(SceneDev
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t < d.N && !gate.skip(vpart_of(d, t))) st3(bb, t, ld3(bb, t) + ld3(yb, t));
   if (gate.skip(cons_part(d, t))) return;
-  adj_local_item(d, t, x, yb, act_all + (size_t)(*step) * d.nseg, slot, gE, gnu, mg, x1, nullptr, tape);
+  adj_local_item(d, t, x, yb, act_all + (size_t)(*step) * d.nseg, slot, gE, gnu, mg, x1, nullptr, tape + threadIdx.x, 128);
 }
 
 // xbar^k = sum of the slots (constraints without x dependence contribute nothing)

@@ -390,6 +390,64 @@ __device__ __forceinline__ Mat3<double> rot_from_quat(const float qf[4]) {
   return R;
 }
 
+// The mixed form's FP32 SVD: svd3's method in explicitly rounded operations,
+// so that its singular vectors, whose FP32 roundings reach the results, are
+// the same bits in every kernel that inlines it (left to itself, the compiler
+// fuses products and sums differently from one kernel to the next).
+__device__ __forceinline__ float rn_dot(Vec3<float> a, Vec3<float> b) {
+  return __fmaf_rn(a.z, b.z, __fmaf_rn(a.x, b.x, __fmul_rn(a.y, b.y)));
+}
+__device__ __forceinline__ Vec3<float> rn_scale(float s, Vec3<float> a) {
+  return {__fmul_rn(s, a.x), __fmul_rn(s, a.y), __fmul_rn(s, a.z)};
+}
+__device__ __forceinline__ Vec3<float> rn_axpy(float s, Vec3<float> a, Vec3<float> b) {  // s a + b
+  return {__fmaf_rn(s, a.x, b.x), __fmaf_rn(s, a.y, b.y), __fmaf_rn(s, a.z, b.z)};
+}
+__device__ __forceinline__ void jacobi_rotate_f(Vec3<float>& bp, Vec3<float>& bq, Vec3<float>& vp, Vec3<float>& vq,
+                                                bool& rotated) {
+  const float a = rn_dot(bp, bp), b = rn_dot(bq, bq), g = rn_dot(bp, bq);
+  if (!(fabsf(g) > __fmul_rn(Eps<float>::rot, __fsqrt_rn(__fmul_rn(a, b))))) return;
+  rotated = true;
+  const float zeta = __fdiv_rn(__fsub_rn(b, a), __fmul_rn(2.0f, g));
+  const float t = __fdiv_rn(zeta >= 0.0f ? 1.0f : -1.0f, __fadd_rn(fabsf(zeta), __fsqrt_rn(__fmaf_rn(zeta, zeta, 1.0f))));
+  const float c = rsqrtf(__fmaf_rn(t, t, 1.0f)), s = __fmul_rn(c, t);
+  const Vec3<float> nbp = rn_axpy(c, bp, rn_scale(-s, bq)), nbq = rn_axpy(c, bq, rn_scale(s, bp));
+  const Vec3<float> nvp = rn_axpy(c, vp, rn_scale(-s, vq)), nvq = rn_axpy(c, vq, rn_scale(s, vp));
+  bp = nbp; bq = nbq; vp = nvp; vq = nvq;
+}
+__device__ __forceinline__ Svd3<float> svd3_f(const Mat3<float>& F) {
+  Svd3<float> o;
+  Vec3<float> b0 = F.c[0], b1 = F.c[1], b2 = F.c[2];
+  Vec3<float> v0 = mk3(1.0f, 0.0f, 0.0f), v1 = mk3(0.0f, 1.0f, 0.0f), v2 = mk3(0.0f, 0.0f, 1.0f);
+#pragma unroll 1
+  for (int sweep = 0; sweep < Eps<float>::sweeps; ++sweep) {
+    bool rotated = false;
+    jacobi_rotate_f(b0, b1, v0, v1, rotated);
+    jacobi_rotate_f(b0, b2, v0, v2, rotated);
+    jacobi_rotate_f(b1, b2, v1, v2, rotated);
+    if (!rotated) break;
+  }
+  float s0 = __fsqrt_rn(rn_dot(b0, b0)), s1 = __fsqrt_rn(rn_dot(b1, b1)), s2 = __fsqrt_rn(rn_dot(b2, b2));
+  auto swap3 = [](float& s, float& t, Vec3<float>& b, Vec3<float>& e, Vec3<float>& v, Vec3<float>& w) {
+    if (s < t) { const float q = s; s = t; t = q; Vec3<float> x = b; b = e; e = x; x = v; v = w; w = x; }
+  };
+  swap3(s0, s1, b0, b1, v0, v1);
+  swap3(s0, s2, b0, b2, v0, v2);
+  swap3(s1, s2, b1, b2, v1, v2);
+  o.s[0] = s0; o.s[1] = s1; o.s[2] = s2;
+  o.v[0] = v0; o.v[1] = v1; o.v[2] = v2;
+  const float tiny = __fmul_rn(Eps<float>::rel, s0);
+  o.u[0] = s0 > 0.0f ? rn_scale(__fdiv_rn(1.0f, s0), b0) : mk3(1.0f, 0.0f, 0.0f);
+  if (s1 > tiny) {
+    o.u[1] = rn_scale(__fdiv_rn(1.0f, s1), b1);
+  } else {  // complete the basis (such an element takes the FP64 branch)
+    const Vec3<float> w = cross3(o.u[0], fabsf(o.u[0].x) < 0.9f ? mk3(1.0f, 0.0f, 0.0f) : mk3(0.0f, 1.0f, 0.0f));
+    o.u[1] = rsqrtf(rn_dot(w, w)) * w;
+  }
+  o.u[2] = s2 > tiny ? rn_scale(__fdiv_rn(1.0f, s2), b2) : cross3(o.u[0], o.u[1]);
+  return o;
+}
+
 // Mixed-form corotated deviations DR = md - F and DV = md_volume - F (columns;
 // the tet's J d - L x is G (wr DR + wv DV)).  Only the SVD runs in FP32; its
 // error enters the deviations at second order:
@@ -410,7 +468,7 @@ __device__ __forceinline__ bool corot_delta_mixed(const Mat3<double>& F, Vec3<do
   Mat3<float> Ff;
 #pragma unroll
   for (int j = 0; j < 3; ++j) Ff.c[j] = mk3((float)F.c[j].x, (float)F.c[j].y, (float)F.c[j].z);
-  const Svd3<float> sv = svd3(Ff);
+  const Svd3<float> sv = svd3_f(Ff);
   const float smax = fmaxf(sv.s[0], fmaxf(sv.s[1], sv.s[2]));
   const float smin = fminf(sv.s[0], fminf(sv.s[1], sv.s[2]));
   if (!(smax > 0.0f) || !(smin >= kDegenerateRatio * smax) || !(det3(F) > 0.0)) return false;
@@ -418,7 +476,7 @@ __device__ __forceinline__ bool corot_delta_mixed(const Mat3<double>& F, Vec3<do
                            {sv.v[0].z, sv.v[1].z, sv.v[2].z}};
   Mat3<float> R0;
 #pragma unroll
-  for (int j = 0; j < 3; ++j) R0.c[j] = vjf[j][0] * sv.u[0] + vjf[j][1] * sv.u[1] + vjf[j][2] * sv.u[2];
+  for (int j = 0; j < 3; ++j) R0.c[j] = rn_axpy(vjf[j][2], sv.u[2], rn_axpy(vjf[j][0], sv.u[0], rn_scale(vjf[j][1], sv.u[1])));
   float q[4];
   quat_from_rot(R0, q);
   const Mat3<double> R = rot_from_quat(q);
