@@ -243,35 +243,49 @@ void block_shares(const BlockPlan& P, int G, std::vector<BlockChunk>& chunks, st
   ptr.assign((size_t)phases * (G + 1), 0);
   for (int p = 0; p < phases; ++p) {
     const bool fwd = p < P.tiers;
-    const int tier = fwd ? p : 2 * P.tiers - 2 - p;
-    // cost of a row: its products plus a fixed part (reduction, epilogue); of a block in a CTA: staging its vector
+    const int tier = fwd ? p : 2 * P.tiers - 2 - p, b0 = P.tier_ptr[tier], b1 = P.tier_ptr[tier + 1], nb = b1 - b0;
+    // a row costs its products and a fixed part (reduction, epilogue)
     auto rows = [&](const BlockInfo& B) { return fwd ? B.n + B.r : B.n; };
     auto width = [&](const BlockInfo& B) { return (fwd ? B.n : B.r) + 64; };
-    double total = 0;
-    for (int b = P.tier_ptr[tier]; b < P.tier_ptr[tier + 1]; ++b) total += (double)rows(P.blk[b]) * width(P.blk[b]);
-    const double share = total / G;
-    int c = 0;
-    double room = share;
-    ptr[(size_t)p * (G + 1)] = (int)chunks.size();
-    for (int b = P.tier_ptr[tier]; b < P.tier_ptr[tier + 1]; ++b) {
-      const int R = rows(P.blk[b]);
-      const double w = width(P.blk[b]);
-      int r0 = 0;
-      while (r0 < R) {
-        int k = (int)std::ceil(room / w - 1e-9);
-        if (c == G - 1) k = R - r0;
-        k = std::max(0, std::min(k, R - r0));
-        if (k > 0) chunks.push_back(BlockChunk{b, r0, k});
-        r0 += k;
-        room -= k * w;
-        if (room <= 1e-6 * share && c < G - 1) {
-          ptr[(size_t)p * (G + 1) + ++c] = (int)chunks.size();
-          room += share;
-          if (room < 0) room = 0;
+    std::vector<double> cost(nb);
+    std::vector<std::vector<BlockChunk>> mine(G);
+    for (int k = 0; k < nb; ++k) cost[k] = (double)rows(P.blk[b0 + k]) * width(P.blk[b0 + k]);
+    if (nb <= G) {
+      // whole CTAs per block, given one by one to the block with the largest
+      // share: a CTA with parts of two blocks would stage twice, and every
+      // phase ends with its slowest CTA
+      std::vector<int> ctas(nb, 1);
+      for (int left = G - nb; left > 0; --left) {
+        int best = -1;
+        for (int k = 0; k < nb; ++k)
+          if (ctas[k] < rows(P.blk[b0 + k]) && (best < 0 || cost[k] / ctas[k] > cost[best] / ctas[best])) best = k;
+        if (best < 0) break;
+        ++ctas[best];
+      }
+      int c = 0;
+      for (int k = 0; k < nb; ++k) {
+        const int R = rows(P.blk[b0 + k]), m = ctas[k];
+        for (int q = 0; q < m; ++q, ++c) {
+          const int r0 = (int)((int64_t)R * q / m), r1 = (int)((int64_t)R * (q + 1) / m);
+          if (r1 > r0) mine[c].push_back(BlockChunk{b0 + k, r0, r1 - r0});
         }
       }
+    } else {  // whole blocks, the largest first, each to the CTA with the least
+      std::vector<int> order(nb);
+      std::iota(order.begin(), order.end(), 0);
+      std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cost[x] > cost[y]; });
+      std::vector<double> load(G, 0.0);
+      for (int k : order) {
+        const int c = (int)(std::min_element(load.begin(), load.end()) - load.begin());
+        load[c] += cost[k];
+        if (rows(P.blk[b0 + k]) > 0) mine[c].push_back(BlockChunk{b0 + k, 0, rows(P.blk[b0 + k])});
+      }
     }
-    while (c < G) ptr[(size_t)p * (G + 1) + ++c] = (int)chunks.size();
+    for (int c = 0; c < G; ++c) {
+      ptr[(size_t)p * (G + 1) + c] = (int)chunks.size();
+      chunks.insert(chunks.end(), mine[c].begin(), mine[c].end());
+    }
+    ptr[(size_t)p * (G + 1) + G] = (int)chunks.size();
   }
 }
 

@@ -864,7 +864,7 @@ static int plan_steps(dfem_scene* sc, int vec, int G, const std::vector<BlockChu
         const BlockInfo& B = P.blk[chunks[k].blk];
         const bool fwd = p < P.tiers;
         ++nch;
-        ti += ((fwd && B.tier > 0) ? 3 : 1) * (fwd ? B.n : B.r);
+        ti += ((fwd && B.tier > 0) ? 3 : 1) * (fwd ? B.n : B.r) + chunks[k].rows;
         rd += (size_t)chunks[k].rows * (fwd ? B.ldx : B.ldr);
       }
     if (nch > kPsChunks) return DFEM_OK;
@@ -873,8 +873,7 @@ static int plan_steps(dfem_scene* sc, int vec, int G, const std::vector<BlockChu
   }
   if (phases > 31) return DFEM_OK;
   sc->ps_tab = std::min((tab + 3) & ~3, kMaxTab);
-  const int ncons = s.T + s.M + s.S + s.B;
-  sc->ps_tape_warps = std::max(1, std::min(8, (ncons + 32 * G - 1) / (32 * G)));
+  sc->ps_tape_warps = std::max(1, std::min(kPsWarps / 2, (s.T + 32 * G - 1) / (32 * G)));
   const size_t fixed = ps_fixed_doubles(vec) + sc->ps_tab / 2, tape = (size_t)kVolTape * 32 * sc->ps_tape_warps;
   if (fixed + tape > kMaxSmem) return DFEM_OK;
   rows = (rows + 1) & ~size_t(1);
@@ -894,6 +893,28 @@ static int plan_steps(dfem_scene* sc, int vec, int G, const std::vector<BlockChu
   CK(sc->ps_partial.alloc(2 * (size_t)G));
   sc->ps_ok = true;
   return DFEM_OK;
+}
+
+// Whether the device schedules a 16-CTA cluster of the solve.
+static bool cluster_fits() {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(kBlockClusterCtas);
+  cfg.blockDim = dim3(kBsThreads);
+  cfg.dynamicSmemBytes = 224 * 1024;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = kBlockClusterCtas;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const void* fn = (const void*)k_pd_adjoint<ClusterBarrier>;
+  int n = 0;
+  const bool ok = raise_smem_limit(fn, cfg.dynamicSmemBytes) == cudaSuccess &&
+                  cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                  cudaOccupancyMaxActiveClusters(&n, fn, &cfg) == cudaSuccess && n >= 1;
+  cudaGetLastError();
+  return ok;
 }
 
 // Buffers, tables and launch shapes of the dense form (block-inverse: single
@@ -922,7 +943,14 @@ static int dense_prepare(dfem_scene* sc, bool* ok) {
     int most = 1;
     for (int t = 0; t < P.tiers; ++t) most = std::max(most, P.tier_tile[t + 1] - P.tier_tile[t]);
     sc->bf_grid = std::min(nsm * occ, most);
-    sc->bl_cluster = getenv("DFEM_CL") && sc->hs.N <= atoi(getenv("DFEM_CL"));
+    // One cluster or the grid: a barrier of the cluster takes 0.25 us, of the
+    // grid 1.2 us, three per iteration, but sixteen SMs run the elements of a
+    // larger scene in turns and stream a larger inverse through less of L2.
+    // Forward + adjoint per iteration, grid / cluster: 144 vertices (cloth)
+    // 26.2 / 20.9 us, 275 (800 tets) 26.9 / 23.1, 396 (1,250 tets) 30.3 /
+    // 27.9, 484 (cloth) 30.9 / 26.9, 961 (cloth) 35.7 / 46.7, 1,029 (3,600
+    // tets) 35.4 / 59.
+    sc->bl_cluster = sc->hs.N <= 512 && sc->hs.T <= 2048 && cluster_fits();
     const int G = sc->bl_cluster ? kBlockClusterCtas : nsm;
     std::vector<BlockChunk> chunks;
     std::vector<int> share;

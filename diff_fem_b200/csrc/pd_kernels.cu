@@ -177,32 +177,8 @@ __device__ __forceinline__ double spring_length(const SceneDev& d, int t, const 
   return c < 0 ? r : r * act_row[c];
 }
 
-// Local step of constraint t (tets, muscles, springs, bending stencils in
-// that order): its projection and its J*d contribution to its slots.  The
-// pointers are not restrict-qualified: a kernel that writes x in an earlier
-// phase of the same launch (k_contact_fused) must not read it through the
-// read-only data path.
-__device__ __forceinline__ void local_item(const SceneDev& d, int t, const double* x, const double* act_row,
-                                           double* slot) {
-  if (t < d.T) {
-    // corotated FEM (CorotateFEMConstraint::EvaluateDVector + EvaluateJMatrix)
-    int4 v = d.tv[t];
-    Vec3<double> xv[4] = {ld3(x, v.x), ld3(x, v.y), ld3(x, v.z), ld3(x, v.w)};
-    double G[4][3];
-    load_g(d.tinv, d.T, t, G);
-    Mat3<double> F = deformation(G, xv), md, mdv;
-    corot_project_polar(F, md, mdv);
-    double wr = d.twr[t], wv = d.twv[t];
-    Vec3<double> P[3];
-#pragma unroll
-    for (int j = 0; j < 3; ++j) P[j] = rn_axpy(wr, md.c[j], rn_scale(wv, mdv.c[j]));
-    int4 sl = d.tslot[t];
-    const int sv[4] = {sl.x, sl.y, sl.z, sl.w};
-#pragma unroll
-    for (int a = 0; a < 4; ++a) st3(slot, sv[a], G[a][0] * P[0] + G[a][1] * P[1] + G[a][2] * P[2]);
-    return;
-  }
-  t -= d.T;
+// Local step of the constraints other than tets: t counts from the first muscle.
+__device__ __forceinline__ void local_rest(const SceneDev& d, int t, const double* x, const double* act_row, double* slot) {
   if (t < d.M) {
     // muscle (LinearMuscleConstraint::Computep0 + EvaluateJMatrix): d = (1-a) F f
     int4 v = d.mv[t];
@@ -251,6 +227,34 @@ __device__ __forceinline__ void local_item(const SceneDev& d, int t, const doubl
     if (ln > 1e-25) dd = (w * d.brest[t] / ln) * lap;
     for (int k = o0; k < o1; ++k) st3(slot, d.bslot[k], (w * d.bbeta[k]) * dd);
   }
+}
+
+// Local step of constraint t (tets, muscles, springs, bending stencils in
+// that order): its projection and its J*d contribution to its slots.  The
+// pointers are not restrict-qualified: a kernel that writes x in an earlier
+// phase of the same launch (k_contact_fused) must not read it through the
+// read-only data path.
+__device__ __forceinline__ void local_item(const SceneDev& d, int t, const double* x, const double* act_row,
+                                           double* slot) {
+  if (t < d.T) {
+    // corotated FEM (CorotateFEMConstraint::EvaluateDVector + EvaluateJMatrix)
+    int4 v = d.tv[t];
+    Vec3<double> xv[4] = {ld3(x, v.x), ld3(x, v.y), ld3(x, v.z), ld3(x, v.w)};
+    double G[4][3];
+    load_g(d.tinv, d.T, t, G);
+    Mat3<double> F = deformation(G, xv), md, mdv;
+    corot_project_polar(F, md, mdv);
+    double wr = d.twr[t], wv = d.twv[t];
+    Vec3<double> P[3];
+#pragma unroll
+    for (int j = 0; j < 3; ++j) P[j] = rn_axpy(wr, md.c[j], rn_scale(wv, mdv.c[j]));
+    int4 sl = d.tslot[t];
+    const int sv[4] = {sl.x, sl.y, sl.z, sl.w};
+#pragma unroll
+    for (int a = 0; a < 4; ++a) st3(slot, sv[a], G[a][0] * P[0] + G[a][1] * P[1] + G[a][2] * P[2]);
+    return;
+  }
+  local_rest(d, t - d.T, x, act_row, slot);
 }
 
 // Local step: every constraint projects and writes its J*d contribution to its
@@ -1241,6 +1245,48 @@ __device__ __noinline__ void muscle_vjp(const SceneDev& d, int t, const double* 
   for (int a = 0; a < 4; ++a) st3(slot, sv[a], ((1.0 - a_act) * c[a]) * db);
 }
 
+// VJP of the constraints other than tets: t counts from the first muscle.
+__device__ __forceinline__ void adj_local_rest(const SceneDev& d, int t, const double* x, const double* yb,
+                                               const double* act_row, double* slot, double* mg) {
+  if (t < d.M) {
+    muscle_vjp(d, t, x, yb, act_row, slot, mg);
+    return;
+  }
+  t -= d.M;
+  if (t < d.S) {
+    int2 v = d.sv[t];
+    double w = d.ssw[t];
+    Vec3<double> db = w * (ld3(yb, v.x) - ld3(yb, v.y));
+    Vec3<double> e = ld3(x, v.x) - ld3(x, v.y);
+    double inv = rsqrt(dot3(e, e));
+    Vec3<double> eh = inv * e;
+    // a pneumatic spring's activation term: d md / d a = rest * eh
+    if (d.sch && d.sch[t] >= 0) mg[d.M + t] = d.srest[t] * dot3(db, eh);
+    Vec3<double> ge = (spring_length(d, t, act_row) * inv) * (db - dot3(eh, db) * eh);
+    int2 sl = d.sslot[t];
+    st3(slot, sl.x, ge);
+    st3(slot, sl.y, (-1.0) * ge);
+    return;
+  }
+  t -= d.S;
+  if (t < d.B) {
+    int o0 = d.boff[t], o1 = d.boff[t + 1];
+    double w = d.bw[t];
+    Vec3<double> db = mk3(0.0, 0.0, 0.0), lap = mk3(0.0, 0.0, 0.0);
+    for (int q = o0; q < o1; ++q) {
+      db = db + (w * d.bbeta[q]) * ld3(yb, d.bv[q]);
+      lap = lap + d.bbeta[q] * ld3(x, d.bv[q]);
+    }
+    double ln = sqrt(dot3(lap, lap));
+    Vec3<double> gl = mk3(0.0, 0.0, 0.0);
+    if (ln > 1e-25) {
+      Vec3<double> lh = (1.0 / ln) * lap;
+      gl = (w * d.brest[t] / ln) * (db - dot3(lh, db) * lh);
+    }
+    for (int q = o0; q < o1; ++q) st3(slot, d.bslot[q], d.bbeta[q] * gl);
+  }
+}
+
 // tape: this thread's first value of the VJP's tape (kVolTape values, stride apart, in shared memory).
 // (Plain pointers: k_cadj_fused writes yb earlier in the same launch; the
 // kernels that call it keep their parameters restrict-qualified.)
@@ -1284,44 +1330,7 @@ __device__ __forceinline__ void adj_local_item(const SceneDev& d, int t, const d
     for (int a = 0; a < 4; ++a) st3(slot, sv[a], G[a][0] * gF.c[0] + G[a][1] * gF.c[1] + G[a][2] * gF.c[2]);
     return;
   }
-  t -= d.T;
-  if (t < d.M) {
-    muscle_vjp(d, t, x, yb, act_row, slot, mg);
-    return;
-  }
-  t -= d.M;
-  if (t < d.S) {
-    int2 v = d.sv[t];
-    double w = d.ssw[t];
-    Vec3<double> db = w * (ld3(yb, v.x) - ld3(yb, v.y));
-    Vec3<double> e = ld3(x, v.x) - ld3(x, v.y);
-    double inv = rsqrt(dot3(e, e));
-    Vec3<double> eh = inv * e;
-    // a pneumatic spring's activation term: d md / d a = rest * eh
-    if (d.sch && d.sch[t] >= 0) mg[d.M + t] = d.srest[t] * dot3(db, eh);
-    Vec3<double> ge = (spring_length(d, t, act_row) * inv) * (db - dot3(eh, db) * eh);
-    int2 sl = d.sslot[t];
-    st3(slot, sl.x, ge);
-    st3(slot, sl.y, (-1.0) * ge);
-    return;
-  }
-  t -= d.S;
-  if (t < d.B) {
-    int o0 = d.boff[t], o1 = d.boff[t + 1];
-    double w = d.bw[t];
-    Vec3<double> db = mk3(0.0, 0.0, 0.0), lap = mk3(0.0, 0.0, 0.0);
-    for (int q = o0; q < o1; ++q) {
-      db = db + (w * d.bbeta[q]) * ld3(yb, d.bv[q]);
-      lap = lap + d.bbeta[q] * ld3(x, d.bv[q]);
-    }
-    double ln = sqrt(dot3(lap, lap));
-    Vec3<double> gl = mk3(0.0, 0.0, 0.0);
-    if (ln > 1e-25) {
-      Vec3<double> lh = (1.0 / ln) * lap;
-      gl = (w * d.brest[t] / ln) * (db - dot3(lh, db) * lh);
-    }
-    for (int q = o0; q < o1; ++q) st3(slot, d.bslot[q], d.bbeta[q] * gl);
-  }
+  adj_local_rest(d, t - d.T, x, yb, act_row, slot, mg);
 }
 
 // Reverse PD iteration k (k read from device memory): local VJP at x^k with

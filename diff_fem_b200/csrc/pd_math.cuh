@@ -241,9 +241,12 @@ __device__ __forceinline__ void rn_cof(const Mat3<double>& a, Mat3<double>& c) {
 // Polar factor of F (C = cof(F) and det = det(F) given); false when the
 // element is near a lower rank (or not finite).
 constexpr int kPolarIterations = 16;
-__device__ __forceinline__ bool polar_newton(const Mat3<double>& F, Mat3<double> C, double det, Mat3<double>& Q) {
+__device__ __forceinline__ bool full_rank(const Mat3<double>& F, double det) {
   const double q = __dmul_rn(rn_dot(F, F), 1.0 / 3.0);
-  if (!(__dmul_rn(det, det) > __dmul_rn(1e-4, __dmul_rn(q, __dmul_rn(q, q)))) || !isfinite(det)) return false;
+  return __dmul_rn(det, det) > __dmul_rn(1e-4, __dmul_rn(q, __dmul_rn(q, q))) && isfinite(det);
+}
+__device__ __forceinline__ bool polar_newton(const Mat3<double>& F, Mat3<double> C, double det, Mat3<double>& Q) {
+  if (!full_rank(F, det)) return false;
   Q = F;
   double d2 = 1.0;
 #pragma unroll 1
@@ -329,6 +332,35 @@ __device__ __forceinline__ void volume_newton(const Mat3<double>& F, Mat3<double
 
 static __device__ __noinline__ void corot_project_svd(const Mat3<double>& F, Mat3<double>& md, Mat3<double>& mdv) {
   corot_project(F, md, mdv);
+}
+
+// The two halves of the projection, for kernels that give them to two threads:
+// md (reflected rotation) and md_volume of an element.
+__device__ __forceinline__ void corot_rotation(const Mat3<double>& F, Mat3<double>& md) {
+  Mat3<double> C;
+  rn_cof(F, C);
+  const double det = rn_dot(F.c[0], C.c[0]);
+  if (!polar_newton(F, C, det, md)) {
+    Mat3<double> f = F, a, b;
+    corot_project_svd(f, a, b);
+    md = a;
+    return;
+  }
+  if (det < 0.0) md.c[2] = rn_scale(-1.0, md.c[2]);
+}
+__device__ __forceinline__ void corot_volume(const Mat3<double>& F, Mat3<double>& mdv) {
+  Mat3<double> C, D;
+  rn_cof(F, C);
+  const double det = rn_dot(F.c[0], C.c[0]);
+  if (!full_rank(F, det)) {
+    Mat3<double> f = F, a, b;
+    corot_project_svd(f, a, b);
+    mdv = b;
+    return;
+  }
+  volume_newton<false>(F, C, det, D, nullptr);
+#pragma unroll
+  for (int j = 0; j < 3; ++j) mdv.c[j] = rn_add(F.c[j], D.c[j]);
 }
 
 // md (reflected rotation) and md_volume of an element.
@@ -629,58 +661,48 @@ static __device__ __noinline__ void corot_adjoint_svd(const Mat3<double>& F, con
 //   volume steps in reverse, D' = c C, c = num / (C : C):
 //     gc = gD' : C,  gC = c gD' + gc / (C : C) (D - 2 c C),
 //     gP = sigma cofT(P, gC) - gc / (C : C) C,  gD = gc / (C : C) C + gP, gF += gP.
-__device__ __forceinline__ void corot_adjoint_polar(const Mat3<double>& F, const Mat3<double>& Y, double wr, double wv,
-                                                    double& yr, double& yv, Mat3<double>& gF, double* tape_sh,
-                                                    int stride) {
-  Mat3<double> C, Q;
-  rn_cof(F, C);
-  const double det = rn_dot(F.c[0], C.c[0]);
-  if (!polar_newton(F, C, det, Q)) {
-    Mat3<double> f = F, y = Y, g;
-    double a, b;
-    corot_adjoint_svd(f, y, wr, wv, a, b, g);
-    yr = a;
-    yv = b;
-    gF = g;
-    return;
-  }
+__device__ __forceinline__ void rotation_vjp(const Mat3<double>& F, const Mat3<double>& Q, double sg, const Mat3<double>& Y,
+                                             double wr, double& yr, Mat3<double>& gF) {
+  const Vec3<double> g2 = rn_scale(sg, Y.c[2]);  // md's column 2 is sigma times Q's
+  yr = __dadd_rn(rn_dot(Y.c[0], Q.c[0]), __dadd_rn(rn_dot(Y.c[1], Q.c[1]), rn_dot(g2, Q.c[2])));
+  const double b0 = __dadd_rn(rn_dot(Q.c[2], Y.c[1]), -rn_dot(Q.c[1], g2));
+  const double b1 = __dadd_rn(rn_dot(Q.c[0], g2), -rn_dot(Q.c[2], Y.c[0]));
+  const double b2 = __dadd_rn(rn_dot(Q.c[1], Y.c[0]), -rn_dot(Q.c[0], Y.c[1]));
+  const double s00 = rn_dot(Q.c[0], F.c[0]), s11 = rn_dot(Q.c[1], F.c[1]), s22 = rn_dot(Q.c[2], F.c[2]);
+  const double k01 = __dmul_rn(-0.5, __dadd_rn(rn_dot(Q.c[0], F.c[1]), rn_dot(Q.c[1], F.c[0])));
+  const double k02 = __dmul_rn(-0.5, __dadd_rn(rn_dot(Q.c[0], F.c[2]), rn_dot(Q.c[2], F.c[0])));
+  const double k12 = __dmul_rn(-0.5, __dadd_rn(rn_dot(Q.c[1], F.c[2]), rn_dot(Q.c[2], F.c[1])));
+  const double k00 = __dadd_rn(s11, s22), k11 = __dadd_rn(s00, s22), k22 = __dadd_rn(s00, s11);
+  // the symmetric 3x3 system by its cofactors
+  const double a00 = __fma_rn(k11, k22, -__dmul_rn(k12, k12)), a01 = __fma_rn(k02, k12, -__dmul_rn(k01, k22));
+  const double a02 = __fma_rn(k01, k12, -__dmul_rn(k02, k11)), a11 = __fma_rn(k00, k22, -__dmul_rn(k02, k02));
+  const double a12 = __fma_rn(k01, k02, -__dmul_rn(k00, k12)), a22 = __fma_rn(k00, k11, -__dmul_rn(k01, k01));
+  const double w = wr / rn_dot(mk3(k00, k01, k02), mk3(a00, a01, a02));
+  const Vec3<double> b = mk3(b0, b1, b2);
+  const double z0 = __dmul_rn(w, rn_dot(mk3(a00, a01, a02), b)), z1 = __dmul_rn(w, rn_dot(mk3(a01, a11, a12), b)),
+               z2 = __dmul_rn(w, rn_dot(mk3(a02, a12, a22), b));
+  gF.c[0] = rn_axpy(z2, Q.c[1], rn_scale(-z1, Q.c[2]));
+  gF.c[1] = rn_axpy(z0, Q.c[2], rn_scale(-z2, Q.c[0]));
+  gF.c[2] = rn_axpy(z1, Q.c[0], rn_scale(-z0, Q.c[1]));
+}
+
+// gF: the volume part of the VJP alone.
+__device__ __forceinline__ void volume_vjp(const Mat3<double>& F, const Mat3<double>& C0, double det, const Mat3<double>& Y,
+                                           double wv, double& yv, Mat3<double>& gF, double* tape_sh, int stride) {
   const double sg = det < 0.0 ? -1.0 : 1.0;
-  {  // rotation
-    const Vec3<double> g2 = rn_scale(sg, Y.c[2]);  // md's column 2 is sigma times Q's
-    yr = __dadd_rn(rn_dot(Y.c[0], Q.c[0]), __dadd_rn(rn_dot(Y.c[1], Q.c[1]), rn_dot(g2, Q.c[2])));
-    const double b0 = __dadd_rn(rn_dot(Q.c[2], Y.c[1]), -rn_dot(Q.c[1], g2));
-    const double b1 = __dadd_rn(rn_dot(Q.c[0], g2), -rn_dot(Q.c[2], Y.c[0]));
-    const double b2 = __dadd_rn(rn_dot(Q.c[1], Y.c[0]), -rn_dot(Q.c[0], Y.c[1]));
-    const double s00 = rn_dot(Q.c[0], F.c[0]), s11 = rn_dot(Q.c[1], F.c[1]), s22 = rn_dot(Q.c[2], F.c[2]);
-    const double k01 = __dmul_rn(-0.5, __dadd_rn(rn_dot(Q.c[0], F.c[1]), rn_dot(Q.c[1], F.c[0])));
-    const double k02 = __dmul_rn(-0.5, __dadd_rn(rn_dot(Q.c[0], F.c[2]), rn_dot(Q.c[2], F.c[0])));
-    const double k12 = __dmul_rn(-0.5, __dadd_rn(rn_dot(Q.c[1], F.c[2]), rn_dot(Q.c[2], F.c[1])));
-    const double k00 = __dadd_rn(s11, s22), k11 = __dadd_rn(s00, s22), k22 = __dadd_rn(s00, s11);
-    // the symmetric 3x3 system by its cofactors
-    const double a00 = __fma_rn(k11, k22, -__dmul_rn(k12, k12)), a01 = __fma_rn(k02, k12, -__dmul_rn(k01, k22));
-    const double a02 = __fma_rn(k01, k12, -__dmul_rn(k02, k11)), a11 = __fma_rn(k00, k22, -__dmul_rn(k02, k02));
-    const double a12 = __fma_rn(k01, k02, -__dmul_rn(k00, k12)), a22 = __fma_rn(k00, k11, -__dmul_rn(k01, k01));
-    const double w = wr / rn_dot(mk3(k00, k01, k02), mk3(a00, a01, a02));
-    const Vec3<double> b = mk3(b0, b1, b2);
-    const double z0 = __dmul_rn(w, rn_dot(mk3(a00, a01, a02), b)), z1 = __dmul_rn(w, rn_dot(mk3(a01, a11, a12), b)),
-                 z2 = __dmul_rn(w, rn_dot(mk3(a02, a12, a22), b));
-    gF.c[0] = rn_axpy(z2, Q.c[1], rn_scale(-z1, Q.c[2]));
-    gF.c[1] = rn_axpy(z0, Q.c[2], rn_scale(-z2, Q.c[0]));
-    gF.c[2] = rn_axpy(z1, Q.c[0], rn_scale(-z0, Q.c[1]));
-  }
+  Mat3<double> C, gD;
   VolTape tape;
   tape.sh = tape_sh;
   tape.stride = stride;
-  Mat3<double> gD;
   {
     Mat3<double> D;
-    volume_newton<true>(F, C, det, D, &tape);
+    volume_newton<true>(F, C0, det, D, &tape);
     yv = 0.0;
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
       yv = __dadd_rn(yv, rn_dot(Y.c[j], rn_add(F.c[j], D.c[j])));
       gD.c[j] = rn_scale(wv, Y.c[j]);
-      gF.c[j] = rn_add(gF.c[j], gD.c[j]);
+      gF.c[j] = gD.c[j];
     }
   }
 #pragma unroll 1
@@ -714,6 +736,59 @@ __device__ __forceinline__ void corot_adjoint_polar(const Mat3<double>& F, const
       gD.c[j] = rn_add(nc, g);
     }
   }
+}
+
+// The two halves for two threads: gF of each (the element's is their sum).
+__device__ __forceinline__ void corot_adjoint_rotation(const Mat3<double>& F, const Mat3<double>& Y, double wr, double& yr,
+                                                       Mat3<double>& gF) {
+  Mat3<double> C, Q;
+  rn_cof(F, C);
+  const double det = rn_dot(F.c[0], C.c[0]);
+  if (!polar_newton(F, C, det, Q)) {
+    Mat3<double> f = F, y = Y, g;
+    double a, b;
+    corot_adjoint_svd(f, y, wr, 0.0, a, b, g);
+    yr = a;
+    gF = g;
+    return;
+  }
+  rotation_vjp(F, Q, det < 0.0 ? -1.0 : 1.0, Y, wr, yr, gF);
+}
+__device__ __forceinline__ void corot_adjoint_volume(const Mat3<double>& F, const Mat3<double>& Y, double wv, double& yv,
+                                                     Mat3<double>& gF, double* tape_sh, int stride) {
+  Mat3<double> C;
+  rn_cof(F, C);
+  const double det = rn_dot(F.c[0], C.c[0]);
+  if (!full_rank(F, det)) {
+    Mat3<double> f = F, y = Y, g;
+    double a, b;
+    corot_adjoint_svd(f, y, 0.0, wv, a, b, g);
+    yv = b;
+    gF = g;
+    return;
+  }
+  volume_vjp(F, C, det, Y, wv, yv, gF, tape_sh, stride);
+}
+
+__device__ __forceinline__ void corot_adjoint_polar(const Mat3<double>& F, const Mat3<double>& Y, double wr, double wv,
+                                                    double& yr, double& yv, Mat3<double>& gF, double* tape_sh,
+                                                    int stride) {
+  Mat3<double> C, Q, gV;
+  rn_cof(F, C);
+  const double det = rn_dot(F.c[0], C.c[0]);
+  if (!polar_newton(F, C, det, Q)) {
+    Mat3<double> f = F, y = Y, g;
+    double a, b;
+    corot_adjoint_svd(f, y, wr, wv, a, b, g);
+    yr = a;
+    yv = b;
+    gF = g;
+    return;
+  }
+  rotation_vjp(F, Q, det < 0.0 ? -1.0 : 1.0, Y, wr, yr, gF);
+  volume_vjp(F, C, det, Y, wv, yv, gV, tape_sh, stride);
+#pragma unroll
+  for (int j = 0; j < 3; ++j) gF.c[j] = rn_add(gF.c[j], gV.c[j]);
 }
 
 }  // namespace dfem

@@ -29,6 +29,8 @@ namespace dfem {
 constexpr int kPsThreads = 512;
 constexpr int kPsWarps = kPsThreads / 32;
 constexpr int kPsChunks = 40;   // row ranges of a CTA over all phases of the solve
+constexpr int kPsPair = kPsThreads / 2;  // tets of a CTA in flight (two threads each)
+constexpr int kPsXch = 20;               // doubles a pair of threads exchanges
 
 struct PdSteps {
   int n, s0;                    // steps, index of the first
@@ -85,6 +87,7 @@ struct PsChunk {
   const int* idx;               // vertices of the staged vector
   const int* v0;                // forward, tiers > 0: their contribution ranges [v0, v1)
   const int* v1;
+  const int* out;               // a row's vertex, or -1 - its contribution slot
 };
 
 struct PsShared {
@@ -93,10 +96,10 @@ struct PsShared {
   double ws[kPsWarps];
 };
 
-// Shared memory: PsShared | staged planes (3 vec) | partial products | tables
-// | rows | tape (adjoint).
+// Shared memory: PsShared | staged planes (3 vec) | partial products | the
+// local step's exchange | tables | tape (adjoint) | rows.
 __host__ __device__ inline size_t ps_fixed_doubles(int vec) {
-  return (sizeof(PsShared) + 15) / 16 * 2 + 3 * (size_t)vec + 3 * kBsRows;
+  return (sizeof(PsShared) + 15) / 16 * 2 + 3 * (size_t)vec + 3 * kBsRows + kPsXch * kPsPair;
 }
 
 // The CTA's chunks, index tables and rows (once per launch).
@@ -128,7 +131,9 @@ __device__ __forceinline__ void ps_setup(const BlockDev& b, PsShared& S, int* ta
       }
       const int* gi = fwd ? b.cols + B.cofs : b.rows + B.rofs;
       const bool ptr = fwd && B.tier > 0;
-      if (ti + (ptr ? 3 : 1) * w <= tab_ints) {
+      const int need = (ptr ? 3 : 1) * w + C.rows;
+      P.out = nullptr;
+      if (ti + need <= tab_ints) {
         int* o = tab + ti;
         for (int q = tid; q < w; q += blockDim.x) {
           const int g = gi[q];
@@ -138,7 +143,13 @@ __device__ __forceinline__ void ps_setup(const BlockDev& b, PsShared& S, int* ta
         P.idx = o;
         P.v0 = ptr ? o + w : nullptr;
         P.v1 = ptr ? o + 2 * w : nullptr;
-        ti += (ptr ? 3 : 1) * w;
+        o += (ptr ? 3 : 1) * w;
+        for (int q = tid; q < C.rows; q += blockDim.x) {
+          const int row = C.row0 + q;
+          o[q] = row < B.n ? b.cols[B.cofs + row] : -1 - b.cslot[B.rofs + row - B.n];
+        }
+        P.out = o;
+        ti += need;
       } else {
         P.idx = gi;
         P.v0 = P.v1 = nullptr;  // read through the vertex
@@ -150,46 +161,64 @@ __device__ __forceinline__ void ps_setup(const BlockDev& b, PsShared& S, int* ta
   __syncthreads();
 }
 
-// Two rows of a chunk times the staged planes, columns [2 q0, 2 q1).
-__device__ __forceinline__ void ps_row_pair(const double2* r0, const double2* r1, const double2* bx, const double2* by,
-                                            const double2* bz, int q0, int q1, double o[2][3]) {
+// R rows (2 or 4; ld apart, the last `valid` - 1 repeated) of a chunk times
+// the staged planes, columns [2 q0, 2 q1): each staged value serves R
+// products.  The warp's sums are folded R values at a time, so that lane group
+// lane / (32 / R) ends with its row's three.
+template <int R>
+__device__ __forceinline__ void ps_rows(const double* mat, int ld, int valid, const double2* bx, const double2* by,
+                                        const double2* bz, int q0, int q1, double o[3]) {
   const int lane = threadIdx.x & 31;
-  double a[2][3] = {{0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}};
-  int q = q0 + lane;
-  for (; q + 96 < q1; q += 128) {
-    double2 u[4], w[4];
+  const double2* row[R];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) { u[k] = r0[q + 32 * k]; w[k] = r1[q + 32 * k]; }
+  for (int r = 0; r < R; ++r) row[r] = reinterpret_cast<const double2*>(mat + (size_t)min(r, valid - 1) * ld);
+  double a[R][3];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const double2 x = bx[q + 32 * k], y = by[q + 32 * k], z = bz[q + 32 * k];
-      a[0][0] += u[k].x * x.x + u[k].y * x.y;
-      a[0][1] += u[k].x * y.x + u[k].y * y.y;
-      a[0][2] += u[k].x * z.x + u[k].y * z.y;
-      a[1][0] += w[k].x * x.x + w[k].y * x.y;
-      a[1][1] += w[k].x * y.x + w[k].y * y.y;
-      a[1][2] += w[k].x * z.x + w[k].y * z.y;
+  for (int r = 0; r < R; ++r) a[r][0] = a[r][1] = a[r][2] = 0.0;
+#pragma unroll 2
+  for (int q = q0 + lane; q < q1; q += 32) {
+    double2 u[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) u[r] = row[r][q];
+    const double2 x = bx[q], y = by[q], z = bz[q];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      a[r][0] = fma(u[r].y, x.y, fma(u[r].x, x.x, a[r][0]));
+      a[r][1] = fma(u[r].y, y.y, fma(u[r].x, y.x, a[r][1]));
+      a[r][2] = fma(u[r].y, z.y, fma(u[r].x, z.x, a[r][2]));
     }
   }
-  for (; q < q1; q += 32) {
-    const double2 u = r0[q], w = r1[q], x = bx[q], y = by[q], z = bz[q];
-    a[0][0] += u.x * x.x + u.y * x.y;
-    a[0][1] += u.x * y.x + u.y * y.y;
-    a[0][2] += u.x * z.x + u.y * z.y;
-    a[1][0] += w.x * x.x + w.y * x.y;
-    a[1][1] += w.x * y.x + w.y * y.y;
-    a[1][2] += w.x * z.x + w.y * z.y;
+  double v[R / 2][3];
+  const bool h16 = lane & 16;
+#pragma unroll
+  for (int r = 0; r < R / 2; ++r)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const double keep = h16 ? a[r + R / 2][c] : a[r][c], send = h16 ? a[r][c] : a[r + R / 2][c];
+      v[r][c] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
+    }
+  if (R == 4) {
+    const bool h8 = lane & 8;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const double keep = h8 ? v[R / 2 - 1][c] : v[0][c], send = h8 ? v[0][c] : v[R / 2 - 1][c];
+      v[0][c] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
+    }
   }
 #pragma unroll
-  for (int r = 0; r < 2; ++r)
+  for (int s = R == 4 ? 4 : 8; s > 0; s >>= 1)
 #pragma unroll
-    for (int c = 0; c < 3; ++c) o[r][c] = warp_sum(a[r][c]);
+    for (int c = 0; c < 3; ++c) v[0][c] += __shfl_xor_sync(0xffffffffu, v[0][c], s);
+#pragma unroll
+  for (int c = 0; c < 3; ++c) o[c] = v[0][c];
 }
 
-// block_solve with the CTA's tables and rows in shared memory.
-template <class BAR, class DONE>
+// block_solve with the CTA's tables and rows in shared memory.  pre(v) loads
+// what done(v, value, loaded) needs before the products, so that its latency
+// is hidden.
+template <class BAR, class PRE, class DONE>
 __device__ __forceinline__ bool ps_solve(const BlockDev& b, BAR& bar, const PsShared& S, const double* rhs, double* y,
-                                         double* planes, DONE done) {
+                                         double* planes, PRE pre, DONE done) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   double* sx = planes;
   double* sy = sx + b.vec;
@@ -197,7 +226,7 @@ __device__ __forceinline__ bool ps_solve(const BlockDev& b, BAR& bar, const PsSh
   double* part = sz + b.vec;
   const int phases = 2 * b.tiers - 1;
   for (int p = 0; p < phases; ++p) {
-    const bool fwd = p < b.tiers;
+    const bool fwd = p < b.tiers, fin = !fwd || p == b.tiers - 1;
     for (int k = S.first[p]; k < S.first[p + 1]; ++k) {
       const PsChunk& C = S.ch[k];
       const int w = fwd ? C.n : C.r, ld = C.ld, w2 = ld / 2;
@@ -210,7 +239,13 @@ __device__ __forceinline__ bool ps_solve(const BlockDev& b, BAR& bar, const PsSh
             v = ld3(rhs, g);
             if (C.tier > 0) {
               const int e = C.v0 ? C.v1[i] : b.vptr[g + 1];
-              for (int q = C.v0 ? C.v0[i] : b.vptr[g]; q < e; ++q) v = v - ld3(b.contrib, q);
+              for (int q = C.v0 ? C.v0[i] : b.vptr[g]; q < e; q += 8) {  // eight in flight, subtracted in order
+                Vec3<double> c[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) c[u] = q + u < e ? ld3(b.contrib, q + u) : mk3(0.0, 0.0, 0.0);
+#pragma unroll
+                for (int u = 0; u < 8; ++u) v = v - c[u];
+              }
             }
           } else {
             v = ld3(y, g);
@@ -218,48 +253,172 @@ __device__ __forceinline__ bool ps_solve(const BlockDev& b, BAR& bar, const PsSh
         }
         sx[i] = v.x; sy[i] = v.y; sz[i] = v.z;
       }
-      __syncthreads();
       for (int base = 0; base < C.rows; base += kBsRows) {
-        const int nr = min(kBsRows, C.rows - base), pairs = (nr + 1) / 2;
-        int seg = 1;  // column segments: power of two, up to one per warp and no shorter than 32 pairs of columns
-        while (2 * seg * pairs <= kPsWarps && 64 * seg <= w2) seg *= 2;
-        const int len = (w2 + seg - 1) / seg;
-        if (base > 0) __syncthreads();
-        for (int u = warp; u < pairs * seg; u += kPsWarps) {
-          const int pr = u / seg, sg = u % seg;
-          const int ra = base + 2 * pr, rb = min(ra + 1, C.rows - 1);
-          double o[2][3];
-          ps_row_pair(reinterpret_cast<const double2*>(C.mat + (size_t)ra * ld),
-                      reinterpret_cast<const double2*>(C.mat + (size_t)rb * ld), reinterpret_cast<const double2*>(sx),
-                      reinterpret_cast<const double2*>(sy), reinterpret_cast<const double2*>(sz), sg * len,
-                      min(w2, (sg + 1) * len), o);
-          if (lane == 0) {
-#pragma unroll
-            for (int r = 0; r < 2; ++r)
-#pragma unroll
-              for (int c = 0; c < 3; ++c)
-                if (2 * pr + r < nr) part[3 * ((2 * pr + r) * seg + sg) + c] = o[r][c];
+        const int nr = min(kBsRows, C.rows - base);
+        int out = 0;
+        Vec3<double> yo = mk3(0.0, 0.0, 0.0);
+        decltype(pre(0)) pl;
+        if (tid < nr) {
+          const int row = C.row0 + base + tid;
+          out = C.out ? C.out[base + tid] : row < C.n ? b.cols[C.cofs + row] : -1 - b.cslot[C.rofs + row - C.n];
+          if (out >= 0 && fin) {
+            if (!fwd) yo = ld3(y, out);
+            pl = pre(out);
           }
         }
         __syncthreads();
-        for (int r = tid; r < nr; r += kPsThreads) {
-          Vec3<double> v = ld3(part, r * seg);
-          for (int sg = 1; sg < seg; ++sg) v = v + ld3(part, r * seg + sg);
-          const int row = C.row0 + base + r;
-          if (fwd && row >= C.n) {
-            st3(b.contrib, b.cslot[C.rofs + row - C.n], v);
-          } else {
-            const int g = b.cols[C.cofs + row];
-            if (!fwd) v = ld3(y, g) - v;
-            if (!fwd || p == b.tiers - 1) done(g, v);
-            else st3(y, g, v);
-          }
+        const int R = nr > 2 ? 4 : 2, groups = nr > 2 ? (nr + 3) >> 2 : 1;
+        int ls = 0;  // log2 of the column segments: up to one per warp and no shorter than 32 pairs of columns
+        while ((2 << ls) * groups <= kPsWarps && (64 << ls) <= w2) ++ls;
+        const int seg = 1 << ls, len = (w2 + seg - 1) >> ls;
+        const double2* bx = reinterpret_cast<const double2*>(sx);
+        const double2* by = reinterpret_cast<const double2*>(sy);
+        const double2* bz = reinterpret_cast<const double2*>(sz);
+        for (int u = warp; u < groups * seg; u += kPsWarps) {
+          const int gr = u >> ls, sg = u & (seg - 1), q0 = sg * len, q1 = min(w2, q0 + len);
+          const double* m = C.mat + (size_t)(base + gr * R) * ld;
+          double o[3];
+          if (R == 4) ps_rows<4>(m, ld, nr - 4 * gr, bx, by, bz, q0, q1, o);
+          else ps_rows<2>(m, ld, nr - 2 * gr, bx, by, bz, q0, q1, o);
+          const int r = gr * R + lane / (32 / R);
+          if (lane % (32 / R) == 0 && r < nr) st3(part, r * seg + sg, mk3(o[0], o[1], o[2]));
+        }
+        __syncthreads();
+        if (tid < nr) {
+          Vec3<double> v = ld3(part, tid * seg);
+          for (int sg = 1; sg < seg; ++sg) v = v + ld3(part, tid * seg + sg);
+          if (out < 0) st3(b.contrib, -1 - out, v);
+          else if (fin) done(out, fwd ? v : yo - v, pl);
+          else st3(y, out, v);
         }
       }
     }
     if (p + 1 < phases && !bar.sync()) return false;
   }
   return true;
+}
+
+// Local step of all constraints by a CTA's sixteen warps.  A tet is given to
+// two threads, eight warps apart: one takes its rotation, the other its
+// volume projection (the two iterations do not depend on one another and are
+// the chain of dependent FP64 operations that bounds a scene with less than a
+// warp per scheduler); the rotation passes through shared memory.
+__device__ __forceinline__ void ps_give(double* xch, bool rot, int me, const Vec3<double> P[3]) {
+  double* o = xch + (rot ? 0 : 9) * kPsPair + me;
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    o[(3 * j) * kPsPair] = P[j].x;
+    o[(3 * j + 1) * kPsPair] = P[j].y;
+    o[(3 * j + 2) * kPsPair] = P[j].z;
+  }
+}
+// P += the other half's (a sum of two: the same bits in both)
+__device__ __forceinline__ void ps_take(const double* xch, bool rot, int me, Vec3<double> P[3]) {
+  const double* o = xch + (rot ? 9 : 0) * kPsPair + me;
+#pragma unroll
+  for (int j = 0; j < 3; ++j)
+    P[j] = rn_add(P[j], mk3(o[(3 * j) * kPsPair], o[(3 * j + 1) * kPsPair], o[(3 * j + 2) * kPsPair]));
+}
+// corners 0, 1 (rotation's thread) or 2, 3 of G P into their slots
+__device__ __forceinline__ void ps_corners(const double G[4][3], const Vec3<double> P[3], int4 sl, bool rot, double* slot) {
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    const double g0 = rot ? G[q][0] : G[q + 2][0], g1 = rot ? G[q][1] : G[q + 2][1], g2 = rot ? G[q][2] : G[q + 2][2];
+    const int o = rot ? (q == 0 ? sl.x : sl.y) : (q == 0 ? sl.z : sl.w);
+    st3(slot, o, g0 * P[0] + g1 * P[1] + g2 * P[2]);
+  }
+}
+
+template <class BAR>
+__device__ __forceinline__ void ps_local(const SceneDev& d, const double* x, const double* act_row, double* slot,
+                                         double* xch, int4 tv0, int first, int stride) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nc = BAR::ctas();
+  const int me = tid & (kPsPair - 1);
+  const bool rot = warp < kPsWarps / 2;
+  for (int base = 0; base < d.T; base += kPsPair * nc) {
+    const int t = base + 32 * ((warp & (kPsWarps / 2 - 1)) * nc + BAR::cta()) + lane;
+    double G[4][3];
+    Vec3<double> P[3];  // this half's part of wr md + wv md_volume
+    if (t < d.T) {
+      const int4 v = base == 0 ? tv0 : d.tv[t];
+      const Vec3<double> xv[4] = {ld3(x, v.x), ld3(x, v.y), ld3(x, v.z), ld3(x, v.w)};
+      load_g(d.tinv, d.T, t, G);
+      const double w = rot ? d.twr[t] : d.twv[t];
+      const Mat3<double> F = deformation(G, xv);
+      Mat3<double> m;
+      if (rot) corot_rotation(F, m);
+      else corot_volume(F, m);
+#pragma unroll
+      for (int j = 0; j < 3; ++j) P[j] = rn_scale(w, m.c[j]);
+      ps_give(xch, rot, me, P);
+    }
+    __syncthreads();
+    if (t < d.T) {  // two corners each
+      ps_take(xch, rot, me, P);
+      ps_corners(G, P, d.tslot[t], rot, slot);
+    }
+    if (base + kPsPair * nc < d.T) __syncthreads();
+  }
+  for (int t = first; t < d.M + d.S + d.B; t += stride) local_rest(d, t, x, act_row, slot);
+}
+
+// Its VJP (with the Hs term of the next iterate x1), split the same way; the
+// volume half's tape takes the threads of tape_warps warps.
+template <class BAR>
+__device__ __forceinline__ void ps_adj_local(const SceneDev& d, const double* x, const double* x1, const double* y,
+                                             const double* act_row, double* slot, double* gE, double* gnu, double* mg,
+                                             bool first_it, double* xch, double* tape, int tape_warps, int4 tv0, int first,
+                                             int stride) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nc = BAR::ctas();
+  const int me = tid & (kPsPair - 1), half = warp & (kPsWarps / 2 - 1);
+  const bool rot = warp < kPsWarps / 2;
+  for (int base = 0; base < d.T; base += 32 * tape_warps * nc) {
+    const int t = half < tape_warps ? base + 32 * (half * nc + BAR::cta()) + lane : d.T;
+    double G[4][3], yv = 0.0;
+    Mat3<double> gF;
+    if (t < d.T) {
+      const int4 v = base == 0 ? tv0 : d.tv[t];
+      const int vi[4] = {v.x, v.y, v.z, v.w};
+      Vec3<double> xv[4], yw[4];
+#pragma unroll
+      for (int a = 0; a < 4; ++a) { xv[a] = ld3(x, vi[a]); yw[a] = ld3(y, vi[a]); }
+      load_g(d.tinv, d.T, t, G);
+      const Mat3<double> F = deformation(G, xv), Y = deformation(G, yw);
+      if (rot) {
+        double yr;
+        corot_adjoint_rotation(F, Y, d.twr[t], yr, gF);
+#pragma unroll
+        for (int a = 0; a < 4; ++a) xv[a] = ld3(x1, vi[a]);
+        const Mat3<double> F1 = deformation(G, xv);
+        double yh = 0;
+#pragma unroll
+        for (int j = 0; j < 3; ++j) yh += dot3(Y.c[j], F1.c[j]);
+        xch[18 * kPsPair + me] = yr;
+        xch[19 * kPsPair + me] = yh;
+      } else {
+        corot_adjoint_volume(F, Y, d.twv[t], yv, gF, tape + 32 * half + lane, 32 * tape_warps);
+      }
+      ps_give(xch, rot, me, gF.c);
+    }
+    __syncthreads();
+    if (t < d.T) {
+      ps_take(xch, rot, me, gF.c);
+      ps_corners(G, gF.c, d.tslot[t], rot, slot);
+      if (!rot) {
+        const double yr = xch[18 * kPsPair + me], yh = xch[19 * kPsPair + me], E = d.tE[t], nu = d.tnu[t], vol = d.tvol[t];
+        const double opn = 1.0 + nu;
+        gE[t] += vol / opn * (yr + nu * yv) - vol * yh;
+        gnu[t] += E * vol / (opn * opn) * (yv - yr);
+      }
+    }
+    if (base + 32 * tape_warps * nc < d.T) __syncthreads();
+  }
+  const int nmg = d.M + (d.sch ? d.S : 0);
+  for (int t = first; t < d.M + d.S + d.B; t += stride) {
+    adj_local_rest(d, t, x, y, act_row, slot, mg);
+    // activation terms: summed over the step's iterations by their constraint's thread
+    if (t < nmg && (t < d.M || d.sch[t - d.M] >= 0)) mg[nmg + t] = first_it ? mg[t] : mg[nmg + t] + mg[t];
+  }
 }
 
 // Sum of v over the grid: the CTA's part goes to partial; after the next
@@ -278,7 +437,13 @@ __device__ __forceinline__ void ps_put(double v, double* ws, double* partial) {
 }
 __device__ __forceinline__ double ps_total(const double* partial, int n) {
   double s = 0;
-  for (int k = threadIdx.x & 31; k < n; k += 32) s += __ldcg(partial + k);
+  for (int k = threadIdx.x & 31; k < n; k += 256) {  // eight loads in flight
+    double v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v[u] = k + 32 * u < n ? __ldcg(partial + k + 32 * u) : 0.0;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) s += v[u];
+  }
   return warp_sum(s);
 }
 
@@ -286,8 +451,16 @@ __device__ __forceinline__ double ps_total(const double* partial, int n) {
 template <class T>
 __device__ __forceinline__ Vec3<double> ps_sum_slots(const T* slot, int k0, int k1) {
   Vec3<double> a = mk3(0.0, 0.0, 0.0);
-  for (int k = k0 + (int)(threadIdx.x & 7); k < k1; k += 8)
-    a = a + mk3((double)slot[3 * (size_t)k], (double)slot[3 * (size_t)k + 1], (double)slot[3 * (size_t)k + 2]);
+  for (int k = k0 + (int)(threadIdx.x & 7); k < k1; k += 32) {  // four loads in flight
+    Vec3<double> v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const size_t q = 3 * (size_t)(k + 8 * u);
+      v[u] = k + 8 * u < k1 ? mk3((double)slot[q], (double)slot[q + 1], (double)slot[q + 2]) : mk3(0.0, 0.0, 0.0);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) a = a + v[u];
+  }
 #pragma unroll
   for (int o = 4; o > 0; o >>= 1) {
     a.x += __shfl_xor_sync(0xffffffffu, a.x, o);
@@ -304,6 +477,7 @@ __global__ void __launch_bounds__(kPsThreads, 1) k_pd_forward(SceneDev d, BlockD
   double* planes = pssh + (sizeof(PsShared) + 15) / 16 * 2;
   int* tab = reinterpret_cast<int*>(pssh + ps_fixed_doubles(b.vec));
   double* res = pssh + ps_fixed_doubles(b.vec) + a.tab_ints / 2;
+  double* xch = planes + 3 * (size_t)b.vec + 3 * kBsRows;
   BAR bar(b.bar, b.status);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, cta = BAR::cta(), nc = BAR::ctas();
   // items are dealt to the CTAs a warp's worth at a time
@@ -322,6 +496,11 @@ __global__ void __launch_bounds__(kPsThreads, 1) k_pd_forward(SceneDev d, BlockD
     }
     if (!bar.sync()) return;
   }
+  // this thread's first tet and vertex: their tables are read once, so that the first loads after a barrier are
+  // the ones that wait for it
+  const int t0 = 32 * ((warp & (kPsWarps / 2 - 1)) * nc + cta) + lane, g0 = min(first >> 3, d.N - 1);
+  const int4 tv0 = t0 < d.T ? d.tv[t0] : make_int4(0, 0, 0, 0);
+  const int vs0 = d.vslot_ptr[g0], vs1 = d.vslot_ptr[g0 + 1];
   int par = 0;
   double* xprev = a.xt;  // positions the step starts from, as every CTA reads them
   double* xk = a.xk;
@@ -331,12 +510,26 @@ __global__ void __launch_bounds__(kPsThreads, 1) k_pd_forward(SceneDev d, BlockD
     double* hist = a.hist + (size_t)s * a.hist_step;
     // begin (after the end of the step before): v_wc, q_n, x^0 = q_n, c0 = M/h^2 q_n - Hs x + J_att d_att
     double q2 = 0.0;
-    for (int i = first; i < d.N; i += stride) {
+    for (int g = first >> 3; g < ((d.N + 3) & ~3); g += stride >> 3) {  // eight lanes per vertex: its row of Hs
+      const int i = min(g, d.N - 1);
+      Vec3<double> acc = mk3(0.0, 0.0, 0.0);
+      if (!MIXED) {
+        const int k1 = d.hs_ptr[i + 1];
+        for (int k = d.hs_ptr[i] + (lane & 7); k < k1; k += 8) acc = acc + d.hs_val[k] * ld3(xprev, d.hs_col[k]);
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) {
+          acc.x += __shfl_xor_sync(0xffffffffu, acc.x, o);
+          acc.y += __shfl_xor_sync(0xffffffffu, acc.y, o);
+          acc.z += __shfl_xor_sync(0xffffffffu, acc.z, o);
+        }
+      }
+      if ((lane & 7) != 0 || g >= d.N) continue;
       Vec3<double> x, v;
       if (st > 0) {
         x = ld3(xprev, i);
         v = (d.damping / d.h) * (x - ld3(a.xt, i));
         if (a.traj) st3(a.traj + (size_t)(s - 1) * 3 * d.N, a.to_user[i], x);
+        st3(a.xt, i, x);
       } else {
         x = ld3(a.xt, i);
         v = ld3(a.vt, i);
@@ -352,24 +545,7 @@ __global__ void __launch_bounds__(kPsThreads, 1) k_pd_forward(SceneDev d, BlockD
       st3(a.qn, i, q);
       st3(xk, i, q);
       st3(hist, i, q);
-      if (!MIXED) {
-        Vec3<double> acc = (d.mass[i] / (d.h * d.h)) * q;
-        const int k1 = d.hs_ptr[i + 1];
-        for (int k = d.hs_ptr[i]; k < k1; k += 8) {  // eight entries in flight, subtracted in order
-          double w[8];
-          Vec3<double> xj[8];
-#pragma unroll
-          for (int u = 0; u < 8; ++u) {
-            const bool in = k + u < k1;
-            w[u] = in ? d.hs_val[k + u] : 0.0;
-            xj[u] = in ? ld3(xprev, d.hs_col[k + u]) : mk3(0.0, 0.0, 0.0);
-          }
-#pragma unroll
-          for (int u = 0; u < 8; ++u) acc = acc - w[u] * xj[u];
-        }
-        st3(a.c0, i, acc + ld3(d.attach_jd, i));
-      }
-      if (st > 0) st3(a.xt, i, x);
+      if (!MIXED) st3(a.c0, i, (d.mass[i] / (d.h * d.h)) * q - acc + ld3(d.attach_jd, i));
       q2 += dot3(q, q);
     }
     ps_put(q2, S.ws, a.partial + par * nc + cta);
@@ -382,14 +558,14 @@ __global__ void __launch_bounds__(kPsThreads, 1) k_pd_forward(SceneDev d, BlockD
     const double* act_row = a.act_all + (size_t)s * d.nseg;
     int k = 0;
     for (; k < a.K && !conv; ++k) {
-      for (int t = first; t < ncons; t += stride) {
-        if (MIXED) force_item(d, t, xk, act_row, reinterpret_cast<float*>(a.slot));
-        else local_item(d, t, xk, act_row, a.slot);
-      }
+      if (MIXED)
+        for (int t = first; t < ncons; t += stride) force_item(d, t, xk, act_row, reinterpret_cast<float*>(a.slot));
+      else
+        ps_local<BAR>(d, xk, act_row, a.slot, xch, tv0, first, stride);
       if (!bar.sync()) return;
       for (int g = first >> 3; g < ((d.N + 3) & ~3); g += stride >> 3) {  // eight lanes per vertex
         const int i = min(g, d.N - 1);
-        const int k0 = d.vslot_ptr[i], k1 = d.vslot_ptr[i + 1];
+        const int k0 = i == g0 ? vs0 : d.vslot_ptr[i], k1 = i == g0 ? vs1 : d.vslot_ptr[i + 1];
         if (MIXED) {
           const Vec3<double> f = ps_sum_slots(reinterpret_cast<const float*>(a.slot), k0, k1);
           if ((lane & 7) == 0 && g < d.N) {
@@ -398,23 +574,25 @@ __global__ void __launch_bounds__(kPsThreads, 1) k_pd_forward(SceneDev d, BlockD
             st3(a.rhs, i, m * (ld3(a.qn, i) - xi) + ld3(d.attach_jd, i) - d.attach_k[i] * xi + f);
           }
         } else {
-          const Vec3<double> f = ps_sum_slots(a.slot, k0, k1);
-          if ((lane & 7) == 0 && g < d.N) st3(a.rhs, i, ld3(a.c0, i) + f);
+          const Vec3<double> c = ld3(a.c0, i), f = ps_sum_slots(a.slot, k0, k1);
+          if ((lane & 7) == 0 && g < d.N) st3(a.rhs, i, c + f);
         }
       }
       if (!bar.sync()) return;
       double e2 = 0.0;
       double* h1 = hist + (size_t)(k + 1) * 3 * d.N;
-      const bool ok = ps_solve(b, bar, S, a.rhs, a.y, planes, [&](int g, Vec3<double> z) {
-        // plain form: x^{k+1} = x_t + z (the reference's delta form); mixed form: x^{k+1} = x^k + z
-        const Vec3<double> xc = ld3(xk, g);
-        const Vec3<double> xn = (MIXED ? xc : ld3(a.xt, g)) + z;
-        const Vec3<double> dl = xn - xc;
-        e2 += dot3(dl, dl);
-        st3(xk, g, xn);
-        st3(h1, g, xn);
-        if (b.tiers > 1) st3(a.y, g, z);  // read by the blocks below
-      });
+      // plain form: x^{k+1} = x_t + z (the reference's delta form); mixed form: x^{k+1} = x^k + z
+      struct Pos { Vec3<double> xc, x0; };
+      const bool ok = ps_solve(
+          b, bar, S, a.rhs, a.y, planes,
+          [&](int g) { return Pos{ld3(xk, g), MIXED ? mk3(0.0, 0.0, 0.0) : ld3(a.xt, g)}; },
+          [&](int g, Vec3<double> z, const Pos& p) {
+            const Vec3<double> xn = (MIXED ? p.xc : p.x0) + z, dl = xn - p.xc;
+            e2 += dot3(dl, dl);
+            st3(xk, g, xn);
+            st3(h1, g, xn);
+            if (b.tiers > 1) st3(a.y, g, z);  // read by the blocks below
+          });
       if (!ok) return;
       ps_put(e2, S.ws, a.partial + par * nc + cta);
       if (!bar.sync()) return;
@@ -457,16 +635,20 @@ __global__ void __launch_bounds__(kPsThreads, 1) k_pd_adjoint(SceneDev d, BlockD
   double* tape = pssh + ps_fixed_doubles(b.vec) + a.tab_ints / 2;
   const int tstride = 32 * a.tape_warps;
   double* res = tape + (size_t)kVolTape * tstride;
+  double* xch = planes + 3 * (size_t)b.vec + 3 * kBsRows;
   BAR bar(b.bar, b.status);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, cta = BAR::cta(), nc = BAR::ctas();
   const int first = 32 * (warp * nc + cta) + lane, stride = kPsThreads * nc;
-  const int ncons = d.T + d.M + d.S + d.B, nmg = d.M + (d.sch ? d.S : 0);
+  const int nmg = d.M + (d.sch ? d.S : 0);
   ps_setup<BAR>(b, S, tab, a.tab_ints, res, a.res_doubles);
   if (a.zero) {
     if (cta == 0 && tid < 4) a.status[tid] = 0;
     for (int t = first; t < d.T; t += stride) { a.gE[t] = 0.0; a.gnu[t] = 0.0; }
     for (int q = first; q < a.n * d.nseg; q += stride) a.gact[(size_t)a.s0 * d.nseg + q] = 0.0;
   }
+  const int t0 = 32 * ((warp & (kPsWarps / 2 - 1)) * nc + cta) + lane, g0 = min(first >> 3, d.N - 1);
+  const int4 tv0 = (warp & (kPsWarps / 2 - 1)) < a.tape_warps && t0 < d.T ? d.tv[t0] : make_int4(0, 0, 0, 0);
+  const int vs0 = d.vslot_ptr[g0], vs1 = d.vslot_ptr[g0 + 1];
   const double c = d.damping / d.h, ih2 = 1.0 / (d.h * d.h);
   for (int st = a.n - 1; st >= 0; --st) {
     const int s = a.s0 + st;
@@ -494,26 +676,21 @@ __global__ void __launch_bounds__(kPsThreads, 1) k_pd_adjoint(SceneDev d, BlockD
     const double* act_row = a.act_all + (size_t)s * d.nseg;
     if (!bar.sync()) return;
     for (int k = nit - 1; k >= 0; --k) {
-      const bool ok = ps_solve(b, bar, S, a.xkb, a.y, planes, [&](int g, Vec3<double> y) {
-        st3(a.y, g, y);
-        st3(a.bb, g, ld3(a.bb, g) + y);
-      });
+      const bool ok = ps_solve(
+          b, bar, S, a.xkb, a.y, planes, [&](int g) { return ld3(a.bb, g); },
+          [&](int g, Vec3<double> y, const Vec3<double>& bb) {
+            st3(a.y, g, y);
+            st3(a.bb, g, bb + y);
+          });
       if (!ok || !bar.sync()) return;
       const double* x = hist + (size_t)k * 3 * d.N;
       const double* x1 = x + 3 * (size_t)d.N;
-      if (warp < a.tape_warps) {
-        for (int t = first; t < ncons; t += tstride * nc) {
-          adj_local_item(d, t, x, a.y, act_row, a.slot, a.gE, a.gnu, a.mg, x1, nullptr, tape + tid, tstride);
-          // activation terms: summed over the step's iterations by their constraint's thread
-          const int m = t - d.T, q = m < d.M ? m : m - d.M;  // muscles, then springs
-          if (m >= 0 && m < nmg && (m < d.M || d.sch[q] >= 0))
-            a.mg[nmg + m] = k == nit - 1 ? a.mg[m] : a.mg[nmg + m] + a.mg[m];
-        }
-      }
+      ps_adj_local<BAR>(d, x, x1, a.y, act_row, a.slot, a.gE, a.gnu, a.mg, k == nit - 1, xch, tape, a.tape_warps, tv0,
+                        first, stride);
       if (!bar.sync()) return;
       for (int g = first >> 3; g < ((d.N + 3) & ~3); g += stride >> 3) {
         const int i = min(g, d.N - 1);
-        const Vec3<double> f = ps_sum_slots(a.slot, d.vslot_ptr[i], d.vslot_ptr[i + 1]);
+        const Vec3<double> f = ps_sum_slots(a.slot, i == g0 ? vs0 : d.vslot_ptr[i], i == g0 ? vs1 : d.vslot_ptr[i + 1]);
         if ((lane & 7) == 0 && g < d.N) st3(a.xkb, i, f);
       }
       if (k == 0)  // the activation gradient of the step
