@@ -161,7 +161,8 @@ struct dfem_scene {
                                                           // best split, cluster, resident, dense
   // block-inverse ("dense") form (solve_cut = -3), built by every refactorisation while it is in use
   bool dense_ok = false;                 // the scene qualifies (single part, the plan fits)
-  bool dense_built = false;              // the products belong to the current moduli
+  bool dense_built = false;              // the form belongs to the current moduli
+  bool blk_built = false;                // mixed scenes: the adjoint's blocks do (built by the first adjoint that needs them)
   bool tri_built = false;                // the supernodal factor does (built on demand while the dense form is in use)
   double dense_build_ms = 0.0;
   // mixed scenes: X = Hs^-1 from the supernodal factor (dense_solve.cuh); FP64 scenes: blocks (block_inverse.cuh)
@@ -754,7 +755,8 @@ static void dense_release(dfem_scene* sc) {
   sc->bl_sol.alloc(0);
   sc->bl_piv.alloc(0);
   sc->bl_contrib.alloc(0);
-  sc->dense_built = false;
+  sc->dense_built = sc->blk_built = false;
+  sc->ps_ok = false;
   sc->bd = BlockDev{};
 }
 
@@ -880,6 +882,12 @@ static int plan_steps(dfem_scene* sc, int vec, int G, const std::vector<BlockChu
   sc->ps_res_f = (int)std::min(rows, kMaxSmem - fixed);
   sc->ps_res_a = (int)std::min(rows, kMaxSmem - fixed - tape);
   sc->ps_smem_f = (fixed + sc->ps_res_f) * sizeof(double);
+  if (dense_is_x(sc)) {  // the forward's solve: planes of N_p, the CTA's rows of X if they fit
+    const size_t np = (size_t)sc->dd.Np, fx = ps_fixed_doubles((int)np) - kPsXch * kPsPair;
+    if (fx > kMaxSmem) return DFEM_OK;
+    sc->ps_res_f = (int)(std::min(((size_t)s.N + G - 1) / G, (kMaxSmem - fx) / np) * np);
+    sc->ps_smem_f = (fx + sc->ps_res_f) * sizeof(double);
+  }
   sc->ps_smem_a = (fixed + tape + sc->ps_res_a) * sizeof(double);
   for (auto fn : {(const void*)k_pd_forward<GridBarrier, false>, (const void*)k_pd_forward<GridBarrier, true>,
                   (const void*)k_pd_forward<ClusterBarrier, false>, (const void*)k_pd_forward<ClusterBarrier, true>})
@@ -919,15 +927,20 @@ static bool cluster_fits() {
 
 // Buffers, tables and launch shapes of the dense form (block-inverse: single
 // scenes whose plan fits an eighth of the free memory); false: not a candidate.
-static int dense_prepare(dfem_scene* sc, bool* ok) {
+static int block_prepare(dfem_scene* sc, bool* ok) {
   *ok = false;
-  if (sc->hs.nparts != 1 || sc->hs.F.nsuper == 0) return DFEM_OK;
-  if (dense_is_x(sc)) return dense_x_prepare(sc, ok);
   BlockPlan& P = sc->bplan;
+  const bool mx = dense_is_x(sc);
   if (sc->bd.blk == nullptr) {
     size_t free_b = 0, total_b = 0;
     CK(cudaMemGetInfo(&free_b, &total_b));
     if (!plan_blocks(sc->hs.F, sc->hs.Hs, (int64_t)(free_b / 8 / sizeof(double)), P)) return DFEM_OK;
+    const bool view = mx && P.tiers == 1;  // the one block is X itself
+    if (view) {
+      P.blk[0].ldx = sc->dd.Np;
+      P.blk[0].xp = 0;
+      P.front_doubles = P.panel_doubles = P.solve_doubles = 0;
+    }
     int vec = 2, coop = 0, nsm = 1, occ = 0;
     for (const BlockInfo& B : P.blk) vec = std::max({vec, B.ldx, B.ldr});
     CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, sc->device));
@@ -979,9 +992,9 @@ static int dense_prepare(dfem_scene* sc, bool* ok) {
     if (e == cudaSuccess) e = sc->bl_contrib.alloc(3 * std::max<size_t>(1, P.rows.size()));
     if (e == cudaSuccess) e = sc->bl_bar.alloc(2);
     if (e == cudaSuccess) e = cudaMemset(sc->bl_bar.p, 0, 2 * sizeof(unsigned));
-    if (e == cudaSuccess) e = cudaMemset(sc->bl_sol.p, 0, P.solve_doubles * sizeof(double));  // the rows' padding stays 0
+    if (e == cudaSuccess && !view) e = cudaMemset(sc->bl_sol.p, 0, P.solve_doubles * sizeof(double));  // the rows' padding stays 0
     if (e != cudaSuccess) {
-      dense_release(sc);
+      if (!mx) dense_release(sc);
       CK(e);
     }
     RC(plan_steps(sc, vec, G, chunks, share));
@@ -990,11 +1003,28 @@ static int dense_prepare(dfem_scene* sc, bool* ok) {
     d.blk = sc->bl_blk.p; d.tiles = sc->bl_tiles.p; d.tier_tile = sc->bl_tier_tile.p; d.kids = sc->bl_kids.p;
     d.hs_idx = sc->bl_hs_idx.p; d.hs_loc = sc->bl_hs_loc.p; d.cols = sc->bl_cols.p; d.rows = sc->bl_rows.p;
     d.rmap = sc->bl_rmap.p; d.cslot = sc->bl_cslot.p; d.vptr = sc->bl_vptr.p; d.chunks = sc->bl_chunks.p;
-    d.share = sc->bl_share.p; d.front = sc->bl_front.p; d.panel = sc->bl_panel.p; d.sol = sc->bl_sol.p;
+    d.share = sc->bl_share.p; d.front = sc->bl_front.p; d.panel = sc->bl_panel.p; d.sol = view ? sc->dn_A.p : sc->bl_sol.p;
     d.piv = sc->bl_piv.p; d.contrib = sc->bl_contrib.p; d.bar = sc->bl_bar.p; d.status = sc->status.p; d.vec = vec;
     sc->bd = d;
   }
   *ok = true;
+  return DFEM_OK;
+}
+
+static int dense_prepare(dfem_scene* sc, bool* ok) {
+  *ok = false;
+  if (sc->hs.nparts != 1 || sc->hs.F.nsuper == 0) return DFEM_OK;
+  if (!dense_is_x(sc)) return block_prepare(sc, ok);
+  RC(dense_x_prepare(sc, ok));
+  if (*ok && !sc->bd.blk) {  // steps in one launch, with the blocks (or X) in the adjoint: left out if they do not fit
+    bool b = false;
+    if (block_prepare(sc, &b) != DFEM_OK || !b) {
+      cudaGetLastError();
+      g_last_error.clear();
+      sc->ps_ok = false;
+      sc->bd = BlockDev{};
+    }
+  }
   return DFEM_OK;
 }
 
@@ -1039,6 +1069,7 @@ static int factor_values(dfem_scene* sc, bool dense) {
     if (!sc->tri_built) RC(factor_values(sc, false));
     RC(dense_x_build(sc));
     sc->dense_built = true;
+    sc->blk_built = false;
     return DFEM_OK;
   }
   std::vector<int> failh(np + 1);
@@ -1073,6 +1104,26 @@ static int ensure_factor(dfem_scene* sc) {
   return factor_values(sc, dense);
 }
 
+// Mixed scenes whose adjoint solves with blocks: built once per material
+// change, by the first adjoint after it (X's regularisation).  *ok: false
+// when a pivot fails, the adjoint then takes the graph form.
+static int ensure_adjoint_blocks(dfem_scene* sc, bool* ok) {
+  *ok = true;
+  if (!dense_is_x(sc) || sc->bplan.tiers == 1 || sc->blk_built) return DFEM_OK;
+  int bad = 0;
+  CK(cudaMemsetAsync(sc->part_fail.p, 0, sizeof(int), sc->stream));
+  RC(dense_build(sc));
+  CK(cudaMemcpyAsync(&bad, sc->part_fail.p, sizeof(int), cudaMemcpyDeviceToHost, sc->stream));
+  CK(cudaStreamSynchronize(sc->stream));
+  *ok = bad == 0;
+  if (bad) {
+    sc->ps_ok = false;
+    invalidate_graphs(sc);
+  }
+  sc->blk_built = bad == 0;
+  return DFEM_OK;
+}
+
 static int ensure_triangular(dfem_scene* sc) {
   if (sc->tri_built) return DFEM_OK;
   CK(cudaMemsetAsync(sc->part_fail.p, 0, sizeof(int) * (sc->hs.nparts + 1), sc->stream));
@@ -1088,7 +1139,7 @@ static int gpu_refactor(dfem_scene* sc) {
   k_hs_values<<<(sc->rd.nnz + 255) / 256, 256, 0, sc->stream>>>(sc->rd);
   sc->launches += (s.T > 0 ? 1 : 0) + 1;
   std::fill(sc->part_reg_h.begin(), sc->part_reg_h.end(), 0.0);
-  sc->dense_built = sc->tri_built = false;
+  sc->dense_built = sc->tri_built = sc->blk_built = false;
   return factor_values(sc, sc->solve_cut == -3);
 }
 
@@ -1818,6 +1869,7 @@ static PdSteps steps_args(dfem_scene* sc, int n, int s0) {
   a.iters = sc->iters.p; a.status = sc->status.p; a.vwc = sc->has_contact ? sc->vwc.p : nullptr;
   a.to_user = sc->to_user.p; a.tab_ints = sc->ps_tab;
   a.xkb = sc->xkb.p; a.xtb = sc->xtb.p; a.bb = sc->bb.p; a.gE = sc->gE.p; a.gnu = sc->gnu.p; a.mg = sc->mg.p;
+  a.X = sc->dn_A.p; a.Np = sc->dd.Np;
   a.gact = sc->gact.p; a.io_a = sc->io_a.p; a.io_b = sc->io_b.p; a.tape_warps = sc->ps_tape_warps;
   return a;
 }
@@ -3010,6 +3062,10 @@ int dfem_step_backward(dfem_scene* sc, const double* gx_out, const double* gv_ou
   if (!sc || !gx_out || !gv_out || !gx || !gv) return fail(DFEM_ERR_INVALID, "null argument");
   if (sc->rec_steps <= 0) return fail(DFEM_ERR_STATE, "dfem_step_backward needs a preceding dfem_step_forward");
   CK(cudaSetDevice(sc->device));
+  if (one_launch(sc)) {
+    bool blocks = true;
+    RC(ensure_adjoint_blocks(sc, &blocks));
+  }
   const int nq = sc->sk_nq;
   // the joint state a replayed step starts from (restored to the forward's final one at the end)
   auto joint_state_at = [&](int st) -> int {

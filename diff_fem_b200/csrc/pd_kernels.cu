@@ -290,8 +290,10 @@ __device__ __forceinline__ Vec3<float> ld3f(const float* p, int i) { return mk3(
 // in FP64 first; each slot is rounded to FP32 once, from an FP64 value, and a
 // vertex's slots are summed in FP64.
 
-// Force slots of constraint t (plain pointers: see local_item).
-__device__ __forceinline__ void force_item(const SceneDev& d, int t, const double* x, const double* act_row, float* slot) {
+// Force slots of constraint t (plain pointers: see local_item).  Not inlined:
+// a force's last bit decides its rounding to FP32, so every kernel calls the
+// one compiled copy of its arithmetic.
+static __device__ __noinline__ void force_item(const SceneDev& d, int t, const double* x, const double* act_row, float* slot) {
   if (t < d.T) {
     int4 v = d.tv[t];
     Vec3<double> xv[4] = {ld3(x, v.x), ld3(x, v.y), ld3(x, v.z), ld3(x, v.w)};
@@ -362,7 +364,8 @@ __device__ __forceinline__ void force_item(const SceneDev& d, int t, const doubl
   }
 }
 
-__global__ void __launch_bounds__(128, DFEM_FORCE_MIN_BLOCKS) k_force_f32(SceneDev d, Gate gate, const double* __restrict__ x,
+__global__ void __launch_bounds__(128, DFEM_FORCE_MIN_BLOCKS) k_force_f32(const __grid_constant__ SceneDev d, Gate gate,
+                                                   const double* __restrict__ x,
                                                    const double* __restrict__ act_all, const int* step,
                                                    float* __restrict__ slot) {
   int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -371,16 +374,30 @@ __global__ void __launch_bounds__(128, DFEM_FORCE_MIN_BLOCKS) k_force_f32(SceneD
 }
 
 // r_i = m_i/h^2 (q_i - x_i) + attach_jd_i - attach_k_i x_i + the sum of vertex i's FP32 force
-// slots, accumulated in FP64 (the slots' own rounding is then the only FP32 error of the rhs)
-__global__ void k_gather_force(SceneDev d, Gate gate, const float* __restrict__ slot, const double* __restrict__ qn,
+// slots, accumulated in FP64 in slot order (the slots' own rounding is then the only FP32 error
+// of the rhs); eight slots in flight.  Not inlined, as force_item.
+static __device__ __noinline__ Vec3<double> force_rhs(const SceneDev& d, int i, const float* slot, const double* qn,
+                                                  const double* x) {
+  const int k1 = d.vslot_ptr[i + 1];
+  Vec3<double> acc = mk3(0.0, 0.0, 0.0);
+  for (int k = d.vslot_ptr[i]; k < k1; k += 8) {
+    Vec3<float> f[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) f[u] = ld3f(slot, min(k + u, k1 - 1));
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (k + u < k1) acc = acc + to_d(f[u]);
+  }
+  const Vec3<double> xi = ld3(x, i);
+  const double m = d.mass[i] / (d.h * d.h);
+  return m * (ld3(qn, i) - xi) + ld3(d.attach_jd, i) - d.attach_k[i] * xi + acc;
+}
+
+__global__ void k_gather_force(const __grid_constant__ SceneDev d, Gate gate, const float* __restrict__ slot, const double* __restrict__ qn,
                                const double* __restrict__ x, double* __restrict__ rhs) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= d.N || gate.skip(vpart_of(d, i))) return;
-  Vec3<double> acc = mk3(0.0, 0.0, 0.0);
-  for (int k = d.vslot_ptr[i]; k < d.vslot_ptr[i + 1]; ++k) acc = acc + to_d(ld3f(slot, k));
-  const Vec3<double> xi = ld3(x, i);
-  const double m = d.mass[i] / (d.h * d.h);
-  st3(rhs, i, m * (ld3(qn, i) - xi) + ld3(d.attach_jd, i) - d.attach_k[i] * xi + acc);
+  st3(rhs, i, force_rhs(d, i, slot, qn, x));
 }
 
 // rhs_i = c0_i + sum of the slots of vertex i

@@ -23,6 +23,7 @@
 #pragma once
 
 // (included by engine.cu after pd_kernels.cu and block_inverse.cuh)
+#include <type_traits>
 
 namespace dfem {
 
@@ -62,6 +63,8 @@ struct PdSteps {
   const double* v_in;
   double* x_out;                // user order, device memory (null: stays in xt / vt)
   double* v_out;
+  const double* X;              // mixed form: Hs^-1, N_p x N_p (dense_solve.cuh)
+  int Np;
   int res_doubles;              // shared memory for the solve's rows
   int tab_ints;                 // ... and for its index tables
   // adjoint
@@ -298,6 +301,68 @@ __device__ __forceinline__ bool ps_solve(const BlockDev& b, BAR& bar, const PsSh
   return true;
 }
 
+// The mixed form's solve: rows cta, cta + nc, ... of X times rhs, every row
+// summed as in k_dense_solve (the same lanes, order and operations: the mixed
+// form's results follow the solve's last bits).  A warp takes one row, or two
+// side by side where the CTA has more rows than warps (each staged value then
+// serves both).  res: the CTA's first nres rows in shared memory.
+template <class DONE>
+__device__ __forceinline__ void ps_dense_rows(const double* X, int Np, const double* res, int nres, int N, int cta, int nc,
+                                              const double* rhs, double* planes, DONE done) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, np2 = Np / 2;
+  double* sx = planes;
+  double* sy = sx + Np;
+  double* sz = sy + Np;
+  for (int j = tid; j < Np; j += kPsThreads) {
+    const Vec3<double> v = j < N ? ld3(rhs, j) : mk3(0.0, 0.0, 0.0);
+    sx[j] = v.x; sy[j] = v.y; sz[j] = v.z;
+  }
+  __syncthreads();
+  const double2* bx = reinterpret_cast<const double2*>(sx);
+  const double2* by = reinterpret_cast<const double2*>(sy);
+  const double2* bz = reinterpret_cast<const double2*>(sz);
+  const int rows = (N - cta + nc - 1) / nc;
+  auto run = [&](auto two, int r0, int r1) {
+    constexpr bool kTwo = decltype(two)::value;
+    const double2* m0 = reinterpret_cast<const double2*>(r0 < nres ? res + (size_t)r0 * Np : X + (size_t)(cta + r0 * nc) * Np);
+    const double2* m1 = reinterpret_cast<const double2*>(r1 < nres ? res + (size_t)r1 * Np : X + (size_t)(cta + r1 * nc) * Np);
+    double a[2][3] = {{0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}};
+    for (int q0 = lane; q0 < np2; q0 += 256) {
+      double2 u[8], w[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const int q = q0 + 32 * k;
+        u[k] = q < np2 ? m0[q] : make_double2(0.0, 0.0);
+        if (kTwo) w[k] = q < np2 ? m1[q] : make_double2(0.0, 0.0);
+      }
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const int q = q0 + 32 * k;
+        if (q < np2) {
+          const double2 x = bx[q], y = by[q], z = bz[q];
+          a[0][0] = __dadd_rn(a[0][0], __fma_rn(u[k].x, x.x, __dmul_rn(u[k].y, x.y)));
+          a[0][1] = __dadd_rn(a[0][1], __fma_rn(u[k].y, y.y, __dmul_rn(u[k].x, y.x)));
+          a[0][2] = __dadd_rn(a[0][2], __fma_rn(u[k].x, z.x, __dmul_rn(u[k].y, z.y)));
+          if (kTwo) {
+            a[1][0] = __dadd_rn(a[1][0], __fma_rn(w[k].x, x.x, __dmul_rn(w[k].y, x.y)));
+            a[1][1] = __dadd_rn(a[1][1], __fma_rn(w[k].y, y.y, __dmul_rn(w[k].x, y.x)));
+            a[1][2] = __dadd_rn(a[1][2], __fma_rn(w[k].x, z.x, __dmul_rn(w[k].y, z.y)));
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < (kTwo ? 2 : 1); ++r) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) a[r][c] = warp_sum(a[r][c]);
+      if (lane == 0) done(cta + (r == 0 ? r0 : r1) * nc, mk3(a[r][0], a[r][1], a[r][2]));
+    }
+  };
+  int r = warp;
+  for (; r + kPsWarps < rows; r += 2 * kPsWarps) run(std::true_type{}, r, r + kPsWarps);
+  if (r < rows) run(std::false_type{}, r, r);
+}
+
 // Local step of all constraints by a CTA's sixteen warps.  A tet is given to
 // two threads, eight warps apart: one takes its rotation, the other its
 // volume projection (the two iterations do not depend on one another and are
@@ -448,15 +513,14 @@ __device__ __forceinline__ double ps_total(const double* partial, int n) {
 }
 
 // Sum of a vertex's slots by eight lanes (lane l adds slots l, l + 8, ..., then a fixed tree).
-template <class T>
-__device__ __forceinline__ Vec3<double> ps_sum_slots(const T* slot, int k0, int k1) {
+__device__ __forceinline__ Vec3<double> ps_sum_slots(const double* slot, int k0, int k1) {
   Vec3<double> a = mk3(0.0, 0.0, 0.0);
   for (int k = k0 + (int)(threadIdx.x & 7); k < k1; k += 32) {  // four loads in flight
     Vec3<double> v[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const size_t q = 3 * (size_t)(k + 8 * u);
-      v[u] = k + 8 * u < k1 ? mk3((double)slot[q], (double)slot[q + 1], (double)slot[q + 2]) : mk3(0.0, 0.0, 0.0);
+      v[u] = k + 8 * u < k1 ? mk3(slot[q], slot[q + 1], slot[q + 2]) : mk3(0.0, 0.0, 0.0);
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u) a = a + v[u];
@@ -471,13 +535,16 @@ __device__ __forceinline__ Vec3<double> ps_sum_slots(const T* slot, int k0, int 
 }
 
 template <class BAR, bool MIXED>
-__global__ void __launch_bounds__(kPsThreads, 1) k_pd_forward(SceneDev d, BlockDev b, PdSteps a) {
+__global__ void __launch_bounds__(kPsThreads, 1) k_pd_forward(const __grid_constant__ SceneDev d, BlockDev b, PdSteps a) {
   extern __shared__ __align__(16) double pssh[];
   PsShared& S = *reinterpret_cast<PsShared*>(pssh);
   double* planes = pssh + (sizeof(PsShared) + 15) / 16 * 2;
-  int* tab = reinterpret_cast<int*>(pssh + ps_fixed_doubles(b.vec));
-  double* res = pssh + ps_fixed_doubles(b.vec) + a.tab_ints / 2;
-  double* xch = planes + 3 * (size_t)b.vec + 3 * kBsRows;
+  // plain form: ps_fixed_doubles, tables, rows; mixed form: three planes of N_p, rows of X
+  const int vec = MIXED ? a.Np : b.vec;
+  int* tab = reinterpret_cast<int*>(pssh + ps_fixed_doubles(vec));
+  double* res = pssh + ps_fixed_doubles(vec) + (MIXED ? 0 : a.tab_ints / 2);
+  double* xch = planes + 3 * (size_t)vec + 3 * kBsRows;
+  if (MIXED) res = xch;  // the mixed form exchanges nothing
   BAR bar(b.bar, b.status);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, cta = BAR::cta(), nc = BAR::ctas();
   // items are dealt to the CTAs a warp's worth at a time
@@ -487,7 +554,19 @@ __global__ void __launch_bounds__(kPsThreads, 1) k_pd_forward(SceneDev d, BlockD
   const int ncons = d.T + d.M + d.S + d.B;
   if (lead && a.zero)
     for (int q = 0; q < 4; ++q) a.status[q] = 0;
-  ps_setup<BAR>(b, S, tab, a.tab_ints, res, a.res_doubles);
+  // mixed form: the first of the CTA's rows cta, cta + nc, ... of X stay in shared memory
+  const int xres = MIXED ? min((d.N - cta + nc - 1) / nc, a.res_doubles / a.Np) : 0;
+  if (MIXED) {
+    {
+      for (int q = tid; q < xres * (a.Np / 2); q += kPsThreads) {
+        const int r = q / (a.Np / 2), c = q % (a.Np / 2);
+        reinterpret_cast<double2*>(res)[q] = __ldcg(reinterpret_cast<const double2*>(a.X + (size_t)(cta + r * nc) * a.Np) + c);
+      }
+    }
+    __syncthreads();
+  } else {
+    ps_setup<BAR>(b, S, tab, a.tab_ints, res, a.res_doubles);
+  }
   if (a.x_in) {
     for (int i = first; i < d.N; i += stride) {
       const int u = a.to_user[i];
@@ -563,37 +642,39 @@ __global__ void __launch_bounds__(kPsThreads, 1) k_pd_forward(SceneDev d, BlockD
       else
         ps_local<BAR>(d, xk, act_row, a.slot, xch, tv0, first, stride);
       if (!bar.sync()) return;
-      for (int g = first >> 3; g < ((d.N + 3) & ~3); g += stride >> 3) {  // eight lanes per vertex
-        const int i = min(g, d.N - 1);
-        const int k0 = i == g0 ? vs0 : d.vslot_ptr[i], k1 = i == g0 ? vs1 : d.vslot_ptr[i + 1];
-        if (MIXED) {
-          const Vec3<double> f = ps_sum_slots(reinterpret_cast<const float*>(a.slot), k0, k1);
-          if ((lane & 7) == 0 && g < d.N) {
-            const Vec3<double> xi = ld3(xk, i);
-            const double m = d.mass[i] / (d.h * d.h);
-            st3(a.rhs, i, m * (ld3(a.qn, i) - xi) + ld3(d.attach_jd, i) - d.attach_k[i] * xi + f);
-          }
-        } else {
-          const Vec3<double> c = ld3(a.c0, i), f = ps_sum_slots(a.slot, k0, k1);
+      if (MIXED) {
+        for (int i = first; i < d.N; i += stride) st3(a.rhs, i, force_rhs(d, i, reinterpret_cast<float*>(a.slot), a.qn, xk));
+      } else {
+        for (int g = first >> 3; g < ((d.N + 3) & ~3); g += stride >> 3) {  // eight lanes per vertex
+          const int i = min(g, d.N - 1);
+          const Vec3<double> c = ld3(a.c0, i);
+          const Vec3<double> f = ps_sum_slots(a.slot, i == g0 ? vs0 : d.vslot_ptr[i], i == g0 ? vs1 : d.vslot_ptr[i + 1]);
           if ((lane & 7) == 0 && g < d.N) st3(a.rhs, i, c + f);
         }
       }
       if (!bar.sync()) return;
       double e2 = 0.0;
       double* h1 = hist + (size_t)(k + 1) * 3 * d.N;
-      // plain form: x^{k+1} = x_t + z (the reference's delta form); mixed form: x^{k+1} = x^k + z
-      struct Pos { Vec3<double> xc, x0; };
-      const bool ok = ps_solve(
-          b, bar, S, a.rhs, a.y, planes,
-          [&](int g) { return Pos{ld3(xk, g), MIXED ? mk3(0.0, 0.0, 0.0) : ld3(a.xt, g)}; },
-          [&](int g, Vec3<double> z, const Pos& p) {
-            const Vec3<double> xn = (MIXED ? p.xc : p.x0) + z, dl = xn - p.xc;
-            e2 += dot3(dl, dl);
-            st3(xk, g, xn);
-            st3(h1, g, xn);
-            if (b.tiers > 1) st3(a.y, g, z);  // read by the blocks below
-          });
-      if (!ok) return;
+      if (MIXED) {  // x^{k+1} = x^k + z
+        ps_dense_rows(a.X, a.Np, res, xres, d.N, cta, nc, a.rhs, planes, [&](int g, Vec3<double> z) {
+          const Vec3<double> xc = ld3(xk, g), xn = xc + z, dl = xn - xc;
+          e2 += dot3(dl, dl);
+          st3(xk, g, xn);
+          st3(h1, g, xn);
+        });
+      } else {  // x^{k+1} = x_t + z (the reference's delta form)
+        struct Pos { Vec3<double> xc, x0; };
+        const bool ok = ps_solve(
+            b, bar, S, a.rhs, a.y, planes, [&](int g) { return Pos{ld3(xk, g), ld3(a.xt, g)}; },
+            [&](int g, Vec3<double> z, const Pos& p) {
+              const Vec3<double> xn = p.x0 + z, dl = xn - p.xc;
+              e2 += dot3(dl, dl);
+              st3(xk, g, xn);
+              st3(h1, g, xn);
+              if (b.tiers > 1) st3(a.y, g, z);  // read by the blocks below
+            });
+        if (!ok) return;
+      }
       ps_put(e2, S.ws, a.partial + par * nc + cta);
       if (!bar.sync()) return;
       tot = ps_total(a.partial + par * nc, nc);

@@ -7,13 +7,16 @@ Against the triangular form (kernel per phase, supernodal factor): iteration
 counts equal, positions to 1e-12 and gradients to 1e-9 of their largest entry
 (explicit inverses against triangular solves, as in test_solve_modes).  Within
 the form everything is exact: n steps in one call are n calls of one step, a
-replayed step and one regenerated from a checkpoint are the recorded one."""
+replayed step and one regenerated from a checkpoint are the recorded one.
+Mixed scenes keep X = Hs^-1 in their forward, whose steps in one launch are
+the kernels launched one by one bit for bit (a batch of two runs those).
+"""
 import dataclasses
 
 import numpy as np
 import pytest
 
-from diff_fem_b200 import scene as S
+from diff_fem_b200 import _capi, scene as S
 from diff_fem_b200.engine import Scene
 
 pytestmark = pytest.mark.gpu
@@ -96,3 +99,29 @@ def test_steps_in_one_launch_are_the_steps_one_by_one(name):
         for k in g:
             assert np.array_equal(q[k], g[k]), (every, budget, k)
         sc.close()
+
+
+@pytest.mark.parametrize("name", ["one_cube", "27", "64", "625", "two_tiers", "cloth", "muscles", "pneumatic"])
+def test_mixed_steps_in_one_launch_are_the_steps_one_by_one(name):
+    """Bits of n steps, of single steps, and of the adjoint's replays; the
+    adjoint (blocks or X) against the triangular form's on the same iterates."""
+    d = dataclasses.replace(SCENES[name](), precision=_capi.DFEM_PREC_MIXED)
+    n = 4
+    x, v, act, gx, gv = inputs(d, n, 11)
+    sc = Scene(d)
+    sc.solve_mode("dense")
+    f, g = run(sc, n, x, v, act, gx, gv)
+    xs, vs = x, v
+    for s in range(n):
+        xs, vs = sc.forward(xs, vs, n_steps=1, act=None if act is None else act[s:s + 1])
+    assert np.array_equal(xs, f["x"]) and np.array_equal(vs, f["v"])
+    sc.set_adjoint_budget(0)
+    h, q = run(sc, n, x, v, act, gx, gv)
+    assert np.array_equal(h["traj"], f["traj"])
+    for k in g:
+        assert np.array_equal(q[k], g[k]), k
+    sc.solve_mode("persistent")
+    _, p = run(sc, n, x, v, act, gx, gv)  # other iterates: equal to the forces' FP32 rounding
+    for k in p:
+        assert rel(g[k], p[k]) < 1e-4, k
+    sc.close()
