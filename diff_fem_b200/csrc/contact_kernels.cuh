@@ -103,7 +103,9 @@ __device__ int ccd_cubic(double a, double b, double c, double d, double x[3]) {
   return i;
 }
 
-__device__ bool vf_impact(Vec3<double> p0, Vec3<double> p1, Vec3<double> q0, Vec3<double> q1, Vec3<double> q2,
+// (Not inlined, like the other parts of the phase that its forms share: one
+// compiled copy gives every form the same bits.)
+static __device__ __noinline__ bool vf_impact(Vec3<double> p0, Vec3<double> p1, Vec3<double> q0, Vec3<double> q1, Vec3<double> q2,
                           double mult, Vec3<double>* n_out) {
   const double thick = kContactThickness * mult;
   // swept vertex box against the face box dilated by the thickness
@@ -236,8 +238,8 @@ __device__ __forceinline__ void contact_basis(Vec3<double> nrm, Vec3<double> B[3
 // L x_t at vertex i (Hs x_t - M/h^2 x_t), the contact rhs's elastic term.
 __device__ __forceinline__ Vec3<double> contact_lxt(const SceneDev& d, int i, const double* xt) {
   Vec3<double> acc = mk3(0.0, 0.0, 0.0);
-  for (int k = d.hs_ptr[i]; k < d.hs_ptr[i + 1]; ++k) acc = acc + d.hs_val[k] * ld3(xt, d.hs_col[k]);
-  return acc - (d.mass[i] / (d.h * d.h)) * ld3(xt, i);
+  for (int k = d.hs_ptr[i]; k < d.hs_ptr[i + 1]; ++k) acc = rn_axpy(d.hs_val[k], ld3(xt, d.hs_col[k]), acc);
+  return rn_axpy(-(d.mass[i] / (d.h * d.h)), ld3(xt, i), acc);
 }
 
 // The step inputs the contact adjoint reads (v_wc and L x_t of the step with
@@ -313,6 +315,22 @@ __device__ __forceinline__ bool bp_candidates(const ContactDev& c, Vec3<double> 
   return true;
 }
 
+// An impact of contact vertex a with face f: refreshes its entry or appends one.
+__device__ __forceinline__ void impact_add(const ContactDev& c, int a, int f, Vec3<double> n, int* status) {
+  const int cnt = c.imp_cnt[a];
+  int slot = -1;
+  for (int q = 0; q < cnt; ++q)
+    if (c.imp_face[a * kMaxImpactsPerVertex + q] == f) slot = q;
+  if (slot < 0) {
+    if (cnt >= c.max_impacts) { cap_reached(status, kCapImpacts); return; }
+    slot = cnt;
+    c.imp_face[a * kMaxImpactsPerVertex + slot] = f;
+    c.imp_cnt[a] = cnt + 1;
+    atomicAdd(&c.state[CS_NOBS], 1);
+  }
+  st3(c.imp_n, a * kMaxImpactsPerVertex + slot, n);
+}
+
 // Detection of contact vertex a against the obstacle faces (the broad
 // phase's candidates, or all of them — in a batch, all of its part's), in
 // ascending face order; true when it hit a face.
@@ -333,17 +351,7 @@ __device__ __forceinline__ bool contact_detect_item(const ContactDev& c, int a, 
     const int* fv = c.obs_f + 3 * f;
     if (!vf_impact(p0, p1, ld3(c.obs_x, fv[0]), ld3(c.obs_x, fv[1]), ld3(c.obs_x, fv[2]), 1.0, &n)) continue;
     any = true;
-    int cnt = c.imp_cnt[a], slot = -1;
-    for (int q = 0; q < cnt; ++q)
-      if (c.imp_face[a * kMaxImpactsPerVertex + q] == f) slot = q;
-    if (slot < 0) {
-      if (cnt >= c.max_impacts) { cap_reached(status, kCapImpacts); continue; }
-      slot = cnt;
-      c.imp_face[a * kMaxImpactsPerVertex + slot] = f;
-      c.imp_cnt[a] = cnt + 1;
-      atomicAdd(&c.state[CS_NOBS], 1);
-    }
-    st3(c.imp_n, a * kMaxImpactsPerVertex + slot, n);
+    impact_add(c, a, f, n, status);
   }
   return any;
 }
@@ -504,6 +512,33 @@ __global__ void k_contact_prep(int N, ContactDev c, double* xk, double* partial,
 // The Jacobi update of vertex i (obstacle contact only): rhs, the friction
 // cone of its impacts, relaxation, x_n1; first: the pass's first iteration;
 // rk: record index (-1: none).
+// Explicitly rounded, so that every form of the phase has the same bits.
+__device__ __forceinline__ Vec3<double> contact_rhs_value(double m, Vec3<double> vwc, double h, Vec3<double> jd,
+                                                          Vec3<double> lxt, Vec3<double> cdx) {
+  return rn_axpy(-h, cdx, rn_axpy(m, vwc, rn_scale(h, rn_axpy(-1.0, lxt, jd))));
+}
+
+// Reaction B r to the force f at an impact with normal nrm; false: take-off.
+static __device__ __noinline__ bool contact_reaction(Vec3<double> nrm, Vec3<double> f, double mu, Vec3<double>* out) {
+  Vec3<double> B[3];
+  contact_basis(nrm, B);
+  const double f0 = dot3(B[0], f), f1 = dot3(B[1], f), f2 = dot3(B[2], f);
+  if (f0 > 0) return false;
+  double r0 = -f0, r1 = -f1, r2 = -f2;
+  const double rt = sqrt(r1 * r1 + r2 * r2);
+  if (rt > mu * r0) { r1 *= mu * r0 / rt; r2 *= mu * r0 / rt; }
+  *out = r0 * B[0] + r1 * B[1] + r2 * B[2];
+  return true;
+}
+
+// relaxation of the right-hand side, and x_n1
+__device__ __forceinline__ Vec3<double> contact_relax(double alpha, Vec3<double> rhs, Vec3<double> prev) {
+  return rn_axpy(alpha, rhs, rn_scale(1.0 - alpha, prev));
+}
+__device__ __forceinline__ Vec3<double> contact_xn1(double h, double hdiag, Vec3<double> prev, Vec3<double> xt) {
+  return rn_axpy(1.0 / (h * hdiag), prev, xt);
+}
+
 __device__ __forceinline__ void contact_rhs_item(const SceneDev& d, const ContactDev& c, int i, const double* slot,
                                                  const double* xt, const double* xk, bool first, int rk) {
   Vec3<double> jd = ld3(d.attach_jd, i);
@@ -511,28 +546,22 @@ __device__ __forceinline__ void contact_rhs_item(const SceneDev& d, const Contac
   Vec3<double> cdx = mk3(0.0, 0.0, 0.0);
   for (int k = d.hs_ptr[i]; k < d.hs_ptr[i + 1]; ++k) {
     int j = d.hs_col[k];
-    if (j != i) cdx = cdx + d.hs_val[k] * (ld3(xk, j) - ld3(xt, j));
+    if (j != i) cdx = rn_axpy(d.hs_val[k], ld3(xk, j) - ld3(xt, j), cdx);
   }
-  Vec3<double> rhs = d.mass[i] * ld3(c.vwc, i) + d.h * (jd - ld3(c.lxt, i)) - d.h * cdx;
+  Vec3<double> rhs = contact_rhs_value(d.mass[i], ld3(c.vwc, i), d.h, jd, ld3(c.lxt, i), cdx);
   Vec3<double> prev = first ? rhs : ld3(c.prev, i);
   int a = c.cidx[i];
   if (a >= 0) {
-    Vec3<double> f = rhs;
-    int cnt = c.imp_cnt[a];
+    const Vec3<double> f = rhs;
+    const int cnt = c.imp_cnt[a];
     for (int q = 0; q < cnt; ++q) {
-      Vec3<double> B[3];
-      contact_basis(ld3(c.imp_n, a * kMaxImpactsPerVertex + q), B);
-      double f0 = dot3(B[0], f), f1 = dot3(B[1], f), f2 = dot3(B[2], f);
-      if (f0 > 0) continue;  // take-off
-      double r0 = -f0, r1 = -f1, r2 = -f2;
-      double rt = sqrt(r1 * r1 + r2 * r2);
-      if (rt > c.mu * r0) { r1 *= c.mu * r0 / rt; r2 *= c.mu * r0 / rt; }
-      rhs = r0 * B[0] + r1 * B[1] + r2 * B[2];
+      Vec3<double> r;
+      if (contact_reaction(ld3(c.imp_n, a * kMaxImpactsPerVertex + q), f, c.mu, &r)) rhs = r;
     }
   }
-  prev = c.alpha * rhs + (1.0 - c.alpha) * prev;
+  prev = contact_relax(c.alpha, rhs, prev);
   st3(c.prev, i, prev);
-  st3(c.xn1, i, ld3(xt, i) + (1.0 / (d.h * c.hdiag[i])) * prev);
+  st3(c.xn1, i, contact_xn1(d.h, c.hdiag[i], prev, ld3(xt, i)));
   st3(c.xold, i, ld3(xk, i));
   if (rk >= 0) {
     st3(c.rec_x + (size_t)rk * 3 * d.N, i, ld3(xk, i));
@@ -563,116 +592,21 @@ __global__ void k_contact_ctl_iter(ContactDev c, int K) {
   if (it >= K) c.state[CS_MODE] = 0;
 }
 
-// ---- the obstacle contact phase in one cooperative launch --------------------
-//
-// The whole phase of a step without soft contact as one kernel whose CTAs are
-// all resident (a cooperative launch): the state machine of the conditional
-// loop of the kernels above — detection; Jacobi iterations until the
-// max-norm change of ori_x drops below EPS or K iterations ran; detection
-// again, until a detection finds no impact — with grid-wide barriers between
-// its phases instead of kernel boundaries (3 barriers per Jacobi iteration, 1
-// per detection, against 6 launches per loop body).  Every phase runs its
-// kernel's per-item code (contact_detect_item, contact_prep_item, local_item,
-// contact_rhs_item) in a grid-stride loop, so the arithmetic and the records
-// for the adjoint are those of the loop of kernels, bit for bit.  Every
-// thread keeps an identical copy of the state machine, updated from values
-// read after a barrier; thread 0 writes the final state (passes, loop-body
-// executions, computed iterations, source iteration) to c.state for the
-// step's record.  The detections' hit flags alternate between two words, so
-// clearing one never races with reading the other.
 __device__ __forceinline__ int rec_index_at(const ContactDev& c, int comp) {
   if (!c.rec_on || *c.rec_on == 0) return -1;
   const int k = *c.rec_base + comp;
   return k < c.rec_cap ? k : -1;
 }
 
-__global__ void __launch_bounds__(128) k_contact_fused(SceneDev d, ContactDev c, const double* xt, double* xk,
-                                                       const double* act_all, const int* step, double* slot,
-                                                       double* partial, int* status) {
-  namespace cg = cooperative_groups;
-  cg::grid_group grid = cg::this_grid();
-  __shared__ double ws[4];
-  __shared__ double s_m;
-  const int tid = blockIdx.x * blockDim.x + threadIdx.x, nthr = gridDim.x * blockDim.x;
-  const bool lead = tid == 0;
-  const double* act_row = act_all + (size_t)(*step) * d.nseg;
-  const int ncons = d.T + d.M + d.S + d.B, nv = max(d.N, c.nc);
-  for (int i = tid; i < nv; i += nthr) contact_begin_item(d, c, i, xt, xk);
-  if (lead)
-    for (int k = 0; k < CS_SIZE; ++k) c.state[k] = 0;
-  if (!(c.nc > 0 && c.nof > 0)) return;  // uniform, before any barrier
-  grid.sync();
-  int mode = 0, pass = 0, it = 0, bodies = 0, comp = 0, src = 0, ndet = 0;
-  const int cap = c.max_passes * (c.K + 2) + 2;
-  for (;;) {
-    bodies += 1;
-    if (mode == 0) {  // detection pass (k_contact_detect, k_contact_ctl_detect)
-      int* flag = c.state + ((ndet & 1) ? CS_FANY1 : CS_FANY0);
-      for (int a = tid; a < c.nc; a += nthr)
-        if (contact_detect_item(c, a, xt, xk, status)) atomicOr(flag, 1);
-      grid.sync();
-      const bool any = *(volatile int*)flag != 0;
-      if (lead) c.state[(ndet & 1) ? CS_FANY0 : CS_FANY1] = 0;  // the other word: read a barrier ago
-      ++ndet;
-      if (!any) break;
-      if (pass >= c.max_passes) {
-        if (lead) cap_reached(status, kCapContactPasses);
-        break;
-      }
-      mode = 1;
-      it = 0;
-      pass += 1;
-    }
-    // one Jacobi iteration (k_contact_prep, k_local, k_contact_rhs, k_contact_ctl_iter)
-    const int rk = rec_index_at(c, comp);
-    double e = 0.0;
-    for (int i = tid; i < nv; i += nthr) e = fmax(e, contact_prep_item(c, i, d.N, xk, rk));
-    for (int o = 16; o > 0; o >>= 1) e = fmax(e, __shfl_xor_sync(0xffffffffu, e, o));
-    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = e;
-    __syncthreads();
-    if (threadIdx.x == 0) partial[blockIdx.x] = fmax(fmax(ws[0], ws[1]), fmax(ws[2], ws[3]));
-    grid.sync();
-    if (threadIdx.x < 32) {  // every CTA forms the same maximum (order-independent)
-      double m = 0.0;
-      for (int b = threadIdx.x; b < (int)gridDim.x; b += 32) m = fmax(m, __ldcg(partial + b));
-      for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-      if (threadIdx.x == 0) s_m = m;
-    }
-    __syncthreads();
-    const bool conv = s_m < kConvergenceEps;
-    src = comp;
-    if (conv) {
-      mode = 0;  // back to detection
-    } else {
-      for (int t = tid; t < ncons; t += nthr) local_item(d, t, xk, act_row, slot);
-      grid.sync();
-      for (int i = tid; i < d.N; i += nthr) contact_rhs_item(d, c, i, slot, xt, xk, it == 0, rk);
-      grid.sync();
-      it += 1;
-      if (lead && c.rec_on && *c.rec_on == 1 && *c.rec_base + comp >= c.rec_cap) atomicExch(status, 6);
-      comp += 1;
-      if (it >= c.K) mode = 0;
-    }
-    if (bodies > cap) {  // unreachable: passes and iterations are bounded above
-      if (lead) cap_reached(status, kCapContactPasses);
-      break;
-    }
-  }
-  if (lead) {
-    c.state[CS_MODE] = mode; c.state[CS_PASS] = pass; c.state[CS_IT] = it; c.state[CS_BODIES] = bodies;
-    c.state[CS_COMP] = comp; c.state[CS_SRC] = src;
-  }
-}
-
 // ---- the obstacle contact phase of a batch ---------------------------------
 //
-// Every part (scene) of a batch runs the state machine of k_contact_fused on
+// Every part (scene) of a batch runs the state machine of k_contact_phase on
 // its own: its own detections, Jacobi iterations, convergence test, passes
 // and records.  One cooperative launch advances all of them in rounds — a
 // detection phase for the parts in detection mode, then one Jacobi iteration
 // for the parts in iteration mode — with grid-wide barriers shared by all
 // parts.  A part's sequence of operations, and so its arithmetic, is the one
-// it has alone (the items are those of k_contact_fused; a part's maximum is
+// it has alone (an item's arithmetic is that of k_contact_phase; a part's maximum is
 // taken over its own vertices).  Each CTA keeps an identical copy of the
 // per-part state in shared memory, updated from values read after a barrier.
 // Records: the computed iteration j of part p is record base + j of its
@@ -1200,9 +1134,9 @@ __global__ void k_contact_rhs_pre(SceneDev d, ContactDev c, const double* __rest
   Vec3<double> cdx = mk3(0.0, 0.0, 0.0);
   for (int k = d.hs_ptr[i]; k < d.hs_ptr[i + 1]; ++k) {
     int j = d.hs_col[k];
-    if (j != i) cdx = cdx + d.hs_val[k] * (ld3(xk, j) - ld3(xt, j));
+    if (j != i) cdx = rn_axpy(d.hs_val[k], ld3(xk, j) - ld3(xt, j), cdx);
   }
-  const Vec3<double> rhs = d.mass[i] * ld3(c.vwc, i) + d.h * (jd - ld3(c.lxt, i)) - d.h * cdx;
+  const Vec3<double> rhs = contact_rhs_value(d.mass[i], ld3(c.vwc, i), d.h, jd, ld3(c.lxt, i), cdx);
   const int a = c.cidx[i];
   const int rk = rec_index(c);
   if (rk >= 0) {
@@ -1212,9 +1146,9 @@ __global__ void k_contact_rhs_pre(SceneDev d, ContactDev c, const double* __rest
   if (a < 0) {
     const bool first = c.state[CS_IT] == 0;
     Vec3<double> prev = first ? rhs : ld3(c.prev, i);
-    prev = c.alpha * rhs + (1.0 - c.alpha) * prev;
+    prev = contact_relax(c.alpha, rhs, prev);
     st3(c.prev, i, prev);
-    st3(c.xn1, i, ld3(xt, i) + (1.0 / (d.h * c.hdiag[i])) * prev);
+    st3(c.xn1, i, contact_xn1(d.h, c.hdiag[i], prev, ld3(xt, i)));
     st3(c.xold, i, ld3(xk, i));
     if (rk >= 0) st3(c.rec_prev + (size_t)rk * 3 * d.N, i, prev);
     return;
@@ -1225,14 +1159,9 @@ __global__ void k_contact_rhs_pre(SceneDev d, ContactDev c, const double* __rest
   int hit = 0;
   const int cnt = c.imp_cnt[a];
   for (int q = 0; q < cnt; ++q) {
-    Vec3<double> B[3];
-    contact_basis(ld3(c.imp_n, a * kMaxImpactsPerVertex + q), B);
-    double f0 = dot3(B[0], f), f1 = dot3(B[1], f), f2 = dot3(B[2], f);
-    if (f0 > 0) continue;  // take-off
-    double r0 = -f0, r1 = -f1, r2 = -f2;
-    double rt = sqrt(r1 * r1 + r2 * r2);
-    if (rt > c.mu * r0) { r1 *= c.mu * r0 / rt; r2 *= c.mu * r0 / rt; }
-    out = r0 * B[0] + r1 * B[1] + r2 * B[2];
+    Vec3<double> r;
+    if (!contact_reaction(ld3(c.imp_n, a * kMaxImpactsPerVertex + q), f, c.mu, &r)) continue;
+    out = r;
     hit = 1;
   }
   c.chit[a] = hit;
@@ -1271,9 +1200,9 @@ __global__ void k_contact_rhs_post(SceneDev d, ContactDev c, const double* xt, c
   }
   const bool first = c.state[CS_IT] == 0;
   Vec3<double> prev = first ? rhs : ld3(c.prev, i);
-  prev = c.alpha * post + (1.0 - c.alpha) * prev;
+  prev = contact_relax(c.alpha, post, prev);
   st3(c.prev, i, prev);
-  st3(c.xn1, i, ld3(xt, i) + (1.0 / (d.h * c.hdiag[i])) * prev);
+  st3(c.xn1, i, contact_xn1(d.h, c.hdiag[i], prev, ld3(xt, i)));
   st3(c.xold, i, ld3(xk, i));
   const int rk = rec_index(c);
   if (rk >= 0) st3(c.rec_prev + (size_t)rk * 3 * d.N, i, prev);
@@ -1390,51 +1319,40 @@ __global__ void k_cadj_start(int N, double cv, double* io_a, double* io_b, Conta
   a.hdb[i] = 0.0;
 }
 
-// slot: J d at ori (k_local); xt: the step's start positions; ori, prev: the
-// recorded iteration j; first: whether it began its pass; rcnt / rn: its impacts.
-__device__ __forceinline__ void cadj_rhs_item(const SceneDev& d, const ContactDev& c, const ContactAdj& a, int i,
-                                              const double* slot, const double* xt, const double* ori,
-                                              const double* prev, int first, const int* rcnt, const double* rn) {
+// The frame W of an impact and the reaction's coefficients r (before the
+// cone's clamp) for the force f; false: take-off.
+static __device__ __noinline__ bool contact_frame(Vec3<double> nrm, Vec3<double> f, Vec3<double> W[3], double r[3]) {
+  Vec3<double> B[3];
+  contact_basis(nrm, B);
+  const double f0 = dot3(B[0], f);
+  if (f0 > 0) return false;
+  W[0] = B[0]; W[1] = B[1]; W[2] = B[2];
+  r[0] = -f0; r[1] = -dot3(B[1], f); r[2] = -dot3(B[2], f);
+  return true;
+}
+
+// Reverse of vertex i's update in a computed iteration: xb = cotangent of its
+// x_n1, pv = its relaxed rhs; hit: an impact's reaction replaced the rhs (W,
+// r: contact_frame of the last one); first: the iteration began its pass.
+static __device__ __noinline__ void cadj_rhs_finish(const SceneDev& d, const ContactDev& c, const ContactAdj& a, int i,
+                                                    Vec3<double> xb, Vec3<double> pv, int first, bool hit,
+                                                    const Vec3<double> W[3], const double r[3], double* yb) {
   const double hd = c.hdiag[i];
-  const Vec3<double> xb = ld3(a.xn1b, i), pv = ld3(prev, i);
   st3(a.cxtb, i, ld3(a.cxtb, i) + xb);
   a.hdb[i] -= dot3(xb, pv) / (d.h * hd * hd);
   const Vec3<double> ptot = ld3(a.pb, i) + (1.0 / (d.h * hd)) * xb;
   Vec3<double> rb = c.alpha * ptot;
-  const int ac = c.cidx[i];
-  if (ac >= 0 && rcnt[ac] > 0) {
-    // rhs_pre of the contact vertex, as in k_contact_rhs
-    Vec3<double> jd = ld3(d.attach_jd, i);
-    for (int k = d.vslot_ptr[i]; k < d.vslot_ptr[i + 1]; ++k) jd = jd + ld3(slot, k);
-    Vec3<double> cdx = mk3(0.0, 0.0, 0.0);
-    for (int k = d.hs_ptr[i]; k < d.hs_ptr[i + 1]; ++k) {
-      const int j = d.hs_col[k];
-      if (j != i) cdx = cdx + d.hs_val[k] * (ld3(ori, j) - ld3(xt, j));
+  if (hit) {  // rhs_post = r0 W0 + r1' W1 + r2' W2 (friction cone clamp)
+    const double r0 = r[0], r1 = r[1], r2 = r[2];
+    const double b0 = dot3(W[0], rb), b1 = dot3(W[1], rb), b2 = dot3(W[2], rb);
+    const double rt = sqrt(r1 * r1 + r2 * r2);
+    double g0 = b0, g1 = b1, g2 = b2;
+    if (rt > c.mu * r0) {
+      g0 = b0 + c.mu * (r1 * b1 + r2 * b2) / rt;
+      g1 = c.mu * r0 * (r2 * r2 * b1 - r1 * r2 * b2) / (rt * rt * rt);
+      g2 = c.mu * r0 * (r1 * r1 * b2 - r1 * r2 * b1) / (rt * rt * rt);
     }
-    const Vec3<double> f = d.mass[i] * ld3(c.vwc, i) + d.h * (jd - ld3(c.lxt, i)) - d.h * cdx;
-    Vec3<double> W[3];
-    bool hit = false;
-    double r0 = 0, r1 = 0, r2 = 0;
-    for (int q = 0; q < rcnt[ac]; ++q) {
-      Vec3<double> B[3];
-      contact_basis(ld3(rn, ac * kMaxImpactsPerVertex + q), B);
-      const double f0 = dot3(B[0], f);
-      if (f0 > 0) continue;
-      hit = true;
-      W[0] = B[0]; W[1] = B[1]; W[2] = B[2];
-      r0 = -f0; r1 = -dot3(B[1], f); r2 = -dot3(B[2], f);
-    }
-    if (hit) {  // rhs_post = r0 W0 + r1' W1 + r2' W2 (friction cone clamp)
-      const double b0 = dot3(W[0], rb), b1 = dot3(W[1], rb), b2 = dot3(W[2], rb);
-      const double rt = sqrt(r1 * r1 + r2 * r2);
-      double g0 = b0, g1 = b1, g2 = b2;
-      if (rt > c.mu * r0) {
-        g0 = b0 + c.mu * (r1 * b1 + r2 * b2) / rt;
-        g1 = c.mu * r0 * (r2 * r2 * b1 - r1 * r2 * b2) / (rt * rt * rt);
-        g2 = c.mu * r0 * (r1 * r1 * b2 - r1 * r2 * b1) / (rt * rt * rt);
-      }
-      rb = (-1.0) * (g0 * W[0] + g1 * W[1] + g2 * W[2]);
-    }
+    rb = (-1.0) * (g0 * W[0] + g1 * W[1] + g2 * W[2]);
   }
   if (first) {
     rb = rb + (1.0 - c.alpha) * ptot;
@@ -1443,7 +1361,32 @@ __device__ __forceinline__ void cadj_rhs_item(const SceneDev& d, const ContactDe
     st3(a.pb, i, (1.0 - c.alpha) * ptot);
   }
   st3(a.vwcb, i, ld3(a.vwcb, i) + d.mass[i] * rb);
-  st3(a.yb, i, d.h * rb);
+  st3(yb, i, d.h * rb);
+}
+
+// slot: J d at ori (k_local); xt: the step's start positions; ori, prev: the
+// recorded iteration j; first: whether it began its pass; rcnt / rn: its impacts.
+__device__ __forceinline__ void cadj_rhs_item(const SceneDev& d, const ContactDev& c, const ContactAdj& a, int i,
+                                              const double* slot, const double* xt, const double* ori,
+                                              const double* prev, int first, const int* rcnt, const double* rn) {
+  const int ac = c.cidx[i];
+  Vec3<double> W[3];
+  double r[3];
+  bool hit = false;
+  if (ac >= 0 && rcnt[ac] > 0) {
+    // rhs_pre of the contact vertex, as in k_contact_rhs
+    Vec3<double> jd = ld3(d.attach_jd, i);
+    for (int k = d.vslot_ptr[i]; k < d.vslot_ptr[i + 1]; ++k) jd = jd + ld3(slot, k);
+    Vec3<double> cdx = mk3(0.0, 0.0, 0.0);
+    for (int k = d.hs_ptr[i]; k < d.hs_ptr[i + 1]; ++k) {
+      const int j = d.hs_col[k];
+      if (j != i) cdx = rn_axpy(d.hs_val[k], ld3(ori, j) - ld3(xt, j), cdx);
+    }
+    const Vec3<double> f = contact_rhs_value(d.mass[i], ld3(c.vwc, i), d.h, jd, ld3(c.lxt, i), cdx);
+    for (int q = 0; q < rcnt[ac]; ++q)
+      if (contact_frame(ld3(rn, ac * kMaxImpactsPerVertex + q), f, W, r)) hit = true;
+  }
+  cadj_rhs_finish(d, c, a, i, ld3(a.xn1b, i), ld3(prev, i), first, hit, W, r, a.yb);
 }
 
 __global__ void k_cadj_rhs(SceneDev d, ContactDev c, ContactAdj a, const double* __restrict__ slot,
@@ -1823,10 +1766,10 @@ __device__ __forceinline__ void cadj_hs_item(const SceneDev& d, const ContactAdj
   double hii = 0.0;
   for (int k = d.hs_ptr[i]; k < d.hs_ptr[i + 1]; ++k) {
     const int j = d.hs_col[k];
-    if (j != i) o = o - d.hs_val[k] * ld3(a.yb, j);
+    if (j != i) o = rn_axpy(-d.hs_val[k], ld3(a.yb, j), o);
     else hii = d.hs_val[k];
   }
-  st3(a.cxtb, i, ld3(a.cxtb, i) + (d.mass[i] / (d.h * d.h) - hii) * ld3(a.yb, i));
+  st3(a.cxtb, i, rn_axpy(d.mass[i] / (d.h * d.h) - hii, ld3(a.yb, i), ld3(a.cxtb, i)));
   st3(a.xn1b, i, o);
 }
 
@@ -1854,75 +1797,13 @@ __global__ void k_cadj_hd(SceneDev d, ContactAdj a, double* gE) {
   cadj_hd_item(d, a, t, gE);
 }
 
-// The reverse sweep of a step's obstacle contact phase (no soft contact) in
-// one cooperative launch: k_cadj_start, then for the recorded computed
-// iterations j = top .. 1 (records base + j - 1) the chain of
-// contact_adjoint_step's kernels — local step at the iteration's input, the
-// rhs VJP, the local VJP, the slot gather with the Hs terms and the
-// segments' activation sums — with grid-wide barriers between them, then
-// the diag(Hs) terms of dL/dE and the PD part's cotangent.  Same per-item
-// code and order as the kernels: bit-identical results.  The records' pass
-// flags are read on the device (the kernels' path copies them to the host).
-__global__ void __launch_bounds__(128) k_cadj_fused(SceneDev d, ContactDev c, ContactAdj a, const double* xt,
-                                                    const double* act_all, const int* step, double* slot, double* gE,
-                                                    double* gnu, double* mg, double* gact, int base, int top, double cv,
-                                                    double* io_a, double* io_b) {
-  __shared__ double tape[kVolTape * 128];
-  namespace cg = cooperative_groups;
-  cg::grid_group grid = cg::this_grid();
-  const int tid = blockIdx.x * blockDim.x + threadIdx.x, nthr = gridDim.x * blockDim.x;
-  const int ncons = d.T + d.M + d.S + d.B;
-  const size_t n3 = 3 * (size_t)d.N;
-  const int st = *step;
-  const double* act_row = act_all + (size_t)st * d.nseg;
-  for (int i = tid; i < d.N; i += nthr) {  // k_cadj_start
-    const Vec3<double> gv = ld3(io_b, i);
-    st3(a.xn1b, i, ld3(io_a, i) + cv * gv);
-    st3(a.cxtb, i, (-cv) * gv);
-    st3(a.vwcb, i, mk3(0.0, 0.0, 0.0));
-    st3(a.pb, i, mk3(0.0, 0.0, 0.0));
-    a.hdb[i] = 0.0;
-  }
-  grid.sync();
-  for (int j = top; j >= 1; --j) {
-    const size_t r = (size_t)base + (j - 1);
-    const double* ori = c.rec_x + r * n3;
-    const double* prev = c.rec_prev + r * n3;
-    const int* rcnt = c.rec_cnt + r * c.nc;
-    const double* rn = c.rec_n + r * c.nc * kMaxImpactsPerVertex * 3;
-    const int first = c.rec_first[r];
-    for (int t = tid; t < ncons; t += nthr) local_item(d, t, ori, act_row, slot);
-    grid.sync();
-    for (int i = tid; i < d.N; i += nthr) cadj_rhs_item(d, c, a, i, slot, xt, ori, prev, first, rcnt, rn);
-    grid.sync();
-    for (int t = tid; t < ncons; t += nthr) adj_local_item(d, t, ori, a.yb, act_row, slot, gE, gnu, mg, nullptr, xt, tape + threadIdx.x, 128);
-    grid.sync();
-    for (int i = tid; i < d.N; i += nthr) {  // k_adj_gather_seq, then k_cadj_hs on the same vertex
-      Vec3<double> acc = mk3(0.0, 0.0, 0.0);
-      for (int k = d.vslot_ptr[i]; k < d.vslot_ptr[i + 1]; ++k) acc = acc + ld3(slot, k);
-      st3(a.orib, i, acc);
-      cadj_hs_item(d, a, i);
-    }
-    for (int q = tid; q < d.nseg; q += nthr) {  // k_seg_reduce
-      double sum = 0;
-      for (int k = d.seg_ptr[q]; k < d.seg_ptr[q + 1]; ++k) sum += mg[member_slot(d.M, d.seg_mus[k])];
-      gact[(size_t)st * d.nseg + q] += sum;
-    }
-    grid.sync();
-  }
-  for (int t = tid; t < d.T; t += nthr) cadj_hd_item(d, a, t, gE);
-  for (int i = tid; i < d.N; i += nthr) {  // k_cadj_to_pd
-    st3(io_a, i, ld3(a.xn1b, i));
-    st3(io_b, i, mk3(0.0, 0.0, 0.0));
-  }
-}
-
 // The reverse sweep of a batch's obstacle contact phase in one cooperative
-// launch: k_cadj_fused for every part, part p reversing its own computed
-// iterations top[p] .. 1 (its records base + j - 1, pass flags
-// rec_first[(base + j - 1) np + p]); the sweeps run side by side, iteration j
-// of every part that has one in the same round.  Same per-item code as
-// k_cadj_fused.
+// launch: k_cadj_start, then part p reverses its own computed iterations
+// top[p] .. 1 (its records base + j - 1, pass flags rec_first[(base + j - 1)
+// np + p]) by the chain of contact_adjoint_step's kernels, with grid-wide
+// barriers between them; the sweeps run side by side, iteration j of every
+// part that has one in the same round.  Then the diag(Hs) terms of dL/dE and
+// the PD part's cotangent.  An item's arithmetic is that of the kernels.
 __global__ void __launch_bounds__(128) k_cadj_fused_parts(SceneDev d, ContactDev c, ContactAdj a, const double* xt,
                                                           const double* act_all, const int* step, double* slot,
                                                           double* gE, double* gnu, double* mg, double* gact, int base,

@@ -28,6 +28,7 @@
 #include "dense_solve.cuh"
 #include "block_inverse.cuh"
 #include "step_kernels.cuh"
+#include "contact_step.cuh"
 #include "resident_plan.h"
 #include "scene.h"
 
@@ -245,15 +246,16 @@ struct dfem_scene {
   bool has_contact = false;
   DBuf<int> cverts, cidx, obs_f, imp_cnt, imp_face, cstate, cpasses;
   DBuf<int> bp_ptr, bp_face;             // broad phase of the obstacle detection
-  // the obstacle contact phase as one cooperative launch (k_contact_fused) or
+  // the obstacle contact phase as one cooperative launch (k_contact_phase) or
   // as the conditional loop of kernels
   bool fused_ok = false;                 // scene has obstacle contact only and the device runs the launch
   bool fused_on = true;                  // dfem_set_option(DFEM_OPTION_FUSED_CONTACT)
   bool split_factor = true;              // dfem_set_option(DFEM_OPTION_SPLIT_FACTOR)
   int gather_form = 0;                   // dfem_set_option(DFEM_OPTION_GATHER): 0 by size, 1 warp, 2 thread
-  int fused_grid = 0;                    // CTAs of k_contact_fused (all resident)
-  int cadj_grid = 0;                     // CTAs of k_cadj_fused (all resident)
-  DBuf<double> fpartial;
+  int fused_grid = 0;                    // CTAs of k_contact_phase (all resident)
+  int cadj_grid = 0;                     // CTAs of k_cadj_phase (all resident)
+  DBuf<double> fpartial, ca_slot;
+  DBuf<unsigned> cbar;                   // the two kernels' barrier counters
   DBuf<double> obs_x, hdiag, imp_n, xn1, xold, cprev, lxt, vwc;
   // soft-soft contact (forward only: the adjoint refuses these scenes)
   bool self_contact = false;
@@ -1424,11 +1426,18 @@ static int upload_scene(dfem_scene* sc) {
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_contact_fused_parts, 128, shm));
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_a, k_cadj_fused_parts, 128, 0));
       } else {
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_contact_fused, 128, 0));
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_a, k_cadj_fused, 128, 0));
+        CK(raise_smem_limit((const void*)k_contact_phase, kCtSmemFwd));
+        CK(raise_smem_limit((const void*)k_cadj_phase, kCtSmemAdj));
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_contact_phase, kPsThreads, kCtSmemFwd));
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_a, k_cadj_phase, kPsThreads, kCtSmemAdj));
+        CK(sc->cbar.alloc(2));
+        CK(cudaMemset(sc->cbar.p, 0, 2 * sizeof(unsigned)));
       }
       const int ncons = s.T + s.M + s.S + s.B;
-      const int want = std::max(1, (std::max(ncons, s.N) + 127) / 128);
+      // (k_contact_phase, k_cadj_phase: one CTA per SM; a small scene gets a
+      // warp's elements and eight lanes per vertex of a warp or two on each)
+      const int want = std::max(1, sc->cnp > 0 ? (std::max(ncons, s.N) + 127) / 128 : (std::max(ncons, 4 * s.N) + 31) / 32);
+      if (sc->cnp <= 0) occ = std::min(occ, 1), occ_a = std::min(occ_a, 1);
       sc->fused_grid = std::min(nsm * occ, want);
       sc->cadj_grid = std::min(nsm * occ_a, want);
       sc->fused_ok = coop != 0 && occ > 0 && occ_a > 0;
@@ -2000,9 +2009,11 @@ static cudaError_t launch_contact_fused(dfem_scene* sc, cudaStream_t st) {
     return cudaLaunchKernelEx(&cfg, k_contact_fused_parts, sc->sd, sc->cd, (const double*)sc->xt.p, sc->xk.p,
                               (const double*)sc->act_all.p, (const int*)sc->step.p, sc->slot.p, sc->status.p);
   }
-  return cudaLaunchKernelEx(&cfg, k_contact_fused, sc->sd, sc->cd, (const double*)sc->xt.p, sc->xk.p,
+  cfg.blockDim = dim3(kPsThreads);
+  cfg.dynamicSmemBytes = kCtSmemFwd;
+  return cudaLaunchKernelEx(&cfg, k_contact_phase, sc->sd, sc->cd, (const double*)sc->xt.p, sc->xk.p,
                             (const double*)sc->act_all.p, (const int*)sc->step.p, sc->slot.p, sc->fpartial.p,
-                            sc->status.p);
+                            sc->cbar.p, sc->status.p);
 }
 
 static void step_post(dfem_scene* sc, cudaStream_t st) {
@@ -2206,6 +2217,7 @@ static int ensure_contact_record(dfem_scene* sc, int cap, int keep = 0) {
   for (DBuf<double>* b : {&sc->ca_xn1b, &sc->ca_pb, &sc->ca_cxtb, &sc->ca_vwcb, &sc->ca_yb, &sc->ca_orib})
     if (!b->p) CK(b->alloc(n3));
   if (!sc->ca_hdb.p) CK(sc->ca_hdb.alloc(std::max(1, s.N)));
+  if (sc->cbar.p && !sc->ca_slot.p) CK(sc->ca_slot.alloc(3 * (size_t)std::max(1, s.nslots)));
   if (sc->self_contact) {
     const int ncf = sc->cd.ncf;
     for (DBuf<double>* b : {&sc->ca_scb, &sc->ca_ptot, &sc->ca_sbp, &sc->ca_gPM})
@@ -2375,18 +2387,9 @@ static int contact_adjoint_step(dfem_scene* sc, int st, bool recorded, int rbase
   }
   if (!sc->self_contact && fused_contact(sc)) {  // the whole reverse sweep in one cooperative launch
     const ContactAdj a = make_cadj(sc);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(sc->cadj_grid);
-    cfg.blockDim = dim3(128);
-    cfg.stream = sc->stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;
-    attr[0].val.cooperative = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    CK(cudaLaunchKernelEx(&cfg, k_cadj_fused, sc->sd, sc->cd, a, xt, (const double*)sc->act_all.p,
-                          (const int*)sc->step.p, sc->slot.p, sc->gE.p, sc->gnu.p, sc->mg.p, sc->gact.p, base, src,
-                          s.damping / s.h, sc->io_a.p, sc->io_b.p));
+    CK(launch_coop(sc->stream, k_cadj_phase, sc->cadj_grid, kPsThreads, kCtSmemAdj, sc->sd, sc->cd, a, xt,
+                   (const double*)sc->act_all.p, (const int*)sc->step.p, sc->slot.p, sc->ca_slot.p, sc->gE.p, sc->gnu.p,
+                   sc->mg.p, sc->gact.p, base, src, s.damping / s.h, sc->io_a.p, sc->io_b.p, sc->cbar.p, sc->status.p));
     sc->launches += 1;
     return DFEM_OK;
   }
@@ -2493,9 +2496,10 @@ static int status_error(const int st4[4]) {
 // status_error for a call's status; a barrier that gave up leaves its counters
 // behind, so they are cleared for the next launch.
 static int check_status(dfem_scene* sc, const int st4[4]) {
-  if (st4[0] == DFEM_ERR_CAP && st4[2] == kWaitGrid && sc->bl_bar.p) {
+  if (st4[0] == DFEM_ERR_CAP && st4[2] == kWaitGrid) {
     CK(cudaStreamSynchronize(sc->stream));
-    CK(cudaMemset(sc->bl_bar.p, 0, 2 * sizeof(unsigned)));
+    for (DBuf<unsigned>* b : {&sc->bl_bar, &sc->cbar})
+      if (b->p) CK(cudaMemset(b->p, 0, 2 * sizeof(unsigned)));
   }
   return status_error(st4);
 }

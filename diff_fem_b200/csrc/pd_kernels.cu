@@ -80,6 +80,14 @@ __device__ __forceinline__ Mat3<double> deformation(const double G[4][3], const 
   return F;
 }
 
+// The same, explicitly rounded: for code that several kernels compile.
+__device__ __forceinline__ Mat3<double> deformation_rn(const double G[4][3], const Vec3<double> xv[4]) {
+  Mat3<double> F;
+#pragma unroll
+  for (int j = 0; j < 3; ++j) F.c[j] = rn_axpy(G[3][j], xv[3], rn_comb(G[0][j], xv[0], G[1][j], xv[1], G[2][j], xv[2]));
+  return F;
+}
+
 // Minimum resident CTAs per SM asked of the register allocator for the
 // heaviest per-constraint kernels (128 threads each): more resident warps hide
 // the FP64 latency chains better than the registers they give up (the mixed
@@ -232,7 +240,7 @@ __device__ __forceinline__ void local_rest(const SceneDev& d, int t, const doubl
 // Local step of constraint t (tets, muscles, springs, bending stencils in
 // that order): its projection and its J*d contribution to its slots.  The
 // pointers are not restrict-qualified: a kernel that writes x in an earlier
-// phase of the same launch (k_contact_fused) must not read it through the
+// phase of the same launch (k_contact_phase) must not read it through the
 // read-only data path.
 __device__ __forceinline__ void local_item(const SceneDev& d, int t, const double* x, const double* act_row,
                                            double* slot) {
@@ -242,7 +250,7 @@ __device__ __forceinline__ void local_item(const SceneDev& d, int t, const doubl
     Vec3<double> xv[4] = {ld3(x, v.x), ld3(x, v.y), ld3(x, v.z), ld3(x, v.w)};
     double G[4][3];
     load_g(d.tinv, d.T, t, G);
-    Mat3<double> F = deformation(G, xv), md, mdv;
+    Mat3<double> F = deformation_rn(G, xv), md, mdv;
     corot_project_polar(F, md, mdv);
     double wr = d.twr[t], wv = d.twv[t];
     Vec3<double> P[3];
@@ -251,7 +259,7 @@ __device__ __forceinline__ void local_item(const SceneDev& d, int t, const doubl
     int4 sl = d.tslot[t];
     const int sv[4] = {sl.x, sl.y, sl.z, sl.w};
 #pragma unroll
-    for (int a = 0; a < 4; ++a) st3(slot, sv[a], G[a][0] * P[0] + G[a][1] * P[1] + G[a][2] * P[2]);
+    for (int a = 0; a < 4; ++a) st3(slot, sv[a], rn_comb(G[a][0], P[0], G[a][1], P[1], G[a][2], P[2]));
     return;
   }
   local_rest(d, t - d.T, x, act_row, slot);
@@ -1304,8 +1312,24 @@ __device__ __forceinline__ void adj_local_rest(const SceneDev& d, int t, const d
   }
 }
 
+// The Hs terms of a tet's E gradient in the contact phase: Y . F and the
+// diagonal's part (explicitly rounded: two forms of the phase evaluate it).
+__device__ __forceinline__ double contact_yh(const double G[4][3], const Mat3<double>& F, const Mat3<double>& Y,
+                                             const Vec3<double> yv[4], const Vec3<double> xv[4], const double* xt,
+                                             const int vi[4]) {
+  double yh = 0;
+#pragma unroll
+  for (int j = 0; j < 3; ++j) yh = __dadd_rn(yh, rn_dot(Y.c[j], F.c[j]));
+#pragma unroll
+  for (int a = 0; a < 4; ++a) {
+    const double gaa = rn_dot(mk3(G[a][0], G[a][1], G[a][2]), mk3(G[a][0], G[a][1], G[a][2]));
+    yh = __fma_rn(gaa, rn_dot(yv[a], ld3(xt, vi[a]) - xv[a]), yh);
+  }
+  return yh;
+}
+
 // tape: this thread's first value of the VJP's tape (kVolTape values, stride apart, in shared memory).
-// (Plain pointers: k_cadj_fused writes yb earlier in the same launch; the
+// (Plain pointers: k_cadj_phase writes yb earlier in the same launch; the
 // kernels that call it keep their parameters restrict-qualified.)
 __device__ __forceinline__ void adj_local_item(const SceneDev& d, int t, const double* x, const double* yb,
                                                const double* act_row, double* slot, double* gE, double* gnu,
@@ -1319,7 +1343,7 @@ __device__ __forceinline__ void adj_local_item(const SceneDev& d, int t, const d
     for (int a = 0; a < 4; ++a) { xv[a] = ld3(x, vi[a]); yv[a] = ld3(yb, vi[a]); }
     double G[4][3];
     load_g(d.tinv, d.T, t, G);
-    const Mat3<double> F = deformation(G, xv), Y = deformation(G, yv);
+    const Mat3<double> F = deformation_rn(G, xv), Y = deformation_rn(G, yv);
     double E = d.tE[t], nu = d.tnu[t], vol = d.tvol[t];
     double yr, yvv, yh = 0;
     Mat3<double> gF;
@@ -1330,13 +1354,7 @@ __device__ __forceinline__ void adj_local_item(const SceneDev& d, int t, const d
 #pragma unroll
       for (int j = 0; j < 3; ++j) yh += dot3(Y.c[j], F1.c[j]);
     } else if (xt) {
-#pragma unroll
-      for (int j = 0; j < 3; ++j) yh += dot3(Y.c[j], F.c[j]);
-#pragma unroll
-      for (int a = 0; a < 4; ++a) {
-        const double gaa = G[a][0] * G[a][0] + G[a][1] * G[a][1] + G[a][2] * G[a][2];
-        yh += gaa * dot3(yv[a], ld3(xt, vi[a]) - xv[a]);
-      }
+      yh = contact_yh(G, F, Y, yv, xv, xt, vi);
     }
     double opn = 1.0 + nu;
     if (gE) gE[t] += vol / opn * (yr + nu * yvv) - vol * yh;
@@ -1344,7 +1362,7 @@ __device__ __forceinline__ void adj_local_item(const SceneDev& d, int t, const d
     int4 sl = d.tslot[t];
     const int sv[4] = {sl.x, sl.y, sl.z, sl.w};
 #pragma unroll
-    for (int a = 0; a < 4; ++a) st3(slot, sv[a], G[a][0] * gF.c[0] + G[a][1] * gF.c[1] + G[a][2] * gF.c[2]);
+    for (int a = 0; a < 4; ++a) st3(slot, sv[a], rn_comb(G[a][0], gF.c[0], G[a][1], gF.c[1], G[a][2], gF.c[2]));
     return;
   }
   adj_local_rest(d, t - d.T, x, yb, act_row, slot, mg);

@@ -229,6 +229,9 @@ __device__ __forceinline__ Vec3<double> rn_scale(double s, Vec3<double> a) {
 __device__ __forceinline__ Vec3<double> rn_axpy(double s, Vec3<double> a, Vec3<double> b) {  // s a + b
   return {__fma_rn(s, a.x, b.x), __fma_rn(s, a.y, b.y), __fma_rn(s, a.z, b.z)};
 }
+__device__ __forceinline__ Vec3<double> rn_comb(double a, Vec3<double> u, double b, Vec3<double> v, double c, Vec3<double> w) {
+  return rn_axpy(c, w, rn_axpy(b, v, rn_scale(a, u)));  // a u + b v + c w
+}
 __device__ __forceinline__ Vec3<double> rn_add(Vec3<double> a, Vec3<double> b) {
   return {__dadd_rn(a.x, b.x), __dadd_rn(a.y, b.y), __dadd_rn(a.z, b.z)};
 }
@@ -770,23 +773,14 @@ __device__ __forceinline__ void corot_adjoint_volume(const Mat3<double>& F, cons
   volume_vjp(F, C, det, Y, wv, yv, gF, tape_sh, stride);
 }
 
+// Both (an element near a lower rank takes the SVD's VJP once for each half,
+// as two threads do).
 __device__ __forceinline__ void corot_adjoint_polar(const Mat3<double>& F, const Mat3<double>& Y, double wr, double wv,
                                                     double& yr, double& yv, Mat3<double>& gF, double* tape_sh,
                                                     int stride) {
-  Mat3<double> C, Q, gV;
-  rn_cof(F, C);
-  const double det = rn_dot(F.c[0], C.c[0]);
-  if (!polar_newton(F, C, det, Q)) {
-    Mat3<double> f = F, y = Y, g;
-    double a, b;
-    corot_adjoint_svd(f, y, wr, wv, a, b, g);
-    yr = a;
-    yv = b;
-    gF = g;
-    return;
-  }
-  rotation_vjp(F, Q, det < 0.0 ? -1.0 : 1.0, Y, wr, yr, gF);
-  volume_vjp(F, C, det, Y, wv, yv, gV, tape_sh, stride);
+  Mat3<double> gV;
+  corot_adjoint_rotation(F, Y, wr, yr, gF);
+  corot_adjoint_volume(F, Y, wv, yv, gV, tape_sh, stride);
 #pragma unroll
   for (int j = 0; j < 3; ++j) gF.c[j] = rn_add(gF.c[j], gV.c[j]);
 }

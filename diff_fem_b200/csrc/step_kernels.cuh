@@ -390,7 +390,7 @@ __device__ __forceinline__ void ps_corners(const double G[4][3], const Vec3<doub
   for (int q = 0; q < 2; ++q) {
     const double g0 = rot ? G[q][0] : G[q + 2][0], g1 = rot ? G[q][1] : G[q + 2][1], g2 = rot ? G[q][2] : G[q + 2][2];
     const int o = rot ? (q == 0 ? sl.x : sl.y) : (q == 0 ? sl.z : sl.w);
-    st3(slot, o, g0 * P[0] + g1 * P[1] + g2 * P[2]);
+    st3(slot, o, rn_comb(g0, P[0], g1, P[1], g2, P[2]));
   }
 }
 
