@@ -32,102 +32,95 @@
 namespace dfem {
 
 constexpr int kCtPlane = 33;                           // 32 values, odd: a vertex's components in different banks
-constexpr int kCtStage = 4 * kCtPlane;                 // doubles of a vertex: 32 slots, or 32 entries of its row (value, x_j)
+constexpr int kCtSlots = 64;                           // slots of a vertex in one round
+constexpr int kCtStage = 3 * kCtSlots + 4 * kCtPlane;  // doubles of a vertex: they, and 32 entries of its row (value, x_j)
 constexpr int kCtWarpStage = 4 * kCtStage;             // four vertices per warp
 constexpr int kCtAdjWarps = kPsWarps / 4;              // warps of a half that run the VJP (as many: the local step)
 constexpr size_t kCtSmemFwd = sizeof(double) * (size_t)(kPsWarps * kCtWarpStage > kPsXch * kPsPair ? kPsWarps * kCtWarpStage : kPsXch * kPsPair);
-constexpr size_t kCtSmemAdj = sizeof(double) * (size_t)(kPsXch * kPsPair + kVolTape * 32 * kCtAdjWarps);
+constexpr int kCtTape = kPsXch * kPsPair;              // adjoint: the exchange, the tape, stages of the local step's warps
+constexpr int kCtFrames = kCtTape + kVolTape * 32 * kCtAdjWarps;
+constexpr size_t kCtSmemAdj = sizeof(double) * (size_t)(kCtFrames + 2 * kCtAdjWarps * kCtWarpStage);
 static_assert(2 * kBroadMaxCandidates * sizeof(int) <= kCtWarpStage * sizeof(double), "a detection's lists");
 static_assert(kMaxImpactsPerVertex <= 8, "one lane per impact");
 static_assert(kCtSmemAdj >= kCtSmemFwd, "the adjoint's shared memory holds the stages");
 
-// init + the slots k0 .. k1 in order, for the four vertices of a warp (eight
-// lanes each; every lane gets its vertex's sum).  w: the warp's stage.
-__device__ __forceinline__ Vec3<double> ct_sum_slots(Vec3<double> init, const double* slot, int k0, int k1, double* w) {
+// Sums of a vertex i (eight lanes each, four vertices per warp; every lane
+// gets its vertex's): ss = init + its slots k0 .. k1 in order; sr = the sum
+// over its row h0 .. h1 of Hs (the diagonal left out unless DIAG) of sign
+// Hs_ij (p_j - q_j) in order (q: DIFF), from zero or (CHAIN) from ss; hii: the
+// diagonal entry.  All reads of a round are in flight before the first sum
+// (the slots go straight to the warp's stage w); the sums run on one lane per
+// component.
+template <bool DIFF, bool CHAIN, bool DIAG>
+__device__ __forceinline__ void ct_sums(const SceneDev& d, int i, int k0, int k1, int h0, int h1, Vec3<double> init,
+                                        const double* slot, const double* p, const double* q, double sign, double* w,
+                                        Vec3<double>& ss, Vec3<double>& sr, double& hii) {
   const int l = threadIdx.x & 7;
   double* g = w + ((threadIdx.x & 31) >> 3) * kCtStage;
-  double acc = l == 0 ? init.x : l == 1 ? init.y : init.z;
-  while (__any_sync(0xffffffffu, k0 < k1)) {
-    const int n = 3 * max(0, min(32, k1 - k0));
-    const double* p = slot + 3 * (size_t)k0;
-    double v[12];
-#pragma unroll
-    for (int u = 0; u < 12; ++u) v[u] = l + 8 * u < n ? p[l + 8 * u] : 0.0;
-#pragma unroll
-    for (int u = 0; u < 12; ++u) g[l + 8 * u] = v[u];
-    __syncwarp();
-    if (l < 3) {
-#pragma unroll 8
-      for (int k = l; k < n; k += 3) acc += g[k];
-    }
-    __syncwarp();
-    k0 += 32;
-  }
-  return mk3(__shfl_sync(0xffffffffu, acc, 0, 8), __shfl_sync(0xffffffffu, acc, 1, 8), __shfl_sync(0xffffffffu, acc, 2, 8));
-}
-
-// init + sum over row i of Hs (entries k0 .. k1, the diagonal left out unless
-// with_diag) of sign Hs_ij x_j in order; x_j = p_j - q_j (q may be null).
-// hii: the diagonal entry.
-__device__ __forceinline__ Vec3<double> ct_sum_row(const SceneDev& d, Vec3<double> init, int i, int k0, int k1, const double* p,
-                                                   const double* q, double sign, bool with_diag, double* w, double* hii) {
-  const int l = threadIdx.x & 7;
-  double* g = w + ((threadIdx.x & 31) >> 3) * kCtStage;
-  double acc = l == 0 ? init.x : l == 1 ? init.y : init.z, h = 0.0;
-  while (__any_sync(0xffffffffu, k0 < k1)) {
-    const int n = max(0, min(32, k1 - k0));
-    int col[4];
+  double* gr = g + 3 * kCtSlots;
+  const unsigned gs = (unsigned)__cvta_generic_to_shared(g);
+  double as = l == 0 ? init.x : l == 1 ? init.y : init.z, ar = 0.0;
+  hii = 0.0;
+  for (bool start = false;;) {
+    const bool last = !__any_sync(0xffffffffu, k1 - k0 > kCtSlots);  // the rest of the slots: rows too
+    const int n = 3 * max(0, min(kCtSlots, k1 - k0)), m = last ? max(0, min(32, h1 - h0)) : 0;
+    const double* ps = slot + 3 * (size_t)k0;
     double val[4];
+    int col[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const bool on = l + 8 * u < n;
-      col[u] = on ? d.hs_col[k0 + l + 8 * u] : i;
-      val[u] = on ? d.hs_val[k0 + l + 8 * u] : 0.0;
+      const bool on = l + 8 * u < m;
+      col[u] = on ? d.hs_col[h0 + l + 8 * u] : i;
+      val[u] = on ? sign * d.hs_val[h0 + l + 8 * u] : 0.0;
     }
+#pragma unroll 4
+    for (int e = l; e < n; e += 8)
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(gs + 8 * e), "l"(ps + e) : "memory");
     Vec3<double> x[4], y[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const bool on = l + 8 * u < n;
+      const bool on = l + 8 * u < m;
       x[u] = on ? ld3(p, col[u]) : mk3(0.0, 0.0, 0.0);
-      y[u] = on && q ? ld3(q, col[u]) : mk3(0.0, 0.0, 0.0);
+      if (DIFF) y[u] = on ? ld3(q, col[u]) : mk3(0.0, 0.0, 0.0);
     }
-    int diag = -1;
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const int e = l + 8 * u;
-      const Vec3<double> v = q ? x[u] - y[u] : x[u];
-      g[e] = sign * val[u];
-      g[kCtPlane + e] = v.x;
-      g[2 * kCtPlane + e] = v.y;
-      g[3 * kCtPlane + e] = v.z;
-      if (e < n && col[u] == i) {
-        diag = e;
-        h = val[u];
+      Vec3<double> v = DIFF ? x[u] - y[u] : x[u];
+      if (!DIAG && e < m && col[u] == i) {  // adds an exact zero
+        hii = sign * val[u];
+        val[u] = 0.0;
+        v = mk3(0.0, 0.0, 0.0);
       }
+      gr[e] = val[u];
+      gr[kCtPlane + e] = v.x;
+      gr[2 * kCtPlane + e] = v.y;
+      gr[3 * kCtPlane + e] = v.z;
     }
-#pragma unroll
-    for (int o = 4; o > 0; o >>= 1) diag = max(diag, __shfl_xor_sync(0xffffffffu, diag, o));
-    if (with_diag) diag = -1;
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncwarp();
     if (l < 3) {
 #pragma unroll 8
-      for (int k = 0; k < n; ++k) {
-        const double a = __fma_rn(g[k], g[kCtPlane * (1 + l) + k], acc);
-        acc = k == diag ? acc : a;
-      }
+      for (int k = l; k < n; k += 3) as += g[k];
+      if (CHAIN && last && !start) ar = as;
+#pragma unroll 8
+      for (int k = 0; k < m; ++k) ar = __fma_rn(gr[k], gr[kCtPlane * (1 + l) + k], ar);
     }
     __syncwarp();
-    k0 += 32;
+    start = start || last;
+    k0 += kCtSlots;
+    h0 += last ? 32 : 0;
+    if (last && !__any_sync(0xffffffffu, h0 < h1)) break;
   }
-  if (hii) {  // one lane of the vertex met it
+  if (!DIAG) {  // one lane of the vertex met it
 #pragma unroll
     for (int o = 4; o > 0; o >>= 1) {
-      const double t = __shfl_xor_sync(0xffffffffu, h, o);
-      h = h != 0.0 ? h : t;
+      const double t = __shfl_xor_sync(0xffffffffu, hii, o);
+      hii = hii != 0.0 ? hii : t;
     }
-    *hii = h;
   }
-  return mk3(__shfl_sync(0xffffffffu, acc, 0, 8), __shfl_sync(0xffffffffu, acc, 1, 8), __shfl_sync(0xffffffffu, acc, 2, 8));
+  ss = mk3(__shfl_sync(0xffffffffu, as, 0, 8), __shfl_sync(0xffffffffu, as, 1, 8), __shfl_sync(0xffffffffu, as, 2, 8));
+  sr = mk3(__shfl_sync(0xffffffffu, ar, 0, 8), __shfl_sync(0xffffffffu, ar, 1, 8), __shfl_sync(0xffffffffu, ar, 2, 8));
 }
 
 // Detection of contact vertex a by a warp (contact_detect_item's result): the
@@ -223,41 +216,50 @@ __device__ __forceinline__ void ct_put_max(double e, double* ws, double* partial
     *partial = m;
   }
 }
-__device__ __forceinline__ double ct_max(const double* partial, int n) {
-  double m = 0.0;
-#pragma unroll 4
-  for (int b = threadIdx.x & 31; b < n; b += 32) m = fmax(m, __ldcg(partial + b));
-  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-  return m;
+// (One warp reads: with all of them the reads of the same few lines queue.)
+__device__ __forceinline__ double ct_max(const double* partial, int n, double* ws) {
+  if (threadIdx.x < 32) {
+    double m = 0.0;
+#pragma unroll 5
+    for (int b = threadIdx.x; b < n; b += 32) m = fmax(m, __ldcg(partial + b));
+    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if (threadIdx.x == 0) ws[0] = m;
+  }
+  __syncthreads();
+  return ws[0];
 }
 __device__ __forceinline__ double ct_norm(Vec3<double> a) { return fmax(fabs(a.x), fmax(fabs(a.y), fabs(a.z))); }
 
 // A half of a tet's local step and its corners' slots after the exchange
 // (local_item's bits: wr md + wv md_volume as one fused multiply-add).
-__device__ __forceinline__ void ct_tet_give(const SceneDev& d, int t, const double* x, bool rot, double* xch, int me,
-                                            double G[4][3], Vec3<double> P[3]) {
-  const int4 v = d.tv[t];
+struct CtTet {
+  double G[4][3], wr;
+  Vec3<double> P[3];
+  int4 sl;
+};
+__device__ __forceinline__ void ct_tet_give(const SceneDev& d, int t, int4 v, const double* x, bool rot, double* xch, int me,
+                                            CtTet& T) {
   const Vec3<double> xv[4] = {ld3(x, v.x), ld3(x, v.y), ld3(x, v.z), ld3(x, v.w)};
-  load_g(d.tinv, d.T, t, G);
+  load_g(d.tinv, d.T, t, T.G);
   const double wv = d.twv[t];
-  const Mat3<double> F = deformation_rn(G, xv);
+  T.wr = d.twr[t];
+  T.sl = d.tslot[t];
+  const Mat3<double> F = deformation_rn(T.G, xv);
   Mat3<double> m;
   if (rot) corot_rotation(F, m);
   else corot_volume(F, m);
 #pragma unroll
-  for (int j = 0; j < 3; ++j) P[j] = rot ? m.c[j] : rn_scale(wv, m.c[j]);
-  ps_give(xch, rot, me, P);
+  for (int j = 0; j < 3; ++j) T.P[j] = rot ? m.c[j] : rn_scale(wv, m.c[j]);
+  ps_give(xch, rot, me, T.P);
 }
-__device__ __forceinline__ void ct_tet_take(const SceneDev& d, int t, bool rot, const double* xch, int me,
-                                            const double G[4][3], Vec3<double> P[3], double* slot) {
+__device__ __forceinline__ void ct_tet_take(bool rot, const double* xch, int me, CtTet& T, double* slot) {
   const double* o = xch + (rot ? 9 : 0) * kPsPair + me;
-  const double wr = d.twr[t];
 #pragma unroll
   for (int j = 0; j < 3; ++j) {
     const Vec3<double> q = mk3(o[(3 * j) * kPsPair], o[(3 * j + 1) * kPsPair], o[(3 * j + 2) * kPsPair]);
-    P[j] = rot ? rn_axpy(wr, P[j], q) : rn_axpy(wr, q, P[j]);
+    T.P[j] = rot ? rn_axpy(T.wr, T.P[j], q) : rn_axpy(T.wr, q, T.P[j]);
   }
-  ps_corners(G, P, d.tslot[t], rot, slot);
+  ps_corners(T.G, T.P, T.sl, rot, slot);
 }
 
 __global__ void __launch_bounds__(kPsThreads, 1) k_contact_phase(const __grid_constant__ SceneDev d,
@@ -275,12 +277,17 @@ __global__ void __launch_bounds__(kPsThreads, 1) k_contact_phase(const __grid_co
   const bool rot = warp < kPsWarps / 2;
   double* stage = dyn + warp * kCtWarpStage;
   const double* act_row = act_all + (size_t)(*step) * d.nseg;
+  const int t0 = 32 * ((warp & (kPsWarps / 2 - 1)) * nc + cta) + lane;  // this thread's first tet
+  const int4 tv0 = t0 < d.T ? d.tv[t0] : make_int4(0, 0, 0, 0);
+  const int rec_on = c.rec_on ? *c.rec_on : 0, rec_base = rec_on ? *c.rec_base : 0;
   // k_contact_begin: L x_t, empty lists; ori_x = x_n1 = the PD result, xold = 0
   double e = 0.0;
   for (int b = 4 * wid; b < d.N; b += 4 * nw) {
     const int i = b + (lane >> 3), ii = min(i, d.N - 1);
-    const Vec3<double> s = ct_sum_row(d, mk3(0.0, 0.0, 0.0), ii, d.hs_ptr[ii], i < d.N ? d.hs_ptr[ii + 1] : 0, xt, nullptr, 1.0,
-                                      true, stage, nullptr);
+    Vec3<double> s, none;
+    double hii;
+    ct_sums<false, false, true>(d, ii, 0, 0, d.hs_ptr[ii], i < d.N ? d.hs_ptr[ii + 1] : 0, mk3(0.0, 0.0, 0.0), slot, xt, xt, 1.0,
+                                stage, none, s, hii);
     if (i < d.N && (lane & 7) == 0) {
       st3(c.lxt, i, rn_axpy(-(d.mass[i] / (d.h * d.h)), ld3(xt, i), s));
       e = fmax(e, ct_norm(ld3(xk, i)));
@@ -295,8 +302,7 @@ __global__ void __launch_bounds__(kPsThreads, 1) k_contact_phase(const __grid_co
   if (!(c.nc > 0 && c.nof > 0)) return;  // uniform, before any barrier
   ct_put_max(e, ws, partial + cta);
   if (!bar.sync()) return;
-  double* buf[2] = {xk, c.xn1};
-  int ori = 0, nxt = 0;  // the buffers of ori_x and x_n1
+  int ori = 0, nxt = 0;  // the buffers of ori_x and x_n1 (xk, c.xn1)
   int mode = 0, pass = 0, it = 0, bodies = 0, comp = 0, src = 0, ndet = 0;
   const int cap = c.max_passes * (c.K + 2) + 2;
   for (;;) {
@@ -305,7 +311,7 @@ __global__ void __launch_bounds__(kPsThreads, 1) k_contact_phase(const __grid_co
       // the hits' flags alternate, so clearing one never races with reading the other
       int* flag = c.state + ((ndet & 1) ? CS_FANY1 : CS_FANY0);
       for (int a = wid; a < c.nc; a += nw)
-        if (ct_detect(c, a, xt, buf[ori], (int*)stage, status) && lane == 0) atomicOr(flag, 1);
+        if (ct_detect(c, a, xt, ori ? c.xn1 : xk, (int*)stage, status) && lane == 0) atomicOr(flag, 1);
       if (!bar.sync()) return;
       const bool any = *(volatile int*)flag != 0;
       if (lead) c.state[(ndet & 1) ? CS_FANY0 : CS_FANY1] = 0;  // the other word: read a barrier ago
@@ -320,21 +326,20 @@ __global__ void __launch_bounds__(kPsThreads, 1) k_contact_phase(const __grid_co
       pass += 1;
     }
     // one Jacobi iteration (k_contact_prep, k_local, k_contact_rhs, k_contact_ctl_iter)
-    const int rk = rec_index_at(c, comp);
+    const int rk = rec_on && rec_base + comp < c.rec_cap ? rec_base + comp : -1;
     ori = nxt;
     src = comp;
-    if (ct_max(partial, nc) < kConvergenceEps) {
+    if (ct_max(partial, nc, ws) < kConvergenceEps) {
       mode = 0;  // back to detection
     } else {
-      const double* x = buf[ori];
-      double* xn = buf[1 - ori];
+      const double* x = ori ? c.xn1 : xk;
+      double* xn = ori ? xk : c.xn1;
       for (int base = 0; base < d.T; base += kPsPair * nc) {
-        const int t = base + 32 * ((warp & (kPsWarps / 2 - 1)) * nc + cta) + lane;
-        double G[4][3];
-        Vec3<double> P[3];
-        if (t < d.T) ct_tet_give(d, t, x, rot, dyn, me, G, P);
+        const int t = base + t0;
+        CtTet T;
+        if (t < d.T) ct_tet_give(d, t, base == 0 ? tv0 : d.tv[t], x, rot, dyn, me, T);
         __syncthreads();
-        if (t < d.T) ct_tet_take(d, t, rot, dyn, me, G, P, slot);
+        if (t < d.T) ct_tet_take(rot, dyn, me, T, slot);
         if (base + kPsPair * nc < d.T) __syncthreads();
       }
       for (int t = nthr - 32 * (wid + 1) + lane; t < d.M + d.S + d.B; t += nthr) local_rest(d, t, x, act_row, slot);
@@ -345,13 +350,15 @@ __global__ void __launch_bounds__(kPsThreads, 1) k_contact_phase(const __grid_co
         const int i = b + (lane >> 3), ii = min(i, d.N - 1), l = lane & 7;
         const bool on = i < d.N;
         const int a = on ? c.cidx[ii] : -1, cnt = a >= 0 ? c.imp_cnt[a] : 0;
-        const Vec3<double> xi = ld3(x, ii), xti = ld3(xt, ii);
-        Vec3<double> nrm = mk3(0.0, 0.0, 0.0);
+        const int k0 = d.vslot_ptr[ii], k1 = on ? d.vslot_ptr[ii + 1] : 0, h0 = d.hs_ptr[ii], h1 = on ? d.hs_ptr[ii + 1] : 0;
+        const Vec3<double> xi = ld3(x, ii), xti = ld3(xt, ii), vwc = ld3(c.vwc, ii), lxt = ld3(c.lxt, ii);
+        const Vec3<double> before = ld3(c.prev, ii);
+        const double mass = d.mass[ii], hdiag = c.hdiag[ii];
+        Vec3<double> nrm = mk3(0.0, 0.0, 0.0), jd, cdx;
         if (l < cnt) nrm = ld3(c.imp_n, a * kMaxImpactsPerVertex + l);
-        const Vec3<double> jd = ct_sum_slots(ld3(d.attach_jd, ii), slot, d.vslot_ptr[ii], on ? d.vslot_ptr[ii + 1] : 0, stage);
-        const Vec3<double> cdx = ct_sum_row(d, mk3(0.0, 0.0, 0.0), ii, d.hs_ptr[ii], on ? d.hs_ptr[ii + 1] : 0, x, xt, 1.0, false,
-                                            stage, nullptr);
-        const Vec3<double> rhs = contact_rhs_value(d.mass[ii], ld3(c.vwc, ii), d.h, jd, ld3(c.lxt, ii), cdx);
+        double hii;
+        ct_sums<true, false, false>(d, ii, k0, k1, h0, h1, ld3(d.attach_jd, ii), slot, x, xt, 1.0, stage, jd, cdx, hii);
+        const Vec3<double> rhs = contact_rhs_value(mass, vwc, d.h, jd, lxt, cdx);
         Vec3<double> post = rhs, r = rhs;
         const bool hit = l < cnt && contact_reaction(nrm, rhs, c.mu, &r);
         const unsigned m = (__ballot_sync(0xffffffffu, hit) >> (lane & 24)) & 0xffu;
@@ -360,8 +367,8 @@ __global__ void __launch_bounds__(kPsThreads, 1) k_contact_phase(const __grid_co
                                     __shfl_sync(0xffffffffu, r.z, win, 8));
         if (m) post = rw;
         if (on && l == 0) {
-          const Vec3<double> prev = contact_relax(c.alpha, post, first ? rhs : ld3(c.prev, i));
-          const Vec3<double> xnew = contact_xn1(d.h, c.hdiag[i], prev, xti);
+          const Vec3<double> prev = contact_relax(c.alpha, post, first ? rhs : before);
+          const Vec3<double> xnew = contact_xn1(d.h, hdiag, prev, xti);
           st3(c.prev, i, prev);
           st3(xn, i, xnew);
           e = fmax(e, ct_norm(xnew - xi));
@@ -380,7 +387,7 @@ __global__ void __launch_bounds__(kPsThreads, 1) k_contact_phase(const __grid_co
       ct_put_max(e, ws, partial + cta);
       if (!bar.sync()) return;
       it += 1;
-      if (lead && c.rec_on && *c.rec_on == 1 && *c.rec_base + comp >= c.rec_cap) atomicExch(status, 6);
+      if (lead && rec_on == 1 && rec_base + comp >= c.rec_cap) atomicExch(status, 6);
       comp += 1;
       if (it >= c.K) mode = 0;
     }
@@ -400,14 +407,25 @@ __global__ void __launch_bounds__(kPsThreads, 1) k_contact_phase(const __grid_co
 
 // Reverse sweep: k_cadj_start, the iterations j = top .. 1 (records base + j -
 // 1; contact_adjoint_step's kernels), the diag(Hs) terms of dL/dE and the PD
-// part's cotangent.  yb and a.orib alternate as the iterations' y-bar; slot2:
-// the local step's slots (slot: the VJP's).
+// part's cotangent.  Round j: the constraints' VJP at iteration j's input, and
+// on other warps the frames of iteration j - 1's impacts and the local step at
+// j - 2's input (both need records only); then the vertices, which gather
+// iteration j and reverse the update of j - 1.  yb and a.orib alternate as the
+// iterations' y-bar, slot2 holds the local step's slots of two iterations
+// (slot: the VJP's).
+struct CtFrames {
+  double* slot2;  // 2 x 3 nslots
+  size_t slots3;
+  double* fr;     // nc x 12: W, r of the winning impact (contact_frame)
+  int* hit;       // nc
+};
+
 __global__ void __launch_bounds__(kPsThreads, 1) k_cadj_phase(const __grid_constant__ SceneDev d,
                                                               const __grid_constant__ ContactDev c,
-                                                              const __grid_constant__ ContactAdj a, const double* xt,
-                                                              const double* act_all, const int* step, double* slot, double* slot2,
-                                                              double* gE, double* gnu, double* mg, double* gact, int base,
-                                                              int top, double cv, double* io_a, double* io_b,
+                                                              const __grid_constant__ ContactAdj a, const CtFrames fr,
+                                                              const double* xt, const double* act_all, const int* step,
+                                                              double* slot, double* gE, double* gnu, double* mg, double* gact,
+                                                              int base, int top, double cv, double* io_a, double* io_b,
                                                               unsigned* counter, int* status) {
   extern __shared__ __align__(16) double dyn[];
   GridBarrier bar(counter, status);
@@ -416,54 +434,100 @@ __global__ void __launch_bounds__(kPsThreads, 1) k_cadj_phase(const __grid_const
   const int tid = wid * 32 + lane, nthr = nw * 32;
   const int me = threadIdx.x & (kPsPair - 1);
   const bool rot = warp < kPsWarps / 2;
-  const int hw = warp & (kPsWarps / 2 - 1);
-  const bool vjp = hw < kCtAdjWarps;  // this warp's tets: the VJP of iteration j, or the local step of j - 1
+  const int hw = warp & (kPsWarps / 2 - 1), hq = hw & (kCtAdjWarps - 1);
+  const bool vjp = hw < kCtAdjWarps;  // this warp's tets: the VJP, or the local step
   double* stage = dyn + warp * kCtWarpStage;
-  double* tape = dyn + kPsXch * kPsPair + 32 * (hw & (kCtAdjWarps - 1)) + lane;
+  double* tape = dyn + kCtTape + 32 * hq + lane;
+  const int fw = (rot ? 0 : kCtAdjWarps) + hq;  // a local-step warp's place among them
+  double* fstage = dyn + kCtFrames + fw * kCtWarpStage;
   const size_t n3 = 3 * (size_t)d.N;
   const int st = *step, rest = d.M + d.S + d.B;
   const double* act_row = act_all + (size_t)st * d.nseg;
-  for (int j = top + 1; j >= 1; --j) {
+  const int t0 = 32 * (hq * nc + cta) + lane;
+  const int4 tv0 = t0 < d.T ? d.tv[t0] : make_int4(0, 0, 0, 0);
+  for (int j = top + 2; j >= 1; --j) {
     const double* yb = (j & 1) ? a.yb : a.orib;   // of iteration j
     double* ybn = (j & 1) ? a.orib : a.yb;        // of j - 1
-    {  // constraints: the VJP at iteration j's input (none at top + 1), the local step at j - 1's
-      const bool do_vjp = j <= top, do_loc = j >= 2;
+    {  // constraints
+      const bool do_vjp = j <= top, do_loc = j >= 3;
       const double* x = c.rec_x + ((size_t)base + (do_vjp ? j - 1 : 0)) * n3;
-      const double* xl = c.rec_x + ((size_t)base + (do_loc ? j - 2 : 0)) * n3;
+      const double* xl = c.rec_x + ((size_t)base + (do_loc ? j - 3 : 0)) * n3;
+      double* lslot = fr.slot2 + (j & 1) * fr.slots3;
       const bool run = vjp ? do_vjp : do_loc;
+      if (!vjp && j >= 2 && j <= top + 1) {  // the frames of iteration j - 1
+        const size_t r = (size_t)base + j - 2;
+        const double* ori = c.rec_x + r * n3;
+        const int* rcnt = c.rec_cnt + r * c.nc;
+        const double* rn = c.rec_n + r * c.nc * kMaxImpactsPerVertex * 3;
+        const double* fslot = fr.slot2 + ((j + 1) & 1) * fr.slots3;
+        for (int b = 4 * (fw * nc + cta); b < c.nc; b += 8 * kCtAdjWarps * nc) {
+          const int ac = b + (lane >> 3), l = lane & 7, cnt = ac < c.nc ? rcnt[ac] : 0;
+          if (!__any_sync(0xffffffffu, cnt > 0)) {
+            if (l == 0 && ac < c.nc) fr.hit[ac] = 0;
+            continue;
+          }
+          const int i = c.cverts[min(ac, c.nc - 1)];
+          const bool on = cnt > 0;
+          const int k0 = d.vslot_ptr[i], k1 = on ? d.vslot_ptr[i + 1] : 0, h0 = d.hs_ptr[i], h1 = on ? d.hs_ptr[i + 1] : 0;
+          const Vec3<double> vwc = ld3(c.vwc, i), lxt = ld3(c.lxt, i);
+          const double mass = d.mass[i];
+          Vec3<double> nrm = mk3(0.0, 0.0, 0.0), jd, cdx, W[3];
+          if (l < cnt) nrm = ld3(rn, ac * kMaxImpactsPerVertex + l);
+          double hii, rc[3];
+          ct_sums<true, false, false>(d, i, k0, k1, h0, h1, ld3(d.attach_jd, i), fslot, ori, xt, 1.0, fstage, jd, cdx, hii);
+          const Vec3<double> f = contact_rhs_value(mass, vwc, d.h, jd, lxt, cdx);
+          const bool hit = l < cnt && contact_frame(nrm, f, W, rc);
+          const unsigned m = (__ballot_sync(0xffffffffu, hit) >> (lane & 24)) & 0xffu;
+          if (ac < c.nc) {
+            if (l == 0) fr.hit[ac] = m != 0;
+            if (m && l == 31 - __clz(m)) {
+              double* o = fr.fr + 12 * (size_t)ac;
+#pragma unroll
+              for (int q = 0; q < 3; ++q) {
+                st3(o, q, W[q]);
+                o[9 + q] = rc[q];
+              }
+            }
+          }
+        }
+      }
       for (int b = 0; b < d.T; b += 32 * kCtAdjWarps * nc) {
-        const int t = run ? b + 32 * ((hw & (kCtAdjWarps - 1)) * nc + cta) + lane : d.T;
-        double G[4][3], yv = 0.0;
-        Mat3<double> gF;
+        const int t = run ? b + t0 : d.T;
+        CtTet T;
+        double yv = 0.0;
         if (t < d.T) {
+          const int4 v = b == 0 ? tv0 : d.tv[t];
           if (vjp) {
-            const int4 v = d.tv[t];
             const int vi[4] = {v.x, v.y, v.z, v.w};
             Vec3<double> xv[4], yw[4];
+            Mat3<double> gF;
 #pragma unroll
             for (int q = 0; q < 4; ++q) { xv[q] = ld3(x, vi[q]); yw[q] = ld3(yb, vi[q]); }
-            load_g(d.tinv, d.T, t, G);
-            const Mat3<double> F = deformation_rn(G, xv), Y = deformation_rn(G, yw);
+            load_g(d.tinv, d.T, t, T.G);
+            T.sl = d.tslot[t];
+            const Mat3<double> F = deformation_rn(T.G, xv), Y = deformation_rn(T.G, yw);
             if (rot) {
               double yr;
               corot_adjoint_rotation(F, Y, d.twr[t], yr, gF);
               dyn[18 * kPsPair + me] = yr;
 #pragma unroll
               for (int q = 0; q < 4; ++q) { xv[q] = ld3(x, vi[q]); yw[q] = ld3(yb, vi[q]); }  // again: fewer live registers
-              dyn[19 * kPsPair + me] = contact_yh(G, F, Y, yw, xv, xt, vi);
+              dyn[19 * kPsPair + me] = contact_yh(T.G, F, Y, yw, xv, xt, vi);
             } else {
               corot_adjoint_volume(F, Y, d.twv[t], yv, gF, tape, 32 * kCtAdjWarps);
             }
-            ps_give(dyn, rot, me, gF.c);
+#pragma unroll
+            for (int q = 0; q < 3; ++q) T.P[q] = gF.c[q];
+            ps_give(dyn, rot, me, T.P);
           } else {
-            ct_tet_give(d, t, xl, rot, dyn, me, G, gF.c);
+            ct_tet_give(d, t, v, xl, rot, dyn, me, T);
           }
         }
         __syncthreads();
         if (t < d.T) {
           if (vjp) {
-            ps_take(dyn, rot, me, gF.c);
-            ps_corners(G, gF.c, d.tslot[t], rot, slot);
+            ps_take(dyn, rot, me, T.P);
+            ps_corners(T.G, T.P, T.sl, rot, slot);
             if (!rot) {
               const double yr = dyn[18 * kPsPair + me], yh = dyn[19 * kPsPair + me], E = d.tE[t], nu = d.tnu[t], vol = d.tvol[t];
               const double opn = 1.0 + nu;
@@ -471,7 +535,7 @@ __global__ void __launch_bounds__(kPsThreads, 1) k_cadj_phase(const __grid_const
               gnu[t] += E * vol / (opn * opn) * (yv - yr);
             }
           } else {
-            ct_tet_take(d, t, rot, dyn, me, G, gF.c, slot2);
+            ct_tet_take(rot, dyn, me, T, lslot);
           }
         }
         if (b + 32 * kCtAdjWarps * nc < d.T) __syncthreads();
@@ -480,23 +544,33 @@ __global__ void __launch_bounds__(kPsThreads, 1) k_cadj_phase(const __grid_const
         if (q < rest) {
           if (do_vjp) adj_local_rest(d, q, x, yb, act_row, slot, mg);
         } else if (do_loc) {
-          local_rest(d, q - rest, xl, act_row, slot2);
+          local_rest(d, q - rest, xl, act_row, lslot);
         }
       }
       if (!bar.sync()) return;
     }
-    // vertices: the gather of iteration j (x_n1 bar of j - 1; at top + 1 the phase's own), the rhs VJP of j - 1
+    if (j > top + 1) continue;
+    // vertices: the gather of iteration j (x_n1 bar of j - 1; at top + 1 the phase's own), the reverse of j - 1's update
     const bool gather = j <= top, rhs = j >= 2;
     const size_t r = (size_t)base + (rhs ? j - 2 : 0);
-    const double* ori = c.rec_x + r * n3;
     const double* prev = c.rec_prev + r * n3;
-    const int* rcnt = c.rec_cnt + r * c.nc;
-    const double* rn = c.rec_n + r * c.nc * kMaxImpactsPerVertex * 3;
     const int first = rhs ? c.rec_first[r] : 0;
     for (int b = 4 * wid; b < d.N; b += 4 * nw) {
       const int i = b + (lane >> 3), ii = min(i, d.N - 1), l = lane & 7;
       const bool on = i < d.N;
       Vec3<double> xb;
+      const int ac = rhs ? c.cidx[ii] : -1;
+      const int hit = ac >= 0 ? fr.hit[ac] : 0;
+      Vec3<double> W[3], pv = mk3(0.0, 0.0, 0.0);
+      double rc[3] = {0.0, 0.0, 0.0};
+      if (rhs) pv = ld3(prev, ii);
+      if (hit) {
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+          W[q] = ld3(fr.fr + 12 * (size_t)ac, q);
+          rc[q] = fr.fr[12 * (size_t)ac + 9 + q];
+        }
+      }
       if (!gather) {
         const Vec3<double> gv = ld3(io_b, ii);
         xb = ld3(io_a, ii) + cv * gv;
@@ -507,35 +581,21 @@ __global__ void __launch_bounds__(kPsThreads, 1) k_cadj_phase(const __grid_const
           a.hdb[i] = 0.0;
         }
       } else {
-        const Vec3<double> yi = ld3(yb, ii);
+        const int k0 = d.vslot_ptr[ii], k1 = on ? d.vslot_ptr[ii + 1] : 0, h0 = d.hs_ptr[ii], h1 = on ? d.hs_ptr[ii + 1] : 0;
+        const Vec3<double> yi = ld3(yb, ii), xtb = ld3(a.cxtb, ii);
+        const double mass = d.mass[ii];
         double hii;
-        xb = ct_sum_slots(mk3(0.0, 0.0, 0.0), slot, d.vslot_ptr[ii], on ? d.vslot_ptr[ii + 1] : 0, stage);
-        xb = ct_sum_row(d, xb, ii, d.hs_ptr[ii], on ? d.hs_ptr[ii + 1] : 0, yb, nullptr, -1.0, false, stage, &hii);
-        if (on && l == 0) st3(a.cxtb, i, rn_axpy(d.mass[i] / (d.h * d.h) - hii, yi, ld3(a.cxtb, i)));
+        Vec3<double> none;
+        ct_sums<false, true, false>(d, ii, k0, k1, h0, h1, mk3(0.0, 0.0, 0.0), slot, yb, yb, -1.0, stage, none, xb, hii);
+        if (on && l == 0) st3(a.cxtb, i, rn_axpy(mass / (d.h * d.h) - hii, yi, xtb));
       }
-      __syncwarp();
-      if (rhs) {
-        const int ac = on ? c.cidx[ii] : -1, cnt = ac >= 0 ? rcnt[ac] : 0;
-        Vec3<double> W[3];
-        double rc[3];
-        int win = 0;
-        bool hit = false;
-        if (__any_sync(0xffffffffu, cnt > 0)) {
-          Vec3<double> nrm = mk3(0.0, 0.0, 0.0);
-          if (l < cnt) nrm = ld3(rn, ac * kMaxImpactsPerVertex + l);
-          const bool need = cnt > 0;
-          const Vec3<double> jd = ct_sum_slots(ld3(d.attach_jd, ii), slot2, d.vslot_ptr[ii], need ? d.vslot_ptr[ii + 1] : 0, stage);
-          const Vec3<double> cdx = ct_sum_row(d, mk3(0.0, 0.0, 0.0), ii, d.hs_ptr[ii], need ? d.hs_ptr[ii + 1] : 0, ori, xt, 1.0,
-                                              false, stage, nullptr);
-          const Vec3<double> f = contact_rhs_value(d.mass[ii], ld3(c.vwc, ii), d.h, jd, ld3(c.lxt, ii), cdx);
-          hit = l < cnt && contact_frame(nrm, f, W, rc);
-          const unsigned m = (__ballot_sync(0xffffffffu, hit) >> (lane & 24)) & 0xffu;
-          win = m ? 31 - __clz(m) : 0;
+      if (on && l == 0) {
+        if (rhs) {
+          cadj_rhs_finish(d, c, a, i, xb, pv, first, hit != 0, W, rc, ybn);
+        } else {  // k_cadj_to_pd
+          st3(io_a, i, xb);
+          st3(io_b, i, mk3(0.0, 0.0, 0.0));
         }
-        if (on && l == win) cadj_rhs_finish(d, c, a, i, xb, ld3(prev, i), first, hit, W, rc, ybn);
-      } else if (on && l == 0) {  // k_cadj_to_pd
-        st3(io_a, i, xb);
-        st3(io_b, i, mk3(0.0, 0.0, 0.0));
       }
       __syncwarp();
     }

@@ -254,7 +254,8 @@ struct dfem_scene {
   int gather_form = 0;                   // dfem_set_option(DFEM_OPTION_GATHER): 0 by size, 1 warp, 2 thread
   int fused_grid = 0;                    // CTAs of k_contact_phase (all resident)
   int cadj_grid = 0;                     // CTAs of k_cadj_phase (all resident)
-  DBuf<double> fpartial, ca_slot;
+  DBuf<double> fpartial, ca_slot, ca_frame;  // (k_cadj_phase: CtFrames)
+  DBuf<int> ca_hit;
   DBuf<unsigned> cbar;                   // the two kernels' barrier counters
   DBuf<double> obs_x, hdiag, imp_n, xn1, xold, cprev, lxt, vwc;
   // soft-soft contact (forward only: the adjoint refuses these scenes)
@@ -2217,7 +2218,11 @@ static int ensure_contact_record(dfem_scene* sc, int cap, int keep = 0) {
   for (DBuf<double>* b : {&sc->ca_xn1b, &sc->ca_pb, &sc->ca_cxtb, &sc->ca_vwcb, &sc->ca_yb, &sc->ca_orib})
     if (!b->p) CK(b->alloc(n3));
   if (!sc->ca_hdb.p) CK(sc->ca_hdb.alloc(std::max(1, s.N)));
-  if (sc->cbar.p && !sc->ca_slot.p) CK(sc->ca_slot.alloc(3 * (size_t)std::max(1, s.nslots)));
+  if (sc->cbar.p) {
+    if (!sc->ca_slot.p) CK(sc->ca_slot.alloc(6 * (size_t)std::max(1, s.nslots)));
+    if (!sc->ca_frame.p) CK(sc->ca_frame.alloc(12 * nc));
+    if (!sc->ca_hit.p) CK(sc->ca_hit.alloc(nc));
+  }
   if (sc->self_contact) {
     const int ncf = sc->cd.ncf;
     for (DBuf<double>* b : {&sc->ca_scb, &sc->ca_ptot, &sc->ca_sbp, &sc->ca_gPM})
@@ -2387,8 +2392,9 @@ static int contact_adjoint_step(dfem_scene* sc, int st, bool recorded, int rbase
   }
   if (!sc->self_contact && fused_contact(sc)) {  // the whole reverse sweep in one cooperative launch
     const ContactAdj a = make_cadj(sc);
-    CK(launch_coop(sc->stream, k_cadj_phase, sc->cadj_grid, kPsThreads, kCtSmemAdj, sc->sd, sc->cd, a, xt,
-                   (const double*)sc->act_all.p, (const int*)sc->step.p, sc->slot.p, sc->ca_slot.p, sc->gE.p, sc->gnu.p,
+    const CtFrames fr{sc->ca_slot.p, 3 * (size_t)std::max(1, s.nslots), sc->ca_frame.p, sc->ca_hit.p};
+    CK(launch_coop(sc->stream, k_cadj_phase, sc->cadj_grid, kPsThreads, kCtSmemAdj, sc->sd, sc->cd, a, fr, xt,
+                   (const double*)sc->act_all.p, (const int*)sc->step.p, sc->slot.p, sc->gE.p, sc->gnu.p,
                    sc->mg.p, sc->gact.p, base, src, s.damping / s.h, sc->io_a.p, sc->io_b.p, sc->cbar.p, sc->status.p));
     sc->launches += 1;
     return DFEM_OK;

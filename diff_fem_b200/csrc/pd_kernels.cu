@@ -228,7 +228,19 @@ __device__ __forceinline__ void local_rest(const SceneDev& d, int t, const doubl
     // bending (BendingConstraint::EvaluateDVector): d = w * lap * rest/|lap|, J = w beta
     int o0 = d.boff[t], o1 = d.boff[t + 1];
     Vec3<double> lap = mk3(0.0, 0.0, 0.0);
-    for (int k = o0; k < o1; ++k) lap = lap + d.bbeta[k] * ld3(x, d.bv[k]);
+    for (int k0 = o0; k0 < o1; k0 += 8) {  // a stencil's reads in flight together, its sum in order
+      const int m = min(8, o1 - k0);
+      double be[8];
+      Vec3<double> xv[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        be[u] = u < m ? d.bbeta[k0 + u] : 0.0;
+        xv[u] = u < m ? ld3(x, d.bv[k0 + u]) : mk3(0.0, 0.0, 0.0);
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (u < m) lap = rn_axpy(be[u], xv[u], lap);
+    }
     double ln = sqrt(dot3(lap, lap));
     double w = d.bw[t];
     Vec3<double> dd = mk3(0.0, 0.0, 0.0);
@@ -1298,9 +1310,23 @@ __device__ __forceinline__ void adj_local_rest(const SceneDev& d, int t, const d
     int o0 = d.boff[t], o1 = d.boff[t + 1];
     double w = d.bw[t];
     Vec3<double> db = mk3(0.0, 0.0, 0.0), lap = mk3(0.0, 0.0, 0.0);
-    for (int q = o0; q < o1; ++q) {
-      db = db + (w * d.bbeta[q]) * ld3(yb, d.bv[q]);
-      lap = lap + d.bbeta[q] * ld3(x, d.bv[q]);
+    for (int q0 = o0; q0 < o1; q0 += 4) {
+      const int m = min(4, o1 - q0);
+      double be[4];
+      Vec3<double> xv[4], yv[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int v = u < m ? d.bv[q0 + u] : 0;
+        be[u] = u < m ? d.bbeta[q0 + u] : 0.0;
+        xv[u] = u < m ? ld3(x, v) : mk3(0.0, 0.0, 0.0);
+        yv[u] = u < m ? ld3(yb, v) : mk3(0.0, 0.0, 0.0);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (u < m) {
+          db = rn_axpy(__dmul_rn(w, be[u]), yv[u], db);
+          lap = rn_axpy(be[u], xv[u], lap);
+        }
     }
     double ln = sqrt(dot3(lap, lap));
     Vec3<double> gl = mk3(0.0, 0.0, 0.0);

@@ -404,7 +404,9 @@ __device__ __forceinline__ void ps_local(const SceneDev& d, const double* x, con
     const int t = base + 32 * ((warp & (kPsWarps / 2 - 1)) * nc + BAR::cta()) + lane;
     double G[4][3];
     Vec3<double> P[3];  // this half's part of wr md + wv md_volume
+    int4 sl;
     if (t < d.T) {
+      sl = d.tslot[t];
       const int4 v = base == 0 ? tv0 : d.tv[t];
       const Vec3<double> xv[4] = {ld3(x, v.x), ld3(x, v.y), ld3(x, v.z), ld3(x, v.w)};
       load_g(d.tinv, d.T, t, G);
@@ -420,7 +422,7 @@ __device__ __forceinline__ void ps_local(const SceneDev& d, const double* x, con
     __syncthreads();
     if (t < d.T) {  // two corners each
       ps_take(xch, rot, me, P);
-      ps_corners(G, P, d.tslot[t], rot, slot);
+      ps_corners(G, P, sl, rot, slot);
     }
     if (base + kPsPair * nc < d.T) __syncthreads();
   }
@@ -441,7 +443,9 @@ __device__ __forceinline__ void ps_adj_local(const SceneDev& d, const double* x,
     const int t = half < tape_warps ? base + 32 * (half * nc + BAR::cta()) + lane : d.T;
     double G[4][3], yv = 0.0;
     Mat3<double> gF;
+    int4 sl;
     if (t < d.T) {
+      sl = d.tslot[t];
       const int4 v = base == 0 ? tv0 : d.tv[t];
       const int vi[4] = {v.x, v.y, v.z, v.w};
       Vec3<double> xv[4], yw[4];
@@ -468,7 +472,7 @@ __device__ __forceinline__ void ps_adj_local(const SceneDev& d, const double* x,
     __syncthreads();
     if (t < d.T) {
       ps_take(xch, rot, me, gF.c);
-      ps_corners(G, gF.c, d.tslot[t], rot, slot);
+      ps_corners(G, gF.c, sl, rot, slot);
       if (!rot) {
         const double yr = xch[18 * kPsPair + me], yh = xch[19 * kPsPair + me], E = d.tE[t], nu = d.tnu[t], vol = d.tvol[t];
         const double opn = 1.0 + nu;
