@@ -134,7 +134,7 @@ struct dfem_scene {
   // factor
   DBuf<int> rseg_ptr, cdst, sn_c0, sn_w, sn_r, sn_rofs, rowidx, sn_lofs, sn_dofs, lvl_sn;
   DBuf<double> contrib, Lcm, Dinv, DinvC;
-  DBuf<SnInfo> sn_info;
+  DBuf<SnInfo> sn_info, sn_info_p;  // (sn_info_p: the persistent form's staging)
   std::vector<int> lvl_ptr;
   // Launch segments of the level-kernel solve: every level of the elimination
   // tree, split into its small supernodes (one warp each, eight per CTA) and
@@ -149,7 +149,7 @@ struct dfem_scene {
   };
   std::vector<LevelSeg> segs;
   // persistent solve (one launch per solve) and the autotuned choice between it and the level kernels
-  DBuf<int> sn_parent, sn_pos, kid_ptr, kid, done_f, done_b, solve_ctl;
+  DBuf<int> sn_pos, kid, done_f, done_b, solve_ctl;
   size_t shm_pers = 0;
   int pers_slots = 1;                    // CTAs of the persistent solve resident at once
   // The solve runs levels 0 .. solve_cut-1 as level kernels and the rest in
@@ -502,14 +502,76 @@ static int upload_factor(dfem_scene* sc) {
   if (sc->hs.nparts > 1)
     for (int q = 0; q < ns; ++q)
       snp[q] = (int)(std::upper_bound(sc->hs.part_v0.begin(), sc->hs.part_v0.end(), F.sn_c0[q]) - sc->hs.part_v0.begin()) - 1;
+  std::vector<int> kp(ns + 1, 0);  // children CSR
+  for (int q = 0; q < ns; ++q)
+    if (F.sn_parent[q] >= 0) kp[F.sn_parent[q] + 1]++;
+  for (int q = 0; q < ns; ++q) kp[q + 1] += kp[q];
   {
     std::vector<SnInfo> info(std::max(1, ns));
     for (int k = 0; k < ns; ++k) {
       const int q = F.lvl_sn[k];
       info[k] = SnInfo{F.sn_c0[q], F.sn_w[q], F.sn_r[q], (int)F.sn_rofs[q], (int)F.sn_lofs[q], (int)F.sn_dofs[q],
-                       F.rseg_ptr[F.sn_c0[q]], nseg[q], q, snp[q], stage[q], chunk[q]};
+                       F.rseg_ptr[F.sn_c0[q]], nseg[q], q, snp[q], stage[q], chunk[q],
+                       F.sn_parent[q], kp[q], kp[q + 1]};
     }
     CK(sc->sn_info.upload(info));
+    // The persistent form's own staging: a batch has many small supernodes,
+    // which bound its solve by items in flight, so two CTAs share an SM when
+    // every diagonal block fits half of it (larger L_{R,s} are streamed); a
+    // single scene's chain of large ones keeps the whole.  24 scenes of
+    // 2,000-12,000 tets, per solve: 0.181 -> 0.148 ms; three per SM would stream
+    // most blocks, 0.185 ms; a single 12,800-tet beam 0.102 -> 0.114 ms.
+    const size_t half = (228 * 1024 / 2 - 1024 - 256) & ~size_t(15);
+    size_t pb = sc->hs.nparts > 1 ? half : budget;
+    for (int q = 0; q < ns && pb == half; ++q) {
+      size_t uf, ub;
+      solve_shm_doubles(F.sn_w[q], F.sn_r[q], nseg[q], false, 0, &uf, &ub);
+      if (8 * std::max(uf, ub) > half) pb = budget;
+    }
+    size_t mp = 0;
+    for (int k = 0; k < ns; ++k) {
+      SnInfo& in = info[k];
+      size_t uf, ub, tf, tb;
+      solve_shm_doubles(in.w, in.r, in.nseg, false, 0, &uf, &ub);
+      solve_shm_doubles(in.w, in.r, in.nseg, true, 0, &tf, &tb);
+      const size_t u = std::max(uf, ub), t = std::max(tf, tb);
+      in.stage = in.r > 0 && 8 * t <= pb;
+      in.cc = 0;
+      size_t nd = in.stage ? t : u;
+      if (!in.stage && in.r > 0 && 8 * u < pb) {
+        const size_t cc = std::min<size_t>(((pb / 8 - u) / (2 * (size_t)in.r)) & ~size_t(1), (size_t)in.w);
+        if (cc >= 2) {
+          in.cc = (int)cc;
+          nd = u + 2 * cc * (size_t)in.r;
+        }
+      }
+      mp = std::max(mp, 8 * nd);
+    }
+    sc->shm_pers = mp;
+    // Items of the whole solve in the order of the longest path of work that
+    // waits for them (a topological order: a child's path holds its parent's).
+    // By level, the long chains started behind every leaf: the same 24 scenes
+    // 0.134 -> 0.121 ms per solve, a single scene's time the same.
+    auto cost = [&](int q) { return 5.0 + 0.05 * F.sn_w[q] + 0.004 * nseg[q]; };  // us of an item and its hand-over
+    std::vector<double> up(ns), down(ns, 0.0);
+    for (int k = ns - 1; k >= 0; --k) {
+      const int q = F.lvl_sn[k], p = F.sn_parent[q];
+      up[q] = cost(q) + (p >= 0 ? up[p] : 0.0);
+    }
+    for (int k = 0; k < ns; ++k) {
+      const int q = F.lvl_sn[k], p = F.sn_parent[q];
+      down[q] += cost(q);
+      if (p >= 0) down[p] = std::max(down[p], down[q]);
+    }
+    std::vector<int> ord(ns);
+    info.resize(std::max(1, 3 * ns));
+    for (int dir = 0; dir < 2; ++dir) {
+      const std::vector<double>& key = dir == 0 ? up : down;
+      for (int k = 0; k < ns; ++k) ord[k] = dir == 0 ? k : ns - 1 - k;
+      std::stable_sort(ord.begin(), ord.end(), [&](int a, int b) { return key[F.lvl_sn[a]] > key[F.lvl_sn[b]]; });
+      for (int k = 0; k < ns; ++k) info[(size_t)(1 + dir) * ns + k] = info[ord[k]];
+    }
+    CK(sc->sn_info_p.upload(info));
   }
   for (auto fn : {(const void*)k_fwd_level<CtaGroup>, (const void*)k_bwd_level<CtaGroup>})
     CK(raise_smem_limit(fn, max_cta_blk));
@@ -517,22 +579,16 @@ static int upload_factor(dfem_scene* sc) {
     CK(raise_smem_limit(fn, max_warp_blk));
   // persistent solve: elimination tree (children CSR), completion stamps, control words
   {
-    std::vector<int> kp(ns + 1, 0), kd(std::max(1, ns));
-    for (int q = 0; q < ns; ++q)
-      if (F.sn_parent[q] >= 0) kp[F.sn_parent[q] + 1]++;
-    for (int q = 0; q < ns; ++q) kp[q + 1] += kp[q];
+    std::vector<int> kd(std::max(1, ns));
     std::vector<int> fill(kp.begin(), kp.end() - 1);
     for (int q = 0; q < ns; ++q)
       if (F.sn_parent[q] >= 0) kd[fill[F.sn_parent[q]]++] = q;
-    CK(sc->sn_parent.upload(F.sn_parent));
-    CK(sc->kid_ptr.upload(kp));
     CK(sc->kid.upload(kd));
     if (sc->done_f.n != (size_t)ns || !sc->done_f.p) {
       CK(sc->done_f.alloc(std::max(1, ns)));
       CK(sc->done_b.alloc(std::max(1, ns)));
       CK(sc->solve_ctl.alloc(4));
     }
-    sc->shm_pers = max_cta;
     CK(raise_smem_limit((const void*)k_solve_persistent, sc->shm_pers));
     int nsm = 1, per_sm = 0;
     CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, sc->device));
@@ -546,8 +602,8 @@ static int upload_factor(dfem_scene* sc) {
     CK(sc->sn_pos.upload(pos));
   }
   RC(plan_resident(sc, nseg, cdst));
-  FactorDev fd{sc->sn_info.p, sc->rseg_ptr.p, sc->cdst.p, sc->contrib.p, sc->rowidx.p, sc->Lcm.p, sc->Dinv.p,
-               sc->DinvC.p, sc->status.p, ns, sc->sn_pos.p, sc->sn_parent.p, sc->kid_ptr.p, sc->kid.p, sc->done_f.p,
+  FactorDev fd{sc->sn_info.p, sc->sn_info_p.p, sc->rseg_ptr.p, sc->cdst.p, sc->contrib.p, sc->rowidx.p, sc->Lcm.p, sc->Dinv.p,
+               sc->DinvC.p, sc->status.p, ns, sc->sn_pos.p, sc->kid.p, sc->done_f.p,
                sc->done_b.p, sc->solve_ctl.p, sc->spin_tries};
   if (std::memcmp(&fd, &sc->fd, sizeof(fd)) != 0) invalidate_graphs(sc);
   sc->fd = fd;

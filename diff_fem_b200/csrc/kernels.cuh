@@ -246,10 +246,15 @@ struct SnInfo {
   int part;       // batch part
   int stage;      // 1: L_{R,s} is staged in shared memory too
   int cc;         // not staged: columns per chunk of L_{R,s} streamed through two shared buffers (0: read from global)
+  int parent;      // elimination tree: the parent (-1: a root), the children f.kid[kid0 .. kid1)
+  int kid0, kid1;
 };
 
 struct FactorDev {
   const SnInfo* info;    // level order
+  // the persistent solve's (its own stage, cc): level order, then the whole
+  // solve's items (forward, backward) by the longest path of work after them
+  const SnInfo* info_p;
   const int* rseg_ptr;   // row -> its contributions: contrib[3 rseg_ptr[i] .. 3 rseg_ptr[i+1]) in a fixed order
   const int* cdst;       // below-diagonal row position (rowidx order) -> its contribution slot
   double* contrib;       // 3 doubles per below-diagonal row of every supernode, grouped by destination row
@@ -261,8 +266,6 @@ struct FactorDev {
   // persistent solve: elimination tree, completion stamps, control words
   int nsuper;
   const int* sn_pos;     // supernode -> its level-order position
-  const int* sn_parent;
-  const int* kid_ptr;
   const int* kid;
   int* done_f;
   int* done_b;

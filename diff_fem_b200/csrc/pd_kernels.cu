@@ -722,31 +722,41 @@ __device__ __forceinline__ bool fwd_supernode(const FactorDev& f, const SnInfo& 
   for (int c = rk; c <= w; c += gs) psh[c] = f.rseg_ptr[c0 + c] - in.seg0;
   for (int k = rk; k < 3 * w; k += gs) tsh[k] = rhs[3 * (size_t)c0 + k];
   G::sync();
-  for (int c = rk; c < w; c += gs) {
-    double a0 = tsh[3 * c], a1 = tsh[3 * c + 1], a2 = tsh[3 * c + 2];
-    for (int k = psh[c]; k < psh[c + 1]; ++k) { a0 -= qsh[3 * k]; a1 -= qsh[3 * k + 1]; a2 -= qsh[3 * k + 2]; }
-    tsh[3 * c] = a0; tsh[3 * c + 1] = a1; tsh[3 * c + 2] = a2;
+  for (int e = rk; e < 3 * w; e += gs) {  // a thread per row and component
+    const int c = e / 3, j = e - 3 * c;
+    double a = tsh[e];
+#pragma unroll 4
+    for (int k = psh[c]; k < psh[c + 1]; ++k) a -= qsh[3 * k + j];
+    tsh[e] = a;
   }
   if (!stage_blocks_wait<G>(f, bar, phase, in.s, 1)) {
     drain_chunks<G>(in, sbar, sph);
     return false;
   }
-  // column-major Dinv: the threads of a warp read consecutive words
-  for (int c = rk; c < w; c += gs) {
-    double a0 = 0, a1 = 0, a2 = 0;
-#pragma unroll 4
-    for (int k = 0; k <= c; ++k) {
-      const double dv = Dsh[k * w + c];
-      a0 += dv * tsh[3 * k]; a1 += dv * tsh[3 * k + 1]; a2 += dv * tsh[3 * k + 2];
-    }
-    ysh[3 * c] = a0; ysh[3 * c + 1] = a1; ysh[3 * c + 2] = a2;
-    double* yo = y + 3 * (size_t)(c0 + c);
-    yo[0] = a0; yo[1] = a1; yo[2] = a2;
+  // column-major Dinv: the threads of a warp read consecutive words; a
+  // component per thread (a row's sum is one chain of dependent operations)
+  for (int e = rk; e < 3 * w; e += gs) {
+    const int j = e / w, c = e - j * w;
+    double a = 0;
+#pragma unroll 8
+    for (int k = 0; k <= c; ++k) a += Dsh[k * w + c] * tsh[3 * k + j];
+    ysh[3 * c + j] = a;
+    y[3 * (size_t)(c0 + c) + j] = a;
   }
   G::sync();
   if (streamed<G>(in)) return fwd_panel_stream<G>(f, in, Lsh, sbar, sph, ysh);
-  const double* Lc = in.stage ? Lsh : f.Lcm + in.lofs;
   const int* dst = f.cdst + in.rofs;
+  if (in.stage) {
+    for (int e = rk; e < 3 * r; e += gs) {
+      const int j = e / r, a = e - j * r, d = dst[a];
+      double s = 0;
+#pragma unroll 8
+      for (int c = 0; c < w; ++c) s += Lsh[c * r + a] * ysh[3 * c + j];
+      f.contrib[3 * (size_t)d + j] = s;
+    }
+    return true;
+  }
+  const double* Lc = f.Lcm + in.lofs;
   for (int a = rk; a < r; a += gs) {
     const int d = dst[a];
     double a0 = 0, a1 = 0, a2 = 0;
@@ -777,7 +787,7 @@ __device__ __forceinline__ bool fwd_supernode(const FactorDev& f, const SnInfo& 
 template <class G>
 __device__ __forceinline__ bool bwd_supernode(const FactorDev& f, const SnInfo& in, double* y, double* sh,
                                               uint64_t* bar, unsigned phase, uint64_t* sbar, unsigned* sph,
-                                              bool issued) {
+                                              bool issued, int row0 = -1) {
   const int c0 = in.c0, w = in.w, r = in.r;
   const int* R = f.rowidx + in.rofs;
   double* Dsh = sh;
@@ -787,7 +797,7 @@ __device__ __forceinline__ bool bwd_supernode(const FactorDev& f, const SnInfo& 
   if (!issued) stage_blocks_issue<G>(f, in, false, Dsh, Lsh, bar, sbar);
   const int rk = G::rank(), gs = G::size();
   for (int a = rk; a < r; a += gs) {
-    const double* q = y + 3 * (size_t)R[a];
+    const double* q = y + 3 * (size_t)(a == rk && row0 >= 0 ? row0 : R[a]);
     xr[3 * a] = __ldcg(q); xr[3 * a + 1] = __ldcg(q + 1); xr[3 * a + 2] = __ldcg(q + 2);
   }
   for (int k = rk; k < 3 * w; k += gs) tsh[k] = __ldcg(y + 3 * (size_t)c0 + k);
@@ -840,15 +850,12 @@ __device__ __forceinline__ bool bwd_supernode(const FactorDev& f, const SnInfo& 
     }
   }
   G::sync();
-  for (int c = rk; c < w; c += gs) {
-    double a0 = 0, a1 = 0, a2 = 0;
-#pragma unroll 4
-    for (int k = c; k < w; ++k) {
-      const double dv = Dsh[k * w + c];
-      a0 += dv * tsh[3 * k]; a1 += dv * tsh[3 * k + 1]; a2 += dv * tsh[3 * k + 2];
-    }
-    double* yo = y + 3 * (size_t)(c0 + c);
-    yo[0] = a0; yo[1] = a1; yo[2] = a2;
+  for (int e = rk; e < 3 * w; e += gs) {  // a thread per column and component
+    const int j = e / w, c = e - j * w;
+    double a = 0;
+#pragma unroll 8
+    for (int k = c; k < w; ++k) a += Dsh[k * w + c] * tsh[3 * k + j];
+    y[3 * (size_t)(c0 + c) + j] = a;
   }
   return true;
 }
@@ -895,7 +902,13 @@ __global__ void __launch_bounds__(256) k_bwd_level(FactorDev f, int lvl_begin, i
 // whole solve.  The CTAs claim work items from a ticket counter: with
 // n = ns - p0, tickets 0 .. n-1 are the forward solves of those supernodes in
 // level order (leaves first), tickets n .. 2n-1 the backward solves in
-// reverse level order (roots first).  A CTA claims its next ticket while it
+// reverse level order (roots first); for p0 = 0 both in the order of the work
+// that waits for them (upload_factor).  What bounds it is the hand-over from
+// item to item, 4-9 us each (a stamp, its poll, the reads that follow it) on
+// the largest scene's chain, and with it the items in flight: a lane per child
+// polls, an item's record holds its parent and children, and a row's sum runs
+// on a thread per component (24 scenes: 0.148 -> 0.134 ms per solve together).
+// A CTA claims its next ticket while it
 // solves the current one (the claim's round trip overlaps the work).  It
 // starts the claimed item's (read-only) block copies, then waits until the
 // supernodes the item reads are done — forward: its children in the
@@ -936,6 +949,28 @@ __device__ __forceinline__ bool wait_epoch(const int* flag, int epoch, const int
   return false;
 }
 
+// Completion wait of a supernode's dependencies by a warp (a lane per child);
+// false, in all its lanes, when one gave up.
+__device__ __forceinline__ bool wait_dependencies(const FactorDev& f, const SnInfo& in, bool fwd, int p0, int epoch) {
+  const int lane = threadIdx.x & 31;
+  bool ok = true;
+  int* ctl = f.ctl;
+  if (fwd) {
+    for (int k = in.kid0 + lane; ok && k < in.kid1; k += 32) {
+      const int kid = f.kid[k];
+      if (p0 == 0 || f.sn_pos[kid] >= p0) ok = wait_epoch(f.done_f + kid, epoch, ctl + 3, f.spin_tries);
+    }
+  } else if (lane == 0) {
+    ok = wait_epoch(in.parent >= 0 ? f.done_b + in.parent : f.done_f + in.s, epoch, ctl + 3, f.spin_tries);
+  }
+  ok = __all_sync(0xffffffffu, ok) != 0;
+  if (!ok && lane == 0) {
+    if (ld_acquire(ctl + 3) == 0) record_gave_up(f, in.s, fwd ? 3 : 4);
+    atomicExch(ctl + 3, 1);
+  }
+  return ok;
+}
+
 __global__ void __launch_bounds__(256) k_solve_persistent(FactorDev f, int p0, Gate gate,
                                                           const double* __restrict__ rhs, double* y) {
   extern __shared__ __align__(16) double sh[];
@@ -967,27 +1002,16 @@ __global__ void __launch_bounds__(256) k_solve_persistent(FactorDev f, int p0, G
     if (!s_go) break;
     const int t = s_ticket;
     const bool fwd = t < n;
-    const SnInfo in = f.info[fwd ? p0 + t : p0 + 2 * n - 1 - t];
+    const SnInfo in = f.info_p[p0 == 0 ? n + t : fwd ? p0 + t : p0 + 2 * n - 1 - t];
     const int s = in.s;
     if (!gate.skip(in.part)) {
       // the factor blocks are read-only: start their copies before waiting on the dependencies
       stage_blocks_issue<CtaGroup>(f, in, fwd, sh, sh + even_count(in.w * in.w), &bar, sbar);
-      if (threadIdx.x == 0) {
-        bool ok = true;
-        if (fwd) {
-          for (int k = f.kid_ptr[s]; ok && k < f.kid_ptr[s + 1]; ++k) {
-            const int kid = f.kid[k];
-            if (f.sn_pos[kid] >= p0) ok = wait_epoch(f.done_f + kid, epoch, ctl + 3, f.spin_tries);
-          }
-        } else {
-          const int p = f.sn_parent[s];
-          ok = wait_epoch(p >= 0 ? f.done_b + p : f.done_f + s, epoch, ctl + 3, f.spin_tries);
-        }
-        if (!ok) {
-          if (ld_acquire(ctl + 3) == 0) record_gave_up(f, s, fwd ? 3 : 4);
-          atomicExch(ctl + 3, 1);
-        }
-        s_go = ok ? 1 : 0;
+      // ... and so is the row whose solution this thread gathers first
+      const int row0 = !fwd && (int)threadIdx.x < in.r ? f.rowidx[in.rofs + threadIdx.x] : -1;
+      if (threadIdx.x < 32) {
+        const bool ok = wait_dependencies(f, in, fwd, p0, epoch);
+        if (threadIdx.x == 0) s_go = ok ? 1 : 0;
       }
       __syncthreads();
       if (!s_go) {  // aborted: let this CTA's copies land before it leaves
@@ -996,7 +1020,7 @@ __global__ void __launch_bounds__(256) k_solve_persistent(FactorDev f, int p0, G
         break;
       }
       const bool ok = fwd ? fwd_supernode<CtaGroup>(f, in, rhs, y, sh, &bar, phase, sbar, sph, true)
-                          : bwd_supernode<CtaGroup>(f, in, y, sh, &bar, phase, sbar, sph, true);
+                          : bwd_supernode<CtaGroup>(f, in, y, sh, &bar, phase, sbar, sph, true, row0);
       phase ^= 1u;
       if (!ok) {
         if (threadIdx.x == 0) atomicExch(ctl + 3, 1);
