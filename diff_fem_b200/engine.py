@@ -240,9 +240,9 @@ class Scene:
         "levels", "persistent", "split" (level kernels below the autotuned
         cut level, one persistent launch above), "cluster" (one thread-block
         cluster walks the levels), "resident" (the factor held in one
-        cluster's shared memory) or "dense" (one product with Hs^-1, rebuilt
-        from the factor after every refactorisation; single scenes up to 4,096
-        vertices).  Returns the form in use and the autotune's ms per solve of
+        cluster's shared memory) or "dense" (single scenes: products with
+        block inverses, or, in the forward of mixed scenes of up to 4,096
+        vertices, one with Hs^-1; rebuilt for every new set of moduli).  Returns the form in use and the autotune's ms per solve of
         each form."""
         req = {None: -1, "auto": 0, "levels": 1, "persistent": 2, "split": 3, "cluster": 4, "resident": 5,
                "dense": 6}[request]

@@ -316,10 +316,12 @@ int dfem_host_factor_solve(const dfem_scene_desc *desc, const double *b, double 
  * up to 16 CTAs: every block stays in shared memory for the launch,
  * contributions and solution values move between the CTAs over distributed
  * shared memory, a cluster barrier between levels), 6 dense (single scenes
- * of at most 4,096 vertices: X = Hs^-1 is formed from the factor after every
- * refactorisation, N_p^2 doubles twice with N_p = N rounded up to 64, and a
- * solve is one product with X; the autotune keeps it when its saving over
- * 100 solves exceeds the rebuild); a form requested with
+ * only: the elimination tree merged into a few tiers of blocks whose inverses
+ * are rebuilt for every new set of moduli, a solve being products with them;
+ * the forward of mixed scenes instead takes one product with X = Hs^-1, formed
+ * from the factor, N_p^2 doubles twice with N_p = N rounded up to 64, at most
+ * 4,096 vertices; the autotune keeps it when its saving over 100 solves
+ * exceeds the rebuild); a form requested with
  * 1-6 is used in every iteration (no per-iteration selection, see
  * dfem_solve_select).  *chosen (may
  * be NULL) receives the form in use (1-6), ms (may be NULL, 2 values)
