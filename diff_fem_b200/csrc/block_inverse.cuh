@@ -18,7 +18,7 @@
 // deterministic.  A pivot that is not positive (or not finite) raises the
 // failure word, as the supernodal factor does; the host retries with the next
 // regularisation.  12,800-tet beam (10 blocks of up to 373 columns and a top
-// one of 693): 34 pivots of 10.5 us, 0.36 ms (a first version: 16 us each).
+// one of 693): 34 pivots of 11.1 us, 0.38 ms (a first version: 16 us each).
 //
 // Solve: 2 tiers - 1 phases of row products, see block_solve.
 #pragma once
@@ -131,26 +131,12 @@ constexpr size_t kBfSmem = sizeof(double) * (kBfOps + 2 * 4 * kBlkPivot + (size_
                            sizeof(BfTile) * kBfOwn;
 static_assert(3 * kBlkTile * kBfLd >= kBlkTile * kBfTld, "a tile past the resident ones is assembled in the operands' space");
 
-// 1 / d by Newton's iteration from the hardware's approximate reciprocal
-// (about 20 bits; a cubic and a quadratic step): a dependent chain of 60
-// cycles where the division takes 111 (the pivots of a sweep follow one
-// another).  d outside the approximation's range gives 0, an infinity or a
-// NaN, which fails the pivot test of the caller.
-__device__ __forceinline__ double newton_recip(double d) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
-  double e = fma(-d, y, 1.0);
-  y = fma(y, fma(e, e, e), y);
-  e = fma(-d, y, 1.0);
-  return fma(y, e, y);
-}
-
 // D = A^-1 of the symmetric positive definite A (32 x 32 at A, row length ld,
 // lower half) by sweeps of 2 x 2 pivots, to out (32 x 32).  Warp w holds rows
 // 2 w and 2 w + 1, a lane two columns of one of them, in registers; the warp
 // that owns a step's pivot rows publishes them, and their products with the
 // inverse of the pivot, through shared memory (zz: 2 x 4 x 32 doubles, used
-// in turn): sixteen dependent steps of one barrier each, 0.25 K cycles a step
+// in turn): sixteen dependent steps of one barrier each, 0.33 K cycles a step
 // (with every warp reading the whole matrix from shared memory and forming
 // the pivot's inverse itself: 0.8 K).  True when a pivot is not positive.
 __device__ __forceinline__ bool invert_pivot(const double* A, int ld, double* zz, double* out) {
@@ -162,7 +148,7 @@ __device__ __forceinline__ bool invert_pivot(const double* A, int ld, double* zz
     const int src = k >> 1;
     const double p = __shfl_sync(0xffffffffu, a0, src), q = __shfl_sync(0xffffffffu, a1, src),
                  r = __shfl_sync(0xffffffffu, a1, 16 + src);
-    const double det = fma(p, r, -q * q), id = newton_recip(det);
+    const double det = fma(p, r, -q * q), id = 1.0 / det;
     bad |= !(p > 0.0) || !(det > 0.0) || !isfinite(det) || !(id > 0.0) || !isfinite(id);
     const bool mine = (lane & 15) == src;
     const double z0 = mine ? (lane < 16 ? -1.0 : 0.0) : a0, z1 = mine ? (lane < 16 ? 0.0 : -1.0) : a1;
