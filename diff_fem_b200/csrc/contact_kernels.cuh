@@ -13,15 +13,17 @@
 #pragma once
 #include <cooperative_groups.h>
 
+#include "contact_flags.h"
 #include "kernels.cuh"
 
 namespace dfem {
 
 // state words: [mode, pass, it, any, active, loop-body executions, computed
 // Jacobi iterations, the computed iteration whose x_n1 the current ori_x is,
-// obstacle impacts in the lists, self groups of this pass, of the last pass]
+// obstacle impacts in the lists, self groups of this pass, of the last pass,
+// k_contact_phase's hit words (contact_flags.h)]
 enum { CS_MODE = 0, CS_PASS = 1, CS_IT = 2, CS_ANY = 3, CS_ACTIVE = 4, CS_BODIES = 5, CS_COMP = 6, CS_SRC = 7,
-       CS_NOBS = 8, CS_NGRP = 9, CS_NGRP_PREV = 10, CS_FANY0 = 11, CS_FANY1 = 12, CS_SIZE = 13 };
+       CS_NOBS = 8, CS_NGRP = 9, CS_NGRP_PREV = 10, CS_HIT = 11, CS_SIZE = CS_HIT + kHitWords };
 
 // per-step record of the phase: [passes, loop-body executions]; while the
 // forward steps record their contact iterations, the step's place in the

@@ -310,13 +310,12 @@ __global__ void __launch_bounds__(kPsThreads, 1) k_contact_phase(const __grid_co
   for (;;) {
     bodies += 1;
     if (mode == 0) {  // detection pass (k_contact_detect, k_contact_ctl_detect)
-      // the hits' flags alternate, so clearing one never races with reading the other
-      int* flag = c.state + ((ndet & 1) ? CS_FANY1 : CS_FANY0);
+      int* flag = c.state + CS_HIT + hit_word(ndet);
       for (int a = wid; a < c.nc; a += nw)
         if (ct_detect(c, a, xt, ori ? c.xn1 : xk, (int*)stage, status) && lane == 0) atomicOr(flag, 1);
       if (!bar.sync()) return;
       const bool any = *(volatile int*)flag != 0;
-      if (lead) c.state[(ndet & 1) ? CS_FANY0 : CS_FANY1] = 0;  // the other word: read a barrier ago
+      if (lead) c.state[CS_HIT + cleared_word(ndet)] = 0;  // (contact_flags.h)
       ++ndet;
       if (!any) break;
       if (pass >= c.max_passes) {
