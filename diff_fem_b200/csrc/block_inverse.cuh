@@ -15,9 +15,9 @@
 // its inverse D go through global memory, and one grid-wide barrier separates
 // sweeps.  The CTA of the tile that holds the next pivot inverts it before
 // the barrier.  All values have one writer and a fixed order: the result is
-// deterministic.  A pivot that is not positive (or not finite) raises the
-// failure word, as the supernodal factor does; the host retries with the next
-// regularisation.  12,800-tet beam (10 blocks of up to 373 columns and a top
+// deterministic.  A pivot that is not positive (or not finite) raises bit 0 of
+// the failure word, as the supernodal factor does; the host retries with the
+// next regularisation.  A barrier that gave up raises bit 1 (kBuildGaveUp).  12,800-tet beam (10 blocks of up to 373 columns and a top
 // one of 693): 34 pivots of 11.1 us, 0.38 ms (a first version: 16 us each).
 //
 // Solve: 2 tiers - 1 phases of row products, see block_solve.
@@ -51,6 +51,7 @@ struct BlockDev {
   double* contrib;                // 3 per row of every block
   unsigned* bar;                  // grid barrier: arrivals, CTAs done
   int* status;
+  int spin_tries;                 // polls of a grid barrier before it gives up
   int vec;                        // doubles of one staged component (largest n or r, even)
 };
 
@@ -58,16 +59,23 @@ struct BlockDev {
 //
 // Barrier over a cooperative launch (every CTA resident): arrivals counted in
 // global memory, thread 0 polls (acquire) until all CTAs of this round have
-// come, at most kSpinTries times.  1.2 us on 148 CTAs; a barrier of one
+// come, at most `tries` times.  1.2 us on 148 CTAs; a barrier of one
 // cluster takes 0.25 us.  sync() is false, in every thread of the CTA, when
-// the wait gave up (status 6, wait kWaitGrid): the caller returns.
+// the wait gave up (status 6, wait kWaitGrid): the caller returns.  The
+// counters are then left as they are until the host has seen the status and
+// cleared both (reset_barriers): a launch that finds the status so on entry
+// returns at once (gave_up).
 constexpr int kWaitGrid = 14;
 
 struct GridBarrier {
   unsigned* c;
   int* status;
+  int tries;
   unsigned target = 0;
-  __device__ GridBarrier(unsigned* c_, int* s_) : c(c_), status(s_) {}
+  __device__ GridBarrier(unsigned* c_, int* s_, int t_) : c(c_), status(s_), tries(t_) {}
+  __device__ static bool gave_up(const int* s) {
+    return __syncthreads_or(threadIdx.x == 0 && *(const volatile int*)(s + 2) == kWaitGrid) != 0;
+  }
   __device__ static int cta() { return blockIdx.x; }
   __device__ static int ctas() { return gridDim.x; }
   __device__ bool sync() {
@@ -77,7 +85,8 @@ struct GridBarrier {
       target += gridDim.x;
       asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(c) : "memory");
       ok = 0;
-      for (int k = 0; k < kSpinTries; ++k) {
+#pragma unroll 1
+      for (int k = 0; k < tries; ++k) {
         unsigned v;
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(c) : "memory");
         if ((int)(v - target) >= 0) { ok = 1; break; }
@@ -105,7 +114,8 @@ struct GridBarrier {
 
 // The same over one thread-block cluster (the grid is one cluster).
 struct ClusterBarrier {
-  __device__ ClusterBarrier(unsigned*, int*) {}
+  __device__ ClusterBarrier(unsigned*, int*, int) {}
+  __device__ static bool gave_up(const int*) { return false; }
   __device__ static int cta() { return (int)cluster_rank(); }
   __device__ static int ctas() { return gridDim.x; }
   __device__ bool sync() {
@@ -117,6 +127,7 @@ struct ClusterBarrier {
 
 // ---------------------------------------------------------------- build ----
 
+constexpr int kBuildGaveUp = 2;
 constexpr int kBfThreads = 512;   // one CTA per SM: sixteen warps, 16 x 16 of a tile's output each
 constexpr int kBfOwn = 32;        // tiles of a CTA whose descriptors are kept in shared memory
 constexpr int kBfRes = 4;         // tiles of a CTA kept in shared memory
@@ -207,7 +218,11 @@ __global__ void __launch_bounds__(kBfThreads, 1) k_block_factor(BlockDev b, cons
   double* zz = bfsh + kBfOps;
   double* res = zz + 2 * 4 * kBlkPivot;
   BfTile* own = reinterpret_cast<BfTile*>(res + (size_t)kBfRes * kBlkTile * kBfTld);
-  GridBarrier bar(b.bar, b.status);
+  if (GridBarrier::gave_up(b.status)) {
+    if (threadIdx.x == 0) atomicOr(fail, kBuildGaveUp);
+    return;
+  }
+  GridBarrier bar(b.bar, b.status, b.spin_tries);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const double reg = reg_p[0];
   bool bad = false;
@@ -257,7 +272,10 @@ __global__ void __launch_bounds__(kBfThreads, 1) k_block_factor(BlockDev b, cons
       write_panel(S, kBfTld, T.I, T.J, 0, b.panel + B.panel);
       if (T.I == 0) bad |= invert_pivot(S, kBfTld, zz, b.piv + (size_t)2 * B.pivofs * kBlkPivot * kBlkPivot);
     }
-    if (!bar.sync()) return;
+    if (!bar.sync()) {
+      if (tid == 0) atomicOr(fail, kBuildGaveUp);
+      return;
+    }
     int steps = 0;
     if (q0 < q1) steps = b.blk[b.tiles[q0].blk].np;  // the tier's first block has the most pivots
     for (int s = 0; s < steps; ++s) {
@@ -389,10 +407,13 @@ __global__ void __launch_bounds__(kBfThreads, 1) k_block_factor(BlockDev b, cons
                 }
               }
         }
-      if (!bar.sync()) return;
+      if (!bar.sync()) {
+        if (tid == 0) atomicOr(fail, kBuildGaveUp);
+        return;
+      }
     }
   }
-  if (bad) atomicExch(fail, 1);
+  if (bad) atomicOr(fail, 1);
   bar.leave();
 }
 
@@ -527,8 +548,8 @@ __device__ __forceinline__ bool block_solve(const BlockDev& b, BAR& bar, const d
 template <class BAR>
 __global__ void __launch_bounds__(kBsThreads, 1) k_block_solve(BlockDev b, Gate gate, const double* rhs, double* y) {
   extern __shared__ __align__(16) double bssh[];
-  if (gate.skip(0)) return;  // uniform, before any barrier
-  BAR bar(b.bar, b.status);
+  if (gate.skip(0) || BAR::gave_up(b.status)) return;  // uniform, before any barrier
+  BAR bar(b.bar, b.status, b.spin_tries);
   if (!block_solve(b, bar, rhs, y, bssh, [&](int g, Vec3<double> v) { st3(y, g, v); })) return;
   bar.leave();
 }

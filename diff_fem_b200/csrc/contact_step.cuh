@@ -267,10 +267,12 @@ __device__ __forceinline__ void ct_tet_take(bool rot, const double* xch, int me,
 __global__ void __launch_bounds__(kPsThreads, 1) k_contact_phase(const __grid_constant__ SceneDev d,
                                                                  const __grid_constant__ ContactDev c, const double* xt,
                                                                  double* xk, const double* act_all, const int* step,
-                                                                 double* slot, double* partial, unsigned* counter, int* status) {
+                                                                 double* slot, double* partial, unsigned* counter, int tries,
+                                                                 int* status) {
   extern __shared__ __align__(16) double dyn[];
   __shared__ double ws[kPsWarps];
-  GridBarrier bar(counter, status);
+  if (GridBarrier::gave_up(status)) return;
+  GridBarrier bar(counter, status, tries);
   const int nc = gridDim.x, cta = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int wid = warp * nc + cta, nw = kPsWarps * nc;  // a warp's share: CTAs first
   const int tid = wid * 32 + lane, nthr = nw * 32;
@@ -427,9 +429,10 @@ __global__ void __launch_bounds__(kPsThreads, 1) k_cadj_phase(const __grid_const
                                                               const double* xt, const double* act_all, const int* step,
                                                               double* slot, double* gE, double* gnu, double* mg, double* gact,
                                                               int base, int top, double cv, double* io_a, double* io_b,
-                                                              unsigned* counter, int* status) {
+                                                              unsigned* counter, int tries, int* status) {
   extern __shared__ __align__(16) double dyn[];
-  GridBarrier bar(counter, status);
+  if (GridBarrier::gave_up(status)) return;
+  GridBarrier bar(counter, status, tries);
   const int nc = gridDim.x, cta = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int wid = warp * nc + cta, nw = kPsWarps * nc;
   const int tid = wid * 32 + lane, nthr = nw * 32;

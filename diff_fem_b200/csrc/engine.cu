@@ -1063,7 +1063,8 @@ static int block_prepare(dfem_scene* sc, bool* ok) {
     d.hs_idx = sc->bl_hs_idx.p; d.hs_loc = sc->bl_hs_loc.p; d.cols = sc->bl_cols.p; d.rows = sc->bl_rows.p;
     d.rmap = sc->bl_rmap.p; d.cslot = sc->bl_cslot.p; d.vptr = sc->bl_vptr.p; d.chunks = sc->bl_chunks.p;
     d.share = sc->bl_share.p; d.front = sc->bl_front.p; d.panel = sc->bl_panel.p; d.sol = view ? sc->dn_A.p : sc->bl_sol.p;
-    d.piv = sc->bl_piv.p; d.contrib = sc->bl_contrib.p; d.bar = sc->bl_bar.p; d.status = sc->status.p; d.vec = vec;
+    d.piv = sc->bl_piv.p; d.contrib = sc->bl_contrib.p; d.bar = sc->bl_bar.p; d.status = sc->status.p; d.spin_tries = sc->spin_tries;
+    d.vec = vec;
     sc->bd = d;
   }
   *ok = true;
@@ -1087,13 +1088,33 @@ static int dense_prepare(dfem_scene* sc, bool* ok) {
   return DFEM_OK;
 }
 
+// A grid barrier that gave up leaves its counters behind: they and the status
+// word are cleared for the next launch.  The caller reports the error.
+static int reset_barriers(dfem_scene* sc) {
+  CK(cudaStreamSynchronize(sc->stream));
+  for (DBuf<unsigned>* b : {&sc->bl_bar, &sc->cbar})
+    if (b->p) CK(cudaMemset(b->p, 0, 2 * sizeof(unsigned)));
+  CK(cudaMemset(sc->status.p, 0, 4 * sizeof(int)));
+  if (!dense_is_x(sc)) sc->dense_built = false;  // a block build among the launches may be incomplete
+  sc->blk_built = false;
+  return DFEM_OK;
+}
+
 // X_B and P_B of every block from the current Hs values (block_inverse.cuh),
-// on the scene's stream; a pivot that is not positive raises part_fail[0].
+// on the scene's stream; a pivot that is not positive raises bit 0 of
+// part_fail[0], a barrier that gave up kBuildGaveUp (check_build).
 static int dense_build(dfem_scene* sc) {
   CK(launch_coop(sc->stream, k_block_factor, sc->bf_grid, kBfThreads, kBfSmem, sc->bd, (const double*)sc->hs_val.p,
                  (const double*)sc->part_reg.p, sc->part_fail.p));
   sc->launches += 1;
   return DFEM_OK;
+}
+
+// DFEM_ERR_CAP when a build reported a barrier that gave up.
+static int check_build(dfem_scene* sc, int failed) {
+  if (!(failed & kBuildGaveUp)) return DFEM_OK;
+  RC(reset_barriers(sc));
+  return fail(DFEM_ERR_CAP, "a grid-wide barrier gave up in the block build");
 }
 
 // Levels of the supernodal factor from the current Hs values.
@@ -1139,6 +1160,7 @@ static int factor_values(dfem_scene* sc, bool dense) {
     CK(cudaMemcpyAsync(failh.data(), sc->part_fail.p, sizeof(int) * (np + 1), cudaMemcpyDeviceToHost, sc->stream));
     CK(cudaStreamSynchronize(sc->stream));
     if (failh[np]) return fail(DFEM_ERR_INVALID, "invalid material (non-finite E or nu, or nu <= -1)");
+    if (dense) RC(check_build(sc, failh[0]));
     bool any = false;
     for (int p = 0; p < np; ++p)
       if (failh[p]) {
@@ -1174,6 +1196,7 @@ static int ensure_adjoint_blocks(dfem_scene* sc, bool* ok) {
   RC(dense_build(sc));
   CK(cudaMemcpyAsync(&bad, sc->part_fail.p, sizeof(int), cudaMemcpyDeviceToHost, sc->stream));
   CK(cudaStreamSynchronize(sc->stream));
+  RC(check_build(sc, bad));
   *ok = bad == 0;
   if (bad) {
     sc->ps_ok = false;
@@ -2070,7 +2093,7 @@ static cudaError_t launch_contact_fused(dfem_scene* sc, cudaStream_t st) {
   cfg.dynamicSmemBytes = kCtSmemFwd;
   return cudaLaunchKernelEx(&cfg, k_contact_phase, sc->sd, sc->cd, (const double*)sc->xt.p, sc->xk.p,
                             (const double*)sc->act_all.p, (const int*)sc->step.p, sc->slot.p, sc->fpartial.p,
-                            sc->cbar.p, sc->status.p);
+                            sc->cbar.p, sc->spin_tries, sc->status.p);
 }
 
 static void step_post(dfem_scene* sc, cudaStream_t st) {
@@ -2451,7 +2474,8 @@ static int contact_adjoint_step(dfem_scene* sc, int st, bool recorded, int rbase
     const CtFrames fr{sc->ca_slot.p, 3 * (size_t)std::max(1, s.nslots), sc->ca_frame.p, sc->ca_hit.p};
     CK(launch_coop(sc->stream, k_cadj_phase, sc->cadj_grid, kPsThreads, kCtSmemAdj, sc->sd, sc->cd, a, fr, xt,
                    (const double*)sc->act_all.p, (const int*)sc->step.p, sc->slot.p, sc->gE.p, sc->gnu.p,
-                   sc->mg.p, sc->gact.p, base, src, s.damping / s.h, sc->io_a.p, sc->io_b.p, sc->cbar.p, sc->status.p));
+                   sc->mg.p, sc->gact.p, base, src, s.damping / s.h, sc->io_a.p, sc->io_b.p, sc->cbar.p, sc->spin_tries,
+                   sc->status.p));
     sc->launches += 1;
     return DFEM_OK;
   }
@@ -2540,7 +2564,7 @@ static int status_error(const int st4[4]) {
   if (st4[0] == DFEM_ERR_CAP && st4[2] > 0 && st4[2] <= 9)
     return fail(DFEM_ERR_CAP, std::string(what[st4[2]]) + " gave up (supernode " + std::to_string(st4[1]) + ", " +
                                   std::to_string(st4[3]) + " blocks)");
-  if (st4[0] == DFEM_ERR_CAP && st4[2] == kWaitGrid)
+  if (st4[2] == kWaitGrid)
     return fail(DFEM_ERR_CAP, "a grid-wide barrier gave up (" + std::to_string(st4[3]) + " blocks)");
   if (st4[0] == DFEM_ERR_CAP && st4[2] == kCapContactPasses)
     return fail(DFEM_ERR_CAP, "the contact phase still found new impacts after its last detection pass (pass cap)");
@@ -2555,13 +2579,12 @@ static int status_error(const int st4[4]) {
   return DFEM_OK;
 }
 
-// status_error for a call's status; a barrier that gave up leaves its counters
-// behind, so they are cleared for the next launch.
+// status_error for a call's status.  After a grid barrier that gave up the
+// call's records are incomplete: no backward of them.
 static int check_status(dfem_scene* sc, const int st4[4]) {
-  if (st4[0] == DFEM_ERR_CAP && st4[2] == kWaitGrid) {
-    CK(cudaStreamSynchronize(sc->stream));
-    for (DBuf<unsigned>* b : {&sc->bl_bar, &sc->cbar})
-      if (b->p) CK(cudaMemset(b->p, 0, 2 * sizeof(unsigned)));
+  if (st4[2] == kWaitGrid) {
+    RC(reset_barriers(sc));
+    sc->rec_steps = 0;
   }
   return status_error(st4);
 }
@@ -2765,7 +2788,7 @@ static int autotune_solve(dfem_scene* sc) {
   RC(rc);
   int st4[4] = {0, 0, 0, 0};
   CK(cudaMemcpy(st4, sc->status.p, sizeof(st4), cudaMemcpyDeviceToHost));
-  RC(status_error(st4));
+  RC(check_status(sc, st4));
   sc->solve_cut = sc->solve_ms[1] < sc->solve_ms[0] ? 0 : L;
   if (sc->split_cut > 0 && sc->solve_ms[2] < std::min(sc->solve_ms[0], sc->solve_ms[1])) sc->solve_cut = sc->split_cut;
   {
@@ -3547,7 +3570,7 @@ int dfem_profile_phases(dfem_scene* sc, int32_t reps, double* ms) {
   int st4[4] = {0, 0, 0, 0};
   CK(cudaMemcpyAsync(st4, sc->status.p, sizeof(st4), cudaMemcpyDeviceToHost, sc->stream));
   CK(cudaStreamSynchronize(sc->stream));
-  RC(status_error(st4));
+  RC(check_status(sc, st4));
   // the solve phase counted one launch per call above
   sc->launches += (int64_t)(reps + 1) * (solve_launches(sc) - 1);
   sc->rec_steps = 0;  // gates and iteration counts were overwritten: no backward of the old forward
@@ -3582,7 +3605,7 @@ int dfem_set_limit(dfem_scene* sc, int32_t which, int64_t value) {
       if (!dflt && (value < 1 || value > kSpinTries))
         return fail(DFEM_ERR_INVALID, "poll limit must be in [1, " + std::to_string(kSpinTries) + "]");
       sc->spin_tries = dflt ? kSpinTries : (int)value;
-      sc->fd.spin_tries = sc->spin_tries;
+      sc->fd.spin_tries = sc->bd.spin_tries = sc->spin_tries;
       break;
     default:
       return fail(DFEM_ERR_INVALID, "unknown limit");

@@ -549,7 +549,8 @@ __global__ void __launch_bounds__(kPsThreads, 1) k_pd_forward(const __grid_const
   double* res = pssh + ps_fixed_doubles(vec) + (MIXED ? 0 : a.tab_ints / 2);
   double* xch = planes + 3 * (size_t)vec + 3 * kBsRows;
   if (MIXED) res = xch;  // the mixed form exchanges nothing
-  BAR bar(b.bar, b.status);
+  if (BAR::gave_up(b.status)) return;
+  BAR bar(b.bar, b.status, b.spin_tries);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, cta = BAR::cta(), nc = BAR::ctas();
   // items are dealt to the CTAs a warp's worth at a time
   const int first = 32 * (warp * nc + cta) + lane, stride = kPsThreads * nc;
@@ -721,7 +722,8 @@ __global__ void __launch_bounds__(kPsThreads, 1) k_pd_adjoint(SceneDev d, BlockD
   const int tstride = 32 * a.tape_warps;
   double* res = tape + (size_t)kVolTape * tstride;
   double* xch = planes + 3 * (size_t)b.vec + 3 * kBsRows;
-  BAR bar(b.bar, b.status);
+  if (BAR::gave_up(b.status)) return;
+  BAR bar(b.bar, b.status, b.spin_tries);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, cta = BAR::cta(), nc = BAR::ctas();
   const int first = 32 * (warp * nc + cta) + lane, stride = kPsThreads * nc;
   const int nmg = d.M + (d.sch ? d.S : 0);

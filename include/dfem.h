@@ -391,7 +391,9 @@ int dfem_profile_phases(dfem_scene *scene, int32_t reps, double *ms);
  *   DFEM_LIMIT_SOFT_IMPACTS_PER_VERTEX  soft faces a contact vertex may hit in a step (0..16)
  *   DFEM_LIMIT_GROUP_MEMBERS            members of one soft-contact face group (0..32)
  *   DFEM_LIMIT_SOLVE_WAIT_POLLS         polls of a dependency wait of the persistent
- *                                       solve form (1..2^22)
+ *                                       solve form, and of a grid-wide barrier of
+ *                                       the kernels that run a build, whole steps
+ *                                       or a contact phase in one launch (1..2^22)
  *   DFEM_LIMIT_BROAD_PHASE_CELLS        grid cells a contact vertex's swept box may
  *                                       cover in the obstacle detection's broad phase
  *                                       before the vertex tests every obstacle face
