@@ -17,7 +17,8 @@
 // the barrier.  All values have one writer and a fixed order: the result is
 // deterministic.  A pivot that is not positive (or not finite) raises bit 0 of
 // the failure word, as the supernodal factor does; the host retries with the
-// next regularisation.  A barrier that gave up raises bit 1 (kBuildGaveUp).  12,800-tet beam (10 blocks of up to 373 columns and a top
+// next regularisation.  A barrier that gave up raises bit 1 (kBuildGaveUp).
+// Invalid materials (the word after it) leave everything as it was.  12,800-tet beam (10 blocks of up to 373 columns and a top
 // one of 693): 34 pivots of 11.1 us, 0.38 ms (a first version: 16 us each).
 //
 // Solve: 2 tiers - 1 phases of row products, see block_solve.
@@ -218,6 +219,7 @@ __global__ void __launch_bounds__(kBfThreads, 1) k_block_factor(BlockDev b, cons
   double* zz = bfsh + kBfOps;
   double* res = zz + 2 * 4 * kBlkPivot;
   BfTile* own = reinterpret_cast<BfTile*>(res + (size_t)kBfRes * kBlkTile * kBfTld);
+  if (fail[1]) return;  // uniform, before any barrier
   if (GridBarrier::gave_up(b.status)) {
     if (threadIdx.x == 0) atomicOr(fail, kBuildGaveUp);
     return;

@@ -165,6 +165,7 @@ struct dfem_scene {
   bool dense_built = false;              // the form belongs to the current moduli
   bool blk_built = false;                // mixed scenes: the adjoint's blocks do (built by the first adjoint that needs them)
   bool tri_built = false;                // the supernodal factor does (built on demand while the dense form is in use)
+  bool moduli_ok = false;                // Hs and a factor follow the last moduli (gpu_refactor)
   double dense_build_ms = 0.0;
   // mixed scenes: X = Hs^-1 from the supernodal factor (dense_solve.cuh); FP64 scenes: blocks (block_inverse.cuh)
   DBuf<double> dn_A, dn_W, dn_T, dn_Linv;
@@ -785,7 +786,7 @@ static int upload_refactor_plan(dfem_scene* sc) {
                        sc->hs_col.p, sc->sn_c0.p, sc->sn_w.p, sc->sn_r.p, sc->sn_rofs.p, sc->rowidx.p,
                        sc->sn_lofs.p, sc->Lcm.p, sc->sn_dofs.p, sc->Dinv.p, sc->DinvC.p, sc->Ldw.p, sc->lvl_sn.p, sc->up_ptr.p,
                        sc->up_d.p, sc->up_a0.p, sc->up_a1.p, np > 1 ? sc->sn_part.p : nullptr, sc->part_reg.p,
-                       sc->part_fail.p};
+                       sc->part_fail.p, sc->part_fail.p + np};
   return DFEM_OK;
 }
 
@@ -1192,7 +1193,7 @@ static int ensure_adjoint_blocks(dfem_scene* sc, bool* ok) {
   *ok = true;
   if (!dense_is_x(sc) || sc->bplan.tiers == 1 || sc->blk_built) return DFEM_OK;
   int bad = 0;
-  CK(cudaMemsetAsync(sc->part_fail.p, 0, sizeof(int), sc->stream));
+  CK(cudaMemsetAsync(sc->part_fail.p, 0, 2 * sizeof(int), sc->stream));
   RC(dense_build(sc));
   CK(cudaMemcpyAsync(&bad, sc->part_fail.p, sizeof(int), cudaMemcpyDeviceToHost, sc->stream));
   CK(cudaStreamSynchronize(sc->stream));
@@ -1213,16 +1214,42 @@ static int ensure_triangular(dfem_scene* sc) {
 }
 
 // Materials from E_in / nu_in (device), Hs values, and the factor on the GPU.
+// Invalid materials are refused before anything changes: the scene, its
+// factor and its recorded forward stay as they are.  After any other failure
+// there is no factor (moduli_ok) until a later call succeeds.
 static int gpu_refactor(dfem_scene* sc) {
   const HostScene& s = sc->hs;
   const int np = s.nparts;
+  const std::vector<double> reg = sc->part_reg_h;
+  const bool dense = sc->dense_built, tri = sc->tri_built, blk = sc->blk_built, ok = sc->moduli_ok;
   CK(cudaMemsetAsync(sc->part_fail.p, 0, sizeof(int) * (np + 1), sc->stream));
-  if (s.T > 0) k_materials<<<(s.T + 127) / 128, 128, 0, sc->stream>>>(sc->rd, sc->E_in.p, sc->nu_in.p, np);
+  if (s.T > 0) {
+    k_check_materials<<<(s.T + 127) / 128, 128, 0, sc->stream>>>(sc->rd, sc->E_in.p, sc->nu_in.p);
+    k_materials<<<(s.T + 127) / 128, 128, 0, sc->stream>>>(sc->rd, sc->E_in.p, sc->nu_in.p);
+  }
   k_hs_values<<<(sc->rd.nnz + 255) / 256, 256, 0, sc->stream>>>(sc->rd);
-  sc->launches += (s.T > 0 ? 1 : 0) + 1;
+  sc->launches += (s.T > 0 ? 2 : 0) + 1;
   std::fill(sc->part_reg_h.begin(), sc->part_reg_h.end(), 0.0);
-  sc->dense_built = sc->tri_built = sc->blk_built = false;
-  return factor_values(sc, sc->solve_cut == -3);
+  sc->dense_built = sc->tri_built = sc->blk_built = sc->moduli_ok = false;
+  const int rc = factor_values(sc, sc->solve_cut == -3);
+  if (rc == DFEM_ERR_INVALID) {
+    sc->part_reg_h = reg;
+    CK(cudaMemcpyAsync(sc->part_reg.p, reg.data(), sizeof(double) * np, cudaMemcpyHostToDevice, sc->stream));
+    sc->dense_built = dense;
+    sc->tri_built = tri;
+    sc->blk_built = blk;
+    sc->moduli_ok = ok;
+  } else if (rc != DFEM_OK) {
+    sc->rec_steps = 0;
+  } else {
+    sc->moduli_ok = true;
+  }
+  return rc;
+}
+
+// Before a solve: a call to dfem_set_materials that failed left no factor.
+static int require_moduli(const dfem_scene* sc) {
+  return sc->moduli_ok ? DFEM_OK : fail(DFEM_ERR_STATE, "the last dfem_set_materials failed: no factor until one succeeds");
 }
 
 // Uniform grid over the static obstacle faces for the detection's broad phase
@@ -2931,6 +2958,7 @@ int dfem_set_materials(dfem_scene* sc, const double* youngs, const double* poiss
     RC(copy_in(sc, poisson, T, sc->nu_in.p, mem));
   }
   RC(gpu_refactor(sc));
+  sc->rec_steps = 0;  // the recorded forward used the old factor
   if (sc->has_contact)
     k_hs_diag<<<sc->nblk_v, 128, 0, sc->stream>>>(s.N, sc->hs_ptr.p, sc->hs_col.p, sc->hs_val.p, sc->hdiag.p);
   // the host factor is used after creation only by the skeleton's Schur
@@ -2947,7 +2975,6 @@ int dfem_set_materials(dfem_scene* sc, const double* youngs, const double* poiss
     if (!update_materials(s, E.data(), nu.data(), err)) return fail(DFEM_ERR_FACTOR, err);
     RC(upload_skeleton(sc));
   }
-  sc->rec_steps = 0;  // the recorded forward used the old factor
   return DFEM_OK;
 }
 
@@ -3006,6 +3033,7 @@ int dfem_step_forward(dfem_scene* sc, const double* x, const double* v, const do
   if (!sc || !x || !v || !x_out || !v_out) return fail(DFEM_ERR_INVALID, "null argument");
   if (n_steps < 1) return fail(DFEM_ERR_INVALID, "n_steps must be >= 1");
   CK(cudaSetDevice(sc->device));
+  RC(require_moduli(sc));
   RC(ensure_steps(sc, n_steps));
   const HostScene& s = sc->hs;
   const size_t n3 = 3 * (size_t)s.N;
@@ -3420,6 +3448,7 @@ int dfem_profile_levels(dfem_scene* sc, int32_t reps, int32_t cap, int32_t* n_se
   const int G = (int)sc->segs.size();
   *n_segments = G;
   if (!ms_fwd || !ms_bwd || cap < G) return DFEM_OK;
+  RC(require_moduli(sc));
   RC(ensure_triangular(sc));
   cudaEvent_t e0, e1;
   CK(cudaEventCreate(&e0));
@@ -3461,6 +3490,7 @@ int dfem_solve_mode(dfem_scene* sc, int32_t request, int32_t* chosen, double* ms
   if (!sc) return fail(DFEM_ERR_INVALID, "null argument");
   if (request < -1 || request > 6) return fail(DFEM_ERR_INVALID, "request must be -1, 0, 1, 2, 3, 4, 5 or 6");
   CK(cudaSetDevice(sc->device));
+  if (request >= 0) RC(require_moduli(sc));
   if (request == 0) {
     CK(cudaStreamSynchronize(sc->stream));
     CK(cudaMemsetAsync(sc->status.p, 0, 4 * sizeof(int), sc->stream));

@@ -63,18 +63,22 @@ struct RefactorDev {
   const int* sn_part;   // null for a single scene
   const double* part_reg;
   int* part_fail;
+  int* invalid;         // part_fail's word past the parts: an invalid material
 };
 
-// part_fail[nparts] (one word past the parts) flags an invalid material
-// (non-finite E or nu, or nu <= -1); the tet then keeps its old values.
-__global__ void k_materials(RefactorDev f, const double* __restrict__ E, const double* __restrict__ nu, int nparts) {
+// An invalid material (non-finite E or nu, or nu <= -1) raises *f.invalid; the
+// kernels after this one then change nothing.
+__global__ void k_check_materials(RefactorDev f, const double* __restrict__ E, const double* __restrict__ nu) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= f.T) return;
   const double e = E[t], n = nu[t];
-  if (!isfinite(e) || !isfinite(n) || !(n > -1.0)) {
-    atomicExch(f.part_fail + nparts, 1);
-    return;
-  }
+  if (!isfinite(e) || !isfinite(n) || !(n > -1.0)) atomicExch(f.invalid, 1);
+}
+
+__global__ void k_materials(RefactorDev f, const double* __restrict__ E, const double* __restrict__ nu) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= f.T || *f.invalid) return;
+  const double e = E[t], n = nu[t];
   f.tE[t] = e;
   f.tnu[t] = n;
   const double wr = e / (1.0 + n) * f.tvol[t];  // CorotateFEMConstraint: mMu = E/(1+nu)
@@ -84,7 +88,7 @@ __global__ void k_materials(RefactorDev f, const double* __restrict__ E, const d
 
 __global__ void k_hs_values(RefactorDev f) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= f.nnz) return;
+  if (k >= f.nnz || *f.invalid) return;
   double v = f.hs_base[k];
   for (int q = f.hc_ptr[k]; q < f.hc_ptr[k + 1]; ++q) v += f.tE[f.hc_tet[q]] * f.hc_coef[q];
   f.hs_val[k] = v;
@@ -337,6 +341,7 @@ __device__ __forceinline__ void fl_trsm(const FlSn& n, const double* X, double* 
 __global__ void __launch_bounds__(256) k_factor_level(RefactorDev f, int lvl_begin) {
   extern __shared__ __align__(16) double fsh[];
   __shared__ int s_bad;
+  if (*f.invalid) return;
   const FlSn n = fl_sn(f, f.lvl_sn[lvl_begin + blockIdx.x]);
   double* L = fsh;
   double* X = fsh + n.w * n.w;
@@ -354,6 +359,7 @@ __global__ void __launch_bounds__(256) k_factor_level(RefactorDev f, int lvl_beg
 // share of the work, gridDim.y shares).
 __global__ void __launch_bounds__(256) k_factor_scatter(RefactorDev f, int lvl_begin) {
   __shared__ int s_bad;
+  if (*f.invalid) return;
   const FlSn n = fl_sn(f, f.lvl_sn[lvl_begin + blockIdx.x]);
   if (threadIdx.x == 0) s_bad = 0;
   __syncthreads();
@@ -365,6 +371,7 @@ __global__ void __launch_bounds__(256) k_factor_scatter(RefactorDev f, int lvl_b
 __global__ void __launch_bounds__(256) k_factor_update(RefactorDev f, int lvl_begin) {
   __shared__ int s_bad;
   __shared__ int rowmap[kRowChunk];
+  if (*f.invalid) return;
   const FlSn n = fl_sn(f, f.lvl_sn[lvl_begin + blockIdx.x]);
   const int rows = n.w + n.r, per = (rows + gridDim.y - 1) / gridDim.y;
   const int lo = blockIdx.y * per, hi = min(rows, lo + per);
@@ -377,6 +384,7 @@ __global__ void __launch_bounds__(256) k_factor_update(RefactorDev f, int lvl_be
 __global__ void __launch_bounds__(256) k_factor_diag(RefactorDev f, int lvl_begin) {
   extern __shared__ __align__(16) double fsh[];
   __shared__ int s_bad;
+  if (*f.invalid) return;
   const FlSn n = fl_sn(f, f.lvl_sn[lvl_begin + blockIdx.x]);
   if (threadIdx.x == 0) s_bad = 0;
   fl_diag(f, n, fsh, fsh + n.w * n.w, &s_bad);
@@ -386,6 +394,7 @@ __global__ void __launch_bounds__(256) k_factor_diag(RefactorDev f, int lvl_begi
 // row chunks y, y + shares, ... of the rows below (X read back from DinvC)
 __global__ void __launch_bounds__(256) k_factor_trsm(RefactorDev f, int lvl_begin) {
   extern __shared__ __align__(16) double fsh[];
+  if (*f.invalid) return;
   const FlSn n = fl_sn(f, f.lvl_sn[lvl_begin + blockIdx.x]);
   if (n.r <= (int)blockIdx.y * kTrsmRows) return;
   double* X = fsh;

@@ -206,7 +206,10 @@ int dfem_scene_destroy(dfem_scene *scene);
 int dfem_scene_get_info(const dfem_scene *scene, dfem_scene_info *info);
 
 /* Per-tet materials; refactors H.  Replaces the COROTATE parameter update +
- * PreComputation of forward_all (python/pydifem.cc:207-221). */
+ * PreComputation of forward_all (python/pydifem.cc:207-221).  Invalid
+ * materials (E or nu not finite, nu <= -1) are refused (DFEM_ERR_INVALID) and
+ * change nothing; after any other error steps return DFEM_ERR_STATE until a
+ * call succeeds. */
 int dfem_set_materials(dfem_scene *scene, const double *youngs, const double *poisson, int mem);
 
 /* Muscle activation per segment for the next forward call(s).  Replaces
