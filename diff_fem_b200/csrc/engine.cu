@@ -1146,6 +1146,8 @@ static int enqueue_triangular_factor(dfem_scene* sc) {
 // other parts keep their regularisation, so their factors are unchanged.
 static int factor_values(dfem_scene* sc, bool dense) {
   const int np = sc->hs.nparts;
+  if (dense && !(dense_is_x(sc) ? (const void*)sc->dd.A : (const void*)sc->bd.blk))
+    return fail(DFEM_ERR_STATE, "the dense form has no buffers");
   if (dense && dense_is_x(sc)) {  // from the supernodal factor
     if (!sc->tri_built) RC(factor_values(sc, false));
     RC(dense_x_build(sc));
@@ -1175,6 +1177,7 @@ static int factor_values(dfem_scene* sc, bool dense) {
     }
     (dense ? sc->tri_built : sc->dense_built) = false;  // the other form's factor has another regularisation
   }
+  std::fill(sc->part_reg_h.begin(), sc->part_reg_h.end(), 0.0);
   return fail(DFEM_ERR_FACTOR, "Cholesky factorisation failed after 25 regularisation retries");
 }
 
@@ -1247,9 +1250,12 @@ static int gpu_refactor(dfem_scene* sc) {
   return rc;
 }
 
-// Before a solve: a call to dfem_set_materials that failed left no factor.
-static int require_moduli(const dfem_scene* sc) {
-  return sc->moduli_ok ? DFEM_OK : fail(DFEM_ERR_STATE, "the last dfem_set_materials failed: no factor until one succeeds");
+// Before a solve: the factor of the form in use.  A call to dfem_set_materials
+// that failed left none; a form whose factor another form's regularisation or
+// a build that gave up has outdated gets it again.
+static int require_factor(dfem_scene* sc) {
+  if (!sc->moduli_ok) return fail(DFEM_ERR_STATE, "the last dfem_set_materials failed: no factor until one succeeds");
+  return ensure_factor(sc);
 }
 
 // Uniform grid over the static obstacle faces for the detection's broad phase
@@ -2689,7 +2695,7 @@ constexpr int kClusterMaxSupernodes = 4096;
 // solves): the CTA size of every level-kernel launch, then the level-kernel
 // form, the persistent form and the split form at every cut level; keep the
 // fastest, then tune the per-iteration selection of batches.
-static int autotune_solve(dfem_scene* sc) {
+static int autotune_forms(dfem_scene* sc) {
   const size_t n3 = 3 * (size_t)sc->hs.N;
   RC(ensure_triangular(sc));
   CK(cudaMemsetAsync(sc->rhs.p, 0, n3 * sizeof(double), sc->stream));
@@ -2828,6 +2834,17 @@ static int autotune_solve(dfem_scene* sc) {
   RC(tune_solve_select(sc));
   invalidate_graphs(sc);
   return DFEM_OK;
+}
+
+static int autotune_solve(dfem_scene* sc) {
+  const int rc = autotune_forms(sc);
+  if (rc) {  // the persistent form, which every scene has
+    sc->solve_cut = 0;
+    sc->solve_select = false;
+    dense_release(sc);
+    invalidate_graphs(sc);
+  }
+  return rc;
 }
 
 // Device side of scene creation, once sc->hs (and sc->parts for a batch) is built.
@@ -3033,7 +3050,7 @@ int dfem_step_forward(dfem_scene* sc, const double* x, const double* v, const do
   if (!sc || !x || !v || !x_out || !v_out) return fail(DFEM_ERR_INVALID, "null argument");
   if (n_steps < 1) return fail(DFEM_ERR_INVALID, "n_steps must be >= 1");
   CK(cudaSetDevice(sc->device));
-  RC(require_moduli(sc));
+  RC(require_factor(sc));
   RC(ensure_steps(sc, n_steps));
   const HostScene& s = sc->hs;
   const size_t n3 = 3 * (size_t)s.N;
@@ -3179,6 +3196,7 @@ int dfem_step_backward(dfem_scene* sc, const double* gx_out, const double* gv_ou
   if (!sc || !gx_out || !gv_out || !gx || !gv) return fail(DFEM_ERR_INVALID, "null argument");
   if (sc->rec_steps <= 0) return fail(DFEM_ERR_STATE, "dfem_step_backward needs a preceding dfem_step_forward");
   CK(cudaSetDevice(sc->device));
+  RC(require_factor(sc));
   if (one_launch(sc)) {
     bool blocks = true;
     RC(ensure_adjoint_blocks(sc, &blocks));
@@ -3448,7 +3466,7 @@ int dfem_profile_levels(dfem_scene* sc, int32_t reps, int32_t cap, int32_t* n_se
   const int G = (int)sc->segs.size();
   *n_segments = G;
   if (!ms_fwd || !ms_bwd || cap < G) return DFEM_OK;
-  RC(require_moduli(sc));
+  if (!sc->moduli_ok) return require_factor(sc);
   RC(ensure_triangular(sc));
   cudaEvent_t e0, e1;
   CK(cudaEventCreate(&e0));
@@ -3490,7 +3508,7 @@ int dfem_solve_mode(dfem_scene* sc, int32_t request, int32_t* chosen, double* ms
   if (!sc) return fail(DFEM_ERR_INVALID, "null argument");
   if (request < -1 || request > 6) return fail(DFEM_ERR_INVALID, "request must be -1, 0, 1, 2, 3, 4, 5 or 6");
   CK(cudaSetDevice(sc->device));
-  if (request >= 0) RC(require_moduli(sc));
+  if (request >= 0 && !sc->moduli_ok) return require_factor(sc);
   if (request == 0) {
     CK(cudaStreamSynchronize(sc->stream));
     CK(cudaMemsetAsync(sc->status.p, 0, 4 * sizeof(int), sc->stream));
@@ -3508,12 +3526,17 @@ int dfem_solve_mode(dfem_scene* sc, int32_t request, int32_t* chosen, double* ms
     }
     const int c = request == 1 ? n_levels(sc) : request == 2 ? 0 : request == 3 ? sc->split_cut : request == 4 ? -1
                 : request == 5 ? -2 : -3;
-    if (c != sc->solve_cut || sc->solve_select) {  // a requested form is used in every iteration
-      sc->solve_cut = c;
+    const int before = sc->solve_cut;
+    sc->solve_cut = c;
+    const int rc = require_factor(sc);  // the forms' factors are built on demand
+    if (rc) {
+      sc->solve_cut = before;
+      return rc;
+    }
+    if (c != before || sc->solve_select) {  // a requested form is used in every iteration
       sc->solve_select = false;
       invalidate_graphs(sc);
     }
-    RC(ensure_factor(sc));  // the forms' factors are built on demand
   }
   if (chosen) *chosen = solve_form(sc);
   if (ms) { ms[0] = sc->solve_ms[0]; ms[1] = sc->solve_ms[1]; }
@@ -3565,6 +3588,7 @@ int dfem_profile_phases(dfem_scene* sc, int32_t reps, double* ms) {
   if (!sc || !ms || reps < 1) return fail(DFEM_ERR_INVALID, "bad argument");
   if (sc->rec_steps <= 0) return fail(DFEM_ERR_STATE, "dfem_profile_phases needs a preceding dfem_step_forward");
   CK(cudaSetDevice(sc->device));
+  RC(require_factor(sc));
   const HostScene& s = sc->hs;
   const int ncons = s.T + s.M + s.S + s.B;
   // every phase is launched ungated on the state of the last forward call (step 0, iteration 0)
