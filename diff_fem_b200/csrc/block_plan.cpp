@@ -46,25 +46,29 @@ void tiers_of(const SupernodalFactor& F, const Tree& t, const std::vector<int>& 
 }
 
 // model cost; the tiers that hold blocks are counted (a limit may leave one empty)
-double cost(const SupernodalFactor& F, const Tree& t, const std::vector<int>& taus) {
-  std::vector<int> tier, root;
-  tiers_of(F, t, taus, tier, root);
-  const int ns = F.nsuper, nt = (int)taus.size() + 1;
-  std::vector<int> n(ns, 0);
-  for (int q = 0; q < ns; ++q) n[root[q]] += F.sn_w[q];
-  double bytes = 0, flops = 0;
-  std::vector<int> piv(nt, 0);
-  for (int q = 0; q < ns; ++q)
-    if (root[q] == q) {
-      const double a = n[q], r = F.sn_r[q];
-      bytes += 8.0 * (a * a + 2 * a * r);
-      flops += 1.5 * (a + r) * (a + r) * a;
-      piv[tier[q]] = std::max(piv[tier[q]], (n[q] + kBlkPivot - 1) / kBlkPivot);
-    }
-  int used = 0, steps = 0;
-  for (int p : piv) { used += p > 0; steps += p; }
-  return (2 * used - 1) * kPhaseUs + bytes / kBytesPerUs + (steps * kPivotUs + flops / kFlopsPerUs) / kSolvesPerBuild;
-}
+struct CostModel {
+  const SupernodalFactor& F;
+  const Tree& t;
+  std::vector<int> tier, root, n;  // scratch: the search asks a few hundred times
+  double operator()(const std::vector<int>& taus) {
+    tiers_of(F, t, taus, tier, root);
+    const int ns = F.nsuper;
+    n.assign(ns, 0);
+    for (int q = 0; q < ns; ++q) n[root[q]] += F.sn_w[q];
+    double bytes = 0, flops = 0;
+    int piv[4] = {0, 0, 0, 0};  // at most three limits
+    for (int q = 0; q < ns; ++q)
+      if (root[q] == q) {
+        const double a = n[q], r = F.sn_r[q];
+        bytes += 8.0 * (a * a + 2 * a * r);
+        flops += 1.5 * (a + r) * (a + r) * a;
+        piv[tier[q]] = std::max(piv[tier[q]], (n[q] + kBlkPivot - 1) / kBlkPivot);
+      }
+    int used = 0, steps = 0;
+    for (int p : piv) { used += p > 0; steps += p; }
+    return (2 * used - 1) * kPhaseUs + bytes / kBytesPerUs + (steps * kPivotUs + flops / kFlopsPerUs) / kSolvesPerBuild;
+  }
+};
 
 int even(int v) { return (v + 1) & ~1; }
 
@@ -182,7 +186,9 @@ bool plan_blocks_with(const SupernodalFactor& F, const SparseSym& Hs, const std:
     P.tier_tile[P.blk[b].tier + 1] = (int)P.tiles.size();
   }
   // entries of Hs: (i, j) with j eliminated first (or in the same block, both halves of a diagonal tile)
-  std::vector<std::vector<std::pair<int, int>>> ent(P.tiles.size());
+  // in the order of their tiles, within a tile in their own order
+  const size_t nnz = (size_t)Hs.ptr[N], nt = P.tiles.size();
+  std::vector<int> at(nnz, -1), loc(nnz), hp(nt + 1, 0);
   for (int i = 0; i < N; ++i)
     for (int64_t k = Hs.ptr[i]; k < Hs.ptr[i + 1]; ++k) {
       const int j = Hs.col[k];
@@ -191,16 +197,28 @@ bool plan_blocks_with(const SupernodalFactor& F, const SparseSym& Hs, const std:
       if (fi < 0 || fj < 0) return false;
       const int I = fi / kBlkTile, J = fj / kBlkTile;
       if (I < J) continue;  // the other half of the symmetric matrix
-      ent[tile0[b] + I * (I + 1) / 2 + J].push_back({(int)k, (fi % kBlkTile) * kBlkTile + fj % kBlkTile});
+      at[k] = tile0[b] + I * (I + 1) / 2 + J;
+      loc[k] = (fi % kBlkTile) * kBlkTile + fj % kBlkTile;
+      hp[at[k] + 1]++;
     }
+  for (size_t q = 0; q < nt; ++q) hp[q + 1] += hp[q];
+  P.hs_idx.resize(hp[nt]);
+  P.hs_loc.resize(hp[nt]);
+  {
+    std::vector<int> f(hp.begin(), hp.end() - 1);
+    for (size_t k = 0; k < nnz; ++k)
+      if (at[k] >= 0) {
+        P.hs_idx[f[at[k]]] = (int)k;
+        P.hs_loc[f[at[k]]++] = loc[k];
+      }
+  }
   std::vector<std::vector<int>> kids(nb);
   for (int b = 0; b < nb; ++b)
     if (P.blk[b].parent >= 0) kids[P.blk[b].parent].push_back(b);
   for (size_t q = 0; q < P.tiles.size(); ++q) {
     BlockTile& T = P.tiles[q];
-    T.hs0 = (int)P.hs_idx.size();
-    for (auto& e : ent[q]) { P.hs_idx.push_back(e.first); P.hs_loc.push_back(e.second); }
-    T.hs1 = (int)P.hs_idx.size();
+    T.hs0 = hp[q];
+    T.hs1 = hp[q + 1];
     T.kid0 = (int)P.kids.size();
     for (int d : kids[T.blk]) {
       const int* m = P.rmap.data() + P.blk[d].rofs;
@@ -211,7 +229,6 @@ bool plan_blocks_with(const SupernodalFactor& F, const SparseSym& Hs, const std:
     }
     T.kid1 = (int)P.kids.size();
   }
-  P.est_us = cost(F, t, taus);
   return true;
 }
 
@@ -221,9 +238,10 @@ bool plan_blocks(const SupernodalFactor& F, const SparseSym& Hs, int64_t max_dou
   for (int c = 48; c < F.n; c = c * 4 / 3 + 1) cand.push_back(c);
   // thin the candidates of scenes with very many supernodes (the search is per candidate tuple and supernode)
   std::vector<int> best;
-  double bc = cost(F, t, {});
+  CostModel cost{F, t, {}, {}, {}};
+  double bc = cost({});
   auto consider = [&](const std::vector<int>& v) {
-    const double c = cost(F, t, v);
+    const double c = cost(v);
     if (c < bc) { bc = c; best = v; }
   };
   const size_t nc = cand.size(), step = F.nsuper > 4000 ? 2 : 1;

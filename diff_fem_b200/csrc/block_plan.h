@@ -70,7 +70,6 @@ struct BlockPlan {
   std::vector<BlockKid> kids;
   std::vector<int> hs_idx, hs_loc;              // entry of Hs (index into its values), place in the tile (row * kBlkTile + col)
   int64_t front_doubles = 0, panel_doubles = 0, solve_doubles = 0;
-  double est_us = 0.0;                          // the model's time per solve, with its share of a rebuild
 };
 
 // Chooses the tiers by the cost model and lays the blocks out.

@@ -172,17 +172,14 @@ struct dfem_scene {
   DenseDev dd{};
   int dense_grid = 1;                    // CTAs of the dense solve (one per SM at most)
   BlockPlan bplan;
-  DBuf<BlockInfo> bl_blk;
-  DBuf<BlockTile> bl_tiles;
-  DBuf<BlockKid> bl_kids;
-  DBuf<BlockChunk> bl_chunks;
-  DBuf<int> bl_tier_tile, bl_hs_idx, bl_hs_loc, bl_cols, bl_rows, bl_rmap, bl_cslot, bl_vptr, bl_share;
-  DBuf<double> bl_front, bl_panel, bl_sol, bl_piv, bl_contrib;
+  DBuf<int> bl_tab;                      // its tables, one behind the other
+  DBuf<double> bl_mem;                   // fronts, panels, products, pivot inverses, contributions
   DBuf<unsigned> bl_bar;
   BlockDev bd{};
   bool bl_cluster = false;               // the solve runs in one cluster (small scenes), else on the whole grid
-  // steps in one launch (step_kernels.cuh)
-  bool ps_ok = false;
+  bool blk_failed = false;               // ... a pivot of theirs failed for the current moduli: the adjoint solves with X
+  // steps in one launch (step_kernels.cuh): the forward, the adjoint
+  bool ps_fwd = false, ps_adj = false;
   int ps_tab = 0, ps_res_f = 0, ps_res_a = 0, ps_tape_warps = 1;
   size_t ps_smem_f = 0, ps_smem_a = 0;
   DBuf<double> xk2, ps_partial;
@@ -804,20 +801,24 @@ constexpr int kDenseMaxN = 4096;
 static bool dense_is_x(const dfem_scene* sc) { return sc->hs.precision == DFEM_PREC_MIXED; }
 constexpr int kBlockClusterCtas = 16;
 
+// The blocks' buffers (all of them: a failed block_prepare leaves none behind).
+static void block_release(dfem_scene* sc) {
+  sc->bl_tab.alloc(0);
+  sc->bl_mem.alloc(0);
+  sc->bplan = BlockPlan();
+  sc->blk_built = sc->ps_adj = false;
+  if (!dense_is_x(sc)) sc->ps_fwd = false;
+  sc->bd.blk = nullptr;
+}
+
 static void dense_release(dfem_scene* sc) {
   sc->dn_A.alloc(0);
   sc->dn_W.alloc(0);
   sc->dn_T.alloc(0);
   sc->dn_Linv.alloc(0);
   sc->dd = DenseDev{};
-  sc->bl_front.alloc(0);
-  sc->bl_panel.alloc(0);
-  sc->bl_sol.alloc(0);
-  sc->bl_piv.alloc(0);
-  sc->bl_contrib.alloc(0);
-  sc->dense_built = sc->blk_built = false;
-  sc->ps_ok = false;
-  sc->bd = BlockDev{};
+  block_release(sc);
+  sc->dense_built = sc->ps_fwd = false;
 }
 
 template <class... Args>
@@ -906,62 +907,7 @@ static int dense_x_build(dfem_scene* sc) {
 
 static size_t block_solve_smem(const dfem_scene* sc) { return sizeof(double) * block_solve_doubles(sc->bd.vec); }
 
-// Shared memory of the step kernels: the index tables and rows of a CTA's
-// shares (as many rows as fit), and the adjoint's tape.
-static int plan_steps(dfem_scene* sc, int vec, int G, const std::vector<BlockChunk>& chunks,
-                      const std::vector<int>& share) {
-  const HostScene& s = sc->hs;
-  const BlockPlan& P = sc->bplan;
-  const int phases = 2 * P.tiers - 1;
-  constexpr size_t kMaxSmem = 224 * 1024 / sizeof(double);  // doubles
-  constexpr int kMaxTab = 8192;
-  sc->ps_ok = false;
-  int tab = 0;
-  size_t rows = 0;
-  for (int c = 0; c < G; ++c) {
-    int nch = 0, ti = 0;
-    size_t rd = 0;
-    for (int p = 0; p < phases; ++p)
-      for (int k = share[(size_t)p * (G + 1) + c]; k < share[(size_t)p * (G + 1) + c + 1]; ++k) {
-        const BlockInfo& B = P.blk[chunks[k].blk];
-        const bool fwd = p < P.tiers;
-        ++nch;
-        ti += ((fwd && B.tier > 0) ? 3 : 1) * (fwd ? B.n : B.r) + chunks[k].rows;
-        rd += (size_t)chunks[k].rows * (fwd ? B.ldx : B.ldr);
-      }
-    if (nch > kPsChunks) return DFEM_OK;
-    tab = std::max(tab, ti);
-    rows = std::max(rows, rd);
-  }
-  if (phases > 31) return DFEM_OK;
-  sc->ps_tab = std::min((tab + 3) & ~3, kMaxTab);
-  sc->ps_tape_warps = std::max(1, std::min(kPsWarps / 2, (s.T + 32 * G - 1) / (32 * G)));
-  const size_t fixed = ps_fixed_doubles(vec) + sc->ps_tab / 2, tape = (size_t)kVolTape * 32 * sc->ps_tape_warps;
-  if (fixed + tape > kMaxSmem) return DFEM_OK;
-  rows = (rows + 1) & ~size_t(1);
-  sc->ps_res_f = (int)std::min(rows, kMaxSmem - fixed);
-  sc->ps_res_a = (int)std::min(rows, kMaxSmem - fixed - tape);
-  sc->ps_smem_f = (fixed + sc->ps_res_f) * sizeof(double);
-  if (dense_is_x(sc)) {  // the forward's solve: planes of N_p, the CTA's rows of X if they fit
-    const size_t np = (size_t)sc->dd.Np, fx = ps_fixed_doubles((int)np) - kPsXch * kPsPair;
-    if (fx > kMaxSmem) return DFEM_OK;
-    sc->ps_res_f = (int)(std::min(((size_t)s.N + G - 1) / G, (kMaxSmem - fx) / np) * np);
-    sc->ps_smem_f = (fx + sc->ps_res_f) * sizeof(double);
-  }
-  sc->ps_smem_a = (fixed + tape + sc->ps_res_a) * sizeof(double);
-  for (auto fn : {(const void*)k_pd_forward<GridBarrier, false>, (const void*)k_pd_forward<GridBarrier, true>,
-                  (const void*)k_pd_forward<ClusterBarrier, false>, (const void*)k_pd_forward<ClusterBarrier, true>})
-    CK(raise_smem_limit(fn, sc->ps_smem_f));
-  for (auto fn : {(const void*)k_pd_adjoint<GridBarrier>, (const void*)k_pd_adjoint<ClusterBarrier>})
-    CK(raise_smem_limit(fn, sc->ps_smem_a));
-  for (auto fn : {(const void*)k_pd_forward<ClusterBarrier, false>, (const void*)k_pd_forward<ClusterBarrier, true>,
-                  (const void*)k_pd_adjoint<ClusterBarrier>})
-    CK(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-  CK(sc->xk2.alloc(3 * (size_t)s.N));
-  CK(sc->ps_partial.alloc(2 * (size_t)G));
-  sc->ps_ok = true;
-  return DFEM_OK;
-}
+constexpr size_t kPsMaxSmem = 224 * 1024 / sizeof(double);  // doubles of a step kernel's CTA
 
 // Whether the device schedules a 16-CTA cluster of the solve.
 static bool cluster_fits() {
@@ -985,106 +931,195 @@ static bool cluster_fits() {
   return ok;
 }
 
-// Buffers, tables and launch shapes of the dense form (block-inverse: single
-// scenes whose plan fits an eighth of the free memory); false: not a candidate.
-static int block_prepare(dfem_scene* sc, bool* ok) {
-  *ok = false;
+// What the step kernels and the block solve share: one cluster or the grid
+// (bd.G CTAs), the barrier, the iterate's other buffer and the partial sums.
+// *ok: false when the device has no cooperative launches.
+static int launch_shape(dfem_scene* sc, bool* ok) {
+  int coop = 0, nsm = 1;
+  CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, sc->device));
+  CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, sc->device));
+  *ok = coop != 0;
+  if (!coop || sc->bd.bar) return DFEM_OK;
+  // One cluster or the grid: a barrier of the cluster takes 0.25 us, of the
+  // grid 1.2 us, three per iteration, but sixteen SMs run the elements of a
+  // larger scene in turns and stream a larger inverse through less of L2.
+  // Forward + adjoint per iteration, grid / cluster: 144 vertices (cloth)
+  // 26.2 / 20.9 us, 275 (800 tets) 26.9 / 23.1, 396 (1,250 tets) 30.3 /
+  // 27.9, 484 (cloth) 30.9 / 26.9, 961 (cloth) 35.7 / 46.7, 1,029 (3,600
+  // tets) 35.4 / 59.
+  sc->bl_cluster = sc->hs.N <= 512 && sc->hs.T <= 2048 && cluster_fits();
+  const int G = sc->bl_cluster ? kBlockClusterCtas : nsm;
+  CK(sc->xk2.alloc(3 * (size_t)sc->hs.N));
+  CK(sc->ps_partial.alloc(2 * (size_t)G));
+  CK(sc->bl_bar.alloc(2));
+  CK(cudaMemset(sc->bl_bar.p, 0, 2 * sizeof(unsigned)));
+  sc->bd.N = sc->hs.N;
+  sc->bd.G = G;
+  sc->bd.bar = sc->bl_bar.p;
+  sc->bd.status = sc->status.p;
+  sc->bd.spin_tries = sc->spin_tries;
+  return DFEM_OK;
+}
+
+// The mixed form's forward in one launch: planes of N_p and as many of a CTA's
+// rows of X as fit.
+static int plan_mixed_forward(dfem_scene* sc) {
+  sc->ps_fwd = false;
+  bool ok = false;
+  RC(launch_shape(sc, &ok));
+  const size_t np = (size_t)sc->dd.Np, G = (size_t)sc->bd.G, fx = ps_fixed_doubles((int)np) - kPsXch * kPsPair;
+  if (!ok || fx > kPsMaxSmem) return DFEM_OK;
+  sc->ps_res_f = (int)(std::min(((size_t)sc->hs.N + G - 1) / G, (kPsMaxSmem - fx) / np) * np);
+  sc->ps_smem_f = (fx + sc->ps_res_f) * sizeof(double);
+  for (auto fn : {(const void*)k_pd_forward<GridBarrier, true>, (const void*)k_pd_forward<ClusterBarrier, true>})
+    CK(raise_smem_limit(fn, sc->ps_smem_f));
+  CK(cudaFuncSetAttribute((const void*)k_pd_forward<ClusterBarrier, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  sc->ps_fwd = true;
+  return DFEM_OK;
+}
+
+// Shared memory of the step kernels that solve with blocks (FP64 forwards,
+// every adjoint): the index tables and rows of a CTA's shares (as many rows as
+// fit), and the adjoint's tape.
+static int plan_steps(dfem_scene* sc, int vec, int G, const std::vector<BlockChunk>& chunks,
+                      const std::vector<int>& share) {
+  const HostScene& s = sc->hs;
+  const BlockPlan& P = sc->bplan;
+  const int phases = 2 * P.tiers - 1;
+  constexpr size_t kMaxSmem = kPsMaxSmem;
+  constexpr int kMaxTab = 8192;
+  const bool mx = dense_is_x(sc);
+  sc->ps_adj = false;
+  if (!mx) sc->ps_fwd = false;
+  int tab = 0;
+  size_t rows = 0;
+  for (int c = 0; c < G; ++c) {
+    int nch = 0, ti = 0;
+    size_t rd = 0;
+    for (int p = 0; p < phases; ++p)
+      for (int k = share[(size_t)p * (G + 1) + c]; k < share[(size_t)p * (G + 1) + c + 1]; ++k) {
+        const BlockInfo& B = P.blk[chunks[k].blk];
+        const bool fwd = p < P.tiers;
+        ++nch;
+        ti += ((fwd && B.tier > 0) ? 3 : 1) * (fwd ? B.n : B.r) + chunks[k].rows;
+        rd += (size_t)chunks[k].rows * (fwd ? B.ldx : B.ldr);
+      }
+    if (nch > kPsChunks) return DFEM_OK;
+    tab = std::max(tab, ti);
+    rows = std::max(rows, rd);
+  }
+  if (phases > 31) return DFEM_OK;
+  sc->ps_tab = std::min((tab + 3) & ~3, kMaxTab);
+  sc->ps_tape_warps = std::max(1, std::min(kPsWarps / 2, (s.T + 32 * G - 1) / (32 * G)));
+  const size_t fixed = ps_fixed_doubles(vec) + sc->ps_tab / 2, tape = (size_t)kVolTape * 32 * sc->ps_tape_warps;
+  if (fixed + tape > kMaxSmem) return DFEM_OK;
+  rows = (rows + 1) & ~size_t(1);
+  if (!mx) {
+    sc->ps_res_f = (int)std::min(rows, kMaxSmem - fixed);
+    sc->ps_smem_f = (fixed + sc->ps_res_f) * sizeof(double);
+    for (auto fn : {(const void*)k_pd_forward<GridBarrier, false>, (const void*)k_pd_forward<ClusterBarrier, false>})
+      CK(raise_smem_limit(fn, sc->ps_smem_f));
+    CK(cudaFuncSetAttribute((const void*)k_pd_forward<ClusterBarrier, false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  }
+  sc->ps_res_a = (int)std::min(rows, kMaxSmem - fixed - tape);
+  sc->ps_smem_a = (fixed + tape + sc->ps_res_a) * sizeof(double);
+  for (auto fn : {(const void*)k_pd_adjoint<GridBarrier>, (const void*)k_pd_adjoint<ClusterBarrier>})
+    CK(raise_smem_limit(fn, sc->ps_smem_a));
+  CK(cudaFuncSetAttribute((const void*)k_pd_adjoint<ClusterBarrier>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  sc->ps_adj = true;
+  if (!mx) sc->ps_fwd = true;
+  return DFEM_OK;
+}
+
+// Plan, tables and buffers of the blocks: the plan has to fit an eighth of the
+// free memory.  *ok: false when the scene has no block form.
+static int block_buffers(dfem_scene* sc, bool* ok) {
   BlockPlan& P = sc->bplan;
   const bool mx = dense_is_x(sc);
-  if (sc->bd.blk == nullptr) {
-    size_t free_b = 0, total_b = 0;
-    CK(cudaMemGetInfo(&free_b, &total_b));
-    if (!plan_blocks(sc->hs.F, sc->hs.Hs, (int64_t)(free_b / 8 / sizeof(double)), P)) return DFEM_OK;
-    const bool view = mx && P.tiers == 1;  // the one block is X itself
-    if (view) {
-      P.blk[0].ldx = sc->dd.Np;
-      P.blk[0].xp = 0;
-      P.front_doubles = P.panel_doubles = P.solve_doubles = 0;
-    }
-    int vec = 2, coop = 0, nsm = 1, occ = 0;
-    for (const BlockInfo& B : P.blk) vec = std::max({vec, B.ldx, B.ldr});
-    CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, sc->device));
-    CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, sc->device));
-    const size_t smem = sizeof(double) * block_solve_doubles(vec);
-    if (!coop || smem > 220 * 1024) return DFEM_OK;
-    CK(raise_smem_limit((const void*)k_block_factor, kBfSmem));
-    CK(raise_smem_limit((const void*)k_block_solve<GridBarrier>, smem));
-    CK(raise_smem_limit((const void*)k_block_solve<ClusterBarrier>, smem));
-    CK(cudaFuncSetAttribute((const void*)k_block_solve<ClusterBarrier>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_block_factor, kBfThreads, kBfSmem));
-    if (occ < 1) return DFEM_OK;
-    int most = 1;
-    for (int t = 0; t < P.tiers; ++t) most = std::max(most, P.tier_tile[t + 1] - P.tier_tile[t]);
-    sc->bf_grid = std::min(nsm * occ, most);
-    // One cluster or the grid: a barrier of the cluster takes 0.25 us, of the
-    // grid 1.2 us, three per iteration, but sixteen SMs run the elements of a
-    // larger scene in turns and stream a larger inverse through less of L2.
-    // Forward + adjoint per iteration, grid / cluster: 144 vertices (cloth)
-    // 26.2 / 20.9 us, 275 (800 tets) 26.9 / 23.1, 396 (1,250 tets) 30.3 /
-    // 27.9, 484 (cloth) 30.9 / 26.9, 961 (cloth) 35.7 / 46.7, 1,029 (3,600
-    // tets) 35.4 / 59.
-    sc->bl_cluster = sc->hs.N <= 512 && sc->hs.T <= 2048 && cluster_fits();
-    const int G = sc->bl_cluster ? kBlockClusterCtas : nsm;
-    std::vector<BlockChunk> chunks;
-    std::vector<int> share;
-    block_shares(P, G, chunks, share);
-    if (chunks.empty()) return DFEM_OK;
-    auto some = [](std::vector<int> v) { if (v.empty()) v.push_back(0); return v; };
-    if (P.kids.empty()) P.kids.push_back(BlockKid{0, 0, 0, 0, 0});
-    CK(sc->bl_blk.upload(P.blk));
-    CK(sc->bl_tiles.upload(P.tiles));
-    CK(sc->bl_kids.upload(P.kids));
-    CK(sc->bl_chunks.upload(chunks));
-    CK(sc->bl_share.upload(share));
-    CK(sc->bl_tier_tile.upload(P.tier_tile));
-    CK(sc->bl_hs_idx.upload(some(P.hs_idx)));
-    CK(sc->bl_hs_loc.upload(some(P.hs_loc)));
-    CK(sc->bl_cols.upload(P.cols));
-    CK(sc->bl_rows.upload(some(P.rows)));
-    CK(sc->bl_rmap.upload(some(P.rmap)));
-    CK(sc->bl_cslot.upload(some(P.cslot)));
-    CK(sc->bl_vptr.upload(P.vptr));
-    // all buffers or none: a failed allocation leaves none behind
-    cudaError_t e = sc->bl_front.alloc(P.front_doubles);
-    if (e == cudaSuccess) e = sc->bl_panel.alloc(P.panel_doubles);
-    if (e == cudaSuccess) e = sc->bl_sol.alloc(P.solve_doubles);
-    if (e == cudaSuccess) e = sc->bl_piv.alloc(2 * P.blk.size() * kBlkPivot * kBlkPivot);
-    if (e == cudaSuccess) e = sc->bl_contrib.alloc(3 * std::max<size_t>(1, P.rows.size()));
-    if (e == cudaSuccess) e = sc->bl_bar.alloc(2);
-    if (e == cudaSuccess) e = cudaMemset(sc->bl_bar.p, 0, 2 * sizeof(unsigned));
-    if (e == cudaSuccess && !view) e = cudaMemset(sc->bl_sol.p, 0, P.solve_doubles * sizeof(double));  // the rows' padding stays 0
-    if (e != cudaSuccess) {
-      if (!mx) dense_release(sc);
-      CK(e);
-    }
-    RC(plan_steps(sc, vec, G, chunks, share));
-    BlockDev d{};
-    d.N = sc->hs.N; d.tiers = P.tiers; d.nblk = (int)P.blk.size(); d.G = G;
-    d.blk = sc->bl_blk.p; d.tiles = sc->bl_tiles.p; d.tier_tile = sc->bl_tier_tile.p; d.kids = sc->bl_kids.p;
-    d.hs_idx = sc->bl_hs_idx.p; d.hs_loc = sc->bl_hs_loc.p; d.cols = sc->bl_cols.p; d.rows = sc->bl_rows.p;
-    d.rmap = sc->bl_rmap.p; d.cslot = sc->bl_cslot.p; d.vptr = sc->bl_vptr.p; d.chunks = sc->bl_chunks.p;
-    d.share = sc->bl_share.p; d.front = sc->bl_front.p; d.panel = sc->bl_panel.p; d.sol = view ? sc->dn_A.p : sc->bl_sol.p;
-    d.piv = sc->bl_piv.p; d.contrib = sc->bl_contrib.p; d.bar = sc->bl_bar.p; d.status = sc->status.p; d.spin_tries = sc->spin_tries;
-    d.vec = vec;
-    sc->bd = d;
+  bool coop = false;
+  RC(launch_shape(sc, &coop));
+  if (!coop) return DFEM_OK;
+  size_t free_b = 0, total_b = 0;
+  CK(cudaMemGetInfo(&free_b, &total_b));
+  if (!plan_blocks(sc->hs.F, sc->hs.Hs, (int64_t)(free_b / 8 / sizeof(double)), P)) return DFEM_OK;
+  const bool view = mx && P.tiers == 1;  // the one block is X itself
+  if (view) {
+    P.blk[0].ldx = sc->dd.Np;
+    P.blk[0].xp = 0;
+    P.front_doubles = P.panel_doubles = P.solve_doubles = 0;
   }
+  int vec = 2, nsm = 1, occ = 0;
+  for (const BlockInfo& B : P.blk) vec = std::max({vec, B.ldx, B.ldr});
+  CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, sc->device));
+  const size_t smem = sizeof(double) * block_solve_doubles(vec);
+  if (smem > 220 * 1024) return DFEM_OK;
+  CK(raise_smem_limit((const void*)k_block_factor, kBfSmem));
+  CK(raise_smem_limit((const void*)k_block_solve<GridBarrier>, smem));
+  CK(raise_smem_limit((const void*)k_block_solve<ClusterBarrier>, smem));
+  CK(cudaFuncSetAttribute((const void*)k_block_solve<ClusterBarrier>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_block_factor, kBfThreads, kBfSmem));
+  if (occ < 1) return DFEM_OK;
+  int most = 1;
+  for (int t = 0; t < P.tiers; ++t) most = std::max(most, P.tier_tile[t + 1] - P.tier_tile[t]);
+  sc->bf_grid = std::min(nsm * occ, most);
+  const int G = sc->bd.G;
+  std::vector<BlockChunk> chunks;
+  std::vector<int> share;
+  block_shares(P, G, chunks, share);
+  if (chunks.empty()) return DFEM_OK;
+  // one allocation and copy for the tables, one for the values (each section on 16 bytes)
+  std::vector<int> tab;
+  auto put = [&](const auto& v) -> size_t {
+    const size_t at = (tab.size() + 3) & ~size_t(3), n = v.size() * sizeof(v[0]) / sizeof(int);
+    tab.resize(at + std::max<size_t>(1, n));
+    if (n) std::memcpy(tab.data() + at, v.data(), n * sizeof(int));
+    return at;
+  };
+  const size_t t_blk = put(P.blk), t_tiles = put(P.tiles), t_kids = put(P.kids), t_chunks = put(chunks),
+               t_share = put(share), t_tt = put(P.tier_tile), t_hsi = put(P.hs_idx), t_hsl = put(P.hs_loc), t_cols = put(P.cols),
+               t_rows = put(P.rows), t_rmap = put(P.rmap), t_cslot = put(P.cslot), t_vptr = put(P.vptr);
+  CK(sc->bl_tab.upload(tab));
+  size_t dn = 0;
+  auto take = [&](size_t n) { const size_t at = dn; dn += (n + 1) & ~size_t(1); return at; };
+  const size_t d_sol = take(P.solve_doubles), d_front = take(P.front_doubles), d_panel = take(P.panel_doubles),
+               d_piv = take(2 * P.blk.size() * kBlkPivot * kBlkPivot), d_con = take(3 * std::max<size_t>(1, P.rows.size()));
+  CK(sc->bl_mem.alloc(dn));
+  if (!view) CK(cudaMemset(sc->bl_mem.p + d_sol, 0, P.solve_doubles * sizeof(double)));  // the rows' padding stays 0
+  RC(plan_steps(sc, vec, G, chunks, share));
+  BlockDev d = sc->bd;
+  d.tiers = P.tiers; d.nblk = (int)P.blk.size();
+  const int* T = sc->bl_tab.p;
+  double* M = sc->bl_mem.p;
+  d.blk = reinterpret_cast<const BlockInfo*>(T + t_blk); d.tiles = reinterpret_cast<const BlockTile*>(T + t_tiles);
+  d.kids = reinterpret_cast<const BlockKid*>(T + t_kids); d.chunks = reinterpret_cast<const BlockChunk*>(T + t_chunks);
+  d.share = T + t_share; d.tier_tile = T + t_tt; d.hs_idx = T + t_hsi; d.hs_loc = T + t_hsl; d.cols = T + t_cols;
+  d.rows = T + t_rows; d.rmap = T + t_rmap; d.cslot = T + t_cslot; d.vptr = T + t_vptr;
+  d.sol = view ? sc->dn_A.p : M + d_sol; d.front = M + d_front; d.panel = M + d_panel; d.piv = M + d_piv; d.contrib = M + d_con;
+  d.vec = vec;
+  sc->bd = d;
   *ok = true;
   return DFEM_OK;
 }
 
+static int block_prepare(dfem_scene* sc, bool* ok) {
+  *ok = sc->bd.blk != nullptr;
+  if (*ok) return DFEM_OK;
+  const int rc = block_buffers(sc, ok);
+  if (!*ok) block_release(sc);
+  return rc;
+}
+
+// Buffers and launch shapes of the dense form (single scenes); false: not a
+// candidate.  Mixed scenes: X, and the forward in one launch if it fits; the
+// adjoint's blocks wait for the first adjoint.
 static int dense_prepare(dfem_scene* sc, bool* ok) {
   *ok = false;
   if (sc->hs.nparts != 1 || sc->hs.F.nsuper == 0) return DFEM_OK;
   if (!dense_is_x(sc)) return block_prepare(sc, ok);
   RC(dense_x_prepare(sc, ok));
-  if (*ok && !sc->bd.blk) {  // steps in one launch, with the blocks (or X) in the adjoint: left out if they do not fit
-    bool b = false;
-    if (block_prepare(sc, &b) != DFEM_OK || !b) {
-      cudaGetLastError();
-      g_last_error.clear();
-      sc->ps_ok = false;
-      sc->bd = BlockDev{};
-    }
+  if (*ok && !sc->ps_fwd && plan_mixed_forward(sc) != DFEM_OK) {
+    cudaGetLastError();
+    g_last_error.clear();
   }
   return DFEM_OK;
 }
@@ -1189,24 +1224,32 @@ static int ensure_factor(dfem_scene* sc) {
   return factor_values(sc, dense);
 }
 
-// Mixed scenes whose adjoint solves with blocks: built once per material
-// change, by the first adjoint after it (X's regularisation).  *ok: false
-// when a pivot fails, the adjoint then takes the graph form.
-static int ensure_adjoint_blocks(dfem_scene* sc, bool* ok) {
-  *ok = true;
-  if (!dense_is_x(sc) || sc->bplan.tiers == 1 || sc->blk_built) return DFEM_OK;
+// Mixed scenes: the blocks their adjoint solves with, prepared by the first
+// adjoint and built once per material change (with X's regularisation).
+// Without them (no room, a failed pivot: tried again after the next material
+// change) the adjoint takes the graph form, with X.
+static int ensure_adjoint_blocks(dfem_scene* sc) {
+  if (!dense_is_x(sc) || sc->blk_failed) return DFEM_OK;
+  if (!sc->bd.blk) {
+    bool ok = false;
+    const int rc = block_prepare(sc, &ok);
+    if (rc != DFEM_OK && rc != DFEM_ERR_NOMEM) return rc;
+    if (!ok) {
+      cudaGetLastError();
+      g_last_error.clear();
+      sc->blk_failed = true;
+      return DFEM_OK;
+    }
+  }
+  if (!sc->ps_adj || sc->bplan.tiers == 1 || sc->blk_built) return DFEM_OK;
   int bad = 0;
   CK(cudaMemsetAsync(sc->part_fail.p, 0, 2 * sizeof(int), sc->stream));
   RC(dense_build(sc));
   CK(cudaMemcpyAsync(&bad, sc->part_fail.p, sizeof(int), cudaMemcpyDeviceToHost, sc->stream));
   CK(cudaStreamSynchronize(sc->stream));
   RC(check_build(sc, bad));
-  *ok = bad == 0;
-  if (bad) {
-    sc->ps_ok = false;
-    invalidate_graphs(sc);
-  }
   sc->blk_built = bad == 0;
+  sc->blk_failed = bad != 0;
   return DFEM_OK;
 }
 
@@ -1224,7 +1267,7 @@ static int gpu_refactor(dfem_scene* sc) {
   const HostScene& s = sc->hs;
   const int np = s.nparts;
   const std::vector<double> reg = sc->part_reg_h;
-  const bool dense = sc->dense_built, tri = sc->tri_built, blk = sc->blk_built, ok = sc->moduli_ok;
+  const bool dense = sc->dense_built, tri = sc->tri_built, blk = sc->blk_built, ok = sc->moduli_ok, bad = sc->blk_failed;
   CK(cudaMemsetAsync(sc->part_fail.p, 0, sizeof(int) * (np + 1), sc->stream));
   if (s.T > 0) {
     k_check_materials<<<(s.T + 127) / 128, 128, 0, sc->stream>>>(sc->rd, sc->E_in.p, sc->nu_in.p);
@@ -1233,7 +1276,7 @@ static int gpu_refactor(dfem_scene* sc) {
   k_hs_values<<<(sc->rd.nnz + 255) / 256, 256, 0, sc->stream>>>(sc->rd);
   sc->launches += (s.T > 0 ? 2 : 0) + 1;
   std::fill(sc->part_reg_h.begin(), sc->part_reg_h.end(), 0.0);
-  sc->dense_built = sc->tri_built = sc->blk_built = sc->moduli_ok = false;
+  sc->dense_built = sc->tri_built = sc->blk_built = sc->moduli_ok = sc->blk_failed = false;
   const int rc = factor_values(sc, sc->solve_cut == -3);
   if (rc == DFEM_ERR_INVALID) {
     sc->part_reg_h = reg;
@@ -1242,6 +1285,7 @@ static int gpu_refactor(dfem_scene* sc) {
     sc->tri_built = tri;
     sc->blk_built = blk;
     sc->moduli_ok = ok;
+    sc->blk_failed = bad;
   } else if (rc != DFEM_OK) {
     sc->rec_steps = 0;
   } else {
@@ -1975,11 +2019,13 @@ static void launch_adj_gather(dfem_scene* sc, cudaStream_t st, Gate g) {
     k_adj_gather<<<(sc->hs.N + 3) / 4, 128, 0, st>>>(sc->hs.N, g, sc->vpart.p, sc->vslot_ptr.p, sc->slot.p, sc->xkb.p);
 }
 
-// Scenes whose steps run in one launch: the block-inverse solve, no links, drag
-// or soft contact.
-static bool one_launch(const dfem_scene* sc) {
-  return sc->solve_cut == -3 && sc->ps_ok && sc->bd.blk && sc->hs.nparts == 1 && !sc->skel_on && sc->nF == 0 && !sc->self_contact;
+// Scenes whose steps (forward, adjoint) run in one launch: the dense form, no
+// links, drag or soft contact.
+static bool step_scene(const dfem_scene* sc) {
+  return sc->solve_cut == -3 && sc->hs.nparts == 1 && !sc->skel_on && sc->nF == 0 && !sc->self_contact;
 }
+static bool one_launch(const dfem_scene* sc) { return step_scene(sc) && sc->ps_fwd; }
+static bool one_launch_adj(const dfem_scene* sc) { return step_scene(sc) && sc->ps_adj && !sc->blk_failed; }
 
 static PdSteps steps_args(dfem_scene* sc, int n, int s0) {
   PdSteps a{};
@@ -2274,8 +2320,8 @@ static int build_loop_graph(dfem_scene* sc, const std::vector<LoopStage>& stages
   return DFEM_OK;
 }
 
-static int ensure_graphs(dfem_scene* sc) {
-  if (one_launch(sc) && !sc->has_contact) return DFEM_OK;  // no graphs: k_pd_forward / k_pd_adjoint
+static int ensure_step_graph(dfem_scene* sc) {
+  if (one_launch(sc) && !sc->has_contact) return DFEM_OK;  // no graph: k_pd_forward
   if (!sc->g_step.exec) {
     std::vector<LoopStage> st;
     if (one_launch(sc)) st.push_back({step_loop, nullptr});
@@ -2283,7 +2329,11 @@ static int ensure_graphs(dfem_scene* sc) {
     if (sc->has_contact && !fused_contact(sc)) st.push_back({contact_pre, contact_body});
     RC(build_loop_graph(sc, st, step_post, &sc->g_step));
   }
-  if (!sc->g_adj.exec && !one_launch(sc)) RC(build_loop_graph(sc, {{adj_pre, adj_body}}, adj_post, &sc->g_adj));
+  return DFEM_OK;
+}
+
+static int ensure_adjoint_graph(dfem_scene* sc) {
+  if (!sc->g_adj.exec && !one_launch_adj(sc)) RC(build_loop_graph(sc, {{adj_pre, adj_body}}, adj_post, &sc->g_adj));
   return DFEM_OK;
 }
 
@@ -2299,7 +2349,7 @@ static int run_step(dfem_scene* sc, int st) {
 
 // The reverse of step st's iterations, in place on io_a / io_b.
 static int run_adjoint(dfem_scene* sc, int st) {
-  if (one_launch(sc)) {
+  if (one_launch_adj(sc)) {
     CK(launch_steps(sc, sc->stream, steps_args(sc, 1, st), true));
     return DFEM_OK;
   }
@@ -2830,7 +2880,7 @@ static int autotune_forms(dfem_scene* sc) {
     if (sc->solve_ms[4] > 0.0 && sc->solve_ms[4] < best) { sc->solve_cut = -2; best = sc->solve_ms[4]; }
     if (sc->solve_ms[5] > 0.0 && (best - sc->solve_ms[5]) * kDenseAmortSolves > sc->dense_build_ms) sc->solve_cut = -3;
   }
-  if (sc->solve_cut != -3 && (sc->bl_sol.p || sc->dn_A.p)) dense_release(sc);
+  if (sc->solve_cut != -3 && (sc->bl_mem.p || sc->dn_A.p)) dense_release(sc);
   RC(tune_solve_select(sc));
   invalidate_graphs(sc);
   return DFEM_OK;
@@ -3138,7 +3188,7 @@ int dfem_step_forward(dfem_scene* sc, const double* x, const double* v, const do
     CK(cudaStreamSynchronize(sc->stream));  // `on` is a host local
   }
   CK(cudaGetLastError());
-  RC(ensure_graphs(sc));
+  RC(ensure_step_graph(sc));
   for (int st = 0; st < n_steps; ++st) CK(cudaGraphLaunch(sc->g_step.exec, sc->stream));
   k_to_user<<<nb, 128, 0, sc->stream>>>(s.N, sc->to_user.p, sc->xt.p, sc->io_a.p);
   k_to_user<<<nb, 128, 0, sc->stream>>>(s.N, sc->to_user.p, sc->vt.p, sc->io_b.p);
@@ -3197,10 +3247,7 @@ int dfem_step_backward(dfem_scene* sc, const double* gx_out, const double* gv_ou
   if (sc->rec_steps <= 0) return fail(DFEM_ERR_STATE, "dfem_step_backward needs a preceding dfem_step_forward");
   CK(cudaSetDevice(sc->device));
   RC(require_factor(sc));
-  if (one_launch(sc)) {
-    bool blocks = true;
-    RC(ensure_adjoint_blocks(sc, &blocks));
-  }
+  if (step_scene(sc)) RC(ensure_adjoint_blocks(sc));
   const int nq = sc->sk_nq;
   // the joint state a replayed step starts from (restored to the forward's final one at the end)
   auto joint_state_at = [&](int st) -> int {
@@ -3256,7 +3303,7 @@ int dfem_step_backward(dfem_scene* sc, const double* gx_out, const double* gv_ou
   const HostScene& s = sc->hs;
   const size_t n3 = 3 * (size_t)s.N;
   const int nb = sc->nblk_v;
-  if (one_launch(sc) && !sc->has_contact && sc->hist_step != 0) {  // every step's iterates are stored: one launch
+  if (one_launch_adj(sc) && !sc->has_contact && sc->hist_step != 0) {  // every step's iterates are stored: one launch
     PdSteps a = steps_args(sc, sc->rec_steps, 0);
     a.zero = 1;
     a.x_in = gx_out; a.v_in = gv_out; a.x_out = gx; a.v_out = gv;
@@ -3292,7 +3339,8 @@ int dfem_step_backward(dfem_scene* sc, const double* gx_out, const double* gv_ou
   k_set_int<<<1, 1, 0, sc->stream>>>(sc->write_traj.p, 0);
   CK(cudaMemsetAsync(sc->status.p, 0, 4 * sizeof(int), sc->stream));
   reset_solve_state(sc);
-  RC(ensure_graphs(sc));
+  RC(ensure_step_graph(sc));
+  RC(ensure_adjoint_graph(sc));
   if (any_contact) {
     k_set_int<<<1, 1, 0, sc->stream>>>(sc->crec_on.p, 1);
     k_set_int<<<1, 1, 0, sc->stream>>>(sc->crec_base.p, rbase);
