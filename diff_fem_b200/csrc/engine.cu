@@ -790,6 +790,12 @@ static int upload_refactor_plan(dfem_scene* sc) {
 // The dense form is kept when its saving per solve, over this many solves,
 // exceeds the time to rebuild it after a refactorisation.
 constexpr double kDenseAmortSolves = 100.0;
+// What an iteration saves besides its solve where the steps then run in one
+// launch: the conditional node's share of an iteration of the graph form.  (A
+// solve alone is timed as a launch of its own; an 8-vertex scene's takes 5.8 us
+// in this form and 6.4 in the resident one, so without this the choice, and
+// with it the scene's time and last bits, would follow the timing's jitter.)
+constexpr double kGraphIterationMs = 0.006;
 // Largest mixed scene (vertices) served by X = Hs^-1: X and its workspace take
 // 2 N_p^2 doubles (268 MB at 4,096 vertices).
 constexpr int kDenseMaxN = 4096;
@@ -2878,7 +2884,10 @@ static int autotune_forms(dfem_scene* sc) {
     double best = sc->solve_cut == 0 ? sc->solve_ms[1] : sc->solve_cut == L ? sc->solve_ms[0] : sc->solve_ms[2];
     if (sc->solve_ms[3] > 0.0 && sc->solve_ms[3] < best) { sc->solve_cut = -1; best = sc->solve_ms[3]; }
     if (sc->solve_ms[4] > 0.0 && sc->solve_ms[4] < best) { sc->solve_cut = -2; best = sc->solve_ms[4]; }
-    if (sc->solve_ms[5] > 0.0 && (best - sc->solve_ms[5]) * kDenseAmortSolves > sc->dense_build_ms) sc->solve_cut = -3;
+    const bool steps = sc->ps_fwd && !sc->skel_on && sc->nF == 0 && !sc->self_contact;
+    if (sc->solve_ms[5] > 0.0 &&
+        (best + (steps ? kGraphIterationMs : 0.0) - sc->solve_ms[5]) * kDenseAmortSolves > sc->dense_build_ms)
+      sc->solve_cut = -3;
   }
   if (sc->solve_cut != -3 && (sc->bl_mem.p || sc->dn_A.p)) dense_release(sc);
   RC(tune_solve_select(sc));
