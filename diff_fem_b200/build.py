@@ -15,7 +15,8 @@ CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libdfem.so")
 SOURCES = ["engine.cu", "noalloc.cu", "scene.cpp", "cholesky.cpp", "resident_plan.cpp", "block_plan.cpp", "obj_writer.cpp"]
 HEADERS = ["pd_kernels.cu", "pd_math.cuh", "kernels.cuh", "factor_kernels.cuh", "contact_kernels.cuh", "tma.cuh",
-           "resident_solve.cuh", "drag_kernels.cuh", "skeleton_kernels.cuh", "skeleton_adjoint.cuh", "dense_solve.cuh", "block_inverse.cuh", "step_kernels.cuh", "contact_step.cuh", "contact_flags.h",
+           "resident_solve.cuh", "drag_kernels.cuh", "skeleton_kernels.cuh", "skeleton_adjoint.cuh", "dense_solve.cuh",
+           "block_inverse.cuh", "step_kernels.cuh", "contact_step.cuh", "contact_flags.h", "pointer_rule.h",
            "scene.h", "cholesky.h", "resident_plan.h", "block_plan.h"]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 

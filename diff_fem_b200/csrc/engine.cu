@@ -29,6 +29,7 @@
 #include "block_inverse.cuh"
 #include "step_kernels.cuh"
 #include "contact_step.cuh"
+#include "pointer_rule.h"
 #include "resident_plan.h"
 #include "scene.h"
 
@@ -2363,15 +2364,30 @@ static int run_adjoint(dfem_scene* sc, int st) {
   return DFEM_OK;
 }
 
+// (device memory: the runtime looks up whose it is, pointer_rule.h)
 static int copy_in(dfem_scene* sc, const double* src, size_t n, double* dst, int mem) {
-  CK(cudaMemcpyAsync(dst, src, n * sizeof(double), mem == DFEM_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
+  CK(cudaMemcpyAsync(dst, src, n * sizeof(double), mem == DFEM_MEM_DEVICE ? cudaMemcpyDefault : cudaMemcpyHostToDevice,
                      sc->stream));
   return DFEM_OK;
 }
 static int copy_out(dfem_scene* sc, const double* src, size_t n, double* dst, int mem) {
-  CK(cudaMemcpyAsync(dst, src, n * sizeof(double), mem == DFEM_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
+  CK(cudaMemcpyAsync(dst, src, n * sizeof(double), mem == DFEM_MEM_DEVICE ? cudaMemcpyDefault : cudaMemcpyDeviceToHost,
                      sc->stream));
   return DFEM_OK;
+}
+
+// Whether the kernels may use every one of a call's buffers (null: not given) in place.
+static bool in_place(const dfem_scene* sc, int mem, std::initializer_list<const double*> ptrs) {
+  if (mem != DFEM_MEM_DEVICE) return false;
+  static_assert(kMemoryTypeDevice == cudaMemoryTypeDevice, "the rule's constant");
+  for (const double* p : ptrs) {
+    if (!p) continue;
+    cudaPointerAttributes at{};
+    const bool known = cudaPointerGetAttributes(&at, p) == cudaSuccess;
+    if (!known) cudaGetLastError();
+    if (!used_in_place(known, at.type, at.device, sc->device)) return false;
+  }
+  return true;
 }
 
 // Record of the contact phase for its adjoint: room for `cap` computed Jacobi
@@ -3127,15 +3143,16 @@ int dfem_step_forward(dfem_scene* sc, const double* x, const double* v, const do
     PdSteps a = steps_args(sc, n_steps, 0);
     a.zero = 1;
     a.x_in = x; a.v_in = v; a.x_out = x_out; a.v_out = v_out;
-    if (mem != DFEM_MEM_DEVICE) {
+    const bool direct = in_place(sc, mem, {x, v, x_out, v_out, traj_x});
+    if (!direct) {
       RC(copy_in(sc, x, n3, sc->io_a.p, mem));
       RC(copy_in(sc, v, n3, sc->io_b.p, mem));
       a.x_in = a.x_out = sc->io_a.p;
       a.v_in = a.v_out = sc->io_b.p;
     }
-    a.traj = traj_x ? (mem == DFEM_MEM_DEVICE ? traj_x : sc->traj.p) : nullptr;
+    a.traj = traj_x ? (direct ? traj_x : sc->traj.p) : nullptr;
     CK(launch_steps(sc, sc->stream, a, false));
-    if (mem != DFEM_MEM_DEVICE) {
+    if (!direct) {
       RC(copy_out(sc, sc->io_a.p, n3, x_out, mem));
       RC(copy_out(sc, sc->io_b.p, n3, v_out, mem));
       if (traj_x) RC(copy_out(sc, sc->traj.p, n3 * n_steps, traj_x, mem));
@@ -3316,7 +3333,8 @@ int dfem_step_backward(dfem_scene* sc, const double* gx_out, const double* gv_ou
     PdSteps a = steps_args(sc, sc->rec_steps, 0);
     a.zero = 1;
     a.x_in = gx_out; a.v_in = gv_out; a.x_out = gx; a.v_out = gv;
-    if (mem == DFEM_MEM_DEVICE) {
+    const bool direct = in_place(sc, mem, {gx_out, gv_out, gx, gv, g_youngs, g_poisson, s.nseg > 0 ? g_act : nullptr});
+    if (direct) {
       a.gE_out = g_youngs; a.gnu_out = g_poisson; a.gact_out = s.nseg > 0 ? g_act : nullptr;
     } else {
       RC(copy_in(sc, gx_out, n3, sc->io_a.p, mem));
@@ -3325,7 +3343,7 @@ int dfem_step_backward(dfem_scene* sc, const double* gx_out, const double* gv_ou
       a.v_in = a.v_out = sc->io_b.p;
     }
     CK(launch_steps(sc, sc->stream, a, true));
-    if (mem != DFEM_MEM_DEVICE) {
+    if (!direct) {
       RC(copy_out(sc, sc->io_a.p, n3, gx, mem));
       RC(copy_out(sc, sc->io_b.p, n3, gv, mem));
       if (g_youngs) RC(copy_out(sc, sc->gE.p, s.T, g_youngs, mem));

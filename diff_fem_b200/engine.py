@@ -25,11 +25,12 @@ def _is_cuda_tensor(a) -> bool:
 
 
 def _sync_torch(*arrays):
-    """Make pending work of torch's current stream visible to the engine's stream."""
+    """Make pending work of torch's current streams visible to the engine's stream."""
+    done = None
     for a in arrays:
-        if _is_cuda_tensor(a):
-            torch.cuda.current_stream(a.device).synchronize()
-            return
+        if _is_cuda_tensor(a) and (done is None or a.device != done):
+            done = a.device
+            torch.cuda.current_stream(done).synchronize()
 
 
 def _ptr(a):
@@ -42,6 +43,27 @@ def _ptr(a):
         return a.data_ptr(), (DFEM_MEM_DEVICE if a.is_cuda else DFEM_MEM_HOST), a
     arr = np.ascontiguousarray(a, dtype=np.float64)
     return arr.ctypes.data, DFEM_MEM_HOST, arr
+
+
+def _inputs(names, sizes, *buffers):
+    """Pointers, memory kind and keepalives of a call's input buffers (None: not
+    given).  The engine's kernels read `size` values at each pointer, all of one
+    kind: buffers of another kind or shorter ones are refused here."""
+    ptrs, keep, kind = [], [], None
+    for a, size in zip(buffers, sizes):
+        p, mem, k = _ptr(a)
+        ptrs.append(p)
+        if k is None:
+            continue
+        keep.append(k)
+        if kind is None:
+            kind = mem
+        elif mem != kind:
+            raise ValueError(f"{names} must live in the same memory")
+        n = k.size if isinstance(k, np.ndarray) else k.numel()
+        if n < size:
+            raise ValueError(f"a buffer of {names} has {n} values, the scene needs {size}")
+    return ptrs, DFEM_MEM_HOST if kind is None else kind, keep
 
 
 class Scene:
@@ -111,15 +133,12 @@ class Scene:
         return {name: getattr(inf, name) for name, _ in inf._fields_}
 
     def set_materials(self, youngs, poisson):
-        pe, me, ke = _ptr(youngs)
-        pn, mn, kn = _ptr(poisson)
-        if me != mn:
-            raise ValueError("youngs and poisson must live in the same memory")
+        (pe, pn), mem, keep = _inputs("youngs and poisson", (self.T, self.T), youngs, poisson)
         _sync_torch(youngs, poisson)
-        check(lib().dfem_set_materials(self._h, pe, pn, me))
+        check(lib().dfem_set_materials(self._h, pe, pn, mem))
 
     def set_activations(self, act):
-        p, m, k = _ptr(act)
+        (p,), m, keep = _inputs("act", (self.nseg,), act)
         check(lib().dfem_set_activations(self._h, p, m))
 
     @property
@@ -153,8 +172,9 @@ class Scene:
     def forward(self, x, v, n_steps: int = 1, act=None, traj: bool = False):
         """Run n_steps steps from (x, v).  Returns (x_out, v_out[, traj]) in the
         input's memory kind (numpy for host input, CUDA tensors for device input)."""
-        dev = _is_cuda_tensor(x)
         n3 = 3 * self.N
+        (px, pv, pa), mx, keep = _inputs("x, v and act", (n3, n3, n_steps * self.nseg), x, v, act)
+        dev = _is_cuda_tensor(x)
         if dev:
             xo = torch.empty(n3, dtype=torch.float64, device=x.device)
             vo = torch.empty_like(xo)
@@ -162,14 +182,9 @@ class Scene:
         else:
             xo, vo = np.empty(n3), np.empty(n3)
             tr = np.empty((n_steps, n3)) if traj else None
-        px, mx, kx = _ptr(x)
-        pv, mv, kv = _ptr(v)
-        pa, ma, ka = _ptr(act)
         pxo, _, _ = _ptr(xo)
         pvo, _, _ = _ptr(vo)
         ptr_, _, _ = _ptr(tr)
-        if mx != mv or (ma is not None and ma != mx):
-            raise ValueError("x, v and act must live in the same memory")
         _sync_torch(x, v, act)
         check(lib().dfem_step_forward(self._h, px, pv, pa, int(n_steps), pxo, pvo, ptr_, mx))
         self._last_steps = n_steps
@@ -180,6 +195,8 @@ class Scene:
         with a skeleton also jq, jqd (the gradient w.r.t. the joint state the
         forward started from; gjq / gjqd: cotangents of its end state, zero
         when omitted)."""
+        n3 = 3 * self.N
+        p_in, mem, keep = _inputs("gx and gv", (n3, n3), gx, gv)
         nq = self.n_joint_state
         if nq and (gjq is not None or gjqd is not None):
             a = np.zeros(nq) if gjq is None else np.ascontiguousarray(gjq, np.float64).reshape(-1)
@@ -189,7 +206,6 @@ class Scene:
             P = lambda t: t.ctypes.data_as(C.POINTER(C.c_double))
             check(lib().dfem_set_joint_state_grad(self._h, P(a), P(b)))
         dev = _is_cuda_tensor(gx)
-        n3 = 3 * self.N
         if dev:
             mk = lambda *s: torch.empty(*s, dtype=torch.float64, device=gx.device)
         else:
@@ -197,8 +213,7 @@ class Scene:
         ox, ov = mk(n3), mk(n3)
         gE, gnu = mk(max(1, self.T)), mk(max(1, self.T))
         ga = mk(max(1, self._last_steps * self.nseg))
-        p = [_ptr(a)[0] for a in (gx, gv, ox, ov, gE, gnu, ga)]
-        mem = _ptr(gx)[1]
+        p = p_in + [_ptr(a)[0] for a in (ox, ov, gE, gnu, ga)]
         _sync_torch(gx, gv)
         check(lib().dfem_step_backward(self._h, p[0], p[1], p[2], p[3], p[4], p[5], p[6] if self.nseg else None, mem))
         act = ga[: self._last_steps * self.nseg]
@@ -213,9 +228,9 @@ class Scene:
 
     def eval_local(self, x):
         """J d(x): the local step's contribution to the global rhs at positions x."""
+        (px,), mx, keep = _inputs("x", (3 * self.N,), x)
         dev = _is_cuda_tensor(x)
         out = torch.empty(3 * self.N, dtype=torch.float64, device=x.device) if dev else np.empty(3 * self.N)
-        px, mx, kx = _ptr(x)
         po, _, _ = _ptr(out)
         _sync_torch(x)
         check(lib().dfem_eval_local(self._h, px, po, mx))
