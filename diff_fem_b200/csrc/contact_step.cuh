@@ -533,10 +533,7 @@ __global__ void __launch_bounds__(kPsThreads, 1) k_cadj_phase(const __grid_const
             ps_take(dyn, rot, me, T.P);
             ps_corners(T.G, T.P, T.sl, rot, slot);
             if (!rot) {
-              const double yr = dyn[18 * kPsPair + me], yh = dyn[19 * kPsPair + me], E = d.tE[t], nu = d.tnu[t], vol = d.tvol[t];
-              const double opn = 1.0 + nu;
-              gE[t] += vol / opn * (yr + nu * yv) - vol * yh;
-              gnu[t] += E * vol / (opn * opn) * (yv - yr);
+              tet_moduli_grad(gE, gnu, t, d.tE[t], d.tnu[t], d.tvol[t], dyn[18 * kPsPair + me], yv, dyn[19 * kPsPair + me]);
             }
           } else {
             ct_tet_take(rot, dyn, me, T, lslot);

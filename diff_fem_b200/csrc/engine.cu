@@ -2015,7 +2015,8 @@ static void launch_gather(dfem_scene* sc, cudaStream_t st, Gate g, const double*
 static void launch_adj_local(dfem_scene* sc, cudaStream_t st, Gate g, const int* kptr) {
   const HostScene& s = sc->hs;
   const int nthr = std::max(s.T + s.M + s.S + s.B, s.N);
-  k_adj_local<<<(nthr + 127) / 128, 128, 0, st>>>(sc->sd, g, kptr, sc->step.p, sc->hist.p, sc->hist_step, sc->y.p, sc->bb.p,
+  auto* fn = s.T >= kAdjManyTets ? k_adj_local<3> : k_adj_local<2>;
+  fn<<<(nthr + 127) / 128, 128, 0, st>>>(sc->sd, g, kptr, sc->step.p, sc->hist.p, sc->hist_step, sc->y.p, sc->bb.p,
                                             sc->act_all.p, sc->slot.p, sc->gE.p, sc->gnu.p, sc->mg.p);
 }
 
@@ -2526,6 +2527,7 @@ static int contact_adjoint_step(dfem_scene* sc, int st, bool recorded, int rbase
     const int jmax = *std::max_element(toph.begin(), toph.end());
     const ContactAdj a = make_cadj(sc);
     Gate g;
+    auto* cadj_local = s.T >= kAdjManyTets ? k_cadj_local<3> : k_cadj_local<2>;
     g.flag = sc->c_pst.p + (size_t)PS_SKIP * np;
     k_cadj_start<<<nb, 128, 0, sc->stream>>>(s.N, s.damping / s.h, sc->io_a.p, sc->io_b.p, a, 0);
     int launches = 1;
@@ -2541,7 +2543,7 @@ static int contact_adjoint_step(dfem_scene* sc, int st, bool recorded, int rbase
       k_cadj_rhs_parts<<<nb, 128, 0, sc->stream>>>(sc->sd, sc->cd, a, sc->slot.p, xt, ori, prev,
                                                    sc->crec_first.p + r * np, rcnt, rn);
       if (ncons > 0)
-        k_cadj_local<<<(ncons + 127) / 128, 128, 0, sc->stream>>>(sc->sd, a, ori, xt, sc->act_all.p, sc->step.p,
+        cadj_local<<<(ncons + 127) / 128, 128, 0, sc->stream>>>(sc->sd, a, ori, xt, sc->act_all.p, sc->step.p,
                                                                   sc->slot.p, sc->gE.p, sc->gnu.p, sc->mg.p, g);
       k_adj_gather_seq<<<nb, 128, 0, sc->stream>>>(s.N, g, sc->vpart.p, sc->vslot_ptr.p, sc->slot.p, a.orib);
       if (s.nseg > 0)
@@ -2596,6 +2598,7 @@ static int contact_adjoint_step(dfem_scene* sc, int st, bool recorded, int rbase
     CK(cudaMemcpy(first.data(), sc->crec_first.p + base, top * sizeof(int), cudaMemcpyDeviceToHost));
   const ContactAdj a = make_cadj(sc);
   k_cadj_start<<<nb, 128, 0, sc->stream>>>(s.N, s.damping / s.h, sc->io_a.p, sc->io_b.p, a, soft ? 1 : 0);
+  auto* cadj_local = s.T >= kAdjManyTets ? k_cadj_local<3> : k_cadj_local<2>;
   int launches = 1;
   for (int j = top; j >= 1; --j) {
     if (soft) {
@@ -2615,7 +2618,7 @@ static int contact_adjoint_step(dfem_scene* sc, int st, bool recorded, int rbase
       k_cadj_self_group<<<(sc->cd.ncf + 127) / 128, 128, 0, sc->stream>>>(sc->cd, a, rv);
       k_cadj_self_b<<<(sc->cd.nc + 127) / 128, 128, 0, sc->stream>>>(sc->sd, sc->cd, a, rv, first[j - 1], rcnt, rn);
       if (ncons > 0)
-        k_cadj_local<<<(ncons + 127) / 128, 128, 0, sc->stream>>>(sc->sd, a, ori, xt, sc->act_all.p, sc->step.p,
+        cadj_local<<<(ncons + 127) / 128, 128, 0, sc->stream>>>(sc->sd, a, ori, xt, sc->act_all.p, sc->step.p,
                                                                   sc->slot.p, sc->gE.p, sc->gnu.p, sc->mg.p, kOpen);
       k_adj_gather_seq<<<nb, 128, 0, sc->stream>>>(s.N, kOpen, sc->vpart.p, sc->vslot_ptr.p, sc->slot.p, a.orib);
       if (s.nseg > 0)
@@ -2634,7 +2637,7 @@ static int contact_adjoint_step(dfem_scene* sc, int st, bool recorded, int rbase
       k_local<<<(ncons + 127) / 128, 128, 0, sc->stream>>>(sc->sd, kOpen, ori, sc->act_all.p, sc->step.p, sc->slot.p);
     k_cadj_rhs<<<nb, 128, 0, sc->stream>>>(sc->sd, sc->cd, a, sc->slot.p, xt, ori, prev, first[j - 1], rcnt, rn);
     if (ncons > 0)
-      k_cadj_local<<<(ncons + 127) / 128, 128, 0, sc->stream>>>(sc->sd, a, ori, xt, sc->act_all.p, sc->step.p,
+      cadj_local<<<(ncons + 127) / 128, 128, 0, sc->stream>>>(sc->sd, a, ori, xt, sc->act_all.p, sc->step.p,
                                                                 sc->slot.p, sc->gE.p, sc->gnu.p, sc->mg.p, kOpen);
     k_adj_gather_seq<<<nb, 128, 0, sc->stream>>>(s.N, kOpen, sc->vpart.p, sc->vslot_ptr.p, sc->slot.p, a.orib);
     if (s.nseg > 0)

@@ -92,17 +92,11 @@ __device__ __forceinline__ Mat3<double> deformation_rn(const double G[4][3], con
 // heaviest per-constraint kernels (128 threads each): more resident warps hide
 // the FP64 latency chains better than the registers they give up (the mixed
 // force step takes 0.311 ms on the 256-scene batch at 96 registers, 0.34 ms at
-// more).  The projection by polar and matrix iterations (pd_math.cuh) needs
-// fewer live values than the SVD it replaced: the adjoint local step runs two
-// CTAs at 222 registers without spills (three CTAs, 168 registers, 128 bytes
-// of spills: the same times); inverse-stiffness beam 14.4 -> 12.3 us per
-// launch, local step 10.3 -> 8.2 us, 24-scene batch 45.6 -> 48.1 and 19.3 ->
-// 19.5 us, where the FP64 pipe bounds both.
+// more).  The projection by polar and matrix iterations (pd_math.cuh) took the
+// local step from 10.3 to 8.2 us on the inverse-stiffness beam and from 0.39 to
+// 0.31 ms on the 256-scene batch.
 #ifndef DFEM_FORCE_MIN_BLOCKS
 #define DFEM_FORCE_MIN_BLOCKS 5
-#endif
-#ifndef DFEM_ADJ_MIN_BLOCKS
-#define DFEM_ADJ_MIN_BLOCKS 2
 #endif
 #ifndef DFEM_LOCAL_MIN_BLOCKS
 #define DFEM_LOCAL_MIN_BLOCKS 5
@@ -1378,6 +1372,31 @@ __device__ __forceinline__ double contact_yh(const double G[4][3], const Mat3<do
   return yh;
 }
 
+// CTAs per SM of the adjoint local steps (a kernel for each: the same bits).
+// Two hold every value in registers, three (168) spill beside the 47 KB of
+// their tapes but cover more of a large scene's reads, for which it waits (the
+// FP64 pipe is 28 % busy); what the end reads is prefetched at the start.
+// us per launch, by the SVD (three CTAs) / two / three: 12,800 tets 14.4 / 10.3
+// / 12.3, 119,000 46.4 / 41.0 / 45.2, 219,000 77.1 / 75.2 / 74.6, 402,000 134.8
+// / 133.2 / 128.8, 1.45 M 448 / 454 / 427, 2.97 M 784 / 857 / 806.
+constexpr int kAdjManyTets = 200000;
+
+// dL/dE and dL/dnu of a tet from yr = Y : md, yv = Y : md_volume and yh, its Hs
+// term (explicitly rounded: several kernels evaluate it).
+__device__ __forceinline__ void tet_moduli_grad(double* gE, double* gnu, int t, double E, double nu, double vol, double yr,
+                                                double yv, double yh) {
+  const double opn = 1.0 + nu;
+  if (gE) gE[t] = __dadd_rn(gE[t], __fma_rn(vol / opn, __fma_rn(nu, yv, yr), -__dmul_rn(vol, yh)));
+  if (gnu) gnu[t] = __fma_rn(__dmul_rn(E, vol) / __dmul_rn(opn, opn), __dadd_rn(yv, -yr), gnu[t]);
+}
+// Y . (deformation at x1): the Hs term of the next iterate
+__device__ __forceinline__ double iterate_yh(const double G[4][3], const Mat3<double>& Y, const Vec3<double> x1[4]) {
+  const Mat3<double> F1 = deformation_rn(G, x1);
+  return rn_dot(Y, F1);
+}
+
+__device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
+
 // tape: this thread's first value of the VJP's tape (kVolTape values, stride apart, in shared memory).
 // (Plain pointers: k_cadj_phase writes yb earlier in the same launch; the
 // kernels that call it keep their parameters restrict-qualified.)
@@ -1393,22 +1412,23 @@ __device__ __forceinline__ void adj_local_item(const SceneDev& d, int t, const d
     for (int a = 0; a < 4; ++a) { xv[a] = ld3(x, vi[a]); yv[a] = ld3(yb, vi[a]); }
     double G[4][3];
     load_g(d.tinv, d.T, t, G);
+    if (gE) prefetch_l1(gE + t);  // read after the projection: on their way to the SM meanwhile
+    if (gnu) prefetch_l1(gnu + t);
+    prefetch_l1(d.tE + t);
+    prefetch_l1(d.tnu + t);
+    prefetch_l1(d.tvol + t);
+    prefetch_l1(d.tslot + t);
     const Mat3<double> F = deformation_rn(G, xv), Y = deformation_rn(G, yv);
-    double E = d.tE[t], nu = d.tnu[t], vol = d.tvol[t];
     double yr, yvv, yh = 0;
     Mat3<double> gF;
     corot_adjoint_polar(F, Y, d.twr[t], d.twv[t], yr, yvv, gF, tape, stride);
     if (x1) {
-      Vec3<double> x1v[4] = {ld3(x1, vi[0]), ld3(x1, vi[1]), ld3(x1, vi[2]), ld3(x1, vi[3])};
-      Mat3<double> F1 = deformation(G, x1v);
-#pragma unroll
-      for (int j = 0; j < 3; ++j) yh += dot3(Y.c[j], F1.c[j]);
+      const Vec3<double> x1v[4] = {ld3(x1, vi[0]), ld3(x1, vi[1]), ld3(x1, vi[2]), ld3(x1, vi[3])};
+      yh = iterate_yh(G, Y, x1v);
     } else if (xt) {
       yh = contact_yh(G, F, Y, yv, xv, xt, vi);
     }
-    double opn = 1.0 + nu;
-    if (gE) gE[t] += vol / opn * (yr + nu * yvv) - vol * yh;
-    if (gnu) gnu[t] += E * vol / (opn * opn) * (yvv - yr);
+    tet_moduli_grad(gE, gnu, t, d.tE[t], d.tnu[t], d.tvol[t], yr, yvv, yh);
     int4 sl = d.tslot[t];
     const int sv[4] = {sl.x, sl.y, sl.z, sl.w};
 #pragma unroll
@@ -1420,7 +1440,8 @@ __device__ __forceinline__ void adj_local_item(const SceneDev& d, int t, const d
 
 // Reverse PD iteration k (k read from device memory): local VJP at x^k with
 // the Hs term of x^{k+1}, and bbar += ybar (b = M/h^2 q_n enters every iteration).
-__global__ void __launch_bounds__(128, DFEM_ADJ_MIN_BLOCKS) k_adj_local(SceneDev d, Gate gate, const int* kptr, const int* step,
+template <int CTAS>
+__global__ void __launch_bounds__(128, CTAS) k_adj_local(SceneDev d, Gate gate, const int* kptr, const int* step,
                                                    const double* __restrict__ hist, long long hist_step,
                                                    const double* __restrict__ yb,
                                                    double* bb, const double* __restrict__ act_all,

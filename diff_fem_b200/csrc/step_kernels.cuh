@@ -458,12 +458,8 @@ __device__ __forceinline__ void ps_adj_local(const SceneDev& d, const double* x,
         corot_adjoint_rotation(F, Y, d.twr[t], yr, gF);
 #pragma unroll
         for (int a = 0; a < 4; ++a) xv[a] = ld3(x1, vi[a]);
-        const Mat3<double> F1 = deformation(G, xv);
-        double yh = 0;
-#pragma unroll
-        for (int j = 0; j < 3; ++j) yh += dot3(Y.c[j], F1.c[j]);
         xch[18 * kPsPair + me] = yr;
-        xch[19 * kPsPair + me] = yh;
+        xch[19 * kPsPair + me] = iterate_yh(G, Y, xv);
       } else {
         corot_adjoint_volume(F, Y, d.twv[t], yv, gF, tape + 32 * half + lane, 32 * tape_warps);
       }
@@ -474,10 +470,7 @@ __device__ __forceinline__ void ps_adj_local(const SceneDev& d, const double* x,
       ps_take(xch, rot, me, gF.c);
       ps_corners(G, gF.c, sl, rot, slot);
       if (!rot) {
-        const double yr = xch[18 * kPsPair + me], yh = xch[19 * kPsPair + me], E = d.tE[t], nu = d.tnu[t], vol = d.tvol[t];
-        const double opn = 1.0 + nu;
-        gE[t] += vol / opn * (yr + nu * yv) - vol * yh;
-        gnu[t] += E * vol / (opn * opn) * (yv - yr);
+        tet_moduli_grad(gE, gnu, t, d.tE[t], d.tnu[t], d.tvol[t], xch[18 * kPsPair + me], yv, xch[19 * kPsPair + me]);
       }
     }
     if (base + 32 * tape_warps * nc < d.T) __syncthreads();
