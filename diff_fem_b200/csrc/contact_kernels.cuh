@@ -1333,37 +1333,44 @@ static __device__ __noinline__ bool contact_frame(Vec3<double> nrm, Vec3<double>
   return true;
 }
 
+// VJP of the friction cone rhs_post = r0 W0 + r1' W1 + r2' W2 (the clamp) for
+// the cotangent rb (one compiled copy, only where an impact replaced the rhs).
+static __device__ __noinline__ Vec3<double> cone_vjp(const Vec3<double> W[3], const double r[3], double mu, Vec3<double> rb) {
+  const double r0 = r[0], r1 = r[1], r2 = r[2];
+  const double b0 = dot3(W[0], rb), b1 = dot3(W[1], rb), b2 = dot3(W[2], rb);
+  const double rt = sqrt(r1 * r1 + r2 * r2);
+  double g0 = b0, g1 = b1, g2 = b2;
+  if (rt > mu * r0) {
+    g0 = b0 + mu * (r1 * b1 + r2 * b2) / rt;
+    g1 = mu * r0 * (r2 * r2 * b1 - r1 * r2 * b2) / (rt * rt * rt);
+    g2 = mu * r0 * (r1 * r1 * b2 - r1 * r2 * b1) / (rt * rt * rt);
+  }
+  return (-1.0) * (g0 * W[0] + g1 * W[1] + g2 * W[2]);
+}
+
 // Reverse of vertex i's update in a computed iteration: xb = cotangent of its
 // x_n1, pv = its relaxed rhs; hit: an impact's reaction replaced the rhs (W,
 // r: contact_frame of the last one); first: the iteration began its pass.
-static __device__ __noinline__ void cadj_rhs_finish(const SceneDev& d, const ContactDev& c, const ContactAdj& a, int i,
-                                                    Vec3<double> xb, Vec3<double> pv, int first, bool hit,
-                                                    const Vec3<double> W[3], const double r[3], double* yb) {
-  const double hd = c.hdiag[i];
-  st3(a.cxtb, i, ld3(a.cxtb, i) + xb);
-  a.hdb[i] -= dot3(xb, pv) / (d.h * hd * hd);
-  const Vec3<double> ptot = ld3(a.pb, i) + (1.0 / (d.h * hd)) * xb;
-  Vec3<double> rb = c.alpha * ptot;
-  if (hit) {  // rhs_post = r0 W0 + r1' W1 + r2' W2 (friction cone clamp)
-    const double r0 = r[0], r1 = r[1], r2 = r[2];
-    const double b0 = dot3(W[0], rb), b1 = dot3(W[1], rb), b2 = dot3(W[2], rb);
-    const double rt = sqrt(r1 * r1 + r2 * r2);
-    double g0 = b0, g1 = b1, g2 = b2;
-    if (rt > c.mu * r0) {
-      g0 = b0 + c.mu * (r1 * b1 + r2 * b2) / rt;
-      g1 = c.mu * r0 * (r2 * r2 * b1 - r1 * r2 * b2) / (rt * rt * rt);
-      g2 = c.mu * r0 * (r1 * r1 * b2 - r1 * r2 * b1) / (rt * rt * rt);
-    }
-    rb = (-1.0) * (g0 * W[0] + g1 * W[1] + g2 * W[2]);
-  }
+// Inlined and explicitly rounded, so that every form of the sweep has the same
+// bits (one called copy, for every vertex whether hit or not, had them too, and
+// cost the backward of 256 scenes on their grounds 579 against 557 ms).
+__device__ __forceinline__ void cadj_rhs_finish(const SceneDev& d, const ContactDev& c, const ContactAdj& a, int i,
+                                                Vec3<double> xb, Vec3<double> pv, int first, bool hit,
+                                                const Vec3<double> W[3], const double r[3], double* yb) {
+  const double hd = c.hdiag[i], hh = __dmul_rn(d.h, hd);
+  st3(a.cxtb, i, rn_add(ld3(a.cxtb, i), xb));
+  a.hdb[i] = __dadd_rn(a.hdb[i], -(rn_dot(xb, pv) / __dmul_rn(hh, hd)));
+  const Vec3<double> ptot = rn_axpy(1.0 / hh, xb, ld3(a.pb, i));
+  Vec3<double> rb = rn_scale(c.alpha, ptot);
+  if (hit) rb = cone_vjp(W, r, c.mu, rb);
   if (first) {
-    rb = rb + (1.0 - c.alpha) * ptot;
+    rb = rn_axpy(1.0 - c.alpha, ptot, rb);
     st3(a.pb, i, mk3(0.0, 0.0, 0.0));
   } else {
-    st3(a.pb, i, (1.0 - c.alpha) * ptot);
+    st3(a.pb, i, rn_scale(1.0 - c.alpha, ptot));
   }
-  st3(a.vwcb, i, ld3(a.vwcb, i) + d.mass[i] * rb);
-  st3(yb, i, d.h * rb);
+  st3(a.vwcb, i, rn_axpy(d.mass[i], rb, ld3(a.vwcb, i)));
+  st3(yb, i, rn_scale(d.h, rb));
 }
 
 // slot: J d at ori (k_local); xt: the step's start positions; ori, prev: the
