@@ -32,17 +32,16 @@ SIM_STEPS = 60
 METRIC = "fwd+adjoint sim steps/s (inverse stiffness 12,800 tets, K=20)"
 
 # DRAM bytes per launch of the global solve on the inverse-stiffness workload,
-# by solve form, from one ncu capture each (dram__bytes_read.sum +
-# dram__bytes_write.sum; the persistent form's factor is largely L2-resident
-# between solves, so its figure is below the algorithmic bytes; the dense
-# form reads Hs^-1 from DRAM once per solve).  Not measured by a bench run.
-SOLVE_DRAM_BYTES = {"persistent": 4.36e6, "dense": 88.51e6 + 2.93e6}
+# from one ncu capture of the persistent form (dram__bytes_read.sum +
+# dram__bytes_write.sum; its factor is largely L2-resident between solves, so
+# the figure is below the algorithmic bytes).  Not measured by a bench run.
+SOLVE_DRAM_BYTES = {"persistent": 4.36e6}
 UNIT = "steps/s"
 
 
 def pin_triangular(sc) -> bool:
     """Put a scene on the fastest of its supernodal triangular-solve forms (the
-    plain form) when the autotune chose the dense inverse; True if it did."""
+    plain form) when the autotune chose the dense form (block inverses); True if it did."""
     info = sc.solve_mode()
     if info["mode"] != "dense":
         return False
@@ -318,14 +317,8 @@ def run_ours(args):
     peak_note = "measured (MEASURED_PEAKS.json hbm_gbs, burst copy)" if "hbm_gbs" in peaks else "fallback 6650 GB/s"
     nnz = int(info["nnz_factor"])
     solve_info = sc.solve_mode()
-    if solve_info["mode"] == "dense":
-        # the dense-inverse form reads the N rows x N_p columns of Hs^-1 (FP64) once; rhs in, y out
-        n_p = -(-N // 64) * 64
-        solve_bytes = N * n_p * 8 + 48 * N
-        solve_note = "per solve (the N x N_p FP64 rows of Hs^-1 once, rhs in, y out; k_dense_solve)"
-    else:
-        solve_bytes = 2 * nnz * 8 + 96 * N                   # 2 sweeps x the factor's FP64 values + in/out vectors
-        solve_note = "per solve (both sweeps)"
+    solve_bytes = 2 * nnz * 8 + 96 * N                       # 2 sweeps x the sparse factor's FP64 values + in/out vectors
+    solve_note = "per solve (both sweeps)"
     local_bytes = T * (16 + 72 + 16) + N * 72                 # tet tables + x, b, rhs per vertex
     dom = max(share, key=share.get)
     if dom == "solve":
@@ -342,6 +335,17 @@ def run_ours(args):
                 if traffic else None, "peak_source": peak_note,
                 "algorithmic_bytes": solve_bytes if dom == "solve" else local_bytes, "per": traffic_note,
                 "phase_ms": ph, "phase_share_ms_per_bench_step": share}
+    if solve_info["mode"] == "dense":
+        # whole calls in one launch each (k_pd_forward, k_pd_adjoint): no phase is a kernel of its own, so
+        # the least bytes of all the step's iterations stand against the timed step
+        step_bytes = n_it * (2 * (local_bytes + solve_bytes) + 8 * T)
+        achieved = step_bytes * args.steps / elapsed / 1e9
+        roofline = {"bound": "latency: grid barriers and L2 reads (what an iteration reads stays in L2 and shared memory)",
+                    "kernel": "k_pd_forward + k_pd_adjoint, with k_block_factor", "solve_form": "dense",
+                    "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm, "peak_source": peak_note,
+                    "algorithmic_bytes": step_bytes, "per": "timed step (tet tables, vertex vectors and the sparse "
+                    "factor's values once per PD iteration, forward and adjoint)",
+                    "phase_ms_as_kernels_of_their_own": ph}
 
     line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": 1e3 * elapsed / args.steps, "higher_is_better": True,
@@ -484,7 +488,7 @@ def comparison_extras(args, local: int) -> dict:
         sample = order[np.linspace(0, len(dd) - 1, min(16, len(dd))).astype(int)]
         vo, so = out["fp64"]["offsets"]["vertices"], out["fp64"]["offsets"]["segments"]
         # the plain form is the supernodal triangular solve (the fastest of its
-        # forms per scene); the dense-inverse form small single scenes may
+        # forms per scene); the dense form small single scenes may
         # take instead is timed beside it
         tsum, tsum_auto, n_dense = 0.0, 0.0, 0
         for q in sample:
@@ -524,7 +528,7 @@ def comparison_extras(args, local: int) -> dict:
                                    "solve": "supernodal triangular solve (fastest of its forms per scene)"},
             "fp64_one_at_a_time_any_form": {"value": plain_auto, "unit": "scene-steps/s",
                                             "scenes_with_dense_inverse": n_dense,
-                                            "solve": "the autotuned form, the dense inverse included"},
+                                            "solve": "the autotuned form, the dense one included"},
             "mixed_batched_over_fp64_one_at_a_time_any_form": out["mixed"]["value"] / plain_auto,
             "mixed_batched_over_fp64_one_at_a_time": out["mixed"]["value"] / plain,
             "fp64_batched_over_fp64_one_at_a_time": out["fp64"]["value"] / plain,
