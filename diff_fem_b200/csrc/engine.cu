@@ -329,9 +329,12 @@ static void parallel_for(int n, Fn f) {
 }
 
 // Captured graphs bake in device pointers; any change of them invalidates the graphs.
+// (Their kernel counts go with them: calls that need no graph count their own launches.)
 static void invalidate_graphs(dfem_scene* sc) {
-  if (sc->g_step.exec) { cudaGraphExecDestroy(sc->g_step.exec); sc->g_step.exec = nullptr; }
-  if (sc->g_adj.exec) { cudaGraphExecDestroy(sc->g_adj.exec); sc->g_adj.exec = nullptr; }
+  for (LoopGraph* g : {&sc->g_step, &sc->g_adj}) {
+    if (g->exec) cudaGraphExecDestroy(g->exec);
+    *g = LoopGraph();
+  }
 }
 
 static void refresh_scene_view(dfem_scene* sc) {
